@@ -143,7 +143,9 @@ KParams make_kparams(const DemSystem* s, uint32_t n) {
 }
 
 // Culling bound: the largest radius, and whether culling is valid for this
-// grid (at least 3 cells per axis, cells wider than any contact distance).
+// grid: at least 3 cells per axis (so at least 4, a power of two) and cells
+// wider than any contact distance.  A cell met across the grid's wrap is then
+// two cells (4 rmax) away, out of reach of the attraction (2.4 rmax) too.
 void set_rmax(KParams& P, float rmax) {
     P.rmax = rmax;
     P.cull = (std::isfinite(rmax) && P.gx >= 3 && P.gy >= 3 && P.cellW > 2.002f * rmax &&

@@ -138,6 +138,7 @@ __device__ __forceinline__ void candidate(const KParams& P, uint32_t j, float2 p
                                           const uint32_t* __restrict__ src, float2& fc,
                                           float& moment, float& pr) {
     const float rj = __ldg(radius + j);
+    if (ATTRACT && attract_out_of_reach(r, rj, d2)) return;
     // velocity, spin and type of candidate j sit at its slot of the previous
     // order (src), or at j when the arrays are all in one order (src null)
     const uint32_t sj = src ? __ldg(src + j) : j;
@@ -280,7 +281,12 @@ __device__ __forceinline__ void collide_one(const KParams& P, uint32_t i, int2 g
 // culled cell adds +0, which changes nothing).  Returns false, without
 // touching the outputs, when the visited columns wrap; the caller then uses
 // collide_one.
-template <bool TYPED>
+//
+// With ATTRACT the filter keeps the candidates within attraction reach
+// (attract_reach2, a superset of the contacts), and a neighbour column or row
+// is skipped beyond the largest such reach (exact where culling is: a cell met
+// across the grid's wrap is at least 4 rmax away).
+template <bool TYPED, bool ATTRACT>
 __device__ __forceinline__ bool collide_rows(const KParams& P, uint32_t i, int2 g, float2 p,
                                              float2 v, float w, float r, uint32_t mat,
                                              const float2* __restrict__ pos,
@@ -291,10 +297,12 @@ __device__ __forceinline__ bool collide_rows(const KParams& P, uint32_t i, int2 
                                              const uint32_t* __restrict__ src,
                                              const uint32_t* __restrict__ cellFirst,
                                              float2& force, float& moment, float& pr) {
+    // a radius that is not positive has no attraction reach (see attract_reach2)
+    if (ATTRACT && !(r > 0.0f)) return false;
     int y0 = -1, y1 = 1, x0 = -1, x1 = 1;
     if (p.x > P.cullMargin && p.x < P.Lx - P.cullMargin && p.y > P.cullMargin &&
         p.y < P.Ly - P.cullMargin) {
-        const float reach = (r + P.rmax) * 1.0001f + P.cullMargin;
+        const float reach = (ATTRACT ? kAttractReach * P.rmax : r + P.rmax) * 1.0001f + P.cullMargin;
         const float X0 = (float)g.x * P.cellW, Y0 = (float)(g.y + P.rowOff) * P.cellH;
         if (p.x - X0 > reach) x0 = 0;
         if (X0 + P.cellW - p.x > reach) x1 = 0;
@@ -351,9 +359,15 @@ __device__ __forceinline__ bool collide_rows(const KParams& P, uint32_t i, int2 
                     const float2 da = f32x2_sub(q[k], p), db = f32x2_sub(q[k + 1], p);
                     const float2 sa = f32x2_mul(da, da), sb = f32x2_mul(db, db);
                     const float d2a = sa.x + sa.y, d2b = sb.x + sb.y;
-                    const float2 cd = f32x2_add(make_float2(r, r), make_float2(rq[k], rq[k + 1]));
-                    const float2 c2 = f32x2_mul(cd, cd);
-                    const float2 bound = f32x2_fma(c2, make_float2(2e-6f, 2e-6f), c2);
+                    float2 bound;
+                    if (ATTRACT) {
+                        bound = make_float2(attract_reach2(r, rq[k]), attract_reach2(r, rq[k + 1]));
+                    } else {
+                        const float2 cd =
+                            f32x2_add(make_float2(r, r), make_float2(rq[k], rq[k + 1]));
+                        const float2 c2 = f32x2_mul(cd, cd);
+                        bound = f32x2_fma(c2, make_float2(2e-6f, 2e-6f), c2);
+                    }
                     if (d2a <= bound.x) m8 |= 1u << k;
                     if (d2b <= bound.y) m8 |= 2u << k;
                 }
@@ -364,15 +378,25 @@ __device__ __forceinline__ bool collide_rows(const KParams& P, uint32_t i, int2 
             while (mask) {
                 const uint32_t j = base + (uint32_t)(__ffs(mask) - 1);
                 mask &= mask - 1u;
-                const float rj = __ldg(radius + j);
-                float4 pc = pc0;
-                const uint32_t sj = __ldg(src + j);
-                if (TYPED) pc = P.pair[mat * P.nmat + __ldg(type + sj)];
-                const float2 f = pair_force(p, __ldg(pos + j), v, __ldg(vel + sj), w, __ldg(omega + sj),
-                                            r, rj, pc, P.dt, moment, pr);
-                if (j >= b2) { f2.x += f.x; f2.y += f.y; }
-                else if (j >= b1) { f1.x += f.x; f1.y += f.y; }
-                else { f0.x += f.x; f0.y += f.y; }
+                float2 fc = j >= b2 ? f2 : (j >= b1 ? f1 : f0);
+                if (ATTRACT) {
+                    const float2 pj = __ldg(pos + j);
+                    const float ax = pj.x - p.x, ay = pj.y - p.y;
+                    candidate<TYPED, true>(P, j, p, v, w, r, mat, pj, ax * ax + ay * ay, vel, omega,
+                                           radius, type, src, fc, moment, pr);
+                } else {
+                    const float rj = __ldg(radius + j);
+                    float4 pc = pc0;
+                    const uint32_t sj = __ldg(src + j);
+                    if (TYPED) pc = P.pair[mat * P.nmat + __ldg(type + sj)];
+                    const float2 f = pair_force(p, __ldg(pos + j), v, __ldg(vel + sj), w,
+                                                __ldg(omega + sj), r, rj, pc, P.dt, moment, pr);
+                    fc.x += f.x;
+                    fc.y += f.y;
+                }
+                if (j >= b2) f2 = fc;
+                else if (j >= b1) f1 = fc;
+                else f0 = fc;
             }
         }
         force.x += f0.x; force.y += f0.y;
@@ -531,10 +555,10 @@ __device__ __forceinline__ void step_particle(const KParams& P, uint32_t i, DynS
     const int2 g = make_int2((int)(local & (P.gx - 1u)), (int)(local >> P.log2gx));
     float2 f;
     float moment, pr;
-    if (ATTRACT || !CULL || !P.cull ||
-        !collide_rows<TYPED>(P, i, g, s.p, s.v, s.w, r, mat, in.pos, in.vel, in.omega,
+    if (!CULL || !P.cull ||
+        !collide_rows<TYPED, ATTRACT>(P, i, g, s.p, s.v, s.w, r, mat, in.pos, in.vel, in.omega,
                              inS.radius, inS.type, src, cellFirst, f, moment, pr)) {
-        if (CULL && P.cull)
+        if (CULL && !ATTRACT && P.cull)
             collide_one<TYPED, ATTRACT, true>(P, i, g, s.p, s.v, s.w, r, mat, in.pos, in.vel,
                                               in.omega, inS.radius, inS.type, src,
                                               PackedCells{cellRange}, f, moment, pr);
@@ -903,11 +927,13 @@ cudaError_t launch_step(const KParams& P, DynSet in, StatSet inS, const uint32_t
         }                                                                                      \
     } while (0)
     if (typed) {
-        if (attract) DEM_STEP(true, true, false);
+        if (attract && cull) DEM_STEP(true, true, true);
+        else if (attract) DEM_STEP(true, true, false);
         else if (cull) DEM_STEP(true, false, true);
         else DEM_STEP(true, false, false);
     } else {
-        if (attract) DEM_STEP(false, true, false);
+        if (attract && cull) DEM_STEP(false, true, true);
+        else if (attract) DEM_STEP(false, true, false);
         else if (cull) DEM_STEP(false, false, true);
         else DEM_STEP(false, false, false);
     }
