@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "dem_bands.cuh"
 #include "dem_common.cuh"
 #include "dem_incsort.cuh"
 #include "dem_kernels.cuh"
@@ -380,6 +381,16 @@ struct DemContext {
     cudaGraphExec_t stepGraph[2] = {};
     int launchesPerStep = 0;
     void* block = nullptr;  // one allocation for every per-particle/per-cell array
+    // The step in bands (dem_bands.cuh): its arrays, in bandBlock (band.bands
+    // == 0: the context steps on the packed path); whether they hold the
+    // current state, and whether cells/first of set cur were made from them;
+    // the step loop, with and without followed rows, and the sort phase alone,
+    // by cur (the set the state is packed into).
+    BandArgs band;
+    void* bandBlock = nullptr;
+    float2* ownPos = nullptr;  // the block's positions: not an adopted set
+    bool bandValid = false, bandCells = false;
+    cudaGraphExec_t bandLoop[2] = {}, bandFollow[2] = {}, bandSort[2] = {};
     // followed-particle staging (device), see dem_get_followed
     float* followRows = nullptr;
     // dem_step_followed: the ids (device copy), the ring of per-step rows,
@@ -457,6 +468,14 @@ KParams scene_kparams(const DemContext* c, uint32_t n) {
     return P;
 }
 
+// The state or its cells are new: keys are recomputed and the next step sorts
+// from scratch.
+void state_replaced(DemContext* c) {
+    c->keysValid = false;
+    c->haveOrder = false;
+    c->bandValid = false;
+}
+
 // rounds of the autotuner: every variant once per round, the first round
 // (cold instruction caches, first graph launches) not counted
 constexpr uint32_t kTuneRounds = 6;
@@ -485,6 +504,10 @@ void drop_loop_graphs(DemContext* c) {
         c->loopGraph[p] = nullptr;
         if (c->followGraph[p]) cudaGraphExecDestroy(c->followGraph[p]);
         c->followGraph[p] = nullptr;
+        for (cudaGraphExec_t* g : {&c->bandLoop[p], &c->bandFollow[p], &c->bandSort[p]}) {
+            if (*g) cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
     }
     drop_adj_graphs(c);
 }
@@ -984,6 +1007,8 @@ int init_context(DemContext* c, uint32_t capacity, uint32_t numCells, DemContext
     // caller's buffers are adopted instead (DEM_CTX_CALLER_STATE)
     const bool ownState = !(c->flags & DEM_CTX_CALLER_STATE);
     size_t total = 0;
+    // single scenes step in bands (dem_bands.cuh)
+    if (!ownState || c->nspec || !band_shape(c->P.gx, numCells, c->band)) c->band = BandArgs{};
     if (ownState) {
         total += 2 * (f8p + f8 + 2 * f4);                    // dyn sets
         total += 2 * (f4p + 2 * f4 + (c->typed ? f4 : 0));   // static sets
@@ -1031,6 +1056,7 @@ int init_context(DemContext* c, uint32_t capacity, uint32_t numCells, DemContext
     c->alpha = reinterpret_cast<float*>(take(f4));
     c->errFlag = reinterpret_cast<uint32_t*>(take(256));
     c->loopCtl = reinterpret_cast<uint32_t*>(take(256));
+    c->ownPos = c->dyn[0].pos;
     c->ss = carve_onesweep_scratch(c->sortScratch, capacity, c->keyBits);
     c->inc = carve_incsort(c->incScratch, capacity, c->numCells);
     c->inc.errFlag = c->errFlag;
@@ -1092,6 +1118,7 @@ extern "C" int dem_destroy(DemContext* c) {
     dev_free(c->resQueue);
     dev_free(c->resWork);
     dev_free(c->clusterWork);
+    dev_free(c->bandBlock);
     dev_free(c->renderOwner);
     dev_free(c->ctlBlock);
     dev_free(c->dTable);
@@ -1117,8 +1144,7 @@ extern "C" int dem_set_system(DemContext* c, const DemSystem* sys) {
     set_rmax(c->P, c->rmax);
     drop_graphs(c);
     // keys depend on the box size; recompute them and sort from scratch
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     return DEM_OK;
 }
 
@@ -1154,8 +1180,7 @@ extern "C" int dem_batch_set_systems(DemContext* c, const DemSystem* specs,
                  "batch table");
     c->hTable.swap(table);
     // keys depend on the boxes; recompute them and sort from scratch
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     return DEM_OK;
 }
 
@@ -1175,8 +1200,11 @@ bool has_state_sets(const DemContext* c) { return c->dyn[0].pos != nullptr; }
 // A new state of n particles is in the current sets (set c->cur, positions
 // in dyn[0].pos): clears the error word, reads the largest radius back and
 // keeps or drops the captured graphs.
+bool steps_in_bands(DemContext* c);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
+    // the band arrays, unless the cluster launch will step this scene
+    if (!(c->flags & DEM_CTX_RESIDENT) || !cluster_scene_fits(n, c->numCells)) steps_in_bands(c);
     // the new state replaces the one any recorded error was about
     DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 4, st), "clear error word");
     const int a = c->cur;
@@ -1193,8 +1221,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     // parameters (and specimen table), so the captured graphs stay valid;
     // only the first step's full sort is forced, as after every new state
     if (n == c->n && n > 0 && memcmp(&rmax, &c->rmax, sizeof(float)) == 0) {
-        c->keysValid = false;
-        c->haveOrder = false;
+        state_replaced(c);
         return DEM_OK;
     }
     c->n = n;
@@ -1210,8 +1237,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
         set_rmax(c->P, c->rmax);
     }
     drop_graphs(c);
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     return DEM_OK;
 }
 }  // namespace
@@ -1359,6 +1385,233 @@ extern "C" int dem_get_state(DemContext* c, float* pos, float* vel, float* theta
     return DEM_OK;
 }
 
+namespace {
+
+// ------------------------------------------------------------ step in bands
+// Own buffers, one scene, no control particle.  The arrays are allocated at
+// the first state a context takes (about 100 B per particle and 8 KB per
+// band, of its capacity); a context whose GPU has no room for them steps on
+// the packed path.
+bool steps_in_bands(DemContext* c) {
+    if (c->band.bands == 0 || c->ctlOn || c->dyn[0].pos != c->ownPos) return false;
+    if (c->bandBlock) return true;
+    const bool pressure = c->flags & DEM_CTX_PRESSURE, accel = c->flags & DEM_CTX_ACCEL;
+    const size_t bytes = band_bytes(c->band, c->capacity, c->typed, pressure, accel);
+    if (dev_alloc(&c->bandBlock, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->bandBlock = nullptr;
+        c->band = BandArgs{};
+        return false;
+    }
+    carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel);
+    c->band.errFlag = c->errFlag;
+    return true;
+}
+
+PackedState packed_state(DemContext* c) {
+    const int a = c->cur;
+    return PackedState{state_dyn(c), c->stat[a], c->loc, c->pressure, c->acc, c->alpha};
+}
+
+// A new layout of the bands from the current state: packed (when the bands
+// hold it), sorted from scratch and spread.
+cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
+    const PackedState s = packed_state(c);
+    cudaError_t e = launch_band_pack(c->band, s, true, st);
+    if (e == cudaSuccess) e = launch_calc_hash(c->P, s.dyn.pos, c->keys, nullptr, c->n, st);
+    uint32_t *ko = nullptr, *vo = nullptr;
+    if (e == cudaSuccess)
+        e = onesweep_sort_pairs(c->keys, c->perm, c->n, c->keyBits, true, c->ss, c->errFlag, st,
+                                &ko, &vo, nullptr);
+    if (e == cudaSuccess) e = launch_band_layout(c->band, s, ko, vo, c->first[c->cur], st);
+    return e;
+}
+
+// The conditional nodes of the step loop, innermost last:
+//   while steps are left: { if (full) layout; while (steps left, not full)
+//                           { kBandPairs pairs of steps } }
+// A step the band layout cannot take (kBandFull) ends the inner loop, and
+// steps of the set that does not hold the state do nothing, so every pass of
+// the outer loop makes at least one step.
+constexpr int kBandPairs = 2;
+
+cudaError_t enqueue_band_pairs(DemContext* c, bool follow, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 2 * kBandPairs && e == cudaSuccess; ++k) {
+        e = launch_band_fix(c->band, k & 1, st);
+        if (e == cudaSuccess) e = launch_band_step(c->P, c->band, k & 1, follow, c->variant, st);
+        if (e == cudaSuccess && follow)
+            e = launch_band_followed(c->band, k & 1, c->followIds, c->loopCtl + kLoopFolCount,
+                                     c->followRing, st);
+    }
+    return e;
+}
+
+// The handle of a conditional node that will be added at the capture point of
+// `st`.
+cudaError_t conditional_handle(cudaStream_t st, cudaGraphConditionalHandle* h) {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamGetCaptureInfo(st, &status, nullptr, &g, nullptr, nullptr);
+    return e == cudaSuccess ? cudaGraphConditionalHandleCreate(h, g, 0, 0) : e;
+}
+
+cudaError_t enqueue_band_loop(DemContext* c, bool follow, cudaStream_t st) {
+    cudaGraphConditionalHandle outer;
+    cudaError_t e = conditional_handle(st, &outer);
+    if (e == cudaSuccess) e = launch_band_next(c->band, outer, true, st);
+    if (e != cudaSuccess) return e;
+    return add_conditional(st, outer, cudaGraphCondTypeWhile, c->loopStream, [&](cudaStream_t ob) {
+        cudaGraphConditionalHandle full, inner;
+        cudaError_t eb = conditional_handle(ob, &full);
+        if (eb == cudaSuccess) eb = conditional_handle(ob, &inner);
+        if (eb == cudaSuccess) eb = launch_band_head(c->band, full, inner, true, ob);
+        if (eb == cudaSuccess)
+            eb = add_if(c, ob, full, [&](cudaStream_t fb) { return enqueue_band_layout(c, fb); });
+        if (eb == cudaSuccess)
+            eb = add_conditional(ob, inner, cudaGraphCondTypeWhile, c->forkStream,
+                                 [&](cudaStream_t ib) {
+                                     cudaError_t ei = enqueue_band_pairs(c, follow, ib);
+                                     return ei == cudaSuccess
+                                                ? launch_band_next(c->band, inner, false, ib)
+                                                : ei;
+                                 });
+        if (eb == cudaSuccess) eb = launch_band_next(c->band, outer, true, ob);
+        return eb;
+    });
+}
+
+// The sort phase of one step alone: a new layout when due, then the fixes (of
+// which one runs).
+cudaError_t enqueue_band_sort(DemContext* c, cudaStream_t st) {
+    cudaGraphConditionalHandle full;
+    cudaError_t e = conditional_handle(st, &full);
+    if (e == cudaSuccess) e = launch_band_head(c->band, full, 0, false, st);
+    if (e == cudaSuccess)
+        e = add_if(c, st, full, [&](cudaStream_t fb) { return enqueue_band_layout(c, fb); });
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) e = launch_band_fix(c->band, q, st);
+    return e;
+}
+
+template <typename Body>
+int build_band_graph(DemContext* c, Body body, cudaGraphExec_t* out) {
+    if (*out) return DEM_OK;
+    DEM_TRY_CUDA(cudaStreamBeginCapture(c->capStream, cudaStreamCaptureModeThreadLocal),
+                 "begin capture");
+    cudaError_t e = body(c->capStream);
+    cudaGraph_t g = nullptr;
+    cudaError_t e2 = cudaStreamEndCapture(c->capStream, &g);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+    if (g) cudaGraphDestroy(g);
+    return e == cudaSuccess ? DEM_OK : cuda_fail(e, "band graph");
+}
+
+// Before a call's steps: the band sizes of this n, and the control words (the
+// call's steps, the row block of its first followed rows; a state the bands
+// do not hold asks for a layout).
+int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t st) {
+    c->band.n = c->n;
+    c->band.slack = band_slack(c->band, c->n);
+    c->band.slots = (uint32_t)band_slots(c->band, c->n);
+    const Words w = c->bandValid ? Words{{nsteps, rowBlock}, 2u}
+                                 : Words{{nsteps, rowBlock, 1u, 0u, 0u}, 5u};
+    DEM_TRY_CUDA(launch_set_words(c->band.ctrl, w, st), "band step count");
+    // as a step of the packed path would have left it
+    state_replaced(c);
+    c->bandValid = true;
+    c->bandCells = false;
+    c->inSortOrder = true;
+    return DEM_OK;
+}
+
+// One step at a time with the host around each: profiling, the tuner, direct
+// launches (the layout decided on the host).
+int band_step_alone(DemContext* c, cudaStream_t st) {
+    int rc = band_begin(c, 1, 0, st);
+    if (rc) return rc;
+    const bool direct = c->flags & DEM_CTX_DIRECT;
+    const int a = c->cur;
+    if (!direct) {
+        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_sort(c, s); },
+                              &c->bandSort[a]);
+        if (rc) return rc;
+    }
+    uint32_t full = 0;
+    if (direct) {
+        DEM_TRY_CUDA(cudaMemcpyAsync(&full, c->band.ctrl + kBandFull, 4, cudaMemcpyDeviceToHost, st),
+                     "read sort path");
+        DEM_TRY_CUDA(cudaStreamSynchronize(st), "sync");
+    }
+    const bool prof = c->profiling && c->evUsed + 3 <= c->evCap;
+    cudaEvent_t* ev = prof ? c->evPool + c->evUsed : nullptr;
+    if (prof) DEM_TRY_CUDA(cudaEventRecord(ev[0], st), "profile event");
+    if (direct) {
+        if (full) DEM_TRY_CUDA(enqueue_band_layout(c, st), "band layout");
+        for (int q = 0; q < 2; ++q) DEM_TRY_CUDA(launch_band_fix(c->band, q, st), "band fix");
+    } else {
+        DEM_TRY_CUDA(cudaGraphLaunch(c->bandSort[a], st), "graph launch");
+    }
+    if (prof) DEM_TRY_CUDA(cudaEventRecord(ev[1], st), "profile event");
+    const uint32_t k = c->tuneStep;
+    const bool tune = c->tuned < 0;
+    if (tune) {
+        rc = tune_prepare(c, false);
+        if (rc) return rc;
+        DEM_TRY_CUDA(cudaEventRecord(c->tuneEv[2 * k], st), "tuner event");
+    }
+    for (int q = 0; q < 2; ++q)
+        DEM_TRY_CUDA(launch_band_step(c->P, c->band, q, false,
+                                      tune ? (int)(k % kStepVariants) : c->variant, st),
+                     "band step");
+    if (tune) {
+        DEM_TRY_CUDA(cudaEventRecord(c->tuneEv[2 * k + 1], st), "tuner event");
+        if (++c->tuneStep == kTuneSteps) {
+            rc = tune_finish(c, false);
+            if (rc) return rc;
+        }
+    }
+    if (prof) {
+        DEM_TRY_CUDA(cudaEventRecord(ev[2], st), "profile event");
+        c->evUsed += 3;
+        ++c->stepsProfiled;
+    }
+    return DEM_OK;
+}
+
+// `nsteps` steps in bands; with `follow`, each step's followed rows at row
+// block rowBlock + step of the ring.  The state is packed at the end.
+int band_steps(DemContext* c, uint32_t nsteps, bool follow, uint32_t rowBlock, cudaStream_t st) {
+    int rc = DEM_OK;
+    uint32_t done = 0;
+    while (done < nsteps && (c->tuned < 0 || c->profiling || (c->flags & DEM_CTX_DIRECT))) {
+        rc = band_step_alone(c, st);
+        if (rc) return rc;
+        ++done;
+    }
+    if (done < nsteps) {
+        rc = band_begin(c, nsteps - done, rowBlock + done, st);
+        if (rc) return rc;
+        cudaGraphExec_t* g = follow ? &c->bandFollow[c->cur] : &c->bandLoop[c->cur];
+        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_loop(c, follow, s); }, g);
+        if (rc) return rc;
+        DEM_TRY_CUDA(cudaGraphLaunch(*g, st), "graph launch");
+    }
+    DEM_TRY_CUDA(launch_band_pack(c->band, packed_state(c), false, st), "band pack");
+    return DEM_OK;
+}
+
+// The packed cell ranges and first-particle array of set cur, made from the
+// bands on the first request after a call.
+int band_cells(DemContext* c, cudaStream_t st) {
+    if (!c->bandValid || c->bandCells) return DEM_OK;
+    DEM_TRY_CUDA(launch_band_cells(c->band, c->cells[c->cur], c->first[c->cur], st), "band cells");
+    c->bandCells = true;
+    return DEM_OK;
+}
+
+}  // namespace
+
 // DEM_CTX_DIRECT: the same kernels launched one by one, the sort path
 // (incremental, or full after a mover overflow) read back on the host each
 // step instead of chosen on the device by conditional graph nodes, so that
@@ -1468,8 +1721,7 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
                                  c->resMaxC, c->resQueue, c->resWork, c->resBlocks, io, c->n,
                                  nsteps, c->errFlag, st),
                  "resident step");
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     c->inSortOrder = false;
     return DEM_OK;
 }
@@ -1504,8 +1756,7 @@ int cluster_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
         return kNotResident;
     }
     DEM_TRY_CUDA(e, "cluster step");
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     c->inSortOrder = false;
     return DEM_OK;
 }
@@ -1532,6 +1783,8 @@ namespace {
 // step loop for pairs of steps (also the steps of dem_step_followed, whose
 // per-step rows are gathered from this path's buffers).
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
+    if (steps_in_bands(c)) return band_steps(c, nsteps, false, 0, st);
+    c->bandValid = false;
     if (!c->keysValid) {
         if (c->nspec)
             DEM_TRY_CUDA(launch_calc_hash_batched(c->dTable, c->spec, c->dyn[0].pos, c->keys, c->n,
@@ -1641,6 +1894,8 @@ extern "C" int dem_get_step_variant(DemContext* c, DemStepVariant* out) {
 extern "C" int dem_get_cells(DemContext* c, uint32_t* cellStart, uint32_t* cellEnd,
                              void* stream) {
     if (!c) return fail(DEM_ERR_INVALID_ARG, "context is NULL");
+    int rc = band_cells(c, (cudaStream_t)stream);
+    if (rc) return rc;
     DEM_TRY_CUDA(launch_unpack_cells(c->cells[c->cur], c->numCells, cellStart, cellEnd,
                                      (cudaStream_t)stream),
                  "unpack cells");
@@ -1664,6 +1919,8 @@ extern "C" int dem_row_slots(DemContext* c, uint32_t rowLo, uint32_t rowHi, uint
     if (!c->inSortOrder)
         return fail(DEM_ERR_INVALID_ARG, "the state is not in the order of a sort: step first");
     cudaStream_t st = (cudaStream_t)stream;
+    int rc = band_cells(c, st);
+    if (rc) return rc;
     const uint32_t* f = c->first[c->cur];
     uint32_t w[2];
     DEM_TRY_CUDA(cudaMemcpyAsync(&w[0], f + (size_t)rowLo * gx, 4, cudaMemcpyDeviceToHost, st),
@@ -1706,6 +1963,7 @@ extern "C" int dem_debug_sort_hold(DemContext* c, uint32_t holdTile, uint32_t sp
 
 extern "C" int dem_kernels_per_step(DemContext* c) {
     if (!c) return -1;
+    if (steps_in_bands(c)) return 2;  // band_fix_kernel, band_step_kernel
     if (!c->sortGraph[1][0] && c->n > 0) {
         if (build_graph(c, 1, 0) != DEM_OK) return -1;
     }
@@ -1798,7 +2056,11 @@ extern "C" int dem_step_followed(DemContext* c, uint32_t nsteps, const uint32_t*
                  "followed count");
     for (uint32_t s = 0; s < nsteps;) {
         const uint32_t m = std::min(chunk, nsteps - s);
-        for (uint32_t j = 0; j < m;) {
+        const bool alone = (c->flags & DEM_CTX_DIRECT) || c->profiling || c->tuned < 0;
+        if (steps_in_bands(c) && !alone) {
+            int rc = band_steps(c, m, true, 0, st);
+            if (rc) return rc;
+        } else for (uint32_t j = 0; j < m;) {
             // pairs of steps with their rows in the device-side loop, as in
             // dem_step; a step with host work around it (the first after
             // dem_set_state, tuning, profiling, direct launches) alone
@@ -2072,8 +2334,7 @@ int restore_checkpoint(DemContext* c, const Snapshot& s, cudaStream_t st) {
     DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].radius, s.radius, 4 * n, cudaMemcpyDeviceToDevice, st), "restore radius");
     DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].mass, s.mass, 4 * n, cudaMemcpyDeviceToDevice, st), "restore mass");
     DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].id, s.id, 4 * n, cudaMemcpyDeviceToDevice, st), "restore id");
-    c->keysValid = false;
-    c->haveOrder = false;
+    state_replaced(c);
     c->inSortOrder = false;
     return DEM_OK;
 }

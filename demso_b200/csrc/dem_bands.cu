@@ -1,0 +1,623 @@
+// The step in bands (see dem_bands.cuh).
+#include "dem_bands.cuh"
+
+#include <algorithm>
+
+#include "dem_collide.cuh"
+#include "dem_sort.cuh"
+
+namespace dem {
+namespace {
+
+inline unsigned blocks_for(size_t n, int t) { return (unsigned)((n + (size_t)t - 1) / (size_t)t); }
+inline size_t al256(size_t b) { return (b + 255u) & ~(size_t)255u; }
+
+// Entries of the sorted a[0, n) below v.
+__device__ __forceinline__ uint32_t lower_count(const uint32_t* a, uint32_t n, uint32_t v) {
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (a[mid] < v) lo = mid + 1u;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// ------------------------------------------------------------------ fix
+// Bound by latency: a band's events, its cells' first slots, then its fields,
+// each once.  512 threads hold a run of 1,024 particles in registers while the
+// next run loads, so a band of any length is rewritten in place: a particle
+// moves by at most kBandEvents slots, so the places a run is stored to have
+// been read by then.
+constexpr int kFixThreads = 512;
+constexpr int kFixItems = 2;
+constexpr uint32_t kFixRun = kFixThreads * kFixItems;
+static_assert(kBandEvents <= kFixRun && kBandEvents <= (uint32_t)kFixThreads,
+              "an event per thread; moves stay within the next run");
+
+template <bool TYPED>
+struct Held {
+    float2 p, v;
+    float th, om, r, m;
+    uint32_t id, key, type, dst;
+};
+
+struct FixShared {
+    uint4 ev[kBandEvents];           // slot, new cell, old cell
+    uint32_t leave[kBandEvents];     // leavers' places in the band, sorted
+    uint32_t leaveCell[kBandEvents]; // their old cells (sorted too)
+    uint32_t arrive[kBandEvents];    // arrivals' 2 * cell + (from a higher cell), sorted
+    uint32_t arriveEv[kBandEvents];
+    uint32_t arriveDst[kBandEvents];
+    uint32_t arriveAt[kBandEvents];  // the old place they go in front of
+    uint32_t nl, na;
+};
+
+template <bool TYPED>
+__device__ __forceinline__ void fix_load(const BandArgs& B, const DynSet& d, const FixShared& S,
+                                         uint32_t base, uint32_t cell0, uint32_t from,
+                                         uint32_t end, uint32_t nl, uint32_t na,
+                                         Held<TYPED> (&h)[kFixItems]) {
+#pragma unroll
+    for (int u = 0; u < kFixItems; ++u) {
+        const uint32_t j = from + (uint32_t)u * kFixThreads + threadIdx.x;
+        h[u].dst = kBandEmpty;
+        if (j >= end) continue;
+        const uint32_t s = base + j;
+        const uint32_t key = B.key[s];
+        const uint32_t rl = lower_count(S.leave, nl, j);
+        if (rl < nl && S.leave[rl] == j) continue;  // it left
+        const uint32_t to = j - rl + lower_count(S.arrive, na, 2u * (key - cell0) + 1u);
+        if (to == j) continue;
+        h[u].dst = to;
+        h[u].key = key;
+        h[u].p = d.pos[s];
+        h[u].v = d.vel[s];
+        h[u].th = d.theta[s];
+        h[u].om = d.omega[s];
+        h[u].r = B.stat.radius[s];
+        h[u].m = B.stat.mass[s];
+        h[u].id = B.stat.id[s];
+        if (TYPED) h[u].type = B.stat.type[s];
+    }
+}
+
+template <bool TYPED>
+__device__ __forceinline__ void put(const BandArgs& B, const DynSet& d, uint32_t s, float2 p,
+                                    float2 v, float th, float om, float r, float m, uint32_t id,
+                                    uint32_t type, uint32_t key) {
+    d.pos[s] = p;
+    d.vel[s] = v;
+    d.theta[s] = th;
+    d.omega[s] = om;
+    B.stat.radius[s] = r;
+    B.stat.mass[s] = m;
+    B.stat.id[s] = id;
+    if (TYPED) B.stat.type[s] = type;
+    B.key[s] = key;
+    B.loc[id] = s;
+}
+
+template <bool TYPED>
+__device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint32_t b) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t cell0 = b << B.shift;
+    const uint32_t base = B.base[b], cnt = B.count[b];
+    const uint32_t ne = min(B.evCnt[b], kBandEvents);
+    const BandEvent* __restrict__ ev = B.ev + (size_t)b * kBandEvents;
+    if (tid < ne) S.ev[tid] = ev[tid].a;
+    if (tid == 0) S.nl = S.na = 0u;
+    __syncthreads();
+    if (tid < ne) {
+        const uint4 e = S.ev[tid];
+        const bool leaves = (e.z >> B.shift) == b, enters = (e.y >> B.shift) == b;
+        const uint32_t k2 = 2u * e.y + (e.z < e.y ? 0u : 1u);
+        uint32_t rl = 0, ra = 0;
+        for (uint32_t f = 0; f < ne; ++f) {
+            const uint4 o = S.ev[f];
+            const uint32_t o2 = 2u * o.y + (o.z < o.y ? 0u : 1u);
+            if ((o.z >> B.shift) == b && o.x < e.x) ++rl;
+            if ((o.y >> B.shift) == b && (o2 < k2 || (o2 == k2 && o.x < e.x))) ++ra;
+        }
+        if (leaves) {
+            S.leave[rl] = e.x - base;
+            S.leaveCell[rl] = e.z - cell0;
+            atomicAdd(&S.nl, 1u);
+        }
+        if (enters) {
+            S.arrive[ra] = k2 - 2u * cell0;
+            S.arriveEv[ra] = tid;
+            atomicAdd(&S.na, 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t nl = S.nl, na = S.na;
+    if (tid < na) {
+        const uint32_t k2 = S.arrive[tid], c = cell0 + (k2 >> 1);
+        // in front of its cell's stayers, or behind them
+        const uint32_t at = B.first[(size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u)) +
+                                    (k2 & 1u)] - base;
+        S.arriveAt[tid] = at;
+        S.arriveDst[tid] = at - lower_count(S.leave, nl, at) + tid;
+    }
+    __syncthreads();
+    // places outside [from, end) keep their particles
+    const uint32_t from = min(nl ? S.leave[0] : cnt, na ? S.arriveAt[0] : cnt);
+    const uint32_t end = nl != na ? cnt
+                                  : max(nl ? S.leave[nl - 1] + 1u : 0u, na ? S.arriveAt[na - 1] : 0u);
+    Held<TYPED> now[kFixItems], next[kFixItems];
+    fix_load<TYPED>(B, d, S, base, cell0, from, end, nl, na, now);
+    for (uint32_t run = from; run < end; run += kFixRun) {
+        fix_load<TYPED>(B, d, S, base, cell0, run + kFixRun, end, nl, na, next);
+        __syncthreads();  // this run and the next are read
+#pragma unroll
+        for (int u = 0; u < kFixItems; ++u) {
+            const Held<TYPED>& h = now[u];
+            if (h.dst != kBandEmpty)
+                put<TYPED>(B, d, base + h.dst, h.p, h.v, h.th, h.om, h.r, h.m, h.id, h.type, h.key);
+        }
+#pragma unroll
+        for (int u = 0; u < kFixItems; ++u) now[u] = next[u];
+    }
+    __syncthreads();
+    if (tid < na) {
+        const BandEvent e = ev[S.arriveEv[tid]];
+        put<TYPED>(B, d, base + S.arriveDst[tid], make_float2(e.b.x, e.b.y),
+                   make_float2(e.b.z, e.b.w), e.c.x, e.c.y, e.c.z, e.c.w, e.a.w, e.d.x, e.a.y);
+    }
+    const uint32_t newCnt = cnt - nl + na;
+    for (uint32_t j = newCnt + tid; j < cnt; j += kFixThreads) B.key[base + j] = kBandEmpty;
+    // first slots: one more for every arrival in a lower cell, one fewer for
+    // every leaver of one
+    const uint32_t rows = 1u << (B.shift - B.log2gx), row0 = cell0 >> B.log2gx;
+    for (uint32_t r = 0; r < rows; ++r)
+        for (uint32_t x = tid; x <= B.gx; x += kFixThreads) {
+            const uint32_t c = r * B.gx + x;
+            const uint32_t up = lower_count(S.arrive, na, 2u * c);
+            const uint32_t down = lower_count(S.leaveCell, nl, c);
+            if (up != down) B.first[(size_t)(row0 + r) * (B.gx + 1u) + x] += up - down;
+        }
+    if (tid == 0) {
+        B.count[b] = newCnt;
+        B.evCnt[b] = 0u;
+    }
+}
+
+template <bool TYPED>
+__global__ void __launch_bounds__(kFixThreads, 2) band_fix_kernel(BandArgs B, DynSet d, uint32_t q) {
+    __shared__ FixShared S;
+    const uint32_t left = B.ctrl[kBandLeft];
+    const bool active = left != 0u && B.ctrl[kBandCur] == q && B.ctrl[kBandFull] == 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        B.ctrl[kBandAct + q] = active ? (left == 1u ? 2u : 1u) : 0u;
+    if (!active) return;
+    const uint32_t nd = min(B.ctrl[kBandDirty + q], B.bands);
+    for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
+        fix_band<TYPED>(B, d, S, B.dirty[q][k]);
+        __syncthreads();
+    }
+}
+
+// ----------------------------------------------------------------- step
+// An event into band b's list; the band's first one puts it on the list of
+// the next step's fix.  A full list, or no free slot for every event, asks
+// for a new layout.
+__device__ __forceinline__ BandEvent* push_event(const BandArgs& B, uint32_t b, uint32_t nextSet) {
+    const uint32_t k = atomicAdd(B.evCnt + b, 1u);
+    if (k == 0u) {
+        const uint32_t w = atomicAdd(B.ctrl + kBandDirty + nextSet, 1u);
+        if (w < B.bands) B.dirty[nextSet][w] = b;
+    }
+    const uint32_t room = B.base[b + 1u] - B.base[b] - B.count[b];
+    if (k >= min(kBandEvents, room)) {
+        B.ctrl[kBandFull] = 1u;
+        return nullptr;
+    }
+    return B.ev + (size_t)b * kBandEvents + k;
+}
+
+template <bool TYPED, bool ATTRACT, bool CULL, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB)
+band_step_kernel(KParams P, BandArgs B, DynSet in, DynSet out, uint32_t q, uint32_t everyStep) {
+    const uint32_t act = B.ctrl[kBandAct + q];
+    const uint32_t i = blockIdx.x * THREADS + threadIdx.x;
+    if (i >= B.slots) return;
+    const uint32_t key = B.key[i];
+    Dyn s;
+    s.p = in.pos[i];
+    const float r = B.stat.radius[i];
+    s.v = in.vel[i];
+    s.w = in.omega[i];
+    s.th = in.theta[i];
+    const float m = B.stat.mass[i];
+    const uint32_t mat = TYPED ? B.stat.type[i] : 0u;
+    if (act == 0u) return;
+    if (i == 0u) {
+        B.ctrl[kBandCur] = q ^ 1u;
+        B.ctrl[kBandLeft] -= 1u;
+        B.ctrl[kBandDone] += 1u;
+        B.ctrl[kBandDirty + q] = 0u;  // taken by the fix before this kernel
+        // a sort whose wait gave up left no order to build on
+        if (*B.errFlag & kSortTimeoutBit) B.ctrl[kBandFull] = 1u;
+    }
+    if (key == kBandEmpty) return;
+    const int2 g = make_int2((int)(key & (P.gx - 1u)), (int)(key >> P.log2gx));
+    float2 f;
+    float moment, pr;
+    if (!CULL || !P.cull ||
+        !collide_rows<TYPED, ATTRACT>(P, i, g, s.p, s.v, s.w, r, mat, in.pos, in.vel, in.omega,
+                                      B.stat.radius, B.stat.type, nullptr, B.first, P.gx + 1u, f,
+                                      moment, pr)) {
+        const RowCells cells{B.first, P.gx, P.log2gx};
+        collide_one<TYPED, ATTRACT, CULL && !ATTRACT>(P, i, g, s.p, s.v, s.w, r, mat, in.pos,
+                                                      in.vel, in.omega, B.stat.radius, B.stat.type,
+                                                      nullptr, cells, f, moment, pr);
+    }
+    // F/m and M/I as the reference divides them; without contacts both are
+    // exactly +0 (see finish_particle)
+    const bool quiet = f.x == 0.0f && f.y == 0.0f && moment == 0.0f && m > 0.0f && m < INFINITY;
+    const float two_mrr = 2.0f * m * r * r;
+    float2 a = make_float2(0.0f, 0.0f);
+    float al = 0.0f;
+    if (!(quiet && two_mrr >= 1e-30f && two_mrr <= 1e30f)) {
+        a = make_float2(f.x / m, f.y / m);
+        al = moment / inertia_of(m, r);
+    }
+    integrate_one(P, s, a, al, r, m, mat, pr);
+    out.pos[i] = s.p;
+    out.vel[i] = s.v;
+    out.theta[i] = s.th;
+    out.omega[i] = s.w;
+    // the next step overwrites these: only the call's last step stores them
+    if (act == 2u || everyStep) {
+        if (B.pressure) B.pressure[i] = pr;
+        if (B.acc) {
+            B.acc[i] = a;
+            B.alpha[i] = al;
+        }
+    }
+    if (!(isfinite(s.p.x) && isfinite(s.p.y))) atomicOr(B.errFlag, 1u);
+    const int2 gn = grid_pos_fast(P, s.p);
+    const uint32_t nk = grid_hash(P, gn.x, gn.y);
+    if (nk != key) {
+        B.key[i] = nk;
+        const uint32_t b0 = key >> B.shift, b1 = nk >> B.shift;
+        const uint32_t id = B.stat.id[i];
+        BandEvent* e = push_event(B, b1, q ^ 1u);
+        if (e) {
+            e->a = make_uint4(i, nk, key, id);
+            e->b = make_float4(s.p.x, s.p.y, s.v.x, s.v.y);
+            e->c = make_float4(s.th, s.w, r, m);
+            e->d = make_uint4(mat, 0u, 0u, 0u);
+        }
+        if (b0 != b1) {
+            e = push_event(B, b0, q ^ 1u);
+            if (e) e->a = make_uint4(i, nk, key, id);
+        }
+    }
+}
+
+// --------------------------------------------------------- pack, layout
+constexpr int kPackThreads = 256;
+
+// Particles of the bands below `b` (every thread gets the sum).
+__device__ __forceinline__ uint32_t packed_base(const uint32_t* __restrict__ count, uint32_t b) {
+    __shared__ uint32_t warpSum[kPackThreads / 32];
+    uint32_t v = 0;
+    for (uint32_t k = threadIdx.x; k < b; k += kPackThreads) v += count[k];
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31u) == 0) warpSum[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < kPackThreads / 32; ++w) t += warpSum[w];
+    return t;
+}
+
+// Blocks (band, share): share y of the band's particles.  Bound by DRAM: 40 B
+// in and 44 B out per particle.
+template <bool TYPED>
+__global__ void __launch_bounds__(kPackThreads)
+band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
+    if (B.ctrl[kBandLaid] == 0u) return;
+    const uint32_t b = blockIdx.x;
+    const uint32_t base = B.base[b], cnt = B.count[b];
+    const uint32_t to = packed_base(B.count, b);
+    const bool one = B.ctrl[kBandCur] != 0u;
+    const float2* __restrict__ pos = one ? B.dyn[1].pos : B.dyn[0].pos;
+    const float2* __restrict__ vel = one ? B.dyn[1].vel : B.dyn[0].vel;
+    const float* __restrict__ theta = one ? B.dyn[1].theta : B.dyn[0].theta;
+    const float* __restrict__ omega = one ? B.dyn[1].omega : B.dyn[0].omega;
+    for (uint32_t k = blockIdx.y * kPackThreads + threadIdx.x; k < cnt;
+         k += gridDim.y * kPackThreads) {
+        const uint32_t s = base + k, i = to + k;
+        // out of range only after a sort whose wait gave up
+        if (s >= B.slots || i >= B.n) break;
+        const uint32_t id = B.stat.id[s];
+        o.dyn.pos[i] = pos[s];
+        o.dyn.vel[i] = vel[s];
+        o.dyn.theta[i] = theta[s];
+        o.dyn.omega[i] = omega[s];
+        o.stat.radius[i] = B.stat.radius[s];
+        o.stat.mass[i] = B.stat.mass[s];
+        o.stat.id[i] = id;
+        if (TYPED) o.stat.type[i] = B.stat.type[s];
+        if (stateOnly) continue;
+        o.loc[id] = i;
+        if (B.pressure) o.pressure[i] = B.pressure[s];
+        if (B.acc) {
+            o.acc[i] = B.acc[s];
+            o.alpha[i] = B.alpha[s];
+        }
+    }
+}
+
+// First particle of every cell in the sorted keys (lower bounds).
+__global__ void band_cell_first_kernel(const uint32_t* __restrict__ keys, uint32_t n,
+                                       uint32_t cells, uint32_t* __restrict__ first) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= cells;
+         c += gridDim.x * blockDim.x)
+        first[c] = lower_count(keys, n, c);
+}
+
+// Bands' bases, counts and first slots from the packed first-particle array
+// f; empty slots' keys; counters.
+__global__ void band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
+    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t s = t0; s < B.slots; s += stride) B.key[s] = kBandEmpty;
+    for (size_t k = t0; k <= B.bands; k += stride) {
+        const uint32_t b = (uint32_t)k;
+        const uint32_t p = f[min((uint64_t)b << B.shift, (uint64_t)B.cells)];
+        B.base[b] = p + b * B.slack;
+        if (b < B.bands) {
+            const uint32_t e = f[min((uint64_t)(b + 1u) << B.shift, (uint64_t)B.cells)];
+            // e < p only after a sort whose wait gave up
+            B.count[b] = e > p ? e - p : 0u;
+            B.evCnt[b] = 0u;
+        }
+    }
+    const uint32_t rows = B.cells >> B.log2gx;
+    for (size_t k = t0; k < (size_t)rows * (B.gx + 1u); k += stride) {
+        const uint32_t row = (uint32_t)(k / (B.gx + 1u)), x = (uint32_t)(k - (size_t)row * (B.gx + 1u));
+        const uint32_t b = (row << B.log2gx) >> B.shift;
+        B.first[k] = f[(row << B.log2gx) + x] + b * B.slack;
+    }
+}
+
+// The packed particles, in sorted order, into the slots of set 0.
+template <bool TYPED>
+__global__ void __launch_bounds__(kPackThreads)
+band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys,
+                   const uint32_t* __restrict__ from) {
+    const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
+    if (i == 0u) {
+        B.ctrl[kBandFull] = 0u;
+        B.ctrl[kBandCur] = 0u;
+        B.ctrl[kBandLaid] = 1u;
+        B.ctrl[kBandDirty] = 0u;
+        B.ctrl[kBandDirty + 1u] = 0u;
+    }
+    if (i >= B.n) return;
+    // in range unless a wait of the sort gave up (stale words)
+    const uint32_t key = min(keys[i], B.cells - 1u), src = min(from[i], B.n - 1u);
+    const uint32_t s = i + (key >> B.shift) * B.slack;
+    put<TYPED>(B, B.dyn[0], s, in.dyn.pos[src], in.dyn.vel[src], in.dyn.theta[src],
+               in.dyn.omega[src], in.stat.radius[src], in.stat.mass[src], in.stat.id[src],
+               TYPED ? in.stat.type[src] : 0u, key);
+}
+
+// Blocks (band): packed (start, end) of every cell and first-particle array.
+__global__ void __launch_bounds__(kPackThreads)
+band_cells_kernel(BandArgs B, uint2* __restrict__ cells, uint32_t* __restrict__ first) {
+    if (B.ctrl[kBandLaid] == 0u) return;
+    const uint32_t b = blockIdx.x;
+    const uint32_t shiftDown = B.base[b] - packed_base(B.count, b);
+    const uint32_t c0 = b << B.shift;
+    for (uint32_t k = threadIdx.x; k < (1u << B.shift); k += kPackThreads) {
+        const uint32_t c = c0 + k;
+        if (c >= B.cells) break;
+        const uint32_t* f = B.first + (size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u));
+        const uint32_t a = f[0] - shiftDown, e = f[1] - shiftDown;
+        first[c] = a;
+        cells[c] = a < e ? make_uint2(a, e) : make_uint2(kEmptyCell, kEmptyCell);
+        if (c == B.cells - 1u) first[B.cells] = e;
+    }
+}
+
+__global__ void band_followed_kernel(BandArgs B, DynSet d, uint32_t q,
+                                     const uint32_t* __restrict__ ids,
+                                     const uint32_t* __restrict__ countWord,
+                                     float* __restrict__ ring) {
+    if (B.ctrl[kBandAct + q] == 0u) return;
+    const uint32_t count = *countWord;
+    float* base = ring + (size_t)(B.ctrl[kBandDone] - 1u) * count * 12;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count;
+         k += gridDim.x * blockDim.x)
+        followed_row(B.loc[ids[k]], base + 12ull * k, d, B.stat, B.acc, B.alpha, B.pressure);
+}
+
+// ---------------------------------------------------------- conditions
+__global__ void band_head_kernel(uint32_t* __restrict__ ctrl, cudaGraphConditionalHandle full,
+                                 cudaGraphConditionalHandle loop, int setLoop) {
+    cudaGraphSetConditional(full, ctrl[kBandFull] ? 1u : 0u);
+    if (setLoop) cudaGraphSetConditional(loop, ctrl[kBandLeft] ? 1u : 0u);
+}
+__global__ void band_next_kernel(uint32_t* __restrict__ ctrl, cudaGraphConditionalHandle loop,
+                                 int whileFull) {
+    const bool go = ctrl[kBandLeft] != 0u && (whileFull || ctrl[kBandFull] == 0u);
+    cudaGraphSetConditional(loop, go ? 1u : 0u);
+}
+
+bool attracts(const KParams& P) {
+    for (uint32_t m = 0; m < P.nmat; ++m)
+        if (P.at[m] != 0.0f) return true;
+    return false;
+}
+
+}  // namespace
+
+bool band_shape(uint32_t gx, uint32_t numCells, BandArgs& b) {
+    if (gx == 0 || gx > kBandMaxRow || numCells < gx) return false;
+    uint32_t per = std::max(kBandMinCells, gx);
+    while ((uint64_t)per * kBandMaxBands < numCells) per <<= 1;
+    per = std::min(per, numCells);
+    b.gx = gx;
+    b.cells = numCells;
+    b.log2gx = b.shift = 0;
+    while ((1u << b.log2gx) < gx) ++b.log2gx;
+    while ((1u << b.shift) < per) ++b.shift;
+    b.bands = (numCells + per - 1u) / per;
+    return true;
+}
+
+uint32_t band_slack(const BandArgs& b, uint32_t n) {
+    return std::max(kBandMinSlack, n / (16u * b.bands));
+}
+size_t band_slots(const BandArgs& b, uint32_t n) {
+    return (size_t)n + (size_t)b.bands * band_slack(b, n);
+}
+
+namespace {
+// The arrays in order: take(bytes) gives each one's address.
+template <typename Take>
+void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel, Take take) {
+    const size_t S = band_slots(b, capacity) + kFilterPad;
+    for (int k = 0; k < 2; ++k) {
+        b.dyn[k].pos = static_cast<float2*>(take(8 * S));
+        b.dyn[k].vel = static_cast<float2*>(take(8 * S));
+        b.dyn[k].theta = static_cast<float*>(take(4 * S));
+        b.dyn[k].omega = static_cast<float*>(take(4 * S));
+    }
+    b.stat.radius = static_cast<float*>(take(4 * S));
+    b.stat.mass = static_cast<float*>(take(4 * S));
+    b.stat.id = static_cast<uint32_t*>(take(4 * S));
+    b.stat.type = typed ? static_cast<uint32_t*>(take(4 * S)) : nullptr;
+    b.key = static_cast<uint32_t*>(take(4 * S));
+    b.loc = static_cast<uint32_t*>(take(4ull * capacity));
+    const size_t rows = b.cells >> b.log2gx;
+    b.first = static_cast<uint32_t*>(take(4 * (rows * (b.gx + 1ull) + 4)));
+    b.base = static_cast<uint32_t*>(take(4ull * (b.bands + 1)));
+    b.count = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.evCnt = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.ev = static_cast<BandEvent*>(take(sizeof(BandEvent) * (size_t)b.bands * kBandEvents));
+    for (int k = 0; k < 2; ++k) b.dirty[k] = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.ctrl = static_cast<uint32_t*>(take(4 * kBandCtrlWords));
+    b.pressure = pressure ? static_cast<float*>(take(4 * S)) : nullptr;
+    b.acc = accel ? static_cast<float2*>(take(8 * S)) : nullptr;
+    b.alpha = accel ? static_cast<float*>(take(4 * S)) : nullptr;
+}
+}  // namespace
+
+size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel) {
+    BandArgs t = b;
+    size_t total = 0;
+    band_arrays(t, capacity, typed, pressure, accel, [&](size_t bytes) -> void* {
+        total += al256(bytes);
+        return nullptr;
+    });
+    return total;
+}
+
+void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure,
+                 bool accel) {
+    char* p = static_cast<char*>(base);
+    band_arrays(b, capacity, typed, pressure, accel, [&](size_t bytes) -> void* {
+        char* q = p;
+        p += al256(bytes);
+        return q;
+    });
+}
+
+cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st) {
+    // two blocks of 512 threads fit on a multiprocessor
+    const unsigned blocks = std::min(b.bands, 296u);
+    if (b.stat.type)
+        band_fix_kernel<true><<<blocks, kFixThreads, 0, st>>>(b, b.dyn[q], (uint32_t)q);
+    else
+        band_fix_kernel<false><<<blocks, kFixThreads, 0, st>>>(b, b.dyn[q], (uint32_t)q);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool everyStep,
+                             int variant, cudaStream_t st) {
+    if (variant < 0 || variant >= kStepVariants) return cudaErrorInvalidValue;
+    const bool typed = b.stat.type != nullptr && P.nmat > 1;
+    const bool attract = attracts(P), cull = P.cull != 0u;
+    const DynSet in = b.dyn[q], out = b.dyn[q ^ 1];
+    const uint32_t e = everyStep ? 1u : 0u;
+#define DEM_BAND_T(T, A, C, TH, MB)                                                          \
+    band_step_kernel<T, A, C, TH, MB><<<blocks_for(b.slots, TH), TH, 0, st>>>(P, b, in, out, \
+                                                                              (uint32_t)q, e)
+#define DEM_BAND(T, A, C)                                    \
+    do {                                                     \
+        switch (variant) {                                   \
+            case 1: DEM_BAND_T(T, A, C, 64, 16); break;      \
+            case 2: DEM_BAND_T(T, A, C, 256, 4); break;      \
+            case 3: DEM_BAND_T(T, A, C, 128, 6); break;      \
+            default: DEM_BAND_T(T, A, C, 128, 8); break;     \
+        }                                                    \
+    } while (0)
+#define DEM_BAND_AC(T)                          \
+    do {                                        \
+        if (attract && cull) DEM_BAND(T, true, true);   \
+        else if (attract) DEM_BAND(T, true, false);     \
+        else if (cull) DEM_BAND(T, false, true);        \
+        else DEM_BAND(T, false, false);                 \
+    } while (0)
+    if (typed) DEM_BAND_AC(true);
+    else DEM_BAND_AC(false);
+#undef DEM_BAND_AC
+#undef DEM_BAND
+#undef DEM_BAND_T
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_followed(const BandArgs& b, int q, const uint32_t* ids,
+                                 const uint32_t* countWord, float* ring, cudaStream_t st) {
+    band_followed_kernel<<<16, 128, 0, st>>>(b, b.dyn[q ^ 1], (uint32_t)q, ids, countWord, ring);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool stateOnly,
+                             cudaStream_t st) {
+    // enough blocks to fill the GPU, a share of a band each
+    const dim3 grid(b.bands, std::max(1u, 1184u / b.bands));
+    if (b.stat.type)
+        band_pack_kernel<true><<<grid, kPackThreads, 0, st>>>(b, out, stateOnly ? 1u : 0u);
+    else
+        band_pack_kernel<false><<<grid, kPackThreads, 0, st>>>(b, out, stateOnly ? 1u : 0u);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_layout(const BandArgs& b, const PackedState& in, const uint32_t* keys,
+                               const uint32_t* from, uint32_t* cellFirst, cudaStream_t st) {
+    band_cell_first_kernel<<<std::min(blocks_for((size_t)b.cells + 1, kPackThreads), 1184u),
+                             kPackThreads, 0, st>>>(keys, b.n, b.cells, cellFirst);
+    band_layout_kernel<<<1184, kPackThreads, 0, st>>>(b, cellFirst);
+    const unsigned g = blocks_for(b.n, kPackThreads);
+    if (b.stat.type)
+        band_spread_kernel<true><<<g, kPackThreads, 0, st>>>(b, in, keys, from);
+    else
+        band_spread_kernel<false><<<g, kPackThreads, 0, st>>>(b, in, keys, from);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_cells(const BandArgs& b, uint2* cells, uint32_t* first, cudaStream_t st) {
+    band_cells_kernel<<<b.bands, kPackThreads, 0, st>>>(b, cells, first);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_head(const BandArgs& b, cudaGraphConditionalHandle full,
+                             cudaGraphConditionalHandle loop, bool setLoop, cudaStream_t st) {
+    band_head_kernel<<<1, 1, 0, st>>>(b.ctrl, full, loop, setLoop ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_next(const BandArgs& b, cudaGraphConditionalHandle loop, bool whileFull,
+                             cudaStream_t st) {
+    band_next_kernel<<<1, 1, 0, st>>>(b.ctrl, loop, whileFull ? 1 : 0);
+    return cudaGetLastError();
+}
+
+}  // namespace dem

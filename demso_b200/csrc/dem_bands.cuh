@@ -1,0 +1,139 @@
+// The step in bands: a layout of the sorted state that a step leaves in place.
+//
+// The reference sorts all particles by cell on every step, although between
+// two steps of a granular scene only a few in a hundred thousand change cell.
+// In a densely packed order each of them shifts every particle behind it, so
+// even an incremental sort rewrites the whole state.  Here the order is kept
+// in bands of whole cell rows with free slots at the end of each: a particle
+// that changes cell shifts only the particles between the two places of its
+// own band, or those behind it in the two bands it left and entered; every
+// other band stays where it is, in every array.  A step is two kernels:
+//
+//   fix   one block per band that a particle left or entered in the last
+//         step: the band's particles in the stable order of their new cells
+//         ([arrivals from lower cells][stayers][arrivals from higher cells],
+//         each in the previous order), in place;
+//   step  collide + integrate + new cell, a thread per slot, from one dynamic
+//         set into the other; radius, mass, id and type stay in place.  A
+//         particle whose cell changed writes an event (its whole state) for
+//         the band it enters and a note for the band it leaves.
+//
+// When a band's events or free slots run out (or there is no band layout yet)
+// the next step first lays the bands out again: the state is packed, sorted
+// with the radix sort and spread into bands.  At the end of a call the state
+// is packed into the context's sorted arrays, so that every reader finds it
+// as after a packed sort: the concatenation of the bands is the reference's
+// sorted order, and the bits are its own.
+//
+// Against the packed incremental sort (six kernels a step, 40 B moved per
+// particle in the sort phase and 88 B in the step; here two kernels, 64 B in
+// the step): a call of 20 steps of 4,194,304 disks 4,623 -> 3,911 us, of
+// 1,000,003 dense disks 1,514 -> 1,279 us, 50 steps of 65,536 1,214 -> 1,024 us,
+// 20 steps of a fast gas of 131,071 607 -> 465 us.
+//
+// The two dynamic sets alternate with the steps; which of them holds the state
+// is a word on the device (kBandCur), since a new layout always starts in set
+// 0.  A kernel of set q does nothing unless kBandCur is q.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "dem_kernels.cuh"
+
+namespace dem {
+
+constexpr uint32_t kBandEmpty = 0xffffffffu;  // key of a free slot
+// Events (particles that left or entered) a band takes in one step.
+constexpr uint32_t kBandEvents = 128;
+// Free slots of a band: at least this, and a sixteenth of its share of n.
+constexpr uint32_t kBandMinSlack = 64;
+// Cells of a band: at least kBandMinCells and a whole row; wider rows than
+// kBandMaxRow cells take the packed path (one block rewrites a band).
+constexpr uint32_t kBandMinCells = 256, kBandMaxRow = 4096, kBandMaxBands = 4096;
+
+// Words of BandArgs::ctrl.
+constexpr uint32_t kBandLeft = 0;   // steps left of the call
+constexpr uint32_t kBandDone = 1;   // steps done (the row block of the followed particles)
+constexpr uint32_t kBandFull = 2;   // the next step needs a new layout
+constexpr uint32_t kBandCur = 3;    // dynamic set holding the state
+constexpr uint32_t kBandLaid = 4;   // the bands hold the state (0: only the packed arrays do)
+constexpr uint32_t kBandAct = 5;    // [2] step of set q: 0 skipped, 1 runs, 2 runs as the call's last
+constexpr uint32_t kBandDirty = 7;  // [2] bands with events, by the set the fix of which takes them
+constexpr uint32_t kBandCtrlWords = 16;
+
+// A particle that changed cell: its slot and cells, and its state.
+struct __align__(16) BandEvent {
+    uint4 a;   // slot, new cell, old cell, id
+    float4 b;  // position, velocity
+    float4 c;  // angle, spin, radius, mass
+    uint4 d;   // type
+};
+
+struct BandArgs {
+    uint32_t bands = 0, shift = 0;  // band of a cell: cell >> shift
+    uint32_t gx = 0, log2gx = 0, cells = 0;
+    uint32_t n = 0, slots = 0, slack = 0;
+    DynSet dyn[2] = {};  // slot-indexed
+    StatSet stat = {};
+    uint32_t* key = nullptr;  // cell of every slot's particle (kBandEmpty: free)
+    uint32_t* loc = nullptr;  // slot by id
+    uint32_t* first = nullptr;  // first slot of every cell, gx + 1 words a row (the last: row end)
+    uint32_t* base = nullptr;   // bands + 1
+    uint32_t* count = nullptr;  // particles of each band
+    uint32_t* evCnt = nullptr;
+    BandEvent* ev = nullptr;
+    uint32_t* dirty[2] = {};
+    uint32_t* ctrl = nullptr;
+    float* pressure = nullptr;  // slot-indexed, null when not kept
+    float2* acc = nullptr;
+    float* alpha = nullptr;
+    uint32_t* errFlag = nullptr;
+};
+
+// The packed arrays: the context's state in sorted order.
+struct PackedState {
+    DynSet dyn;
+    StatSet stat;
+    uint32_t* loc;
+    float* pressure;
+    float2* acc;
+    float* alpha;
+};
+
+// Shape of the bands of a grid (bands, shift, gx, log2gx, cells); false when
+// the grid takes the packed path.
+bool band_shape(uint32_t gx, uint32_t numCells, BandArgs& b);
+// Free slots per band, and slots in all, for n particles.
+uint32_t band_slack(const BandArgs& b, uint32_t n);
+size_t band_slots(const BandArgs& b, uint32_t n);
+// Bytes of the band arrays of `capacity` particles, and their addresses.
+size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel);
+void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure, bool accel);
+
+// The kernels; `q` is the dynamic set they step from.
+cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st);
+// everyStep: pressure and accelerations are stored on every step, not only on
+// the call's last one.
+cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool everyStep,
+                             int variant, cudaStream_t st);
+cudaError_t launch_band_followed(const BandArgs& b, int q, const uint32_t* ids,
+                                 const uint32_t* countWord, float* ring, cudaStream_t st);
+// The state into the packed arrays (with pressure and accelerations unless
+// stateOnly); nothing when the bands hold no state.
+cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool stateOnly,
+                             cudaStream_t st);
+// New layout from the packed arrays, sorted by `keys` (their particles in
+// order `from`); cellFirst: numCells + 1 words of scratch.
+cudaError_t launch_band_layout(const BandArgs& b, const PackedState& in, const uint32_t* keys,
+                               const uint32_t* from, uint32_t* cellFirst, cudaStream_t st);
+// Packed cell ranges and first-particle array of the current state.
+cudaError_t launch_band_cells(const BandArgs& b, uint2* cells, uint32_t* first, cudaStream_t st);
+
+// Conditions of the step loop's graph nodes.
+cudaError_t launch_band_head(const BandArgs& b, cudaGraphConditionalHandle full,
+                             cudaGraphConditionalHandle loop, bool setLoop, cudaStream_t st);
+cudaError_t launch_band_next(const BandArgs& b, cudaGraphConditionalHandle loop, bool whileFull,
+                             cudaStream_t st);
+
+}  // namespace dem

@@ -22,6 +22,29 @@ struct StatSet {
     uint32_t* type;  // may be null (single material)
 };
 
+// One row of the reference's followed-particle output (functions.cu:630-654)
+// for the particle in slot i: id, type, pos, vel, acc, theta, omega, alpha,
+// pressure.
+__device__ __forceinline__ void followed_row(uint32_t i, float* __restrict__ r, const DynSet& d,
+                                             const StatSet& s, const float2* __restrict__ acc,
+                                             const float* __restrict__ alpha,
+                                             const float* __restrict__ pressure) {
+    r[0] = __uint_as_float(s.id[i]);
+    r[1] = __uint_as_float(s.type ? s.type[i] : 0u);
+    const float2 p = d.pos[i], v = d.vel[i];
+    r[2] = p.x;
+    r[3] = p.y;
+    r[4] = v.x;
+    r[5] = v.y;
+    const float2 a = acc ? acc[i] : make_float2(0.0f, 0.0f);
+    r[6] = a.x;
+    r[7] = a.y;
+    r[8] = d.theta[i];
+    r[9] = d.omega[i];
+    r[10] = alpha ? alpha[i] : 0.0f;
+    r[11] = pressure ? pressure[i] : 0.0f;
+}
+
 constexpr uint32_t kFollowBatch = 64;
 struct FollowIds {
     uint32_t count;
