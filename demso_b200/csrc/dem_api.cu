@@ -389,7 +389,7 @@ struct DemContext {
     BandArgs band;
     void* bandBlock = nullptr;
     float2* ownPos = nullptr;  // the block's positions: not an adopted set
-    bool bandValid = false, bandCells = false;
+    bool bandValid = false, bandCells = false, bandInit = false;
     cudaGraphExec_t bandLoop[2] = {}, bandFollow[2] = {}, bandSort[2] = {};
     // followed-particle staging (device), see dem_get_followed
     float* followRows = nullptr;
@@ -1514,6 +1514,13 @@ int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t s
     c->band.n = c->n;
     c->band.slack = band_slack(c->band, c->n);
     c->band.slots = (uint32_t)band_slots(c->band, c->n);
+    c->band.skin = c->P.cull ? kSkin * c->P.rmax : 0.0f;
+    if (!c->bandInit) {
+        // stamps start below the first step's number
+        DEM_TRY_CUDA(cudaMemsetAsync(c->band.stamp, 0, 4ull * c->band.cells, st), "band stamps");
+        DEM_TRY_CUDA(launch_set_words(c->band.ctrl + kBandStep, Words{{1u}, 1u}, st), "band step");
+        c->bandInit = true;
+    }
     const Words w = c->bandValid ? Words{{nsteps, rowBlock}, 2u}
                                  : Words{{nsteps, rowBlock, 1u, 0u, 0u}, 5u};
     DEM_TRY_CUDA(launch_set_words(c->band.ctrl, w, st), "band step count");

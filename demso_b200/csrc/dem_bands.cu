@@ -25,12 +25,14 @@ __device__ __forceinline__ uint32_t lower_count(const uint32_t* a, uint32_t n, u
 
 // ------------------------------------------------------------------ fix
 // Bound by latency: a band's events, its cells' first slots, then its fields,
-// each once.  512 threads hold a run of 1,024 particles in registers while the
+// each once.  512 threads hold a run of 512 particles in registers while the
 // next run loads, so a band of any length is rewritten in place: a particle
 // moves by at most kBandEvents slots, so the places a run is stored to have
-// been read by then.
+// been read by then.  Two such blocks fit on a multiprocessor, so 296 bands
+// are rewritten at once; runs of 1,024 (one block) measured 162 against 154 us
+// a step at 4,194,304 disks, 256 threads 165.
 constexpr int kFixThreads = 512;
-constexpr int kFixItems = 2;
+constexpr int kFixItems = 1;
 constexpr uint32_t kFixRun = kFixThreads * kFixItems;
 static_assert(kBandEvents <= kFixRun && kBandEvents <= (uint32_t)kFixThreads,
               "an event per thread; moves stay within the next run");
@@ -40,6 +42,7 @@ struct Held {
     float2 p, v;
     float th, om, r, m;
     uint32_t id, key, type, dst;
+    unsigned long long cand;
 };
 
 struct FixShared {
@@ -78,6 +81,7 @@ __device__ __forceinline__ void fix_load(const BandArgs& B, const DynSet& d, con
         h[u].r = B.stat.radius[s];
         h[u].m = B.stat.mass[s];
         h[u].id = B.stat.id[s];
+        h[u].cand = B.cand[s];
         if (TYPED) h[u].type = B.stat.type[s];
     }
 }
@@ -85,7 +89,7 @@ __device__ __forceinline__ void fix_load(const BandArgs& B, const DynSet& d, con
 template <bool TYPED>
 __device__ __forceinline__ void put(const BandArgs& B, const DynSet& d, uint32_t s, float2 p,
                                     float2 v, float th, float om, float r, float m, uint32_t id,
-                                    uint32_t type, uint32_t key) {
+                                    uint32_t type, uint32_t key, unsigned long long cand) {
     d.pos[s] = p;
     d.vel[s] = v;
     d.theta[s] = th;
@@ -95,6 +99,7 @@ __device__ __forceinline__ void put(const BandArgs& B, const DynSet& d, uint32_t
     B.stat.id[s] = id;
     if (TYPED) B.stat.type[s] = type;
     B.key[s] = key;
+    B.cand[s] = cand;
     B.loc[id] = s;
 }
 
@@ -154,7 +159,8 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
         for (int u = 0; u < kFixItems; ++u) {
             const Held<TYPED>& h = now[u];
             if (h.dst != kBandEmpty)
-                put<TYPED>(B, d, base + h.dst, h.p, h.v, h.th, h.om, h.r, h.m, h.id, h.type, h.key);
+                put<TYPED>(B, d, base + h.dst, h.p, h.v, h.th, h.om, h.r, h.m, h.id, h.type, h.key,
+                           h.cand);
         }
 #pragma unroll
         for (int u = 0; u < kFixItems; ++u) now[u] = next[u];
@@ -163,7 +169,8 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
     if (tid < na) {
         const BandEvent e = ev[S.arriveEv[tid]];
         put<TYPED>(B, d, base + S.arriveDst[tid], make_float2(e.b.x, e.b.y),
-                   make_float2(e.b.z, e.b.w), e.c.x, e.c.y, e.c.z, e.c.w, e.a.w, e.d.x, e.a.y);
+                   make_float2(e.b.z, e.b.w), e.c.x, e.c.y, e.c.z, e.c.w, e.a.w, e.d.x, e.a.y,
+                   kCandNone);
     }
     const uint32_t newCnt = cnt - nl + na;
     for (uint32_t j = newCnt + tid; j < cnt; j += kFixThreads) B.key[base + j] = kBandEmpty;
@@ -188,9 +195,24 @@ __global__ void __launch_bounds__(kFixThreads, 2) band_fix_kernel(BandArgs B, Dy
     __shared__ FixShared S;
     const uint32_t left = B.ctrl[kBandLeft];
     const bool active = left != 0u && B.ctrl[kBandCur] == q && B.ctrl[kBandFull] == 0u;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         B.ctrl[kBandAct + q] = active ? (left == 1u ? 2u : 1u) : 0u;
+        B.ctrl[kBandNow + q] = B.ctrl[kBandStep];
+    }
     if (!active) return;
+    // how far pairs may have approached since their bands searched
+    for (uint32_t b = blockIdx.x * kFixThreads + threadIdx.x; b < B.bands;
+         b += gridDim.x * kFixThreads) {
+        const uint32_t lo = b ? b - 1u : B.bands - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
+        const float own = __uint_as_float(B.moved[q][b]);
+        // as bits, so that a NaN is the largest
+        const float any = __uint_as_float(max(B.moved[q][b], max(B.moved[q][lo], B.moved[q][hi])));
+        const float grown = B.grown[b] + (own + any) * 1.0001f;
+        const bool keep = grown <= 0.99f * B.skin;
+        B.grown[b] = keep ? grown : 0.0f;
+        B.search[b] = keep ? 0u : 1u;
+        B.moved[q ^ 1u][b] = 0u;  // the step of this set collects it
+    }
     const uint32_t nd = min(B.ctrl[kBandDirty + q], B.bands);
     for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
         fix_band<TYPED>(B, d, S, B.dirty[q][k]);
@@ -216,12 +238,264 @@ __device__ __forceinline__ BandEvent* push_event(const BandArgs& B, uint32_t b, 
     return B.ev + (size_t)b * kBandEvents + k;
 }
 
+// Reach of a particle's search: contacts (or attraction) plus the skin.
+template <bool ATTRACT>
+__device__ __forceinline__ float search_bound(float r, float rj, float skin) {
+    const float d = (ATTRACT ? kAttractReach * fmaxf(r, rj) : r + rj) + skin;
+    return d * d * 1.00001f;
+}
+
+// The kept candidates of a particle (see kCandNone): one bit for every
+// candidate within reach plus the skin, row by row.  A cell met across the
+// wrap of the grid's columns is only checked: a candidate there, as a row
+// interval of more than kCandBits, keeps none.
+template <bool ATTRACT>
+__device__ __noinline__ unsigned long long
+search_candidates(const KParams& P, uint32_t i, uint32_t key, float2 p, float r, float skin,
+                  const float2* __restrict__ pos, const float* __restrict__ radius,
+                  const uint32_t* __restrict__ first) {
+    if (ATTRACT && !(r > 0.0f)) return kCandNone;
+    const int gx = (int)(key & (P.gx - 1u)), gy = (int)(key >> P.log2gx);
+    int y0 = -1, y1 = 1;
+    if (p.y > P.cullMargin && p.y < P.Ly - P.cullMargin && p.x > P.cullMargin &&
+        p.x < P.Lx - P.cullMargin) {
+        const float reach =
+            (ATTRACT ? kAttractReach * P.rmax : r + P.rmax) * 1.0001f + P.cullMargin + skin;
+        const float Y0 = (float)(gy + P.rowOff) * P.cellH;
+        if (p.y - Y0 > reach) y0 = 0;
+        if (Y0 + P.cellH - p.y > reach) y1 = 0;
+    }
+    const int xb = max(gx - 1, 0), xe = min(gx + 1, (int)P.gx - 1);
+    unsigned long long kept = 0ull;
+#pragma unroll 1
+    for (int dy = y0; dy <= y1; ++dy) {
+        const uint32_t* __restrict__ f =
+            first + (size_t)((gy + dy) & (int)(P.gy - 1u)) * (P.gx + 1u);
+        const uint32_t a = __ldg(f + xb), n = __ldg(f + xe + 1) - a;
+        if (n > kCandBits) return kCandNone;
+        uint32_t bits = 0u;
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < n; k0 += 4u) {
+            float2 q[4];
+            float rq[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                q[k] = __ldg(pos + (a + k0 + k));
+                rq[k] = __ldg(radius + (a + k0 + k));
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float dx = q[k].x - p.x, dy2 = q[k].y - p.y;
+                if (dx * dx + dy2 * dy2 <= search_bound<ATTRACT>(r, rq[k], skin))
+                    bits |= 1u << (k0 + k);
+            }
+        }
+        bits &= (1u << n) - 1u;  // groups are read whole
+        if (i - a < n) bits &= ~(1u << (i - a));
+        kept |= (unsigned long long)bits << (kCandBits * (uint32_t)(dy + 1));
+        if (xe - xb != 2) {
+            const int w = gx == 0 ? (int)P.gx - 1 : 0;
+            for (uint32_t j = __ldg(f + w), e = __ldg(f + w + 1); j < e; ++j) {
+                const float2 q = __ldg(pos + j);
+                const float dx = q.x - p.x, dy2 = q.y - p.y;
+                if (dx * dx + dy2 * dy2 <= search_bound<ATTRACT>(r, __ldg(radius + j), skin))
+                    return kCandNone;
+            }
+        }
+    }
+    return kept;
+}
+
+struct Pull {
+    float2 f;
+    float moment, pr;
+};
+
+// The search and the law together, for slots that keep no candidates.
+template <bool TYPED, bool ATTRACT, bool CULL>
+__device__ __noinline__ Pull collide_slot(const KParams& P, const BandArgs& B, const DynSet& in,
+                                          uint32_t i, uint32_t key, float2 p, float2 v, float w,
+                                          float r, uint32_t mat) {
+    const int2 g = make_int2((int)(key & (P.gx - 1u)), (int)(key >> P.log2gx));
+    Pull o;
+    if (!CULL || !P.cull ||
+        !collide_rows<TYPED, ATTRACT>(P, i, g, p, v, w, r, mat, in.pos, in.vel, in.omega,
+                                      B.stat.radius, B.stat.type, nullptr, B.first, P.gx + 1u,
+                                      o.f, o.moment, o.pr)) {
+        const RowCells cells{B.first, P.gx, P.log2gx};
+        collide_one<TYPED, ATTRACT, CULL && !ATTRACT>(P, i, g, p, v, w, r, mat, in.pos, in.vel,
+                                                      in.omega, B.stat.radius, B.stat.type,
+                                                      nullptr, cells, o.f, o.moment, o.pr);
+    }
+    return o;
+}
+
+// A warp's contacts, dealt to its lanes.  The contact law is some two hundred
+// instructions (five IEEE divisions, four square roots, a double division) and
+// the particles of a warp touch 0 to 6 others, so lane by lane it ran at a
+// third of the lanes.  Instead a turn takes up to kDeal kept candidates of
+// every lane, whose loads are in flight together, and writes the touching ones
+// into a list in shared memory; the warp evaluates the list 32 at a time, and
+// each lane adds up its own results in its own order.  With the kept candidates
+// (kSkin), a call of 20 steps: 1,000,003 dense disks 54.1 M warp instructions a
+// step at 11 active lanes -> 30 M at 19; 4,194,304 disks 3,911 -> 3,327 us,
+// 250,007 cohesive disks 1,339 -> 1,019 us, 50 steps of 65,536 disks
+// 1,024 -> 885 us.  What bounds the step now is the latency of its four or five
+// rounds of dependent loads (42 % of issue slots used at 4,194,304 disks).
+constexpr int kDeal = 4;
+template <bool ATTRACT>
+struct Deal {
+    uint32_t j[kDeal * 32];  // [candidate of the turn][lane]: the neighbour, then the force's x
+    float fy[kDeal * 32], moment[kDeal * 32];
+    double q[kDeal * 32];
+    float ax[ATTRACT ? kDeal * 32 : 1], ay[ATTRACT ? kDeal * 32 : 1];
+    double aq[ATTRACT ? kDeal * 32 : 1];
+    uint8_t code[kDeal * 32];  // the list: index into the arrays above
+};
+
+// First slot of each of the three row intervals around the cell of `key`, for
+// the rows with candidates in `cand`.
+struct RowBase {
+    uint32_t a[3];
+};
+__device__ __forceinline__ const uint32_t* row_first(const KParams& P, const BandArgs& B,
+                                                     uint32_t key, uint32_t row) {
+    const uint32_t x = key & (P.gx - 1u), y = (key >> P.log2gx) + row - 1u;
+    return B.first + (size_t)(y & (P.gy - 1u)) * (P.gx + 1u) + (x ? x - 1u : 0u);
+}
+__device__ __forceinline__ RowBase row_bases(const KParams& P, const BandArgs& B, uint32_t key,
+                                             unsigned long long cand) {
+    RowBase o;
+#pragma unroll
+    for (uint32_t k = 0; k < 3u; ++k) {
+        const uint32_t bits = (uint32_t)(cand >> (kCandBits * k)) & ((1u << kCandBits) - 1u);
+        o.a[k] = bits ? __ldg(row_first(P, B, key, k)) : 0u;
+    }
+    return o;
+}
+
+// Forces on the particles of a warp from their kept candidates `rem` (0 for a
+// lane without any), in index order, one subtotal per cell, the subtotals
+// added in cell order (an empty cell adds +0).  Every lane calls it.
+template <bool TYPED, bool ATTRACT>
+__device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B, const DynSet& in,
+                                             Deal<ATTRACT>& S, unsigned long long rem,
+                                             const RowBase& base, uint32_t key, float2 p, float2 v,
+                                             float w, float r, uint32_t mat, Pull& o) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t cell = 15u;  // cell of the subtotal
+    float2 sub = make_float2(0.0f, 0.0f);
+    while (__any_sync(kAll, rem != 0ull)) {
+        uint32_t at[kDeal], row[kDeal];
+        float2 qp[kDeal];
+        float qr[kDeal];
+        unsigned have = 0u;
+#pragma unroll
+        for (int k = 0; k < kDeal; ++k) {
+            at[k] = row[k] = 0u;
+            if (rem != 0ull) {
+                const uint32_t bit = (uint32_t)__ffsll((long long)rem) - 1u;
+                rem &= rem - 1ull;
+                row[k] = bit >= 2u * kCandBits ? 2u : (bit >= kCandBits ? 1u : 0u);
+                at[k] = (row[k] == 2u ? base.a[2] : (row[k] == 1u ? base.a[1] : base.a[0])) +
+                        (bit - row[k] * kCandBits);
+                have |= 1u << k;
+            }
+            qp[k] = __ldg(in.pos + at[k]);
+            qr[k] = __ldg(B.stat.radius + at[k]);
+        }
+        uint32_t total = 0u, cells = 0u, mine = 0u;
+#pragma unroll
+        for (int k = 0; k < kDeal; ++k) {
+            const float dx = qp[k].x - p.x, dy = qp[k].y - p.y;
+            const float d2 = dx * dx + dy * dy;
+            const float cd = r + qr[k];
+            // beyond: sqrtf(d2) >= cd after rounding (or both attraction
+            // ranges), no force
+            const bool hit = ((have >> k) & 1u) && (ATTRACT ? !attract_out_of_reach(r, qr[k], d2)
+                                                            : d2 <= cd * cd * 1.000002f);
+            const unsigned hits = __ballot_sync(kAll, hit);
+            if (hit) {
+                const uint32_t* __restrict__ f = row_first(P, B, key, row[k]);
+                S.j[k * 32 + lane] = at[k];
+                S.code[total + __popc(hits & ((1u << lane) - 1u))] = (uint8_t)(k * 32 + lane);
+                cells |= (3u * row[k] + (at[k] >= __ldg(f + 1) ? 1u : 0u) +
+                          (at[k] >= __ldg(f + 2) ? 1u : 0u)) << (4 * k);
+                mine |= 1u << k;
+            }
+            total += (uint32_t)__popc(hits);
+        }
+        if (total == 0u) continue;
+        __syncwarp();
+        for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
+            const uint32_t e = e0 + lane;
+            const uint32_t code = e < total ? S.code[e] : lane;
+            const int own = (int)(code & 31u);
+            const float2 pA = make_float2(__shfl_sync(kAll, p.x, own), __shfl_sync(kAll, p.y, own));
+            const float2 vA = make_float2(__shfl_sync(kAll, v.x, own), __shfl_sync(kAll, v.y, own));
+            const float wA = __shfl_sync(kAll, w, own), rA = __shfl_sync(kAll, r, own);
+            const uint32_t mA = TYPED ? __shfl_sync(kAll, mat, own) : 0u;
+            if (e < total) {
+                const uint32_t j = S.j[code];
+                const uint32_t mB = TYPED ? __ldg(B.stat.type + j) : 0u;
+                const float4 pc = TYPED ? P.pair[mA * P.nmat + mB] : P.pair[0];
+                const float2 pB = __ldg(in.pos + j);
+                const float rB = __ldg(B.stat.radius + j);
+                float2 f;
+                float m;
+                double q;
+                pair_terms(pA, pB, vA, __ldg(in.vel + j), wA, __ldg(in.omega + j), rA, rB, pc,
+                           P.dt, f, m, q);
+                S.j[code] = __float_as_uint(f.x);
+                S.fy[code] = f.y;
+                S.moment[code] = m;
+                S.q[code] = q;
+                if (ATTRACT) {
+                    const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB], q);
+                    S.ax[code] = g.x;
+                    S.ay[code] = g.y;
+                    S.aq[code] = q;
+                }
+            }
+        }
+        __syncwarp();
+        while (mine) {
+            const uint32_t k = (uint32_t)__ffs(mine) - 1u, x = k * 32u + lane;
+            mine &= mine - 1u;
+            const uint32_t c = (cells >> (4u * k)) & 15u;
+            if (c != cell) {
+                o.f.x += sub.x;
+                o.f.y += sub.y;
+                sub = make_float2(0.0f, 0.0f);
+                cell = c;
+            }
+            sub.x += __uint_as_float(S.j[x]);
+            sub.y += S.fy[x];
+            o.moment += S.moment[x];
+            o.pr = (float)((double)o.pr + S.q[x]);
+            if (ATTRACT) {
+                sub.x += S.ax[x];
+                sub.y += S.ay[x];
+                o.pr = (float)((double)o.pr + S.aq[x]);
+            }
+        }
+        __syncwarp();  // the results are read
+    }
+    o.f.x += sub.x;
+    o.f.y += sub.y;
+}
+
 template <bool TYPED, bool ATTRACT, bool CULL, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
-band_step_kernel(KParams P, BandArgs B, DynSet in, DynSet out, uint32_t q, uint32_t everyStep) {
+band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ BandArgs B,
+                 const __grid_constant__ DynSet in, const __grid_constant__ DynSet out, uint32_t q,
+                 uint32_t everyStep) {
+    __shared__ Deal<ATTRACT> deal[CULL ? THREADS / 32 : 1];
     const uint32_t act = B.ctrl[kBandAct + q];
-    const uint32_t i = blockIdx.x * THREADS + threadIdx.x;
-    if (i >= B.slots) return;
+    const uint32_t slot = blockIdx.x * THREADS + threadIdx.x;
+    // the lanes past the last slot stand by as copies of it
+    const uint32_t i = min(slot, B.slots - 1u);
     const uint32_t key = B.key[i];
     Dyn s;
     s.p = in.pos[i];
@@ -231,57 +505,85 @@ band_step_kernel(KParams P, BandArgs B, DynSet in, DynSet out, uint32_t q, uint3
     s.th = in.theta[i];
     const float m = B.stat.mass[i];
     const uint32_t mat = TYPED ? B.stat.type[i] : 0u;
+    unsigned long long cand = CULL ? B.cand[i] : kCandNone;
     if (act == 0u) return;
-    if (i == 0u) {
+    const uint32_t now = B.ctrl[kBandNow + q];
+    if (slot == 0u) {
         B.ctrl[kBandCur] = q ^ 1u;
         B.ctrl[kBandLeft] -= 1u;
         B.ctrl[kBandDone] += 1u;
+        B.ctrl[kBandStep] = now + 1u;
         B.ctrl[kBandDirty + q] = 0u;  // taken by the fix before this kernel
         // a sort whose wait gave up left no order to build on
         if (*B.errFlag & kSortTimeoutBit) B.ctrl[kBandFull] = 1u;
     }
-    if (key == kBandEmpty) return;
-    const int2 g = make_int2((int)(key & (P.gx - 1u)), (int)(key >> P.log2gx));
-    float2 f;
-    float moment, pr;
-    if (!CULL || !P.cull ||
-        !collide_rows<TYPED, ATTRACT>(P, i, g, s.p, s.v, s.w, r, mat, in.pos, in.vel, in.omega,
-                                      B.stat.radius, B.stat.type, nullptr, B.first, P.gx + 1u, f,
-                                      moment, pr)) {
-        const RowCells cells{B.first, P.gx, P.log2gx};
-        collide_one<TYPED, ATTRACT, CULL && !ATTRACT>(P, i, g, s.p, s.v, s.w, r, mat, in.pos,
-                                                      in.vel, in.omega, B.stat.radius, B.stat.type,
-                                                      nullptr, cells, f, moment, pr);
+    const bool mine = slot < B.slots && key != kBandEmpty;
+    if (!__any_sync(0xffffffffu, mine)) return;
+    Pull o{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
+    RowBase base{};
+    if (!mine) {
+        cand = 0ull;
+    } else {
+        // one round of loads: whether to search, and the rows of the candidates
+        // kept so far
+        if (CULL) base = row_bases(P, B, key, cand & kCandNone ? 0ull : cand);
+        if (CULL && ((cand & kCandNone) || B.stamp[key] == now || B.search[key >> B.shift])) {
+            cand = search_candidates<ATTRACT>(P, i, key, s.p, r, B.skin, in.pos, B.stat.radius,
+                                              B.first);
+            B.cand[i] = cand;
+            base = row_bases(P, B, key, cand & kCandNone ? 0ull : cand);
+        }
+        if (cand & kCandNone) {
+            o = collide_slot<TYPED, ATTRACT, CULL>(P, B, in, i, key, s.p, s.v, s.w, r, mat);
+            cand = 0ull;
+        }
     }
+    if (CULL)
+        collide_warp<TYPED, ATTRACT>(P, B, in, deal[threadIdx.x >> 5], cand, base, key, s.p, s.v,
+                                     s.w, r, mat, o);
+    if (!mine) return;
     // F/m and M/I as the reference divides them; without contacts both are
     // exactly +0 (see finish_particle)
-    const bool quiet = f.x == 0.0f && f.y == 0.0f && moment == 0.0f && m > 0.0f && m < INFINITY;
+    const bool quiet =
+        o.f.x == 0.0f && o.f.y == 0.0f && o.moment == 0.0f && m > 0.0f && m < INFINITY;
     const float two_mrr = 2.0f * m * r * r;
     float2 a = make_float2(0.0f, 0.0f);
     float al = 0.0f;
     if (!(quiet && two_mrr >= 1e-30f && two_mrr <= 1e30f)) {
-        a = make_float2(f.x / m, f.y / m);
-        al = moment / inertia_of(m, r);
+        a = make_float2(o.f.x / m, o.f.y / m);
+        al = o.moment / inertia_of(m, r);
     }
-    integrate_one(P, s, a, al, r, m, mat, pr);
+    const float2 was = s.p;
+    integrate_one(P, s, a, al, r, m, mat, o.pr);
     out.pos[i] = s.p;
     out.vel[i] = s.v;
     out.theta[i] = s.th;
     out.omega[i] = s.w;
     // the next step overwrites these: only the call's last step stores them
     if (act == 2u || everyStep) {
-        if (B.pressure) B.pressure[i] = pr;
+        if (B.pressure) B.pressure[i] = o.pr;
         if (B.acc) {
             B.acc[i] = a;
             B.alpha[i] = al;
         }
     }
     if (!(isfinite(s.p.x) && isfinite(s.p.y))) atomicOr(B.errFlag, 1u);
+    const uint32_t b0 = key >> B.shift;
+    if (CULL) {
+        // the band's largest displacement, one atomic a warp while it grows
+        uint32_t far = __float_as_uint(fabsf(s.p.x - was.x) + fabsf(s.p.y - was.y)) & 0x7fffffffu;
+        const unsigned lanes = __activemask();
+        if (__all_sync(lanes, b0 == __shfl_sync(lanes, b0, __ffs(lanes) - 1))) {
+            far = __reduce_max_sync(lanes, far);
+            if ((threadIdx.x & 31u) != (uint32_t)(__ffs(lanes) - 1)) far = 0u;
+        }
+        if (far) atomicMax(B.moved[q ^ 1u] + b0, far);
+    }
     const int2 gn = grid_pos_fast(P, s.p);
     const uint32_t nk = grid_hash(P, gn.x, gn.y);
     if (nk != key) {
         B.key[i] = nk;
-        const uint32_t b0 = key >> B.shift, b1 = nk >> B.shift;
+        const uint32_t b1 = nk >> B.shift;
         const uint32_t id = B.stat.id[i];
         BandEvent* e = push_event(B, b1, q ^ 1u);
         if (e) {
@@ -293,6 +595,16 @@ band_step_kernel(KParams P, BandArgs B, DynSet in, DynSet out, uint32_t q, uint3
         if (b0 != b1) {
             e = push_event(B, b0, q ^ 1u);
             if (e) e->a = make_uint4(i, nk, key, id);
+        }
+        // row intervals around both cells change: the slots there search anew
+        if (CULL) {
+#pragma unroll 1
+            for (int k = 0; k < 18; ++k) {
+                const uint32_t c = k < 9 ? key : nk;
+                const int x = (int)(c & (P.gx - 1u)) + k % 3 - 1;
+                const int y = (int)(c >> P.log2gx) + k / 3 % 3 - 1;
+                B.stamp[cell_index(P, x, y)] = now + 1u;
+            }
         }
     }
 }
@@ -375,6 +687,8 @@ __global__ void band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
             // e < p only after a sort whose wait gave up
             B.count[b] = e > p ? e - p : 0u;
             B.evCnt[b] = 0u;
+            B.moved[0][b] = B.moved[1][b] = 0u;
+            B.grown[b] = 0.0f;  // no slot keeps candidates: every one searches
         }
     }
     const uint32_t rows = B.cells >> B.log2gx;
@@ -404,7 +718,7 @@ band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys
     const uint32_t s = i + (key >> B.shift) * B.slack;
     put<TYPED>(B, B.dyn[0], s, in.dyn.pos[src], in.dyn.vel[src], in.dyn.theta[src],
                in.dyn.omega[src], in.stat.radius[src], in.stat.mass[src], in.stat.id[src],
-               TYPED ? in.stat.type[src] : 0u, key);
+               TYPED ? in.stat.type[src] : 0u, key, kCandNone);
 }
 
 // Blocks (band): packed (start, end) of every cell and first-particle array.
@@ -502,6 +816,11 @@ void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool
     b.evCnt = static_cast<uint32_t*>(take(4ull * b.bands));
     b.ev = static_cast<BandEvent*>(take(sizeof(BandEvent) * (size_t)b.bands * kBandEvents));
     for (int k = 0; k < 2; ++k) b.dirty[k] = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.cand = static_cast<unsigned long long*>(take(8 * S));
+    b.stamp = static_cast<uint32_t*>(take(4ull * b.cells));
+    for (int k = 0; k < 2; ++k) b.moved[k] = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.grown = static_cast<float*>(take(4ull * b.bands));
+    b.search = static_cast<uint32_t*>(take(4ull * b.bands));
     b.ctrl = static_cast<uint32_t*>(take(4 * kBandCtrlWords));
     b.pressure = pressure ? static_cast<float*>(take(4 * S)) : nullptr;
     b.acc = accel ? static_cast<float2*>(take(8 * S)) : nullptr;
@@ -530,8 +849,7 @@ void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pr
 }
 
 cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st) {
-    // two blocks of 512 threads fit on a multiprocessor
-    const unsigned blocks = std::min(b.bands, 296u);
+    const unsigned blocks = std::min(b.bands, 296u);  // two to a multiprocessor
     if (b.stat.type)
         band_fix_kernel<true><<<blocks, kFixThreads, 0, st>>>(b, b.dyn[q], (uint32_t)q);
     else

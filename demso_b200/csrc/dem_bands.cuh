@@ -60,7 +60,24 @@ constexpr uint32_t kBandCur = 3;    // dynamic set holding the state
 constexpr uint32_t kBandLaid = 4;   // the bands hold the state (0: only the packed arrays do)
 constexpr uint32_t kBandAct = 5;    // [2] step of set q: 0 skipped, 1 runs, 2 runs as the call's last
 constexpr uint32_t kBandDirty = 7;  // [2] bands with events, by the set the fix of which takes them
+constexpr uint32_t kBandStep = 9;   // steps since the context was made
+constexpr uint32_t kBandNow = 10;   // [2] kBandStep as the step of set q sees it
 constexpr uint32_t kBandCtrlWords = 16;
+
+// Kept candidates.  The search for neighbours (row intervals, radii and
+// distances of some twenty candidates) finds almost the same few pairs step
+// after step.  Every slot keeps a bit for each candidate within reach plus a
+// skin of kSkin * rmax, counted from the first slot of its row interval, 21
+// bits for each of the three rows; a step then meets only those.  The bits
+// are a superset of the contacts until a pair of the band or its neighbour
+// bands may have closed the skin -- the sum over the steps since of the
+// largest displacement of the band and of the largest of the three bands --
+// or a particle enters or leaves a cell of the slot's 3 x 3, which stamps the
+// cells around it for the next step.  Then the slot searches again.  Slots
+// whose bits do not fit search on every step.
+constexpr float kSkin = 0.1f;
+constexpr uint32_t kCandBits = 21;
+constexpr unsigned long long kCandNone = 1ull << 63;  // no bits kept: search
 
 // A particle that changed cell: its slot and cells, and its state.
 struct __align__(16) BandEvent {
@@ -84,6 +101,12 @@ struct BandArgs {
     uint32_t* evCnt = nullptr;
     BandEvent* ev = nullptr;
     uint32_t* dirty[2] = {};
+    unsigned long long* cand = nullptr;  // kept candidates of every slot
+    float skin = 0.0f;
+    uint32_t* stamp = nullptr;      // per cell: the step that searches anew there
+    uint32_t* moved[2] = {};        // per band: largest |dx| + |dy| of a step (float bits)
+    float* grown = nullptr;         // per band: bound on a pair's approach since the search
+    uint32_t* search = nullptr;     // per band: this step searches anew
     uint32_t* ctrl = nullptr;
     float* pressure = nullptr;  // slot-indexed, null when not kept
     float2* acc = nullptr;

@@ -114,64 +114,84 @@ __device__ __forceinline__ uint32_t grid_hash(const KParams& P, int x, int y) {
     return cell_index(P, x, y - P.rowOff);
 }
 
+// `length(force) / (4*M_PI*r*r)`, the term added to the pressure.
+__device__ __forceinline__ double pressure_term(float flen, float r) {
+    const double den = 4.0 * 3.14159265358979323846 * (double)r * (double)r;
+    return (double)flen / den;
+}
+
 // `pressure += length(force) / (4*M_PI*r*r)` -- the reference does this sum in
 // double and stores the float result.
 __device__ __forceinline__ float add_pressure(float pr, float flen, float r) {
-    const double den = 4.0 * 3.14159265358979323846 * (double)r * (double)r;
-    return (float)((double)pr + (double)flen / den);
+    return (float)((double)pr + pressure_term(flen, r));
 }
 
 // One particle pair, particles_kernel.cuh:236-307 (collideSpheres).  A is the
-// particle being updated, B the neighbour.  Returns the force on A; adds the
-// moment and the pressure contribution.
-__device__ __forceinline__ float2 pair_force(float2 pA, float2 pB, float2 vA, float2 vB, float wA,
-                                             float wB, float rA, float rB, float4 pc, float dt,
-                                             float& moment, float& pressure) {
+// particle being updated, B the neighbour.  Returns whether they touch, with
+// the force on A and the terms of A's moment and pressure.
+__device__ __forceinline__ bool pair_terms(float2 pA, float2 pB, float2 vA, float2 vB, float wA,
+                                           float wB, float rA, float rB, float4 pc, float dt,
+                                           float2& f, float& moment, double& pressure) {
     const float relx = pB.x - pA.x, rely = pB.y - pA.y;
     const float dist = len2(relx, rely);
     const float cd = rA + rB;
-    float2 f = make_float2(0.0f, 0.0f);
-    if (dist < cd) {
-        const float nx = relx / dist, ny = rely / dist;
-        const float tx = -ny, ty = nx;
-        const float rvx = vB.x - vA.x, rvy = vB.y - vA.y;
-        const float vn = rvx * nx + rvy * ny;
-        const float vtx = rvx - vn * nx, vty = rvy - vn * ny;
-        const float fs = -pc.x * (cd - dist);
-        f.x = fs * nx;
-        f.y = fs * ny;
-        if (vn < 0.0f) {
-            const float c = pc.z * vn;
-            f.x += c * nx;
-            f.y += c * ny;
+    f = make_float2(0.0f, 0.0f);
+    moment = 0.0f;
+    pressure = 0.0;
+    if (!(dist < cd)) return false;
+    const float nx = relx / dist, ny = rely / dist;
+    const float tx = -ny, ty = nx;
+    const float rvx = vB.x - vA.x, rvy = vB.y - vA.y;
+    const float vn = rvx * nx + rvy * ny;
+    const float vtx = rvx - vn * nx, vty = rvy - vn * ny;
+    const float fs = -pc.x * (cd - dist);
+    f.x = fs * nx;
+    f.y = fs * ny;
+    if (vn < 0.0f) {
+        const float c = pc.z * vn;
+        f.x += c * nx;
+        f.y += c * ny;
+    }
+    pressure = pressure_term(len2(f.x, f.y), rA);
+    if (pc.w != 0.0f) {
+        const float sw = rA * wA + rB * wB;
+        const float vcx = vtx - sw * tx, vcy = vty - sw * ty;
+        const float ftrx = pc.y * vcx * dt, ftry = pc.y * vcy * dt;
+        const float ftmax = pc.w * len2(f.x, f.y);
+        float ftx, fty;
+        if (len2(ftrx, ftry) < ftmax) {
+            ftx = ftrx;
+            fty = ftry;
+        } else {
+            const float l = len2(vcx, vcy);
+            ftx = ftmax * vcx / l;
+            fty = ftmax * vcy / l;
         }
-        pressure = add_pressure(pressure, len2(f.x, f.y), rA);
-        if (pc.w != 0.0f) {
-            const float sw = rA * wA + rB * wB;
-            const float vcx = vtx - sw * tx, vcy = vty - sw * ty;
-            const float ftrx = pc.y * vcx * dt, ftry = pc.y * vcy * dt;
-            const float ftmax = pc.w * len2(f.x, f.y);
-            float ftx, fty;
-            if (len2(ftrx, ftry) < ftmax) {
-                ftx = ftrx;
-                fty = ftry;
-            } else {
-                const float l = len2(vcx, vcy);
-                ftx = ftmax * vcx / l;
-                fty = ftmax * vcy / l;
-            }
-            f.x += ftx;
-            f.y += fty;
-            moment += rA * (ftx * tx + fty * ty);
-        }
+        f.x += ftx;
+        f.y += fty;
+        moment = rA * (ftx * tx + fty * ty);
+    }
+    return true;
+}
+
+// The same, added to A's running moment and pressure.
+__device__ __forceinline__ float2 pair_force(float2 pA, float2 pB, float2 vA, float2 vB, float wA,
+                                             float wB, float rA, float rB, float4 pc, float dt,
+                                             float& moment, float& pressure) {
+    float2 f;
+    float m;
+    double q;
+    if (pair_terms(pA, pB, vA, vB, wA, wB, rA, rB, pc, dt, f, m, q)) {
+        pressure = (float)((double)pressure + q);
+        if (pc.w != 0.0f) moment += m;
     }
     return f;
 }
 
 // particles_kernel.cuh:311-342 (attractSpheres), only compiled into the
 // attraction variants of the collide kernels.
-__device__ __forceinline__ float2 pair_attract(float2 pA, float2 pB, float rA, float rB, float aA,
-                                               float aB, float& pressure) {
+__device__ __forceinline__ float2 pair_attract_terms(float2 pA, float2 pB, float rA, float rB,
+                                                     float aA, float aB, double& pressure) {
     const float relx = pB.x - pA.x, rely = pB.y - pA.y;
     const float dist = len2(relx, rely);
     const float dA = (float)((double)(rA * 2.0f) * 1.2);
@@ -188,7 +208,14 @@ __device__ __forceinline__ float2 pair_attract(float2 pA, float2 pB, float rA, f
         f.x += c * nx;
         f.y += c * ny;
     }
-    pressure = add_pressure(pressure, len2(f.x, f.y), rA);
+    pressure = pressure_term(len2(f.x, f.y), rA);
+    return f;
+}
+__device__ __forceinline__ float2 pair_attract(float2 pA, float2 pB, float rA, float rB, float aA,
+                                               float aB, float& pressure) {
+    double q;
+    const float2 f = pair_attract_terms(pA, pB, rA, rB, aA, aB, q);
+    pressure = (float)((double)pressure + q);
     return f;
 }
 
