@@ -36,7 +36,7 @@ struct SortScratch {
     uint32_t* altKeys;   // n
     uint32_t* altVals;   // n
     uint32_t* hist;      // sort_hist_words
-    uint32_t* partials;  // sort_scan_partials
+    uint32_t* partials;  // sort_scan_partials words, spare (the size query is part of the ABI)
 };
 
 // Bytes of scratch for the layout carve_sort_scratch produces.
@@ -80,9 +80,5 @@ cudaError_t onesweep_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint
                                 bool identityVals, const OnesweepScratch& s, uint32_t* errFlag,
                                 cudaStream_t stream, uint32_t** keysOut, uint32_t** valsOut,
                                 int* launches);
-
-// Exclusive scan of `len` words in place; partials holds sort_scan_partials(len).
-cudaError_t exclusive_scan_u32(uint32_t* data, size_t len, uint32_t* partials,
-                               cudaStream_t stream, int* launches);
 
 }  // namespace dem

@@ -14,8 +14,7 @@
 // (other streams, other host threads, same device) race on it and corrupt
 // each other's results; order them on one stream or synchronise between
 // them.  Every scratch word is written before it is read within a call (the
-// per-tile histograms, the scan partials and the alternate key/value
-// buffers), so nothing left from an earlier call needs clearing.
+// per-tile histograms and the alternate key/value buffers), so nothing left from an earlier call needs clearing.
 #include <cstdio>
 #include <mutex>
 
