@@ -306,11 +306,6 @@ search_candidates(const KParams& P, uint32_t i, uint32_t key, float2 p, float r,
     return kept;
 }
 
-struct Pull {
-    float2 f;
-    float moment, pr;
-};
-
 // The search and the law together, for slots that keep no candidates.
 template <bool TYPED, bool ATTRACT, bool CULL>
 __device__ __noinline__ Pull collide_slot(const KParams& P, const BandArgs& B, const DynSet& in,
@@ -329,29 +324,6 @@ __device__ __noinline__ Pull collide_slot(const KParams& P, const BandArgs& B, c
     }
     return o;
 }
-
-// A warp's contacts, dealt to its lanes.  The contact law is some two hundred
-// instructions (five IEEE divisions, four square roots, a double division) and
-// the particles of a warp touch 0 to 6 others, so lane by lane it ran at a
-// third of the lanes.  Instead a turn takes up to kDeal kept candidates of
-// every lane, whose loads are in flight together, and writes the touching ones
-// into a list in shared memory; the warp evaluates the list 32 at a time, and
-// each lane adds up its own results in its own order.  With the kept candidates
-// (kSkin), a call of 20 steps: 1,000,003 dense disks 54.1 M warp instructions a
-// step at 11 active lanes -> 30 M at 19; 4,194,304 disks 3,911 -> 3,327 us,
-// 250,007 cohesive disks 1,339 -> 1,019 us, 50 steps of 65,536 disks
-// 1,024 -> 885 us.  What bounds the step now is the latency of its four or five
-// rounds of dependent loads (42 % of issue slots used at 4,194,304 disks).
-constexpr int kDeal = 4;
-template <bool ATTRACT>
-struct Deal {
-    uint32_t j[kDeal * 32];  // [candidate of the turn][lane]: the neighbour, then the force's x
-    float fy[kDeal * 32], moment[kDeal * 32];
-    double q[kDeal * 32];
-    float ax[ATTRACT ? kDeal * 32 : 1], ay[ATTRACT ? kDeal * 32 : 1];
-    double aq[ATTRACT ? kDeal * 32 : 1];
-    uint8_t code[kDeal * 32];  // the list: index into the arrays above
-};
 
 // First slot of each of the three row intervals around the cell of `key`, for
 // the rows with candidates in `cand`.
@@ -384,8 +356,8 @@ __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B
                                              float w, float r, uint32_t mat, Pull& o) {
     constexpr unsigned kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t cell = 15u;  // cell of the subtotal
-    float2 sub = make_float2(0.0f, 0.0f);
+    Sums sum;
+    sum.o = o;  // of a lane that met its neighbours without kept candidates
     while (__any_sync(kAll, rem != 0ull)) {
         uint32_t at[kDeal], row[kDeal];
         float2 qp[kDeal];
@@ -427,63 +399,10 @@ __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B
             total += (uint32_t)__popc(hits);
         }
         if (total == 0u) continue;
-        __syncwarp();
-        for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
-            const uint32_t e = e0 + lane;
-            const uint32_t code = e < total ? S.code[e] : lane;
-            const int own = (int)(code & 31u);
-            const float2 pA = make_float2(__shfl_sync(kAll, p.x, own), __shfl_sync(kAll, p.y, own));
-            const float2 vA = make_float2(__shfl_sync(kAll, v.x, own), __shfl_sync(kAll, v.y, own));
-            const float wA = __shfl_sync(kAll, w, own), rA = __shfl_sync(kAll, r, own);
-            const uint32_t mA = TYPED ? __shfl_sync(kAll, mat, own) : 0u;
-            if (e < total) {
-                const uint32_t j = S.j[code];
-                const uint32_t mB = TYPED ? __ldg(B.stat.type + j) : 0u;
-                const float4 pc = TYPED ? P.pair[mA * P.nmat + mB] : P.pair[0];
-                const float2 pB = __ldg(in.pos + j);
-                const float rB = __ldg(B.stat.radius + j);
-                float2 f;
-                float m;
-                double q;
-                pair_terms(pA, pB, vA, __ldg(in.vel + j), wA, __ldg(in.omega + j), rA, rB, pc,
-                           P.dt, f, m, q);
-                S.j[code] = __float_as_uint(f.x);
-                S.fy[code] = f.y;
-                S.moment[code] = m;
-                S.q[code] = q;
-                if (ATTRACT) {
-                    const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB], q);
-                    S.ax[code] = g.x;
-                    S.ay[code] = g.y;
-                    S.aq[code] = q;
-                }
-            }
-        }
-        __syncwarp();
-        while (mine) {
-            const uint32_t k = (uint32_t)__ffs(mine) - 1u, x = k * 32u + lane;
-            mine &= mine - 1u;
-            const uint32_t c = (cells >> (4u * k)) & 15u;
-            if (c != cell) {
-                o.f.x += sub.x;
-                o.f.y += sub.y;
-                sub = make_float2(0.0f, 0.0f);
-                cell = c;
-            }
-            sub.x += __uint_as_float(S.j[x]);
-            sub.y += S.fy[x];
-            o.moment += S.moment[x];
-            o.pr = (float)((double)o.pr + S.q[x]);
-            if (ATTRACT) {
-                sub.x += S.ax[x];
-                sub.y += S.ay[x];
-                o.pr = (float)((double)o.pr + S.aq[x]);
-            }
-        }
-        __syncwarp();  // the results are read
+        deal_law<TYPED, ATTRACT>(P, S, total, mine, cells, p, v, w, r, mat, in.pos, in.vel,
+                                 in.omega, B.stat.radius, B.stat.type, nullptr, sum);
     }
-    o.f.x += sub.x;
-    o.f.y += sub.y;
+    o = sum.close();
 }
 
 template <bool TYPED, bool ATTRACT, bool CULL, int THREADS, int MINB>

@@ -73,6 +73,157 @@ __device__ __forceinline__ float2 f32x2_fma(float2 a, float2 b, float2 c) {
     return d;
 }
 
+// A bit for each of the 8 candidates at pq (radii pr) that may touch a particle
+// at p of radius r (ATTRACT: that is within attraction reach).  Two candidates
+// share each packed f32x2 operation.  d2 is the law's own
+// rn(rn(dx^2) + rn(dy^2)); the bound cd^2 (1 + 2e-6) is a fused multiply-add,
+// within 2e-7 relative of the exact value, so a rejected candidate still has
+// sqrtf(d2) >= rA + rB in the law's arithmetic (the law itself is unchanged).
+template <bool ATTRACT>
+__device__ __forceinline__ uint32_t filter8(const float2* __restrict__ pq,
+                                            const float* __restrict__ pr, float2 p, float r) {
+    float2 q[8];
+    float rq[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        q[k] = __ldg(pq + k);
+        rq[k] = __ldg(pr + k);
+    }
+    uint32_t m8 = 0u;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const float2 da = f32x2_sub(q[k], p), db = f32x2_sub(q[k + 1], p);
+        const float2 sa = f32x2_mul(da, da), sb = f32x2_mul(db, db);
+        const float d2a = sa.x + sa.y, d2b = sb.x + sb.y;
+        float2 bound;
+        if (ATTRACT) {
+            bound = make_float2(attract_reach2(r, rq[k]), attract_reach2(r, rq[k + 1]));
+        } else {
+            const float2 cd = f32x2_add(make_float2(r, r), make_float2(rq[k], rq[k + 1]));
+            const float2 c2 = f32x2_mul(cd, cd);
+            bound = f32x2_fma(c2, make_float2(2e-6f, 2e-6f), c2);
+        }
+        if (d2a <= bound.x) m8 |= 1u << k;
+        if (d2b <= bound.y) m8 |= 2u << k;
+    }
+    return m8;
+}
+
+// Force, moment and pressure of one particle.
+struct Pull {
+    float2 f;
+    float moment, pr;
+};
+
+// The running sums of one particle: a subtotal per cell, added to the force
+// when the next cell begins (an empty cell adds +0).
+struct Sums {
+    Pull o{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
+    float2 sub = make_float2(0.0f, 0.0f);
+    uint32_t cell = 15u;
+    __device__ __forceinline__ void begin(uint32_t c) {
+        if (c == cell) return;
+        o.f.x += sub.x;
+        o.f.y += sub.y;
+        sub = make_float2(0.0f, 0.0f);
+        cell = c;
+    }
+    __device__ __forceinline__ Pull close() {
+        begin(15u);
+        return o;
+    }
+};
+
+// A warp's contacts, dealt to its lanes.  The contact law is some two hundred
+// instructions (five IEEE divisions, four square roots, a double division) and
+// the particles of a warp touch 0 to 6 others, so lane by lane it ran at a
+// third of the lanes.  Instead a turn takes up to kDeal kept candidates of
+// every lane, whose loads are in flight together, and writes the touching ones
+// into a list in shared memory; the warp evaluates the list 32 at a time, and
+// each lane adds up its own results in its own order.  In the band step, with
+// its kept candidates, a call of 20 steps: 1,000,003 dense disks 54.1 M warp instructions a
+// step at 11 active lanes -> 30 M at 19; 4,194,304 disks 3,911 -> 3,327 us,
+// 250,007 cohesive disks 1,339 -> 1,019 us, 50 steps of 65,536 disks
+// 1,024 -> 885 us.  What bounds the step now is the latency of its four or five
+// rounds of dependent loads (42 % of issue slots used at 4,194,304 disks).
+constexpr int kDeal = 4;
+template <bool ATTRACT>
+struct Deal {
+    uint32_t j[kDeal * 32];  // [candidate of the turn][lane]: the neighbour, then the force's x
+    float fy[kDeal * 32], moment[kDeal * 32];
+    double q[kDeal * 32];
+    float ax[ATTRACT ? kDeal * 32 : 1], ay[ATTRACT ? kDeal * 32 : 1];
+    double aq[ATTRACT ? kDeal * 32 : 1];
+    uint8_t code[kDeal * 32];  // the list: index into the arrays above
+};
+
+// The turn's `total` listed contacts through the law, then each lane's own (bit
+// k of `mine`: its candidate k; four bits of `cells` each: the cell) into its
+// sums.  The neighbours' velocity, spin and type are read through `src` where
+// the arrays are in the previous order.  Every lane calls it.
+template <bool TYPED, bool ATTRACT>
+__device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, uint32_t total,
+                                         uint32_t mine, uint32_t cells, float2 p, float2 v,
+                                         float w, float r, uint32_t mat,
+                                         const float2* __restrict__ pos,
+                                         const float2* __restrict__ vel,
+                                         const float* __restrict__ omega,
+                                         const float* __restrict__ radius,
+                                         const uint32_t* __restrict__ type,
+                                         const uint32_t* __restrict__ src, Sums& sum) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
+        const uint32_t e = e0 + lane;
+        const uint32_t code = e < total ? S.code[e] : lane;
+        const int own = (int)(code & 31u);
+        const float2 pA = make_float2(__shfl_sync(kAll, p.x, own), __shfl_sync(kAll, p.y, own));
+        const float2 vA = make_float2(__shfl_sync(kAll, v.x, own), __shfl_sync(kAll, v.y, own));
+        const float wA = __shfl_sync(kAll, w, own), rA = __shfl_sync(kAll, r, own);
+        const uint32_t mA = TYPED ? __shfl_sync(kAll, mat, own) : 0u;
+        if (e < total) {
+            const uint32_t j = S.j[code];
+            const uint32_t sj = src ? __ldg(src + j) : j;
+            const uint32_t mB = TYPED ? __ldg(type + sj) : 0u;
+            const float4 pc = TYPED ? P.pair[mA * P.nmat + mB] : P.pair[0];
+            const float2 pB = __ldg(pos + j);
+            const float rB = __ldg(radius + j);
+            float2 f;
+            float m;
+            double q;
+            pair_terms(pA, pB, vA, __ldg(vel + sj), wA, __ldg(omega + sj), rA, rB, pc, P.dt, f, m,
+                       q);
+            S.j[code] = __float_as_uint(f.x);
+            S.fy[code] = f.y;
+            S.moment[code] = m;
+            S.q[code] = q;
+            if (ATTRACT) {
+                const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB], q);
+                S.ax[code] = g.x;
+                S.ay[code] = g.y;
+                S.aq[code] = q;
+            }
+        }
+    }
+    __syncwarp();
+    while (mine) {
+        const uint32_t k = (uint32_t)__ffs(mine) - 1u, x = k * 32u + lane;
+        mine &= mine - 1u;
+        sum.begin((cells >> (4u * k)) & 15u);
+        sum.sub.x += __uint_as_float(S.j[x]);
+        sum.sub.y += S.fy[x];
+        sum.o.moment += S.moment[x];
+        sum.o.pr = (float)((double)sum.o.pr + S.q[x]);
+        if (ATTRACT) {
+            sum.sub.x += S.ax[x];
+            sum.sub.y += S.ay[x];
+            sum.o.pr = (float)((double)sum.o.pr + S.aq[x]);
+        }
+    }
+    __syncwarp();  // the results are read
+}
+
 // Contact test and force of one candidate j (the reference's collideSpheres
 // and, with ATTRACT, attractSpheres) added to the cell subtotal fc.
 template <bool TYPED, bool ATTRACT>
@@ -281,45 +432,15 @@ __device__ __forceinline__ bool collide_rows(const KParams& P, uint32_t i, int2 
         // filter: a bit per candidate that may touch, then the contact law on
         // the set bits in index order.  Groups of 8 candidates are read whole
         // (the arrays are padded by kFilterPad), the bits past the interval
-        // and the particle's own bit are cleared per chunk.  Two candidates
-        // share each packed f32x2 operation.  d2 is the law's own
-        // rn(rn(dx^2) + rn(dy^2)); the bound cd^2 (1 + 2e-6) is a fused
-        // multiply-add, within 2e-7 relative of the exact value, so a
-        // rejected candidate still has sqrtf(d2) >= rA + rB in the law's
-        // arithmetic (the law itself is unchanged).
+        // and the particle's own bit are cleared per chunk.
 #pragma unroll 1
         for (uint32_t base = a; base < b; base += 32u) {
             const uint32_t cnt = min(b - base, 32u);
             uint32_t mask = 0u;
 #pragma unroll 1
             for (uint32_t k0 = 0; k0 < cnt; k0 += 8) {
-                float2 q[8];
-                float rq[8];
-                const float2* __restrict__ pq = pos + (base + k0);
-                const float* __restrict__ pr8 = radius + (base + k0);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    q[k] = __ldg(pq + k);
-                    rq[k] = __ldg(pr8 + k);
-                }
-                uint32_t m8 = 0u;
-#pragma unroll
-                for (int k = 0; k < 8; k += 2) {
-                    const float2 da = f32x2_sub(q[k], p), db = f32x2_sub(q[k + 1], p);
-                    const float2 sa = f32x2_mul(da, da), sb = f32x2_mul(db, db);
-                    const float d2a = sa.x + sa.y, d2b = sb.x + sb.y;
-                    float2 bound;
-                    if (ATTRACT) {
-                        bound = make_float2(attract_reach2(r, rq[k]), attract_reach2(r, rq[k + 1]));
-                    } else {
-                        const float2 cd =
-                            f32x2_add(make_float2(r, r), make_float2(rq[k], rq[k + 1]));
-                        const float2 c2 = f32x2_mul(cd, cd);
-                        bound = f32x2_fma(c2, make_float2(2e-6f, 2e-6f), c2);
-                    }
-                    if (d2a <= bound.x) m8 |= 1u << k;
-                    if (d2b <= bound.y) m8 |= 2u << k;
-                }
+                const uint32_t m8 =
+                    filter8<ATTRACT>(pos + (base + k0), radius + (base + k0), p, r);
                 mask |= m8 << k0;
             }
             if (cnt < 32u) mask &= (1u << cnt) - 1u;

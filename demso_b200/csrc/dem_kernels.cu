@@ -70,32 +70,123 @@ reorder_kernel(uint32_t* __restrict__ cellStart, uint32_t* __restrict__ cellEnd,
     if (TYPED) sS.type[i] = oS.type[src];
 }
 
+// collideD on the caller's sorted arrays and cell ranges (any ranges: nothing
+// is assumed of positions and cells beyond what the reference reads).  Bound
+// by issue: about 36 candidates and 3 contacts a particle in a dense packing.
+// The three ranges of a cell row load together; where they follow one another,
+// as sorted particles' do, they are one interval, walked eight candidates at a
+// time, and the touching ones are dealt over the warp (deal_law).  1,048,576
+// disks at area fraction 0.78: 143 -> about 90 us (one step through the five
+// stages 193 -> 163 us).
 template <bool TYPED, bool ATTRACT>
-__global__ void __launch_bounds__(kCollideThreads)
-collide_kernel(KParams P, const float2* __restrict__ pos, const float2* __restrict__ vel,
-               const float* __restrict__ omega, const float* __restrict__ radius,
-               const float* __restrict__ mass, const uint32_t* __restrict__ type,
-               const uint32_t* __restrict__ cellStart, const uint32_t* __restrict__ cellEnd,
-               float2* __restrict__ acc, float* __restrict__ alpha, float* __restrict__ pressure,
-               uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__global__ void __launch_bounds__(kCollideThreads, 8)
+collide_kernel(const __grid_constant__ KParams P, const float2* __restrict__ pos,
+               const float2* __restrict__ vel, const float* __restrict__ omega,
+               const float* __restrict__ radius, const float* __restrict__ mass,
+               const uint32_t* __restrict__ type, const uint32_t* __restrict__ cellStart,
+               const uint32_t* __restrict__ cellEnd, float2* __restrict__ acc,
+               float* __restrict__ alpha, float* __restrict__ pressure, uint32_t n) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ Deal<ATTRACT> deal[kCollideThreads / 32];
+    Deal<ATTRACT>& S = deal[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool mine = slot < n;
+    const uint32_t i = min(slot, n - 1u);  // lanes past the end stand by
     const float2 p = pos[i];
     const float2 v = vel[i];
     const float w = omega[i];
     const float r = radius[i];
     const uint32_t mat = TYPED ? type[i] : 0u;
-    float2 f;
-    float moment, pr;
     int2 g = grid_pos(P, p);
-    g.y -= P.rowOff;  // collide_one takes the cell in the context's rows
-    collide_one<TYPED, ATTRACT, false>(P, i, g, p, v, w, r, mat, pos, vel, omega,
-                                       radius, type, nullptr, SplitCells{cellStart, cellEnd}, f,
-                                       moment, pr);
+    g.y -= P.rowOff;
+    Sums sum;
+    uint32_t held = 0u, cells = 0u, total = 0u;  // candidates of the turn
+    auto flush = [&]() {
+        deal_law<TYPED, ATTRACT>(P, S, total, (1u << held) - 1u, cells, p, v, w, r, mat, pos, vel,
+                                 omega, radius, type, nullptr, sum);
+        held = cells = total = 0u;
+    };
+#pragma unroll 1
+    for (int dy = -1; dy <= 1; ++dy) {
+        uint32_t s[3], e[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t h = cell_index(P, g.x + k - 1, g.y + dy);
+            s[k] = __ldg(cellStart + h);
+            e[k] = __ldg(cellEnd + h);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            // an empty cell's end is unspecified; an empty range holds nothing
+            if (!mine || s[k] == kEmptyCell || e[k] <= s[k]) s[k] = e[k] = 0u;
+        }
+        // one interval when each range that holds something starts where the
+        // last one ended
+        const bool h0 = e[0] != 0u, h1 = e[1] != 0u, h2 = e[2] != 0u;
+        const bool joined = (!h0 || !h1 || s[1] == e[0]) &&
+                            (!h2 || !(h0 || h1) || s[2] == (h1 ? e[1] : e[0]));
+        const uint32_t last = h2 ? e[2] : (h1 ? e[1] : e[0]);
+        const uint32_t b2 = h2 ? s[2] : last, b1 = h1 ? s[1] : b2;
+#pragma unroll 1
+        for (int pass = 0; pass < 3; ++pass) {
+            uint32_t a = 0u, b = 0u;
+            if (joined) {
+                if (pass == 0) {
+                    a = h0 ? s[0] : b1;
+                    b = last;
+                }
+            } else {
+                a = pass == 0 ? s[0] : (pass == 1 ? s[1] : s[2]);
+                b = pass == 0 ? e[0] : (pass == 1 ? e[1] : e[2]);
+            }
+            if (!__any_sync(kAll, a < b)) continue;
+#pragma unroll 1
+            for (; __any_sync(kAll, a < b); a += 8u) {
+                uint32_t hits = 0u;
+                if (a < b) {
+                    if (n - a >= 8u) {
+                        hits = filter8<ATTRACT>(pos + a, radius + a, p, r);
+                    } else {  // the arrays end within the group
+                        for (uint32_t k = 0; k < n - a; ++k) {
+                            const float2 q = __ldg(pos + a + k);
+                            const float rq = __ldg(radius + a + k);
+                            const float dx = q.x - p.x, dq = q.y - p.y;
+                            const float d2 = dx * dx + dq * dq, cd = r + rq;
+                            if (d2 <= (ATTRACT ? attract_reach2(r, rq) : cd * cd * 1.000002f))
+                                hits |= 1u << k;
+                        }
+                    }
+                    // groups are read whole
+                    if (b - a < 8u) hits &= (1u << (b - a)) - 1u;
+                    if (i - a < 8u) hits &= ~(1u << (i - a));
+                }
+                while (__any_sync(kAll, hits != 0u)) {
+                    if (__any_sync(kAll, held == (uint32_t)kDeal)) flush();
+                    const unsigned take = __ballot_sync(kAll, hits != 0u);
+                    if (hits) {
+                        const uint32_t j = a + (uint32_t)__ffs(hits) - 1u;
+                        hits &= hits - 1u;
+                        const uint32_t x = joined ? (j >= b1 ? 1u : 0u) + (j >= b2 ? 1u : 0u)
+                                                  : (uint32_t)pass;
+                        S.j[held * 32u + lane] = j;
+                        S.code[total + __popc(take & ((1u << lane) - 1u))] =
+                            (uint8_t)(held * 32u + lane);
+                        cells |= (3u * (uint32_t)(dy + 1) + x) << (4u * held);
+                        ++held;
+                    }
+                    total += (uint32_t)__popc(take);
+                }
+            }
+        }
+    }
+    if (__any_sync(kAll, held != 0u)) flush();
+    if (!mine) return;
+    const Pull o = sum.close();
     const float m = mass[i];
-    acc[i] = make_float2(f.x / m, f.y / m);
-    alpha[i] = moment / inertia_of(m, r);
-    if (pressure) pressure[i] = pr;
+    acc[i] = make_float2(o.f.x / m, o.f.y / m);
+    alpha[i] = o.moment / inertia_of(m, r);
+    if (pressure) pressure[i] = o.pr;
 }
 
 template <bool TYPED>
