@@ -41,40 +41,6 @@ constexpr int kCoef = DEM_ADJ_NUM_COEF;  // kn, kt, cn, mu (pairs), cn, mu, kt (
 inline unsigned blocks_for(uint32_t n, int t) { return (n + (uint32_t)t - 1u) / (uint32_t)t; }
 inline size_t al256(size_t b) { return (b + 255u) & ~(size_t)255u; }
 
-// One recorded step: the sorted state the step kernel read, its cell ranges
-// and the accelerations it computed.
-struct StepRec {
-    float2* pos;
-    float2* vel;
-    float* omega;
-    float* radius;
-    float* mass;
-    uint32_t* id;
-    float2* acc;
-    float* alpha;
-    uint2* cells;
-};
-
-template <typename T>
-__device__ __forceinline__ T* bump(T* p, size_t off) {
-    return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + off);
-}
-// The record `at` names (see RecSlot), from the one at the window's base.
-__device__ __forceinline__ StepRec rec_at(StepRec r, RecSlot at) {
-    if (!at.slot) return r;
-    const size_t off = at.stride * (size_t)(*at.slot + at.add);
-    r.pos = bump(r.pos, off);
-    r.vel = bump(r.vel, off);
-    r.omega = bump(r.omega, off);
-    r.radius = bump(r.radius, off);
-    r.mass = bump(r.mass, off);
-    r.id = bump(r.id, off);
-    r.acc = bump(r.acc, off);
-    r.alpha = bump(r.alpha, off);
-    r.cells = bump(r.cells, off);
-    return r;
-}
-
 // Adds a thread's coefficient cotangents to the per-slot accumulators
 // acc[k * n + slot]: the values of a warp are reduced over runs of equal
 // `seg` (slots of one specimen are contiguous) in a fixed pattern, and the
@@ -89,6 +55,7 @@ __device__ __forceinline__ void warp_add_coef(const double (&v)[kCoef], uint32_t
 #pragma unroll
     for (int k = 0; k < kCoef; ++k) {
         double x = v[k];
+        if (!__any_sync(0xffffffffu, x != 0.0)) continue;  // zeros add up to zero
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double y = __shfl_down_sync(0xffffffffu, x, o);
@@ -108,6 +75,7 @@ adj_integrate_kernel(KParams P0, const KParams* __restrict__ table,
                      float2* __restrict__ lv, float* __restrict__ lw, float2* __restrict__ lamF,
                      float* __restrict__ lamM, double* __restrict__ acc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at.slot && (int32_t)(*at.slot + at.add) < 0) return;  // past the first step
     double coef[kCoef] = {0, 0, 0, 0, 0, 0, 0};
     const uint32_t seg = i < n ? (table ? spec[i] : 0u) : 0xffffffffu;
     if (i < n) {
@@ -186,6 +154,7 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
                  float2* __restrict__ lamX, float2* __restrict__ lamV, float* __restrict__ lamW,
                  double* __restrict__ acc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at.slot && (int32_t)(*at.slot + at.add) < 0) return;  // past the first step
     double coef[kCoef] = {0, 0, 0, 0, 0, 0, 0};
     const uint32_t seg = i < n ? (table ? spec[i] : 0u) : 0xffffffffu;
     if (i < n) {
@@ -196,10 +165,21 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
         const float2 lFi = lamF[i];
         const float lMi = lamM[i];
         const float4 pc = P.pair[0];
-        const int2 g = grid_pos(P, p);
+        // the neighbour columns and rows within reach, as the forward visits them
+        const int2 g = grid_pos_fast(P, p);
+        int y0 = -1, y1 = 1, x0 = -1, x1 = 1;
+        if (P.cull && p.x > P.cullMargin && p.x < P.Lx - P.cullMargin && p.y > P.cullMargin &&
+            p.y < P.Ly - P.cullMargin) {
+            const float reach = (r + P.rmax) * 1.0001f + P.cullMargin;
+            const float X0 = (float)g.x * P.cellW, Y0 = (float)g.y * P.cellH;
+            if (p.x - X0 > reach) x0 = 0;
+            if (X0 + P.cellW - p.x > reach) x1 = 0;
+            if (p.y - Y0 > reach) y0 = 0;
+            if (Y0 + P.cellH - p.y > reach) y1 = 0;
+        }
         float gx = 0, gy = 0, gvx = 0, gvy = 0, gw = 0;
-        for (int dy = -1; dy <= 1; ++dy) {
-            for (int dx = -1; dx <= 1; ++dx) {
+        for (int dy = y0; dy <= y1; ++dy) {
+            for (int dx = x0; dx <= x1; ++dx) {
                 const uint2 se = rec.cells[grid_hash(P, g.x + dx, g.y + dy)];
                 const uint32_t end = se.x < se.y ? se.y : 0u;
                 for (uint32_t j = se.x < se.y ? se.x : 0u; j < end; ++j) {
@@ -219,10 +199,10 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
                         using D = Dual<float, 5>;
                         D fx, fy, dm;
                         unsigned fl;
-                        pair_law<D>(seed<float, 5>(p.x, 0), seed<float, 5>(p.y, 1), D(q.x), D(q.y),
-                                    seed<float, 5>(v.x, 2), seed<float, 5>(v.y, 3), D(vj.x),
-                                    D(vj.y), seed<float, 5>(w, 4), D(wj), D(r), D(rj), D(pc.x),
-                                    D(pc.y), D(pc.z), D(pc.w), D(P.dt), fx, fy, dm, fl);
+                        pair_law(seed<float, 5>(p.x, 0), seed<float, 5>(p.y, 1), q.x, q.y,
+                                 seed<float, 5>(v.x, 2), seed<float, 5>(v.y, 3), vj.x, vj.y,
+                                 seed<float, 5>(w, 4), wj, r, rj, pc.x, pc.y, pc.z, pc.w, P.dt,
+                                 fx, fy, dm, fl);
                         gx += fx.d[0] * wfx + fy.d[0] * wfy + dm.d[0] * wd;
                         gy += fx.d[1] * wfx + fy.d[1] * wfy + dm.d[1] * wd;
                         gvx += fx.d[2] * wfx + fy.d[2] * wfy + dm.d[2] * wd;
@@ -233,10 +213,10 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
                         using D = Dual<float, 4>;
                         D fx, fy, dm;
                         unsigned fl;
-                        pair_law<D>(D(p.x), D(p.y), D(q.x), D(q.y), D(v.x), D(v.y), D(vj.x),
-                                    D(vj.y), D(w), D(wj), D(r), D(rj), seed<float, 4>(pc.x, 0),
-                                    seed<float, 4>(pc.y, 1), seed<float, 4>(pc.z, 2),
-                                    seed<float, 4>(pc.w, 3), D(P.dt), fx, fy, dm, fl);
+                        pair_law(p.x, p.y, q.x, q.y, v.x, v.y, vj.x, vj.y, w, wj, r, rj,
+                                 seed<float, 4>(pc.x, 0), seed<float, 4>(pc.y, 1),
+                                 seed<float, 4>(pc.z, 2), seed<float, 4>(pc.w, 3), P.dt, fx, fy,
+                                 dm, fl);
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             coef[k] += (double)fx.d[k] * wfx + (double)fy.d[k] * wfy +
@@ -254,7 +234,7 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
     warp_add_coef(coef, seg, i, n, acc);
 }
 
-// Per specimen s: the sum of acc[k * n + slot] over its slots
+// Per specimen s and coefficient k: the sum of acc[k * n + slot] over its slots
 // [first[s], first[s + 1]), in a fixed order (strided per thread, then a
 // fixed-shape block reduction).
 constexpr int kSumThreads = 256;
@@ -265,7 +245,8 @@ adj_coef_sum_kernel(const double* __restrict__ acc, uint32_t n, const uint32_t* 
     const uint32_t s = blockIdx.x;
     const uint32_t a = first ? first[s] : 0u, b = first ? first[s + 1] : n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < kCoef; ++k) {
+    {
+        const int k = (int)blockIdx.y;
         double x = 0.0;
         for (uint32_t j = a + threadIdx.x; j < b; j += kSumThreads) x += acc[(size_t)k * n + j];
 #pragma unroll
@@ -277,7 +258,6 @@ adj_coef_sum_kernel(const double* __restrict__ acc, uint32_t n, const uint32_t* 
             for (int w = 0; w < kSumThreads / 32; ++w) t += red[w];
             out[(size_t)s * kCoef + k] = t;
         }
-        __syncthreads();
     }
 }
 
@@ -353,7 +333,7 @@ cudaError_t adj_backward_step(const KParams& P, const KParams* table, const uint
 
 cudaError_t adj_sum_coef(const double* acc, uint32_t n, const uint32_t* first, uint32_t numSpecimens,
                          double* out, cudaStream_t st) {
-    adj_coef_sum_kernel<<<numSpecimens, kSumThreads, 0, st>>>(acc, n, first, out);
+    adj_coef_sum_kernel<<<dim3(numSpecimens, kCoef), kSumThreads, 0, st>>>(acc, n, first, out);
     return cudaGetLastError();
 }
 

@@ -391,6 +391,7 @@ struct DemContext {
     float2* ownPos = nullptr;  // the block's positions: not an adopted set
     bool bandValid = false, bandCells = false, bandInit = false;
     cudaGraphExec_t bandLoop[2] = {}, bandFollow[2] = {}, bandSort[2] = {};
+    cudaGraphExec_t bandRec[2] = {};  // the loop recording every step for the adjoint
     // followed-particle staging (device), see dem_get_followed
     float* followRows = nullptr;
     // dem_step_followed: the ids (device copy), the ring of per-step rows,
@@ -491,8 +492,10 @@ void drop_tune_graphs(DemContext* c) {
 
 void drop_adj_graphs(DemContext* c) {
     for (int p = 0; p < 2; ++p) {
-        if (c->adjRecLoop[p]) cudaGraphExecDestroy(c->adjRecLoop[p]);
-        c->adjRecLoop[p] = nullptr;
+        for (cudaGraphExec_t* g : {&c->adjRecLoop[p], &c->bandRec[p]}) {
+            if (*g) cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
     }
     if (c->adjRevLoop) cudaGraphExecDestroy(c->adjRevLoop);
     c->adjRevLoop = nullptr;
@@ -1435,14 +1438,22 @@ cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
 // the outer loop makes at least one step.
 constexpr int kBandPairs = 2;
 
-cudaError_t enqueue_band_pairs(DemContext* c, bool follow, cudaStream_t st) {
+// What follows every step of a call: nothing, its followed rows, its record for
+// the adjoint.
+enum class BandAfter { kNothing, kFollowed, kRecord };
+
+cudaError_t enqueue_band_pairs(DemContext* c, BandAfter after, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < 2 * kBandPairs && e == cudaSuccess; ++k) {
-        e = launch_band_fix(c->band, k & 1, st);
-        if (e == cudaSuccess) e = launch_band_step(c->P, c->band, k & 1, follow, c->variant, st);
-        if (e == cudaSuccess && follow)
-            e = launch_band_followed(c->band, k & 1, c->followIds, c->loopCtl + kLoopFolCount,
+        const int q = k & 1;
+        e = launch_band_fix(c->band, q, st);
+        if (e == cudaSuccess)
+            e = launch_band_step(c->P, c->band, q, after != BandAfter::kNothing, c->variant, st);
+        if (e == cudaSuccess && after == BandAfter::kFollowed)
+            e = launch_band_followed(c->band, q, c->followIds, c->loopCtl + kLoopFolCount,
                                      c->followRing, st);
+        if (e == cudaSuccess && after == BandAfter::kRecord)
+            e = launch_band_record(c->band, q, c->adjRec, c->adjRevStepBytes, st);
     }
     return e;
 }
@@ -1456,7 +1467,7 @@ cudaError_t conditional_handle(cudaStream_t st, cudaGraphConditionalHandle* h) {
     return e == cudaSuccess ? cudaGraphConditionalHandleCreate(h, g, 0, 0) : e;
 }
 
-cudaError_t enqueue_band_loop(DemContext* c, bool follow, cudaStream_t st) {
+cudaError_t enqueue_band_loop(DemContext* c, BandAfter after, cudaStream_t st) {
     cudaGraphConditionalHandle outer;
     cudaError_t e = conditional_handle(st, &outer);
     if (e == cudaSuccess) e = launch_band_next(c->band, outer, true, st);
@@ -1471,7 +1482,7 @@ cudaError_t enqueue_band_loop(DemContext* c, bool follow, cudaStream_t st) {
         if (eb == cudaSuccess)
             eb = add_conditional(ob, inner, cudaGraphCondTypeWhile, c->forkStream,
                                  [&](cudaStream_t ib) {
-                                     cudaError_t ei = enqueue_band_pairs(c, follow, ib);
+                                     cudaError_t ei = enqueue_band_pairs(c, after, ib);
                                      return ei == cudaSuccess
                                                 ? launch_band_next(c->band, inner, false, ib)
                                                 : ei;
@@ -1586,21 +1597,24 @@ int band_step_alone(DemContext* c, cudaStream_t st) {
     return DEM_OK;
 }
 
-// `nsteps` steps in bands; with `follow`, each step's followed rows at row
-// block rowBlock + step of the ring.  The state is packed at the end.
-int band_steps(DemContext* c, uint32_t nsteps, bool follow, uint32_t rowBlock, cudaStream_t st) {
+// `nsteps` steps in bands, with the row or record blocks of what follows each
+// from `block` on.  The state is packed at the end.
+int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, cudaStream_t st) {
     int rc = DEM_OK;
     uint32_t done = 0;
-    while (done < nsteps && (c->tuned < 0 || c->profiling || (c->flags & DEM_CTX_DIRECT))) {
+    while (after == BandAfter::kNothing && done < nsteps &&
+           (c->tuned < 0 || c->profiling || (c->flags & DEM_CTX_DIRECT))) {
         rc = band_step_alone(c, st);
         if (rc) return rc;
         ++done;
     }
     if (done < nsteps) {
-        rc = band_begin(c, nsteps - done, rowBlock + done, st);
+        rc = band_begin(c, nsteps - done, block + done, st);
         if (rc) return rc;
-        cudaGraphExec_t* g = follow ? &c->bandFollow[c->cur] : &c->bandLoop[c->cur];
-        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_loop(c, follow, s); }, g);
+        cudaGraphExec_t* g = after == BandAfter::kFollowed ? &c->bandFollow[c->cur]
+                             : after == BandAfter::kRecord ? &c->bandRec[c->cur]
+                                                           : &c->bandLoop[c->cur];
+        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_loop(c, after, s); }, g);
         if (rc) return rc;
         DEM_TRY_CUDA(cudaGraphLaunch(*g, st), "graph launch");
     }
@@ -1790,7 +1804,7 @@ namespace {
 // step loop for pairs of steps (also the steps of dem_step_followed, whose
 // per-step rows are gathered from this path's buffers).
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (steps_in_bands(c)) return band_steps(c, nsteps, false, 0, st);
+    if (steps_in_bands(c)) return band_steps(c, nsteps, BandAfter::kNothing, 0, st);
     c->bandValid = false;
     if (!c->keysValid) {
         if (c->nspec)
@@ -2065,7 +2079,7 @@ extern "C" int dem_step_followed(DemContext* c, uint32_t nsteps, const uint32_t*
         const uint32_t m = std::min(chunk, nsteps - s);
         const bool alone = (c->flags & DEM_CTX_DIRECT) || c->profiling || c->tuned < 0;
         if (steps_in_bands(c) && !alone) {
-            int rc = band_steps(c, m, true, 0, st);
+            int rc = band_steps(c, m, BandAfter::kFollowed, 0, st);
             if (rc) return rc;
         } else for (uint32_t j = 0; j < m;) {
             // pairs of steps with their rows in the device-side loop, as in
@@ -2402,6 +2416,58 @@ extern "C" int dem_adj_forward(DemContext* c, uint32_t nsteps, uint32_t every, v
     return DEM_OK;
 }
 
+namespace {
+// Steps of one pass of the reverse loop; those past slot 0 do nothing.
+constexpr uint32_t kRevSteps = 4;
+
+// A window's `k` steps re-run from the restored checkpoint on the packed path,
+// each recorded: the first sorts from scratch (host-launched, record slot 0),
+// the rest run in pairs inside the recompute loop, recorded at the loop's
+// slot, and an odd last step is host-launched.
+int rerun_recorded(DemContext* c, uint32_t k, size_t stepBytes, char* rec, cudaStream_t st) {
+    const uint32_t n = c->n;
+    if (!c->keysValid) {
+        DEM_TRY_CUDA(c->nspec ? launch_calc_hash_batched(c->dTable, c->spec, c->dyn[0].pos, c->keys,
+                                                         n, st)
+                              : launch_calc_hash(c->P, c->dyn[0].pos, c->keys, nullptr, n, st),
+                     "hash");
+        c->keysValid = true;
+        c->haveOrder = false;
+    }
+    int rc = DEM_OK;
+    for (int pp = 0; pp < 2 && rc == DEM_OK; ++pp) {
+        for (int kk = 0; kk < 2 && rc == DEM_OK; ++kk)
+            if (!c->sortGraph[kk][pp]) rc = build_graph(c, kk, pp);
+        if (rc == DEM_OK && !c->stepGraph[pp]) rc = build_graph(c, 2, pp);
+    }
+    if (rc == DEM_OK) rc = step_recorded(c, st, rec);
+    if (rc) return rc;
+    const uint32_t pairs = (k - 1) / 2;
+    DEM_TRY_CUDA(launch_set_words(c->loopCtl + kLoopRecReq, Words{{pairs, 0u, 1u}, 3u}, st),
+                 "recompute loop count");
+    if (pairs) {
+        const int p = c->cur;
+        if (!c->adjRecLoop[p]) {
+            rc = build_while_graph(
+                c, kLoopRecReq, kLoopRecSlot, 2,
+                [&](cudaStream_t bs) {
+                    return enqueue_step_pair(c, p, bs, [&](int j, cudaStream_t s2) {
+                        return adj_record_step(
+                            rec, RecSlot{c->loopCtl + kLoopRecSlot, (uint32_t)j, stepBytes}, n,
+                            c->numCells, step_in(c, p ^ j), step_in_static(c, p ^ j), c->src,
+                            c->cells[p ^ j ^ 1], c->acc, c->alpha, s2);
+                    });
+                },
+                &c->adjRecLoop[p]);
+            if (rc) return rc;
+        }
+        DEM_TRY_CUDA(cudaGraphLaunch(c->adjRecLoop[p], st), "graph launch");
+    }
+    if ((k - 1) & 1) return step_recorded(c, st, rec + stepBytes * (k - 1));
+    return DEM_OK;
+}
+}  // namespace
+
 extern "C" int dem_adj_backward(DemContext* c, float* lamPos, float* lamVel, float* lamOmega,
                                 double* grad, void* stream) {
     int rc = adj_check_context(c);
@@ -2463,68 +2529,37 @@ extern "C" int dem_adj_backward(DemContext* c, float* lamPos, float* lamVel, flo
     if (e == cudaSuccess && first)
         e = cudaMemcpyAsync(first, c->partOff.data(), 4ull * (ns + 1), cudaMemcpyHostToDevice, st);
     const size_t snap = snapshot_bytes(n);
-    cudaGraphExec_t* recLoop = c->adjRecLoop;
     cudaGraphExec_t& revLoop = c->adjRevLoop;
     for (int w = (int)c->adjWindows - 1; w >= 0 && rc == DEM_OK && e == cudaSuccess; --w) {
         rc = restore_checkpoint(c, carve_snapshot(static_cast<char*>(c->adjCheck) + snap * w, n),
                                 st);
         if (rc) break;
         const uint32_t k = std::min(c->adjEvery, c->adjSteps - (uint32_t)w * c->adjEvery);
-        if (!c->keysValid) {
-            e = c->nspec ? launch_calc_hash_batched(c->dTable, c->spec, c->dyn[0].pos, c->keys, n, st)
-                         : launch_calc_hash(c->P, c->dyn[0].pos, c->keys, nullptr, n, st);
-            c->keysValid = true;
-            c->haveOrder = false;
-        }
-        for (int pp = 0; pp < 2 && rc == DEM_OK; ++pp) {
-            for (int kk = 0; kk < 2 && rc == DEM_OK; ++kk)
-                if (!c->sortGraph[kk][pp]) rc = build_graph(c, kk, pp);
-            if (rc == DEM_OK && !c->stepGraph[pp]) rc = build_graph(c, 2, pp);
-        }
-        if (rc != DEM_OK || e != cudaSuccess) break;
-        // The window's first step sorts from scratch (host-launched, record
-        // slot 0); the rest run in pairs inside the recompute loop, each
-        // recorded at the loop's slot, and an odd last step is host-launched.
-        // The reversed steps then run in the reverse loop, slot k - 1 down
-        // to 0.  Both loops are graphs of this call (they hold its buffers).
-        rc = step_recorded(c, st, rec);
-        if (rc) break;
-        const uint32_t pairs = (k - 1) / 2;
-        e = launch_set_words(c->loopCtl + kLoopRecReq, Words{{pairs, 0u, 1u, k, 0u, k - 1u}, 6u},
-                             st);
-        if (e != cudaSuccess) break;
-        if (pairs) {
-            const int p = c->cur;
-            if (!recLoop[p]) {
-                rc = build_while_graph(
-                    c, kLoopRecReq, kLoopRecSlot, 2,
-                    [&](cudaStream_t bs) {
-                        return enqueue_step_pair(c, p, bs, [&](int k, cudaStream_t s2) {
-                            return adj_record_step(
-                                rec, RecSlot{c->loopCtl + kLoopRecSlot, (uint32_t)k, stepBytes},
-                                c->n, c->numCells, step_in(c, p ^ k), step_in_static(c, p ^ k),
-                                c->src, c->cells[p ^ k ^ 1], c->acc, c->alpha, s2);
-                        });
-                    },
-                    &recLoop[p]);
-                if (rc) break;
-            }
-            e = cudaGraphLaunch(recLoop[p], st);
-            if (e != cudaSuccess) break;
-        }
-        if ((k - 1) & 1) {
-            rc = step_recorded(c, st, rec + stepBytes * (k - 1));
+        const bool bands = steps_in_bands(c);
+        if (bands) {
+            rc = band_steps(c, k, BandAfter::kRecord, 0, st);
             if (rc) break;
         }
+        if (!bands) {
+            rc = rerun_recorded(c, k, stepBytes, rec, st);
+            if (rc) break;
+        }
+        // the reversed steps, slot k - 1 down to 0, in the reverse loop
+        e = launch_set_words(c->loopCtl + kLoopRevReq,
+                             Words{{(k + kRevSteps - 1u) / kRevSteps, 0u, k - 1u}, 3u}, st);
+        if (e != cudaSuccess) break;
         if (!revLoop) {
             rc = build_while_graph(
-                c, kLoopRevReq, kLoopRevSlot, -1,
+                c, kLoopRevReq, kLoopRevSlot, -(int32_t)kRevSteps,
                 [&](cudaStream_t bs) {
-                    return adj_backward_step(c->P, c->nspec ? c->dTable : nullptr, c->spec, rec,
-                                             RecSlot{c->loopCtl + kLoopRevSlot, 0u, stepBytes}, n,
-                                             c->numCells, reinterpret_cast<float2*>(lamPos),
-                                             reinterpret_cast<float2*>(lamVel), lamOmega, tlx,
-                                             tlv, tlw, lamF, lamM, acc, bs);
+                    cudaError_t er = cudaSuccess;
+                    for (uint32_t j = 0; j < kRevSteps && er == cudaSuccess; ++j)
+                        er = adj_backward_step(c->P, c->nspec ? c->dTable : nullptr, c->spec, rec,
+                                               RecSlot{c->loopCtl + kLoopRevSlot, 0u - j, stepBytes},
+                                               n, c->numCells, reinterpret_cast<float2*>(lamPos),
+                                               reinterpret_cast<float2*>(lamVel), lamOmega, tlx,
+                                               tlv, tlw, lamF, lamM, acc, bs);
+                    return er;
                 },
                 &revLoop);
             if (rc) break;

@@ -583,6 +583,43 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     }
 }
 
+// Packed (start, end) of cell c and first slot of the one after it, the slots
+// of its band `down` above their packed places.
+__device__ __forceinline__ uint2 packed_cell(const BandArgs& B, uint32_t c, uint32_t down) {
+    const uint32_t* f = B.first + (size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u));
+    return make_uint2(f[0] - down, f[1] - down);
+}
+
+// Blocks (band, share), as band_pack_kernel: the state the step of set q
+// stepped (its set is intact, its slots move only in the next fix) and the
+// accelerations it stored.
+__global__ void __launch_bounds__(kPackThreads)
+band_record_kernel(BandArgs B, DynSet d, uint32_t q, StepRec rec, size_t stride) {
+    if (B.ctrl[kBandAct + q] == 0u) return;
+    const StepRec r = rec_shifted(rec, B.ctrl[kBandDone] - 1u, stride);
+    const uint32_t b = blockIdx.x;
+    const uint32_t base = B.base[b], cnt = B.count[b];
+    const uint32_t to = packed_base(B.count, b);
+    const uint32_t t0 = blockIdx.y * kPackThreads + threadIdx.x, step = gridDim.y * kPackThreads;
+    for (uint32_t k = t0; k < cnt; k += step) {
+        const uint32_t s = base + k, i = to + k;
+        // out of range only after a sort whose wait gave up
+        if (s >= B.slots || i >= B.n) break;
+        r.pos[i] = d.pos[s];
+        r.vel[i] = d.vel[s];
+        r.omega[i] = d.omega[s];
+        r.radius[i] = B.stat.radius[s];
+        r.mass[i] = B.stat.mass[s];
+        r.id[i] = B.stat.id[s];
+        r.acc[i] = B.acc[s];
+        r.alpha[i] = B.alpha[s];
+    }
+    for (uint32_t k = t0; k < (1u << B.shift); k += step) {
+        const uint32_t c = (b << B.shift) + k;
+        if (c < B.cells) r.cells[c] = packed_cell(B, c, base - to);
+    }
+}
+
 // First particle of every cell in the sorted keys (lower bounds).
 __global__ void band_cell_first_kernel(const uint32_t* __restrict__ keys, uint32_t n,
                                        uint32_t cells, uint32_t* __restrict__ first) {
@@ -650,11 +687,10 @@ band_cells_kernel(BandArgs B, uint2* __restrict__ cells, uint32_t* __restrict__ 
     for (uint32_t k = threadIdx.x; k < (1u << B.shift); k += kPackThreads) {
         const uint32_t c = c0 + k;
         if (c >= B.cells) break;
-        const uint32_t* f = B.first + (size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u));
-        const uint32_t a = f[0] - shiftDown, e = f[1] - shiftDown;
-        first[c] = a;
-        cells[c] = a < e ? make_uint2(a, e) : make_uint2(kEmptyCell, kEmptyCell);
-        if (c == B.cells - 1u) first[B.cells] = e;
+        const uint2 r = packed_cell(B, c, shiftDown);
+        first[c] = r.x;
+        cells[c] = r.x < r.y ? r : make_uint2(kEmptyCell, kEmptyCell);
+        if (c == B.cells - 1u) first[B.cells] = r.y;
     }
 }
 
@@ -824,6 +860,14 @@ cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool sta
         band_pack_kernel<true><<<grid, kPackThreads, 0, st>>>(b, out, stateOnly ? 1u : 0u);
     else
         band_pack_kernel<false><<<grid, kPackThreads, 0, st>>>(b, out, stateOnly ? 1u : 0u);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_band_record(const BandArgs& b, int q, void* recBase, size_t stride,
+                               cudaStream_t st) {
+    const dim3 grid(b.bands, std::max(1u, 592u / b.bands));
+    band_record_kernel<<<grid, kPackThreads, 0, st>>>(b, b.dyn[q], (uint32_t)q,
+                                                      carve_step(recBase, b.n, b.cells), stride);
     return cudaGetLastError();
 }
 

@@ -142,6 +142,10 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
                              int variant, cudaStream_t st);
 cudaError_t launch_band_followed(const BandArgs& b, int q, const uint32_t* ids,
                                  const uint32_t* countWord, float* ring, cudaStream_t st);
+// The record of the step of set q (adj_record_step's, packed) at record block
+// kBandDone - 1 from recBase, records `stride` bytes apart.
+cudaError_t launch_band_record(const BandArgs& b, int q, void* recBase, size_t stride,
+                               cudaStream_t st);
 // The state into the packed arrays (with pressure and accelerations unless
 // stateOnly); nothing when the bands hold no state.
 cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool stateOnly,

@@ -182,6 +182,21 @@ cudaError_t launch_set_words(uint32_t* dst, Words w, cudaStream_t st);
 
 // Adjoint (dem_adjoint.cu).
 size_t adj_step_bytes(uint32_t n, uint32_t numCells);
+// One recorded step: the sorted state the step kernel read, its cell ranges
+// and the accelerations it computed.
+struct StepRec {
+    float2* pos;
+    float2* vel;
+    float* omega;
+    float* radius;
+    float* mass;
+    uint32_t* id;
+    float2* acc;
+    float* alpha;
+    uint2* cells;
+};
+// The arrays of the record at `base` (adj_step_bytes long).
+StepRec carve_step(void* base, uint32_t n, uint32_t numCells);
 // Writes the record of one forward step at recBase in one launch: the sorted
 // state the step kernel stepped (d, s and src as launch_step's in, inS and
 // src), its cell ranges and the acceleration and angular acceleration it
@@ -195,6 +210,28 @@ struct RecSlot {
     uint32_t add = 0;
     size_t stride = 0;
 };
+template <typename T>
+__device__ __forceinline__ T* rec_shift(T* p, size_t off) {
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + off);
+}
+// The record `k` places after r, records `stride` bytes apart.
+__device__ __forceinline__ StepRec rec_shifted(StepRec r, uint32_t k, size_t stride) {
+    const size_t off = stride * (size_t)k;
+    r.pos = rec_shift(r.pos, off);
+    r.vel = rec_shift(r.vel, off);
+    r.omega = rec_shift(r.omega, off);
+    r.radius = rec_shift(r.radius, off);
+    r.mass = rec_shift(r.mass, off);
+    r.id = rec_shift(r.id, off);
+    r.acc = rec_shift(r.acc, off);
+    r.alpha = rec_shift(r.alpha, off);
+    r.cells = rec_shift(r.cells, off);
+    return r;
+}
+// The record `at` names, from the one at the window's base.
+__device__ __forceinline__ StepRec rec_at(StepRec r, RecSlot at) {
+    return at.slot ? rec_shifted(r, *at.slot + at.add, at.stride) : r;
+}
 cudaError_t adj_record_step(void* recBase, RecSlot at, uint32_t n, uint32_t numCells, DynSet d,
                             StatSet s, const uint32_t* src, const uint2* cells, const float2* acc,
                             const float* alpha, cudaStream_t st);
