@@ -24,8 +24,10 @@ __device__ __forceinline__ uint32_t lower_count(const uint32_t* a, uint32_t n, u
 }
 
 // ------------------------------------------------------------------ fix
-// Bound by latency: a band's events, its cells' first slots, then its fields,
-// each once.  512 threads hold a run of 512 particles in registers while the
+// Bound by latency: four rounds of loads (the control words; the band's words
+// and events; its cells' first slots; its fields), each begun together: 153.8 ->
+// 150.4 us a step at 4,194,304 disks, 18.1 -> 17.4 at 131,071 fast ones, against
+// a load at a time.  512 threads hold a run of 512 particles in registers while the
 // next run loads, so a band of any length is rewritten in place: a particle
 // moves by at most kBandEvents slots, so the places a run is stored to have
 // been read by then.  Two such blocks fit on a multiprocessor, so 296 bands
@@ -51,8 +53,8 @@ struct FixShared {
     uint32_t leaveCell[kBandEvents]; // their old cells (sorted too)
     uint32_t arrive[kBandEvents];    // arrivals' 2 * cell + (from a higher cell), sorted
     uint32_t arriveEv[kBandEvents];
-    uint32_t arriveDst[kBandEvents];
-    uint32_t arriveAt[kBandEvents];  // the old place they go in front of
+    uint32_t arriveDst[kBandEvents];  // by event
+    uint32_t arriveAt[kBandEvents];   // the old place they go in front of
     uint32_t nl, na;
 };
 
@@ -67,13 +69,7 @@ __device__ __forceinline__ void fix_load(const BandArgs& B, const DynSet& d, con
         h[u].dst = kBandEmpty;
         if (j >= end) continue;
         const uint32_t s = base + j;
-        const uint32_t key = B.key[s];
-        const uint32_t rl = lower_count(S.leave, nl, j);
-        if (rl < nl && S.leave[rl] == j) continue;  // it left
-        const uint32_t to = j - rl + lower_count(S.arrive, na, 2u * (key - cell0) + 1u);
-        if (to == j) continue;
-        h[u].dst = to;
-        h[u].key = key;
+        h[u].key = B.key[s];
         h[u].p = d.pos[s];
         h[u].v = d.vel[s];
         h[u].th = d.theta[s];
@@ -83,6 +79,10 @@ __device__ __forceinline__ void fix_load(const BandArgs& B, const DynSet& d, con
         h[u].id = B.stat.id[s];
         h[u].cand = B.cand[s];
         if (TYPED) h[u].type = B.stat.type[s];
+        const uint32_t rl = lower_count(S.leave, nl, j);
+        if (rl < nl && S.leave[rl] == j) continue;  // it left
+        const uint32_t to = j - rl + lower_count(S.arrive, na, 2u * (h[u].key - cell0) + 1u);
+        if (to != j) h[u].dst = to;
     }
 }
 
@@ -107,26 +107,32 @@ template <bool TYPED>
 __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint32_t b) {
     const uint32_t tid = threadIdx.x;
     const uint32_t cell0 = b << B.shift;
+    // the band's words and the events, whether or not there are that many, in
+    // one round of loads
     const uint32_t base = B.base[b], cnt = B.count[b];
     const uint32_t ne = min(B.evCnt[b], kBandEvents);
-    const BandEvent* __restrict__ ev = B.ev + (size_t)b * kBandEvents;
-    if (tid < ne) S.ev[tid] = ev[tid].a;
+    BandEvent e{};
+    if (tid < kBandEvents) {
+        e = B.ev[(size_t)b * kBandEvents + tid];
+        S.ev[tid] = e.a;
+    }
     if (tid == 0) S.nl = S.na = 0u;
     __syncthreads();
-    if (tid < ne) {
-        const uint4 e = S.ev[tid];
-        const bool leaves = (e.z >> B.shift) == b, enters = (e.y >> B.shift) == b;
-        const uint32_t k2 = 2u * e.y + (e.z < e.y ? 0u : 1u);
+    const bool mine = tid < ne;
+    const bool enters = mine && (e.a.y >> B.shift) == b;
+    if (mine) {
+        const bool leaves = (e.a.z >> B.shift) == b;
+        const uint32_t k2 = 2u * e.a.y + (e.a.z < e.a.y ? 0u : 1u);
         uint32_t rl = 0, ra = 0;
         for (uint32_t f = 0; f < ne; ++f) {
             const uint4 o = S.ev[f];
             const uint32_t o2 = 2u * o.y + (o.z < o.y ? 0u : 1u);
-            if ((o.z >> B.shift) == b && o.x < e.x) ++rl;
-            if ((o.y >> B.shift) == b && (o2 < k2 || (o2 == k2 && o.x < e.x))) ++ra;
+            if ((o.z >> B.shift) == b && o.x < e.a.x) ++rl;
+            if ((o.y >> B.shift) == b && (o2 < k2 || (o2 == k2 && o.x < e.a.x))) ++ra;
         }
         if (leaves) {
-            S.leave[rl] = e.x - base;
-            S.leaveCell[rl] = e.z - cell0;
+            S.leave[rl] = e.a.x - base;
+            S.leaveCell[rl] = e.a.z - cell0;
             atomicAdd(&S.nl, 1u);
         }
         if (enters) {
@@ -143,7 +149,7 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
         const uint32_t at = B.first[(size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u)) +
                                     (k2 & 1u)] - base;
         S.arriveAt[tid] = at;
-        S.arriveDst[tid] = at - lower_count(S.leave, nl, at) + tid;
+        S.arriveDst[S.arriveEv[tid]] = at - lower_count(S.leave, nl, at) + tid;
     }
     __syncthreads();
     // places outside [from, end) keep their particles
@@ -152,6 +158,16 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
                                   : max(nl ? S.leave[nl - 1] + 1u : 0u, na ? S.arriveAt[na - 1] : 0u);
     Held<TYPED> now[kFixItems], next[kFixItems];
     fix_load<TYPED>(B, d, S, base, cell0, from, end, nl, na, now);
+    // first slots (beside the loads): one more for every arrival in a lower
+    // cell, one fewer for every leaver of one
+    const uint32_t rows = 1u << (B.shift - B.log2gx), row0 = cell0 >> B.log2gx;
+    for (uint32_t r = 0; r < rows; ++r)
+        for (uint32_t x = tid; x <= B.gx; x += kFixThreads) {
+            const uint32_t c = r * B.gx + x;
+            const uint32_t up = lower_count(S.arrive, na, 2u * c);
+            const uint32_t down = lower_count(S.leaveCell, nl, c);
+            if (up != down) B.first[(size_t)(row0 + r) * (B.gx + 1u) + x] += up - down;
+        }
     for (uint32_t run = from; run < end; run += kFixRun) {
         fix_load<TYPED>(B, d, S, base, cell0, run + kFixRun, end, nl, na, next);
         __syncthreads();  // this run and the next are read
@@ -166,24 +182,12 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
         for (int u = 0; u < kFixItems; ++u) now[u] = next[u];
     }
     __syncthreads();
-    if (tid < na) {
-        const BandEvent e = ev[S.arriveEv[tid]];
+    if (enters)
         put<TYPED>(B, d, base + S.arriveDst[tid], make_float2(e.b.x, e.b.y),
                    make_float2(e.b.z, e.b.w), e.c.x, e.c.y, e.c.z, e.c.w, e.a.w, e.d.x, e.a.y,
                    kCandNone);
-    }
     const uint32_t newCnt = cnt - nl + na;
     for (uint32_t j = newCnt + tid; j < cnt; j += kFixThreads) B.key[base + j] = kBandEmpty;
-    // first slots: one more for every arrival in a lower cell, one fewer for
-    // every leaver of one
-    const uint32_t rows = 1u << (B.shift - B.log2gx), row0 = cell0 >> B.log2gx;
-    for (uint32_t r = 0; r < rows; ++r)
-        for (uint32_t x = tid; x <= B.gx; x += kFixThreads) {
-            const uint32_t c = r * B.gx + x;
-            const uint32_t up = lower_count(S.arrive, na, 2u * c);
-            const uint32_t down = lower_count(S.leaveCell, nl, c);
-            if (up != down) B.first[(size_t)(row0 + r) * (B.gx + 1u) + x] += up - down;
-        }
     if (tid == 0) {
         B.count[b] = newCnt;
         B.evCnt[b] = 0u;
@@ -191,17 +195,28 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
 }
 
 template <bool TYPED>
-__global__ void __launch_bounds__(kFixThreads, 2) band_fix_kernel(BandArgs B, DynSet d, uint32_t q) {
+__global__ void __launch_bounds__(kFixThreads, 2)
+band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynSet d, uint32_t q) {
     __shared__ FixShared S;
-    const uint32_t left = B.ctrl[kBandLeft];
-    const bool active = left != 0u && B.ctrl[kBandCur] == q && B.ctrl[kBandFull] == 0u;
+    // left, done, full, cur; the first band of this block, if there is one
+    const uint4 c = *reinterpret_cast<const uint4*>(B.ctrl);
+    const uint32_t nd = min(B.ctrl[kBandDirty + q], B.bands);
+    uint32_t band = blockIdx.x < B.bands ? B.dirty[q][blockIdx.x] : 0u;
+    static_assert(kBandLeft == 0 && kBandFull == 2 && kBandCur == 3, "one load of 16 bytes");
+    const bool active = c.x != 0u && c.w == q && c.z == 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        B.ctrl[kBandAct + q] = active ? (left == 1u ? 2u : 1u) : 0u;
+        B.ctrl[kBandAct + q] = active ? (c.x == 1u ? 2u : 1u) : 0u;
         B.ctrl[kBandNow + q] = B.ctrl[kBandStep];
     }
     if (!active) return;
-    // how far pairs may have approached since their bands searched
-    for (uint32_t b = blockIdx.x * kFixThreads + threadIdx.x; b < B.bands;
+    for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
+        if (k != blockIdx.x) band = B.dirty[q][k];
+        fix_band<TYPED>(B, d, S, band);
+        __syncthreads();
+    }
+    // how far pairs may have approached since their bands searched, by the
+    // blocks from the last on (the first ones have the events)
+    for (uint32_t b = (gridDim.x - 1u - blockIdx.x) * kFixThreads + threadIdx.x; b < B.bands;
          b += gridDim.x * kFixThreads) {
         const uint32_t lo = b ? b - 1u : B.bands - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
         const float own = __uint_as_float(B.moved[q][b]);
@@ -212,11 +227,6 @@ __global__ void __launch_bounds__(kFixThreads, 2) band_fix_kernel(BandArgs B, Dy
         B.grown[b] = keep ? grown : 0.0f;
         B.search[b] = keep ? 0u : 1u;
         B.moved[q ^ 1u][b] = 0u;  // the step of this set collects it
-    }
-    const uint32_t nd = min(B.ctrl[kBandDirty + q], B.bands);
-    for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
-        fix_band<TYPED>(B, d, S, B.dirty[q][k]);
-        __syncthreads();
     }
 }
 
@@ -351,7 +361,8 @@ __device__ __forceinline__ RowBase row_bases(const KParams& P, const BandArgs& B
 // added in cell order (an empty cell adds +0).  Every lane calls it.
 template <bool TYPED, bool ATTRACT>
 __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B, const DynSet& in,
-                                             Deal<ATTRACT>& S, unsigned long long rem,
+                                             Deal<ATTRACT>& S, bool wantPr,
+                                             unsigned long long rem,
                                              const RowBase& base, uint32_t key, float2 p, float2 v,
                                              float w, float r, uint32_t mat, Pull& o) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -399,7 +410,7 @@ __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B
             total += (uint32_t)__popc(hits);
         }
         if (total == 0u) continue;
-        deal_law<TYPED, ATTRACT>(P, S, total, mine, cells, p, v, w, r, mat, in.pos, in.vel,
+        deal_law<TYPED, ATTRACT>(P, S, wantPr, total, mine, cells, p, v, w, r, mat, in.pos, in.vel,
                                  in.omega, B.stat.radius, B.stat.type, nullptr, sum);
     }
     o = sum.close();
@@ -411,7 +422,7 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
                  const __grid_constant__ DynSet in, const __grid_constant__ DynSet out, uint32_t q,
                  uint32_t everyStep) {
     __shared__ Deal<ATTRACT> deal[CULL ? THREADS / 32 : 1];
-    const uint32_t act = B.ctrl[kBandAct + q];
+    const uint32_t act = B.ctrl[kBandAct + q], now = B.ctrl[kBandNow + q];
     const uint32_t slot = blockIdx.x * THREADS + threadIdx.x;
     // the lanes past the last slot stand by as copies of it
     const uint32_t i = min(slot, B.slots - 1u);
@@ -426,7 +437,6 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
     const uint32_t mat = TYPED ? B.stat.type[i] : 0u;
     unsigned long long cand = CULL ? B.cand[i] : kCandNone;
     if (act == 0u) return;
-    const uint32_t now = B.ctrl[kBandNow + q];
     if (slot == 0u) {
         B.ctrl[kBandCur] = q ^ 1u;
         B.ctrl[kBandLeft] -= 1u;
@@ -437,6 +447,9 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
         if (*B.errFlag & kSortTimeoutBit) B.ctrl[kBandFull] = 1u;
     }
     const bool mine = slot < B.slots && key != kBandEmpty;
+    // the next step overwrites the pressure and the accelerations: only the
+    // call's last step makes and stores them
+    const bool store = act == 2u || everyStep;
     if (!__any_sync(0xffffffffu, mine)) return;
     Pull o{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
     RowBase base{};
@@ -458,8 +471,8 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
         }
     }
     if (CULL)
-        collide_warp<TYPED, ATTRACT>(P, B, in, deal[threadIdx.x >> 5], cand, base, key, s.p, s.v,
-                                     s.w, r, mat, o);
+        collide_warp<TYPED, ATTRACT>(P, B, in, deal[threadIdx.x >> 5], store && B.pressure, cand,
+                                     base, key, s.p, s.v, s.w, r, mat, o);
     if (!mine) return;
     // F/m and M/I as the reference divides them; without contacts both are
     // exactly +0 (see finish_particle)
@@ -478,8 +491,7 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
     out.vel[i] = s.v;
     out.theta[i] = s.th;
     out.omega[i] = s.w;
-    // the next step overwrites these: only the call's last step stores them
-    if (act == 2u || everyStep) {
+    if (store) {
         if (B.pressure) B.pressure[i] = o.pr;
         if (B.acc) {
             B.acc[i] = a;

@@ -160,10 +160,11 @@ struct Deal {
 // The turn's `total` listed contacts through the law, then each lane's own (bit
 // k of `mine`: its candidate k; four bits of `cells` each: the cell) into its
 // sums.  The neighbours' velocity, spin and type are read through `src` where
-// the arrays are in the previous order.  Every lane calls it.
+// the arrays are in the previous order.  The pressure, which nothing but a
+// caller reads, is summed only with `wantPr`.  Every lane calls it.
 template <bool TYPED, bool ATTRACT>
-__device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, uint32_t total,
-                                         uint32_t mine, uint32_t cells, float2 p, float2 v,
+__device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, bool wantPr,
+                                         uint32_t total, uint32_t mine, uint32_t cells, float2 p, float2 v,
                                          float w, float r, uint32_t mat,
                                          const float2* __restrict__ pos,
                                          const float2* __restrict__ vel,
@@ -190,19 +191,18 @@ __device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, uin
             const float2 pB = __ldg(pos + j);
             const float rB = __ldg(radius + j);
             float2 f;
-            float m;
-            double q;
+            float m, flen;
             pair_terms(pA, pB, vA, __ldg(vel + sj), wA, __ldg(omega + sj), rA, rB, pc, P.dt, f, m,
-                       q);
+                       flen);
             S.j[code] = __float_as_uint(f.x);
             S.fy[code] = f.y;
             S.moment[code] = m;
-            S.q[code] = q;
+            if (wantPr) S.q[code] = flen != 0.0f ? pressure_term(flen, rA) : 0.0;
             if (ATTRACT) {
-                const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB], q);
+                const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB]);
                 S.ax[code] = g.x;
                 S.ay[code] = g.y;
-                S.aq[code] = q;
+                if (wantPr) S.aq[code] = pressure_term(len2(g.x, g.y), rA);
             }
         }
     }
@@ -214,11 +214,11 @@ __device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, uin
         sum.sub.x += __uint_as_float(S.j[x]);
         sum.sub.y += S.fy[x];
         sum.o.moment += S.moment[x];
-        sum.o.pr = (float)((double)sum.o.pr + S.q[x]);
+        if (wantPr) sum.o.pr = (float)((double)sum.o.pr + S.q[x]);
         if (ATTRACT) {
             sum.sub.x += S.ax[x];
             sum.sub.y += S.ay[x];
-            sum.o.pr = (float)((double)sum.o.pr + S.aq[x]);
+            if (wantPr) sum.o.pr = (float)((double)sum.o.pr + S.aq[x]);
         }
     }
     __syncwarp();  // the results are read

@@ -128,16 +128,17 @@ __device__ __forceinline__ float add_pressure(float pr, float flen, float r) {
 
 // One particle pair, particles_kernel.cuh:236-307 (collideSpheres).  A is the
 // particle being updated, B the neighbour.  Returns whether they touch, with
-// the force on A and the terms of A's moment and pressure.
+// the force on A, the term of A's moment, and the length of the force that
+// enters A's pressure (pressure_term).
 __device__ __forceinline__ bool pair_terms(float2 pA, float2 pB, float2 vA, float2 vB, float wA,
                                            float wB, float rA, float rB, float4 pc, float dt,
-                                           float2& f, float& moment, double& pressure) {
+                                           float2& f, float& moment, float& flen) {
     const float relx = pB.x - pA.x, rely = pB.y - pA.y;
     const float dist = len2(relx, rely);
     const float cd = rA + rB;
     f = make_float2(0.0f, 0.0f);
     moment = 0.0f;
-    pressure = 0.0;
+    flen = 0.0f;
     if (!(dist < cd)) return false;
     const float nx = relx / dist, ny = rely / dist;
     const float tx = -ny, ty = nx;
@@ -152,12 +153,12 @@ __device__ __forceinline__ bool pair_terms(float2 pA, float2 pB, float2 vA, floa
         f.x += c * nx;
         f.y += c * ny;
     }
-    pressure = pressure_term(len2(f.x, f.y), rA);
+    flen = len2(f.x, f.y);
     if (pc.w != 0.0f) {
         const float sw = rA * wA + rB * wB;
         const float vcx = vtx - sw * tx, vcy = vty - sw * ty;
         const float ftrx = pc.y * vcx * dt, ftry = pc.y * vcy * dt;
-        const float ftmax = pc.w * len2(f.x, f.y);
+        const float ftmax = pc.w * flen;
         float ftx, fty;
         if (len2(ftrx, ftry) < ftmax) {
             ftx = ftrx;
@@ -179,10 +180,9 @@ __device__ __forceinline__ float2 pair_force(float2 pA, float2 pB, float2 vA, fl
                                              float wB, float rA, float rB, float4 pc, float dt,
                                              float& moment, float& pressure) {
     float2 f;
-    float m;
-    double q;
-    if (pair_terms(pA, pB, vA, vB, wA, wB, rA, rB, pc, dt, f, m, q)) {
-        pressure = (float)((double)pressure + q);
+    float m, flen;
+    if (pair_terms(pA, pB, vA, vB, wA, wB, rA, rB, pc, dt, f, m, flen)) {
+        pressure = add_pressure(pressure, flen, rA);
         if (pc.w != 0.0f) moment += m;
     }
     return f;
@@ -191,7 +191,7 @@ __device__ __forceinline__ float2 pair_force(float2 pA, float2 pB, float2 vA, fl
 // particles_kernel.cuh:311-342 (attractSpheres), only compiled into the
 // attraction variants of the collide kernels.
 __device__ __forceinline__ float2 pair_attract_terms(float2 pA, float2 pB, float rA, float rB,
-                                                     float aA, float aB, double& pressure) {
+                                                     float aA, float aB) {
     const float relx = pB.x - pA.x, rely = pB.y - pA.y;
     const float dist = len2(relx, rely);
     const float dA = (float)((double)(rA * 2.0f) * 1.2);
@@ -208,14 +208,12 @@ __device__ __forceinline__ float2 pair_attract_terms(float2 pA, float2 pB, float
         f.x += c * nx;
         f.y += c * ny;
     }
-    pressure = pressure_term(len2(f.x, f.y), rA);
     return f;
 }
 __device__ __forceinline__ float2 pair_attract(float2 pA, float2 pB, float rA, float rB, float aA,
                                                float aB, float& pressure) {
-    double q;
-    const float2 f = pair_attract_terms(pA, pB, rA, rB, aA, aB, q);
-    pressure = (float)((double)pressure + q);
+    const float2 f = pair_attract_terms(pA, pB, rA, rB, aA, aB);
+    pressure = add_pressure(pressure, len2(f.x, f.y), rA);
     return f;
 }
 
