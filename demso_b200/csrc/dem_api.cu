@@ -384,14 +384,20 @@ struct DemContext {
     // The step in bands (dem_bands.cuh): its arrays, in bandBlock (band.bands
     // == 0: the context steps on the packed path); whether they hold the
     // current state, and whether cells/first of set cur were made from them;
-    // the step loop, with and without followed rows, and the sort phase alone,
-    // by cur (the set the state is packed into).
+    // the step loop, with and without followed rows, one step, and a step's
+    // sort phase alone, by cur (the set the state is packed into) and bandSet.
     BandArgs band;
+    std::vector<BandGeo> bandGeo;
     void* bandBlock = nullptr;
     float2* ownPos = nullptr;  // the block's positions: not an adopted set
     bool bandValid = false, bandCells = false, bandInit = false;
-    cudaGraphExec_t bandLoop[2] = {}, bandFollow[2] = {}, bandSort[2] = {};
-    cudaGraphExec_t bandRec[2] = {};  // the loop recording every step for the adjoint
+    int bandSet = 0;  // the dynamic set of the bands that holds the state
+    // band_call: short calls in a row that stepped in bands; steps of longer
+    // calls on the packed path since
+    uint32_t shortCalls = 0, packedSteps = 0;
+    cudaGraphExec_t bandLoop[2][2] = {}, bandOne[2][2] = {}, bandFollow[2][2] = {};
+    cudaGraphExec_t bandSort[2][2] = {};
+    cudaGraphExec_t bandRec[2][2] = {};  // the loop recording every step for the adjoint
     // followed-particle staging (device), see dem_get_followed
     float* followRows = nullptr;
     // dem_step_followed: the ids (device copy), the ring of per-step rows,
@@ -492,7 +498,7 @@ void drop_tune_graphs(DemContext* c) {
 
 void drop_adj_graphs(DemContext* c) {
     for (int p = 0; p < 2; ++p) {
-        for (cudaGraphExec_t* g : {&c->adjRecLoop[p], &c->bandRec[p]}) {
+        for (cudaGraphExec_t* g : {&c->adjRecLoop[p], &c->bandRec[p][0], &c->bandRec[p][1]}) {
             if (*g) cudaGraphExecDestroy(*g);
             *g = nullptr;
         }
@@ -507,10 +513,12 @@ void drop_loop_graphs(DemContext* c) {
         c->loopGraph[p] = nullptr;
         if (c->followGraph[p]) cudaGraphExecDestroy(c->followGraph[p]);
         c->followGraph[p] = nullptr;
-        for (cudaGraphExec_t* g : {&c->bandLoop[p], &c->bandFollow[p], &c->bandSort[p]}) {
-            if (*g) cudaGraphExecDestroy(*g);
-            *g = nullptr;
-        }
+        for (int q = 0; q < 2; ++q)
+            for (cudaGraphExec_t* g : {&c->bandLoop[p][q], &c->bandOne[p][q], &c->bandFollow[p][q],
+                                       &c->bandSort[p][q]}) {
+                if (*g) cudaGraphExecDestroy(*g);
+                *g = nullptr;
+            }
     }
     drop_adj_graphs(c);
 }
@@ -1011,7 +1019,17 @@ int init_context(DemContext* c, uint32_t capacity, uint32_t numCells, DemContext
     const bool ownState = !(c->flags & DEM_CTX_CALLER_STATE);
     size_t total = 0;
     // single scenes step in bands (dem_bands.cuh)
-    if (!ownState || c->nspec || !band_shape(c->P.gx, numCells, c->band)) c->band = BandArgs{};
+    if (ownState) {
+        std::vector<KParams> grids{c->P};
+        std::vector<uint32_t> counts{0u};
+        if (c->nspec) {
+            grids = c->hTable;
+            for (uint32_t s = 1; s < c->nspec; ++s) counts.push_back(0u);
+            for (uint32_t s = 0; s < c->nspec; ++s) counts[s] = c->partOff[s + 1] - c->partOff[s];
+        }
+        if (!band_shape(grids, counts, c->nspec != 0, c->band, c->bandGeo)) c->band = BandArgs{};
+        for (uint32_t s = 0; s < c->nspec; ++s) c->hTable[s].firstOff = grids[s].firstOff;
+    }
     if (ownState) {
         total += 2 * (f8p + f8 + 2 * f4);                    // dyn sets
         total += 2 * (f4p + 2 * f4 + (c->typed ? f4 : 0));   // static sets
@@ -1170,6 +1188,7 @@ extern "C" int dem_batch_set_systems(DemContext* c, const DemSystem* specs,
             return fail(DEM_ERR_INVALID_ARG, "specimen %u: material layout is fixed", s);
         table[s] = make_kparams(&specs[s], specs[s].numParticles);
         table[s].cellOff = old.cellOff;
+        table[s].firstOff = old.firstOff;
         set_rmax(table[s], c->rmax);
         bool attract = false;
         for (uint32_t m = 0; m < table[s].nmat; ++m) attract = attract || table[s].at[m] != 0.0f;
@@ -1206,8 +1225,9 @@ bool has_state_sets(const DemContext* c) { return c->dyn[0].pos != nullptr; }
 bool steps_in_bands(DemContext* c);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
-    // the band arrays, unless the cluster launch will step this scene
-    if (!(c->flags & DEM_CTX_RESIDENT) || !cluster_scene_fits(n, c->numCells)) steps_in_bands(c);
+    // the band arrays, unless a resident launch may step this scene or batch
+    if (!(c->flags & DEM_CTX_RESIDENT) || (!c->nspec && !cluster_scene_fits(n, c->numCells)))
+        steps_in_bands(c);
     // the new state replaces the one any recorded error was about
     DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 4, st), "clear error word");
     const int a = c->cur;
@@ -1391,7 +1411,7 @@ extern "C" int dem_get_state(DemContext* c, float* pos, float* vel, float* theta
 namespace {
 
 // ------------------------------------------------------------ step in bands
-// Own buffers, one scene, no control particle.  The arrays are allocated at
+// Own buffers, no control particle.  The arrays are allocated at
 // the first state a context takes (about 100 B per particle and 8 KB per
 // band, of its capacity); a context whose GPU has no room for them steps on
 // the packed path.
@@ -1399,16 +1419,43 @@ bool steps_in_bands(DemContext* c) {
     if (c->band.bands == 0 || c->ctlOn || c->dyn[0].pos != c->ownPos) return false;
     if (c->bandBlock) return true;
     const bool pressure = c->flags & DEM_CTX_PRESSURE, accel = c->flags & DEM_CTX_ACCEL;
-    const size_t bytes = band_bytes(c->band, c->capacity, c->typed, pressure, accel);
+    const size_t bytes = band_bytes(c->band, c->capacity, c->typed, pressure, accel, c->nspec != 0);
     if (dev_alloc(&c->bandBlock, bytes) != cudaSuccess) {
         (void)cudaGetLastError();
         c->bandBlock = nullptr;
         c->band = BandArgs{};
         return false;
     }
-    carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel);
+    carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel, c->nspec != 0);
+    c->band.table = c->dTable;  // null for a single scene
     c->band.errFlag = c->errFlag;
     return true;
+}
+
+// Whether a call of `nsteps` steps goes through the bands.  Packing the state at
+// the end of a call costs about a third of a step, and a change of path a sort
+// from scratch (one to two steps).  A call of fewer than kShortCall steps
+// therefore stays where the state is, and starts a new state on the packed
+// path (one step: 79 against 115 us at 1,000,003 disks, 232 against 263 at
+// 4,194,304; five steps: 385 against 373, 1,151 against 896); longer ones leave
+// the packed path once they have made enough steps to earn the sort, and
+// kShortRun short calls in a row leave the bands.
+constexpr uint32_t kShortCall = 4, kPackedSteps = 16, kShortRun = 16;
+bool band_call(DemContext* c, uint32_t nsteps) {
+    if (!steps_in_bands(c)) return false;
+    if (c->profiling || c->tuned < 0) return true;  // the bands' kernels are what is timed
+    const bool packedOrder = c->keysValid && c->haveOrder;
+    if (nsteps >= kShortCall) {
+        c->shortCalls = 0;
+        c->packedSteps += std::min(nsteps, kPackedSteps);
+        if (!c->bandValid && packedOrder && c->packedSteps < kPackedSteps) return false;
+        c->packedSteps = 0;
+        return true;
+    }
+    if (!c->bandValid) return false;
+    if (++c->shortCalls < kShortRun) return true;
+    c->shortCalls = 0;
+    return false;
 }
 
 PackedState packed_state(DemContext* c) {
@@ -1421,7 +1468,9 @@ PackedState packed_state(DemContext* c) {
 cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
     const PackedState s = packed_state(c);
     cudaError_t e = launch_band_pack(c->band, s, true, st);
-    if (e == cudaSuccess) e = launch_calc_hash(c->P, s.dyn.pos, c->keys, nullptr, c->n, st);
+    if (e == cudaSuccess)
+        e = c->nspec ? launch_calc_hash_batched(c->dTable, c->spec, s.dyn.pos, c->keys, c->n, st)
+                     : launch_calc_hash(c->P, s.dyn.pos, c->keys, nullptr, c->n, st);
     uint32_t *ko = nullptr, *vo = nullptr;
     if (e == cudaSuccess)
         e = onesweep_sort_pairs(c->keys, c->perm, c->n, c->keyBits, true, c->ss, c->errFlag, st,
@@ -1437,6 +1486,7 @@ cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
 // steps of the set that does not hold the state do nothing, so every pass of
 // the outer loop makes at least one step.
 constexpr int kBandPairs = 2;
+constexpr uint32_t kSkipDisks = 1u << 20;
 
 // What follows every step of a call: nothing, its followed rows, its record for
 // the adjoint.
@@ -1445,7 +1495,7 @@ enum class BandAfter { kNothing, kFollowed, kRecord };
 cudaError_t enqueue_band_pairs(DemContext* c, BandAfter after, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < 2 * kBandPairs && e == cudaSuccess; ++k) {
-        const int q = k & 1;
+        const int q = c->bandSet ^ (k & 1);
         e = launch_band_fix(c->band, q, st);
         if (e == cudaSuccess)
             e = launch_band_step(c->P, c->band, q, after != BandAfter::kNothing, c->variant, st);
@@ -1492,15 +1542,17 @@ cudaError_t enqueue_band_loop(DemContext* c, BandAfter after, cudaStream_t st) {
     });
 }
 
-// The sort phase of one step alone: a new layout when due, then the fixes (of
-// which one runs).
-cudaError_t enqueue_band_sort(DemContext* c, cudaStream_t st) {
+// The sort phase of one step alone: a new layout when due, then the fix; with
+// `step` the step too.
+cudaError_t enqueue_band_sort(DemContext* c, bool step, cudaStream_t st) {
     cudaGraphConditionalHandle full;
     cudaError_t e = conditional_handle(st, &full);
     if (e == cudaSuccess) e = launch_band_head(c->band, full, 0, false, st);
     if (e == cudaSuccess)
         e = add_if(c, st, full, [&](cudaStream_t fb) { return enqueue_band_layout(c, fb); });
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) e = launch_band_fix(c->band, q, st);
+    if (e == cudaSuccess) e = launch_band_fix(c->band, c->bandSet, st);
+    if (e == cudaSuccess && step)
+        e = launch_band_step(c->P, c->band, c->bandSet, false, c->variant, st);
     return e;
 }
 
@@ -1525,15 +1577,19 @@ int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t s
     c->band.n = c->n;
     c->band.slack = band_slack(c->band, c->n);
     c->band.slots = (uint32_t)band_slots(c->band, c->n);
-    c->band.skin = c->P.cull ? kSkin * c->P.rmax : 0.0f;
+    c->band.skin = std::isfinite(c->rmax) ? kSkin * c->rmax : 0.0f;
     if (!c->bandInit) {
         // stamps start below the first step's number
         DEM_TRY_CUDA(cudaMemsetAsync(c->band.stamp, 0, 4ull * c->band.cells, st), "band stamps");
+        DEM_TRY_CUDA(cudaMemcpyAsync(const_cast<BandGeo*>(c->band.geo), c->bandGeo.data(),
+                                     sizeof(BandGeo) * c->bandGeo.size(), cudaMemcpyHostToDevice, st),
+                     "bands");
+        if (c->band.cellBand) DEM_TRY_CUDA(launch_band_cell_table(c->band, st), "band cells");
         DEM_TRY_CUDA(launch_set_words(c->band.ctrl + kBandStep, Words{{1u}, 1u}, st), "band step");
         c->bandInit = true;
     }
     const Words w = c->bandValid ? Words{{nsteps, rowBlock}, 2u}
-                                 : Words{{nsteps, rowBlock, 1u, 0u, 0u}, 5u};
+                                 : Words{{nsteps, rowBlock, 1u, (uint32_t)c->bandSet, 0u}, 5u};
     DEM_TRY_CUDA(launch_set_words(c->band.ctrl, w, st), "band step count");
     // as a step of the packed path would have left it
     state_replaced(c);
@@ -1551,8 +1607,8 @@ int band_step_alone(DemContext* c, cudaStream_t st) {
     const bool direct = c->flags & DEM_CTX_DIRECT;
     const int a = c->cur;
     if (!direct) {
-        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_sort(c, s); },
-                              &c->bandSort[a]);
+        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_sort(c, false, s); },
+                              &c->bandSort[a][c->bandSet]);
         if (rc) return rc;
     }
     uint32_t full = 0;
@@ -1566,9 +1622,9 @@ int band_step_alone(DemContext* c, cudaStream_t st) {
     if (prof) DEM_TRY_CUDA(cudaEventRecord(ev[0], st), "profile event");
     if (direct) {
         if (full) DEM_TRY_CUDA(enqueue_band_layout(c, st), "band layout");
-        for (int q = 0; q < 2; ++q) DEM_TRY_CUDA(launch_band_fix(c->band, q, st), "band fix");
+        DEM_TRY_CUDA(launch_band_fix(c->band, c->bandSet, st), "band fix");
     } else {
-        DEM_TRY_CUDA(cudaGraphLaunch(c->bandSort[a], st), "graph launch");
+        DEM_TRY_CUDA(cudaGraphLaunch(c->bandSort[a][c->bandSet], st), "graph launch");
     }
     if (prof) DEM_TRY_CUDA(cudaEventRecord(ev[1], st), "profile event");
     const uint32_t k = c->tuneStep;
@@ -1578,10 +1634,10 @@ int band_step_alone(DemContext* c, cudaStream_t st) {
         if (rc) return rc;
         DEM_TRY_CUDA(cudaEventRecord(c->tuneEv[2 * k], st), "tuner event");
     }
-    for (int q = 0; q < 2; ++q)
-        DEM_TRY_CUDA(launch_band_step(c->P, c->band, q, false,
-                                      tune ? (int)(k % kStepVariants) : c->variant, st),
-                     "band step");
+    DEM_TRY_CUDA(launch_band_step(c->P, c->band, c->bandSet, false,
+                                  tune ? (int)(k % kStepVariants) : c->variant, st),
+                 "band step");
+    c->bandSet ^= 1;
     if (tune) {
         DEM_TRY_CUDA(cudaEventRecord(c->tuneEv[2 * k + 1], st), "tuner event");
         if (++c->tuneStep == kTuneSteps) {
@@ -1608,15 +1664,33 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
         if (rc) return rc;
         ++done;
     }
-    if (done < nsteps) {
-        rc = band_begin(c, nsteps - done, block + done, st);
+    // Whole passes of the loop, then the last few steps one by one where that is
+    // cheaper: a step the loop skips costs its empty launches (7 us at 65,536
+    // disks, 26 at 4,194,304), a graph of one step 12 us more than a step in the
+    // loop.
+    const uint32_t pass = c->n >= kSkipDisks ? 2u * kBandPairs : 1u;
+    const int a = c->cur;
+    while (done < nsteps) {
+        uint32_t m = nsteps - done;
+        if (after == BandAfter::kNothing && m != 1u) m = m >= pass ? m - m % pass : 1u;
+        rc = band_begin(c, m, block + done, st);
         if (rc) return rc;
-        cudaGraphExec_t* g = after == BandAfter::kFollowed ? &c->bandFollow[c->cur]
-                             : after == BandAfter::kRecord ? &c->bandRec[c->cur]
-                                                           : &c->bandLoop[c->cur];
-        rc = build_band_graph(c, [&](cudaStream_t s) { return enqueue_band_loop(c, after, s); }, g);
+        const int q = c->bandSet;
+        cudaGraphExec_t* g = after == BandAfter::kFollowed ? &c->bandFollow[a][q]
+                             : after == BandAfter::kRecord ? &c->bandRec[a][q]
+                             : m == 1u                     ? &c->bandOne[a][q]
+                                                           : &c->bandLoop[a][q];
+        rc = build_band_graph(c,
+                              [&](cudaStream_t s) {
+                                  return m == 1u && after == BandAfter::kNothing
+                                             ? enqueue_band_sort(c, true, s)
+                                             : enqueue_band_loop(c, after, s);
+                              },
+                              g);
         if (rc) return rc;
         DEM_TRY_CUDA(cudaGraphLaunch(*g, st), "graph launch");
+        done += m;
+        c->bandSet ^= (int)(m & 1u);
     }
     DEM_TRY_CUDA(launch_band_pack(c->band, packed_state(c), false, st), "band pack");
     return DEM_OK;
@@ -1691,6 +1765,19 @@ bool has_attraction_host(const KParams& P);
 
 constexpr int kNotResident = -1;
 
+// The resident launch steps a bin per multiprocessor at a time, whatever else
+// the GPU could do; the bands share all of it.  The launch is faster only with
+// about one bin for every multiprocessor, over enough steps to load and store
+// the bins: per step, resident against bands, 512 specimens (144 bins) 60.5 / 66
+// us, 4,096 (1,145 bins) 405 / 380, 32 (9 bins) 58 / 20; calls of one, three and
+// five steps of the 512, 155, 266 and 383 against 104, 317 and 421.
+constexpr uint32_t kResidentSteps = 2;
+bool resident_bins_fill(const DemContext* c) {
+    int sms = 148;
+    (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    return 8u * c->resBins >= 7u * (uint32_t)sms && c->resBins <= (uint32_t)sms;
+}
+
 // A multi-step call of a batch created with DEM_CTX_RESIDENT as one
 // persistent launch (dem_resident.cu).  Returns kNotResident, having done
 // nothing, when the batch has types, attraction, a control particle, stage
@@ -1699,7 +1786,7 @@ constexpr int kNotResident = -1;
 // graph path, but no mover record exists: the next graph-path step sorts
 // from scratch (the same permutation, the sort being stable).
 int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) ||
+    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) || nsteps < kResidentSteps ||
         c->partOff.size() != (size_t)c->nspec + 1 || c->partOff.back() != c->n)
         return kNotResident;
     for (uint32_t s = 0; s < c->nspec; ++s)
@@ -1734,7 +1821,7 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
         c->resMaxC = maxC;
         c->resBlocks = blocks;
     }
-    if (c->resBins == 0) return kNotResident;
+    if (c->resBins == 0 || !resident_bins_fill(c)) return kNotResident;
     const int a = c->cur;
     ResIO io{c->dyn[0].pos, c->dyn[a].vel, c->dyn[a].theta, c->dyn[a].omega, c->stat[a].radius,
              c->stat[a].mass, c->stat[a].id, c->loc, c->pressure, c->acc, c->alpha};
@@ -1751,7 +1838,7 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
 // cluster launch (dem_resident.cu): every block of the cluster holds the
 // whole scene in shared memory and steps its share of the slots.  Returns
 // kNotResident, having done nothing, for scenes it does not take (more than
-// 8,192 disks or cells, types, attraction, a control particle, profiling) or
+// 1,536 disks or 8,192 cells, types, attraction, a control particle, profiling) or
 // when no such cluster can be resident on this GPU; the graph path steps
 // those.  The next graph-path step sorts from scratch.
 int cluster_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
@@ -1804,7 +1891,7 @@ namespace {
 // step loop for pairs of steps (also the steps of dem_step_followed, whose
 // per-step rows are gathered from this path's buffers).
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (steps_in_bands(c)) return band_steps(c, nsteps, BandAfter::kNothing, 0, st);
+    if (band_call(c, nsteps)) return band_steps(c, nsteps, BandAfter::kNothing, 0, st);
     c->bandValid = false;
     if (!c->keysValid) {
         if (c->nspec)
@@ -2078,7 +2165,7 @@ extern "C" int dem_step_followed(DemContext* c, uint32_t nsteps, const uint32_t*
     for (uint32_t s = 0; s < nsteps;) {
         const uint32_t m = std::min(chunk, nsteps - s);
         const bool alone = (c->flags & DEM_CTX_DIRECT) || c->profiling || c->tuned < 0;
-        if (steps_in_bands(c) && !alone) {
+        if (!alone && band_call(c, m)) {
             int rc = band_steps(c, m, BandAfter::kFollowed, 0, st);
             if (rc) return rc;
         } else for (uint32_t j = 0; j < m;) {

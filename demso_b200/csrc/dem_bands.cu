@@ -23,6 +23,10 @@ __device__ __forceinline__ uint32_t lower_count(const uint32_t* a, uint32_t n, u
     return lo;
 }
 
+__device__ __forceinline__ uint32_t band_of(const BandArgs& B, uint32_t cell) {
+    return B.cellBand ? __ldg(B.cellBand + cell) : cell >> B.shift;
+}
+
 // ------------------------------------------------------------------ fix
 // Bound by latency: four rounds of loads (the control words; the band's words
 // and events; its cells' first slots; its fields), each begun together: 153.8 ->
@@ -106,9 +110,10 @@ __device__ __forceinline__ void put(const BandArgs& B, const DynSet& d, uint32_t
 template <bool TYPED>
 __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint32_t b) {
     const uint32_t tid = threadIdx.x;
-    const uint32_t cell0 = b << B.shift;
     // the band's words and the events, whether or not there are that many, in
     // one round of loads
+    const BandGeo geo = B.geo[b];
+    const uint32_t cell0 = geo.cell0, gx = 1u << geo.log2gx;
     const uint32_t base = B.base[b], cnt = B.count[b];
     const uint32_t ne = min(B.evCnt[b], kBandEvents);
     BandEvent e{};
@@ -119,16 +124,16 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
     if (tid == 0) S.nl = S.na = 0u;
     __syncthreads();
     const bool mine = tid < ne;
-    const bool enters = mine && (e.a.y >> B.shift) == b;
+    const bool enters = mine && e.a.y - cell0 < geo.cells;
     if (mine) {
-        const bool leaves = (e.a.z >> B.shift) == b;
+        const bool leaves = e.a.z - cell0 < geo.cells;
         const uint32_t k2 = 2u * e.a.y + (e.a.z < e.a.y ? 0u : 1u);
         uint32_t rl = 0, ra = 0;
         for (uint32_t f = 0; f < ne; ++f) {
             const uint4 o = S.ev[f];
             const uint32_t o2 = 2u * o.y + (o.z < o.y ? 0u : 1u);
-            if ((o.z >> B.shift) == b && o.x < e.a.x) ++rl;
-            if ((o.y >> B.shift) == b && (o2 < k2 || (o2 == k2 && o.x < e.a.x))) ++ra;
+            if (o.z - cell0 < geo.cells && o.x < e.a.x) ++rl;
+            if (o.y - cell0 < geo.cells && (o2 < k2 || (o2 == k2 && o.x < e.a.x))) ++ra;
         }
         if (leaves) {
             S.leave[rl] = e.a.x - base;
@@ -144,9 +149,9 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
     __syncthreads();
     const uint32_t nl = S.nl, na = S.na;
     if (tid < na) {
-        const uint32_t k2 = S.arrive[tid], c = cell0 + (k2 >> 1);
+        const uint32_t k2 = S.arrive[tid], c = k2 >> 1;
         // in front of its cell's stayers, or behind them
-        const uint32_t at = B.first[(size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u)) +
+        const uint32_t at = B.first[geo.first + (c >> geo.log2gx) * (gx + 1u) + (c & (gx - 1u)) +
                                     (k2 & 1u)] - base;
         S.arriveAt[tid] = at;
         S.arriveDst[S.arriveEv[tid]] = at - lower_count(S.leave, nl, at) + tid;
@@ -160,13 +165,13 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
     fix_load<TYPED>(B, d, S, base, cell0, from, end, nl, na, now);
     // first slots (beside the loads): one more for every arrival in a lower
     // cell, one fewer for every leaver of one
-    const uint32_t rows = 1u << (B.shift - B.log2gx), row0 = cell0 >> B.log2gx;
+    const uint32_t rows = geo.cells >> geo.log2gx;
     for (uint32_t r = 0; r < rows; ++r)
-        for (uint32_t x = tid; x <= B.gx; x += kFixThreads) {
-            const uint32_t c = r * B.gx + x;
+        for (uint32_t x = tid; x <= gx; x += kFixThreads) {
+            const uint32_t c = r * gx + x;
             const uint32_t up = lower_count(S.arrive, na, 2u * c);
             const uint32_t down = lower_count(S.leaveCell, nl, c);
-            if (up != down) B.first[(size_t)(row0 + r) * (B.gx + 1u) + x] += up - down;
+            if (up != down) B.first[geo.first + r * (gx + 1u) + x] += up - down;
         }
     for (uint32_t run = from; run < end; run += kFixRun) {
         fix_load<TYPED>(B, d, S, base, cell0, run + kFixRun, end, nl, na, next);
@@ -174,6 +179,7 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
 #pragma unroll
         for (int u = 0; u < kFixItems; ++u) {
             const Held<TYPED>& h = now[u];
+            if (h.dst != kBandEmpty && B.slotSpec) B.slotSpec[base + h.dst] = geo.spec;
             if (h.dst != kBandEmpty)
                 put<TYPED>(B, d, base + h.dst, h.p, h.v, h.th, h.om, h.r, h.m, h.id, h.type, h.key,
                            h.cand);
@@ -182,6 +188,7 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
         for (int u = 0; u < kFixItems; ++u) now[u] = next[u];
     }
     __syncthreads();
+    if (enters && B.slotSpec) B.slotSpec[base + S.arriveDst[tid]] = geo.spec;
     if (enters)
         put<TYPED>(B, d, base + S.arriveDst[tid], make_float2(e.b.x, e.b.y),
                    make_float2(e.b.z, e.b.w), e.c.x, e.c.y, e.c.z, e.c.w, e.a.w, e.d.x, e.a.y,
@@ -215,10 +222,11 @@ band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynS
         __syncthreads();
     }
     // how far pairs may have approached since their bands searched, by the
-    // blocks from the last on (the first ones have the events)
+    // blocks from the last on (the first ones have the events).  Rows across a
+    // grid's wrap are out of reach, so the bands beside a band are enough.
     for (uint32_t b = (gridDim.x - 1u - blockIdx.x) * kFixThreads + threadIdx.x; b < B.bands;
          b += gridDim.x * kFixThreads) {
-        const uint32_t lo = b ? b - 1u : B.bands - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
+        const uint32_t lo = b ? b - 1u : 0u, hi = min(b + 1u, B.bands - 1u);
         const float own = __uint_as_float(B.moved[q][b]);
         // as bits, so that a NaN is the largest
         const float any = __uint_as_float(max(B.moved[q][b], max(B.moved[q][lo], B.moved[q][hi])));
@@ -264,7 +272,9 @@ __device__ __noinline__ unsigned long long
 search_candidates(const KParams& P, uint32_t i, uint32_t key, float2 p, float r, float skin,
                   const float2* __restrict__ pos, const float* __restrict__ radius,
                   const uint32_t* __restrict__ first) {
-    if (ATTRACT && !(r > 0.0f)) return kCandNone;
+    if (!P.cull || (ATTRACT && !(r > 0.0f))) return kCandNone;
+    key -= P.cellOff;
+    first += P.firstOff;
     const int gx = (int)(key & (P.gx - 1u)), gy = (int)(key >> P.log2gx);
     int y0 = -1, y1 = 1;
     if (p.y > P.cullMargin && p.y < P.Ly - P.cullMargin && p.x > P.cullMargin &&
@@ -321,16 +331,24 @@ template <bool TYPED, bool ATTRACT, bool CULL>
 __device__ __noinline__ Pull collide_slot(const KParams& P, const BandArgs& B, const DynSet& in,
                                           uint32_t i, uint32_t key, float2 p, float2 v, float w,
                                           float r, uint32_t mat) {
+    key -= P.cellOff;
     const int2 g = make_int2((int)(key & (P.gx - 1u)), (int)(key >> P.log2gx));
+    // collide_rows counts a row's words from cellOff
+    const uint32_t* __restrict__ first = B.first + P.firstOff;
     Pull o;
     if (!CULL || !P.cull ||
         !collide_rows<TYPED, ATTRACT>(P, i, g, p, v, w, r, mat, in.pos, in.vel, in.omega,
-                                      B.stat.radius, B.stat.type, nullptr, B.first, P.gx + 1u,
-                                      o.f, o.moment, o.pr)) {
-        const RowCells cells{B.first, P.gx, P.log2gx};
-        collide_one<TYPED, ATTRACT, CULL && !ATTRACT>(P, i, g, p, v, w, r, mat, in.pos, in.vel,
-                                                      in.omega, B.stat.radius, B.stat.type,
-                                                      nullptr, cells, o.f, o.moment, o.pr);
+                                      B.stat.radius, B.stat.type, nullptr, first - P.cellOff,
+                                      P.gx + 1u, o.f, o.moment, o.pr)) {
+        const RowCells cells{first, P.gx, P.log2gx, P.cellOff};
+        if (CULL && !ATTRACT && P.cull)
+            collide_one<TYPED, ATTRACT, CULL && !ATTRACT>(P, i, g, p, v, w, r, mat, in.pos, in.vel,
+                                                          in.omega, B.stat.radius, B.stat.type,
+                                                          nullptr, cells, o.f, o.moment, o.pr);
+        else
+            collide_one<TYPED, ATTRACT, false>(P, i, g, p, v, w, r, mat, in.pos, in.vel, in.omega,
+                                               B.stat.radius, B.stat.type, nullptr, cells, o.f,
+                                               o.moment, o.pr);
     }
     return o;
 }
@@ -342,8 +360,9 @@ struct RowBase {
 };
 __device__ __forceinline__ const uint32_t* row_first(const KParams& P, const BandArgs& B,
                                                      uint32_t key, uint32_t row) {
+    key -= P.cellOff;
     const uint32_t x = key & (P.gx - 1u), y = (key >> P.log2gx) + row - 1u;
-    return B.first + (size_t)(y & (P.gy - 1u)) * (P.gx + 1u) + (x ? x - 1u : 0u);
+    return B.first + P.firstOff + (size_t)(y & (P.gy - 1u)) * (P.gx + 1u) + (x ? x - 1u : 0u);
 }
 __device__ __forceinline__ RowBase row_bases(const KParams& P, const BandArgs& B, uint32_t key,
                                              unsigned long long cand) {
@@ -359,12 +378,12 @@ __device__ __forceinline__ RowBase row_bases(const KParams& P, const BandArgs& B
 // Forces on the particles of a warp from their kept candidates `rem` (0 for a
 // lane without any), in index order, one subtotal per cell, the subtotals
 // added in cell order (an empty cell adds +0).  Every lane calls it.
-template <bool TYPED, bool ATTRACT>
+template <bool TYPED, bool ATTRACT, bool BATCH>
 __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B, const DynSet& in,
                                              Deal<ATTRACT>& S, bool wantPr,
                                              unsigned long long rem,
-                                             const RowBase& base, uint32_t key, float2 p, float2 v,
-                                             float w, float r, uint32_t mat, Pull& o) {
+                                             const RowBase& base, uint32_t key, uint32_t spec,
+                                             float2 p, float2 v, float w, float r, uint32_t mat, Pull& o) {
     constexpr unsigned kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
     Sums sum;
@@ -410,15 +429,18 @@ __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B
             total += (uint32_t)__popc(hits);
         }
         if (total == 0u) continue;
-        deal_law<TYPED, ATTRACT>(P, S, wantPr, total, mine, cells, p, v, w, r, mat, in.pos, in.vel,
-                                 in.omega, B.stat.radius, B.stat.type, nullptr, sum);
+        deal_law<TYPED, ATTRACT>(P, BATCH ? B.table : nullptr, spec, S, wantPr, total, mine, cells,
+                                 p, v, w, r, mat, in.pos, in.vel, in.omega, B.stat.radius,
+                                 B.stat.type, nullptr, sum);
     }
     o = sum.close();
 }
 
-template <bool TYPED, bool ATTRACT, bool CULL, int THREADS, int MINB>
+// BATCH: the parameters are those of the slot's specimen (P0's only choose the
+// kernel).
+template <bool TYPED, bool ATTRACT, bool CULL, bool BATCH, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
-band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ BandArgs B,
+band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ BandArgs B,
                  const __grid_constant__ DynSet in, const __grid_constant__ DynSet out, uint32_t q,
                  uint32_t everyStep) {
     __shared__ Deal<ATTRACT> deal[CULL ? THREADS / 32 : 1];
@@ -427,6 +449,8 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
     // the lanes past the last slot stand by as copies of it
     const uint32_t i = min(slot, B.slots - 1u);
     const uint32_t key = B.key[i];
+    const uint32_t spec = BATCH ? B.slotSpec[i] : 0u;
+    const KParams& P = BATCH ? B.table[spec] : P0;
     Dyn s;
     s.p = in.pos[i];
     const float r = B.stat.radius[i];
@@ -453,13 +477,15 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
     if (!__any_sync(0xffffffffu, mine)) return;
     Pull o{make_float2(0.0f, 0.0f), 0.0f, 0.0f};
     RowBase base{};
+    uint32_t b0 = 0u;  // the slot's band
     if (!mine) {
         cand = 0ull;
     } else {
+        b0 = band_of(B, key);
         // one round of loads: whether to search, and the rows of the candidates
         // kept so far
         if (CULL) base = row_bases(P, B, key, cand & kCandNone ? 0ull : cand);
-        if (CULL && ((cand & kCandNone) || B.stamp[key] == now || B.search[key >> B.shift])) {
+        if (CULL && ((cand & kCandNone) || B.stamp[key] == now || B.search[b0])) {
             cand = search_candidates<ATTRACT>(P, i, key, s.p, r, B.skin, in.pos, B.stat.radius,
                                               B.first);
             B.cand[i] = cand;
@@ -471,8 +497,8 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
         }
     }
     if (CULL)
-        collide_warp<TYPED, ATTRACT>(P, B, in, deal[threadIdx.x >> 5], store && B.pressure, cand,
-                                     base, key, s.p, s.v, s.w, r, mat, o);
+        collide_warp<TYPED, ATTRACT, BATCH>(P, B, in, deal[threadIdx.x >> 5], store && B.pressure,
+                                            cand, base, key, spec, s.p, s.v, s.w, r, mat, o);
     if (!mine) return;
     // F/m and M/I as the reference divides them; without contacts both are
     // exactly +0 (see finish_particle)
@@ -499,7 +525,6 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
         }
     }
     if (!(isfinite(s.p.x) && isfinite(s.p.y))) atomicOr(B.errFlag, 1u);
-    const uint32_t b0 = key >> B.shift;
     if (CULL) {
         // the band's largest displacement, one atomic a warp while it grows
         uint32_t far = __float_as_uint(fabsf(s.p.x - was.x) + fabsf(s.p.y - was.y)) & 0x7fffffffu;
@@ -514,7 +539,7 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
     const uint32_t nk = grid_hash(P, gn.x, gn.y);
     if (nk != key) {
         B.key[i] = nk;
-        const uint32_t b1 = nk >> B.shift;
+        const uint32_t b1 = band_of(B, nk);
         const uint32_t id = B.stat.id[i];
         BandEvent* e = push_event(B, b1, q ^ 1u);
         if (e) {
@@ -531,7 +556,7 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
         if (CULL) {
 #pragma unroll 1
             for (int k = 0; k < 18; ++k) {
-                const uint32_t c = k < 9 ? key : nk;
+                const uint32_t c = (k < 9 ? key : nk) - P.cellOff;
                 const int x = (int)(c & (P.gx - 1u)) + k % 3 - 1;
                 const int y = (int)(c >> P.log2gx) + k / 3 % 3 - 1;
                 B.stamp[cell_index(P, x, y)] = now + 1u;
@@ -543,11 +568,12 @@ band_step_kernel(const __grid_constant__ KParams P, const __grid_constant__ Band
 // --------------------------------------------------------- pack, layout
 constexpr int kPackThreads = 256;
 
-// Particles of the bands below `b` (every thread gets the sum).
-__device__ __forceinline__ uint32_t packed_base(const uint32_t* __restrict__ count, uint32_t b) {
+// Packed slot of band b's first particle: those of its scene's or specimen's
+// bands below it are counted (every thread gets the sum).
+__device__ __forceinline__ uint32_t packed_base(const BandArgs& B, uint32_t b, const BandGeo& geo) {
     __shared__ uint32_t warpSum[kPackThreads / 32];
-    uint32_t v = 0;
-    for (uint32_t k = threadIdx.x; k < b; k += kPackThreads) v += count[k];
+    uint32_t v = threadIdx.x == 0 ? geo.scenePart : 0u;
+    for (uint32_t k = geo.sceneBand + threadIdx.x; k < b; k += kPackThreads) v += B.count[k];
     v = __reduce_add_sync(0xffffffffu, v);
     if ((threadIdx.x & 31u) == 0) warpSum[threadIdx.x >> 5] = v;
     __syncthreads();
@@ -565,7 +591,7 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     if (B.ctrl[kBandLaid] == 0u) return;
     const uint32_t b = blockIdx.x;
     const uint32_t base = B.base[b], cnt = B.count[b];
-    const uint32_t to = packed_base(B.count, b);
+    const uint32_t to = packed_base(B, b, B.geo[b]);
     const bool one = B.ctrl[kBandCur] != 0u;
     const float2* __restrict__ pos = one ? B.dyn[1].pos : B.dyn[0].pos;
     const float2* __restrict__ vel = one ? B.dyn[1].vel : B.dyn[0].vel;
@@ -595,10 +621,12 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     }
 }
 
-// Packed (start, end) of cell c and first slot of the one after it, the slots
-// of its band `down` above their packed places.
-__device__ __forceinline__ uint2 packed_cell(const BandArgs& B, uint32_t c, uint32_t down) {
-    const uint32_t* f = B.first + (size_t)(c >> B.log2gx) * (B.gx + 1u) + (c & (B.gx - 1u));
+// Packed range of the band's cell c, the slots of the band `down` above their
+// packed places.
+__device__ __forceinline__ uint2 packed_cell(const BandArgs& B, const BandGeo& geo, uint32_t c,
+                                             uint32_t down) {
+    const uint32_t* f = B.first + geo.first + (c >> geo.log2gx) * ((1u << geo.log2gx) + 1u) +
+                        (c & ((1u << geo.log2gx) - 1u));
     return make_uint2(f[0] - down, f[1] - down);
 }
 
@@ -611,7 +639,8 @@ band_record_kernel(BandArgs B, DynSet d, uint32_t q, StepRec rec, size_t stride)
     const StepRec r = rec_shifted(rec, B.ctrl[kBandDone] - 1u, stride);
     const uint32_t b = blockIdx.x;
     const uint32_t base = B.base[b], cnt = B.count[b];
-    const uint32_t to = packed_base(B.count, b);
+    const BandGeo geo = B.geo[b];
+    const uint32_t to = packed_base(B, b, geo);
     const uint32_t t0 = blockIdx.y * kPackThreads + threadIdx.x, step = gridDim.y * kPackThreads;
     for (uint32_t k = t0; k < cnt; k += step) {
         const uint32_t s = base + k, i = to + k;
@@ -626,10 +655,8 @@ band_record_kernel(BandArgs B, DynSet d, uint32_t q, StepRec rec, size_t stride)
         r.acc[i] = B.acc[s];
         r.alpha[i] = B.alpha[s];
     }
-    for (uint32_t k = t0; k < (1u << B.shift); k += step) {
-        const uint32_t c = (b << B.shift) + k;
-        if (c < B.cells) r.cells[c] = packed_cell(B, c, base - to);
-    }
+    for (uint32_t c = t0; c < geo.cells; c += step)
+        r.cells[geo.cell0 + c] = packed_cell(B, geo, c, base - to);
 }
 
 // First particle of every cell in the sorted keys (lower bounds).
@@ -640,34 +667,41 @@ __global__ void band_cell_first_kernel(const uint32_t* __restrict__ keys, uint32
         first[c] = lower_count(keys, n, c);
 }
 
-// Bands' bases, counts and first slots from the packed first-particle array
-// f; empty slots' keys; counters.
-__global__ void band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
-    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t s = t0; s < B.slots; s += stride) B.key[s] = kBandEmpty;
-    for (size_t k = t0; k <= B.bands; k += stride) {
-        const uint32_t b = (uint32_t)k;
-        const uint32_t p = f[min((uint64_t)b << B.shift, (uint64_t)B.cells)];
-        B.base[b] = p + b * B.slack;
-        if (b < B.bands) {
-            const uint32_t e = f[min((uint64_t)(b + 1u) << B.shift, (uint64_t)B.cells)];
-            // e < p only after a sort whose wait gave up
-            B.count[b] = e > p ? e - p : 0u;
-            B.evCnt[b] = 0u;
-            B.moved[0][b] = B.moved[1][b] = 0u;
-            B.grown[b] = 0.0f;  // no slot keeps candidates: every one searches
-        }
+// A block per band: its base, count and first slots from the packed
+// first-particle array f; its empty slots; its counters.
+__global__ void __launch_bounds__(kPackThreads)
+band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
+    const uint32_t b = blockIdx.x, tid = threadIdx.x;
+    const BandGeo geo = B.geo[b];
+    const uint32_t p = f[geo.cell0], e = f[geo.cell0 + geo.cells];
+    const uint32_t base = min(p + b * B.slack, B.slots);
+    // e < p only after a sort whose wait gave up
+    if (tid == 0) {
+        B.base[b] = base;
+        if (b == B.bands - 1u) B.base[B.bands] = B.slots;
+        B.count[b] = e > p ? e - p : 0u;
+        B.evCnt[b] = 0u;
+        B.moved[0][b] = B.moved[1][b] = 0u;
+        B.grown[b] = 0.0f;  // no slot keeps candidates: every one searches
     }
-    const uint32_t rows = B.cells >> B.log2gx;
-    for (size_t k = t0; k < (size_t)rows * (B.gx + 1u); k += stride) {
-        const uint32_t row = (uint32_t)(k / (B.gx + 1u)), x = (uint32_t)(k - (size_t)row * (B.gx + 1u));
-        const uint32_t b = (row << B.log2gx) >> B.shift;
-        B.first[k] = f[(row << B.log2gx) + x] + b * B.slack;
+    for (uint32_t s = b * kPackThreads + tid; s < B.slots; s += B.bands * kPackThreads) {
+        B.key[s] = kBandEmpty;
+        if (B.slotSpec) B.slotSpec[s] = 0u;
+    }
+    const uint32_t gx = 1u << geo.log2gx, words = (geo.cells >> geo.log2gx) * (gx + 1u);
+    for (uint32_t k = tid; k < words; k += kPackThreads) {
+        const uint32_t row = k / (gx + 1u), x = k - row * (gx + 1u);
+        B.first[geo.first + k] = f[geo.cell0 + row * gx + x] + b * B.slack;
     }
 }
 
-// The packed particles, in sorted order, into the slots of set 0.
+__global__ void __launch_bounds__(kPackThreads) band_cell_table_kernel(BandArgs B) {
+    const BandGeo geo = B.geo[blockIdx.x];
+    for (uint32_t c = threadIdx.x; c < geo.cells; c += kPackThreads)
+        B.cellBand[geo.cell0 + c] = blockIdx.x;
+}
+
+// The packed particles, in sorted order, into the slots of the current set.
 template <bool TYPED>
 __global__ void __launch_bounds__(kPackThreads)
 band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys,
@@ -675,7 +709,6 @@ band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys
     const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
     if (i == 0u) {
         B.ctrl[kBandFull] = 0u;
-        B.ctrl[kBandCur] = 0u;
         B.ctrl[kBandLaid] = 1u;
         B.ctrl[kBandDirty] = 0u;
         B.ctrl[kBandDirty + 1u] = 0u;
@@ -683,8 +716,13 @@ band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys
     if (i >= B.n) return;
     // in range unless a wait of the sort gave up (stale words)
     const uint32_t key = min(keys[i], B.cells - 1u), src = min(from[i], B.n - 1u);
-    const uint32_t s = i + (key >> B.shift) * B.slack;
-    put<TYPED>(B, B.dyn[0], s, in.dyn.pos[src], in.dyn.vel[src], in.dyn.theta[src],
+    const uint32_t band = band_of(B, key), s = i + band * B.slack;
+    // a specimen's slots are its own: the fixes keep within a band
+    if (B.slotSpec) B.slotSpec[s] = B.geo[band].spec;
+    const bool one = B.ctrl[kBandCur] != 0u;
+    const DynSet d{one ? B.dyn[1].pos : B.dyn[0].pos, one ? B.dyn[1].vel : B.dyn[0].vel,
+                   one ? B.dyn[1].theta : B.dyn[0].theta, one ? B.dyn[1].omega : B.dyn[0].omega};
+    put<TYPED>(B, d, s, in.dyn.pos[src], in.dyn.vel[src], in.dyn.theta[src],
                in.dyn.omega[src], in.stat.radius[src], in.stat.mass[src], in.stat.id[src],
                TYPED ? in.stat.type[src] : 0u, key, kCandNone);
 }
@@ -694,12 +732,11 @@ __global__ void __launch_bounds__(kPackThreads)
 band_cells_kernel(BandArgs B, uint2* __restrict__ cells, uint32_t* __restrict__ first) {
     if (B.ctrl[kBandLaid] == 0u) return;
     const uint32_t b = blockIdx.x;
-    const uint32_t shiftDown = B.base[b] - packed_base(B.count, b);
-    const uint32_t c0 = b << B.shift;
-    for (uint32_t k = threadIdx.x; k < (1u << B.shift); k += kPackThreads) {
-        const uint32_t c = c0 + k;
-        if (c >= B.cells) break;
-        const uint2 r = packed_cell(B, c, shiftDown);
+    const BandGeo geo = B.geo[b];
+    const uint32_t shiftDown = B.base[b] - packed_base(B, b, geo);
+    for (uint32_t k = threadIdx.x; k < geo.cells; k += kPackThreads) {
+        const uint32_t c = geo.cell0 + k;
+        const uint2 r = packed_cell(B, geo, k, shiftDown);
         first[c] = r.x;
         cells[c] = r.x < r.y ? r : make_uint2(kEmptyCell, kEmptyCell);
         if (c == B.cells - 1u) first[B.cells] = r.y;
@@ -738,18 +775,33 @@ bool attracts(const KParams& P) {
 
 }  // namespace
 
-bool band_shape(uint32_t gx, uint32_t numCells, BandArgs& b) {
-    if (gx == 0 || gx > kBandMaxRow || numCells < gx) return false;
-    uint32_t per = std::max(kBandMinCells, gx);
-    while ((uint64_t)per * kBandMaxBands < numCells) per <<= 1;
-    per = std::min(per, numCells);
-    b.gx = gx;
-    b.cells = numCells;
-    b.log2gx = b.shift = 0;
-    while ((1u << b.log2gx) < gx) ++b.log2gx;
-    while ((1u << b.shift) < per) ++b.shift;
-    b.bands = (numCells + per - 1u) / per;
-    return true;
+bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, bool batch,
+                BandArgs& b, std::vector<BandGeo>& geo) {
+    geo.clear();
+    uint64_t cell = 0, first = 0, part = 0;
+    for (size_t s = 0; s < P.size(); ++s) {
+        const uint32_t gx = P[s].gx, cells = P[s].gx * P[s].gy;
+        if (gx > kBandMaxRow) return false;
+        uint32_t per = std::max(batch ? kBandBatchCells : kBandMinCells, gx);
+        while (!batch && (uint64_t)per * kBandMaxBands < cells) per <<= 1;
+        per = std::min(per, cells);  // both powers of two
+        P[s].firstOff = (uint32_t)first;
+        const uint32_t sceneBand = (uint32_t)geo.size();
+        for (uint32_t c = 0; c < cells; c += per) {
+            geo.push_back(BandGeo{(uint32_t)cell + c, per, (uint32_t)(first + (c / gx) * (gx + 1ull)),
+                                  P[s].log2gx, sceneBand, (uint32_t)part, (uint32_t)s, 0u});
+        }
+        b.shift = 0;
+        while ((1u << b.shift) < per) ++b.shift;
+        cell += cells;
+        first += (uint64_t)P[s].gy * (gx + 1ull);
+        part += count[s];
+        if (first >= (1ull << 32)) return false;
+    }
+    b.cells = (uint32_t)cell;
+    b.firstWords = (uint32_t)first;
+    b.bands = (uint32_t)geo.size();
+    return b.bands != 0;
 }
 
 uint32_t band_slack(const BandArgs& b, uint32_t n) {
@@ -762,7 +814,8 @@ size_t band_slots(const BandArgs& b, uint32_t n) {
 namespace {
 // The arrays in order: take(bytes) gives each one's address.
 template <typename Take>
-void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel, Take take) {
+void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel, bool batch,
+                 Take take) {
     const size_t S = band_slots(b, capacity) + kFilterPad;
     for (int k = 0; k < 2; ++k) {
         b.dyn[k].pos = static_cast<float2*>(take(8 * S));
@@ -776,8 +829,12 @@ void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool
     b.stat.type = typed ? static_cast<uint32_t*>(take(4 * S)) : nullptr;
     b.key = static_cast<uint32_t*>(take(4 * S));
     b.loc = static_cast<uint32_t*>(take(4ull * capacity));
-    const size_t rows = b.cells >> b.log2gx;
-    b.first = static_cast<uint32_t*>(take(4 * (rows * (b.gx + 1ull) + 4)));
+    b.first = static_cast<uint32_t*>(take(4 * (b.firstWords + 4ull)));
+    b.geo = static_cast<const BandGeo*>(take(sizeof(BandGeo) * (size_t)b.bands));
+    if (batch) {
+        b.cellBand = static_cast<uint32_t*>(take(4ull * b.cells));
+        b.slotSpec = static_cast<uint32_t*>(take(4 * S));
+    }
     b.base = static_cast<uint32_t*>(take(4ull * (b.bands + 1)));
     b.count = static_cast<uint32_t*>(take(4ull * b.bands));
     b.evCnt = static_cast<uint32_t*>(take(4ull * b.bands));
@@ -795,24 +852,30 @@ void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool
 }
 }  // namespace
 
-size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel) {
+size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel,
+                  bool batch) {
     BandArgs t = b;
     size_t total = 0;
-    band_arrays(t, capacity, typed, pressure, accel, [&](size_t bytes) -> void* {
+    band_arrays(t, capacity, typed, pressure, accel, batch, [&](size_t bytes) -> void* {
         total += al256(bytes);
         return nullptr;
     });
     return total;
 }
 
-void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure,
-                 bool accel) {
+void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure, bool accel,
+                 bool batch) {
     char* p = static_cast<char*>(base);
-    band_arrays(b, capacity, typed, pressure, accel, [&](size_t bytes) -> void* {
+    band_arrays(b, capacity, typed, pressure, accel, batch, [&](size_t bytes) -> void* {
         char* q = p;
         p += al256(bytes);
         return q;
     });
+}
+
+cudaError_t launch_band_cell_table(const BandArgs& b, cudaStream_t st) {
+    band_cell_table_kernel<<<b.bands, kPackThreads, 0, st>>>(b);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st) {
@@ -828,12 +891,20 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
                              int variant, cudaStream_t st) {
     if (variant < 0 || variant >= kStepVariants) return cudaErrorInvalidValue;
     const bool typed = b.stat.type != nullptr && P.nmat > 1;
-    const bool attract = attracts(P), cull = P.cull != 0u;
+    const bool attract = attracts(P), batch = b.table != nullptr;
+    const bool cull = batch || P.cull != 0u;  // a specimen without culling searches in full
     const DynSet in = b.dyn[q], out = b.dyn[q ^ 1];
     const uint32_t e = everyStep ? 1u : 0u;
-#define DEM_BAND_T(T, A, C, TH, MB)                                                          \
-    band_step_kernel<T, A, C, TH, MB><<<blocks_for(b.slots, TH), TH, 0, st>>>(P, b, in, out, \
-                                                                              (uint32_t)q, e)
+#define DEM_BAND_T(T, A, C, TH, MB)                                                            \
+    do {                                                                                       \
+        const unsigned g = blocks_for(b.slots, TH);                                            \
+        if (batch)                                                                             \
+            band_step_kernel<T, A, true, true, TH, MB><<<g, TH, 0, st>>>(P, b, in, out,        \
+                                                                         (uint32_t)q, e);      \
+        else                                                                                   \
+            band_step_kernel<T, A, C, false, TH, MB><<<g, TH, 0, st>>>(P, b, in, out,          \
+                                                                       (uint32_t)q, e);        \
+    } while (0)
 #define DEM_BAND(T, A, C)                                    \
     do {                                                     \
         switch (variant) {                                   \
@@ -843,8 +914,8 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
             default: DEM_BAND_T(T, A, C, 128, 8); break;     \
         }                                                    \
     } while (0)
-#define DEM_BAND_AC(T)                          \
-    do {                                        \
+#define DEM_BAND_AC(T)                                  \
+    do {                                                \
         if (attract && cull) DEM_BAND(T, true, true);   \
         else if (attract) DEM_BAND(T, true, false);     \
         else if (cull) DEM_BAND(T, false, true);        \
@@ -887,7 +958,7 @@ cudaError_t launch_band_layout(const BandArgs& b, const PackedState& in, const u
                                const uint32_t* from, uint32_t* cellFirst, cudaStream_t st) {
     band_cell_first_kernel<<<std::min(blocks_for((size_t)b.cells + 1, kPackThreads), 1184u),
                              kPackThreads, 0, st>>>(keys, b.n, b.cells, cellFirst);
-    band_layout_kernel<<<1184, kPackThreads, 0, st>>>(b, cellFirst);
+    band_layout_kernel<<<b.bands, kPackThreads, 0, st>>>(b, cellFirst);
     const unsigned g = blocks_for(b.n, kPackThreads);
     if (b.stat.type)
         band_spread_kernel<true><<<g, kPackThreads, 0, st>>>(b, in, keys, from);

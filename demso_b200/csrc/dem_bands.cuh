@@ -27,17 +27,21 @@
 //
 // Against the packed incremental sort (six kernels a step, 40 B moved per
 // particle in the sort phase and 88 B in the step; here two kernels, 64 B in
-// the step): a call of 20 steps of 4,194,304 disks 4,623 -> 3,911 us, of
-// 1,000,003 dense disks 1,514 -> 1,279 us, 50 steps of 65,536 1,214 -> 1,024 us,
-// 20 steps of a fast gas of 131,071 607 -> 465 us.
+// the step), with the kept candidates below: a call of 20 steps of 4,194,304
+// disks 4,651 -> 3,199 us, of 1,000,003 dense disks 1,534 -> 1,225 us, 50 steps of
+// 65,536 1,235 -> 885 us, 20 steps of a fast gas of 131,071 587 -> 410 us, of 256
+// specimens of two materials 1,278 -> 1,007 us.  A batch's specimens keep their
+// own bands, so a slot never changes specimen.
 //
-// The two dynamic sets alternate with the steps; which of them holds the state
-// is a word on the device (kBandCur), since a new layout always starts in set
-// 0.  A kernel of set q does nothing unless kBandCur is q.
+// The two dynamic sets alternate with the steps (kBandCur: the one that holds
+// the state; a new layout keeps it, so the host knows it from the step count).
+// A kernel of set q does nothing unless kBandCur is q: when a step of the loop
+// below is skipped for a new layout, the next one of its set takes its place.
 #pragma once
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "dem_kernels.cuh"
 
@@ -48,9 +52,12 @@ constexpr uint32_t kBandEmpty = 0xffffffffu;  // key of a free slot
 constexpr uint32_t kBandEvents = 128;
 // Free slots of a band: at least this, and a sixteenth of its share of n.
 constexpr uint32_t kBandMinSlack = 64;
-// Cells of a band: at least kBandMinCells and a whole row; wider rows than
-// kBandMaxRow cells take the packed path (one block rewrites a band).
-constexpr uint32_t kBandMinCells = 256, kBandMaxRow = 4096, kBandMaxBands = 4096;
+// Cells of a band: a whole row and at least kBandMinCells (a batch's, whose
+// bands do not span specimens, kBandBatchCells where a specimen has them);
+// scenes with wider rows than kBandMaxRow cells take the packed path (one block
+// rewrites a band).
+constexpr uint32_t kBandMinCells = 256, kBandBatchCells = 1024;
+constexpr uint32_t kBandMaxRow = 4096, kBandMaxBands = 4096;
 
 // Words of BandArgs::ctrl.
 constexpr uint32_t kBandLeft = 0;   // steps left of the call
@@ -87,9 +94,21 @@ struct __align__(16) BandEvent {
     uint4 d;   // type
 };
 
+// A band: its cells, its first row in the first-slot array, and the bands and
+// packed slots of its scene or specimen before it.
+struct BandGeo {
+    uint32_t cell0, cells, first, log2gx;
+    uint32_t sceneBand, scenePart, spec, pad;
+};
+
 struct BandArgs {
-    uint32_t bands = 0, shift = 0;  // band of a cell: cell >> shift
-    uint32_t gx = 0, log2gx = 0, cells = 0;
+    uint32_t bands = 0, shift = 0;  // band of a cell of a single scene: cell >> shift
+    uint32_t cells = 0, firstWords = 0;
+    const BandGeo* geo = nullptr;
+    uint32_t* cellBand = nullptr;  // batches: band of a cell
+    // batches: the specimens' parameters, the specimen of every slot
+    const KParams* table = nullptr;
+    uint32_t* slotSpec = nullptr;
     uint32_t n = 0, slots = 0, slack = 0;
     DynSet dyn[2] = {};  // slot-indexed
     StatSet stat = {};
@@ -124,15 +143,22 @@ struct PackedState {
     float* alpha;
 };
 
-// Shape of the bands of a grid (bands, shift, gx, log2gx, cells); false when
-// the grid takes the packed path.
-bool band_shape(uint32_t gx, uint32_t numCells, BandArgs& b);
+// The bands of the grids `P` (one scene, or a batch's specimens of `count`
+// particles each), with the grids' firstOff; false when a grid takes the packed
+// path.
+bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, bool batch,
+                BandArgs& b, std::vector<BandGeo>& geo);
 // Free slots per band, and slots in all, for n particles.
 uint32_t band_slack(const BandArgs& b, uint32_t n);
 size_t band_slots(const BandArgs& b, uint32_t n);
 // Bytes of the band arrays of `capacity` particles, and their addresses.
-size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel);
-void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure, bool accel);
+size_t band_bytes(const BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel,
+                  bool batch);
+void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pressure, bool accel,
+                 bool batch);
+
+// Band of every cell of a batch (once, after the arrays are made).
+cudaError_t launch_band_cell_table(const BandArgs& b, cudaStream_t st);
 
 // The kernels; `q` is the dynamic set they step from.
 cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st);

@@ -23,11 +23,13 @@ struct PackedCells {
     const uint2* __restrict__ range;
     __device__ __forceinline__ uint2 get(uint32_t h) const { return __ldg(range + h); }
 };
-// First-particle array of gx + 1 words a row, the last one the row's end.
+// First-particle array of gx + 1 words a row, the last one the row's end, of
+// the grid whose cells are numbered from cellOff.
 struct RowCells {
     const uint32_t* __restrict__ first;
-    uint32_t gx, log2gx;
+    uint32_t gx, log2gx, cellOff;
     __device__ __forceinline__ uint2 get(uint32_t h) const {
+        h -= cellOff;
         const uint32_t* __restrict__ f = first + (size_t)(h >> log2gx) * (gx + 1u) + (h & (gx - 1u));
         return make_uint2(__ldg(f), __ldg(f + 1));
     }
@@ -161,9 +163,12 @@ struct Deal {
 // k of `mine`: its candidate k; four bits of `cells` each: the cell) into its
 // sums.  The neighbours' velocity, spin and type are read through `src` where
 // the arrays are in the previous order.  The pressure, which nothing but a
-// caller reads, is summed only with `wantPr`.  Every lane calls it.
+// caller reads, is summed only with `wantPr`.  The parameters are P, or with
+// `table` those of the particle's specimen `spec` (a warp may hold particles of
+// several).  Every lane calls it.
 template <bool TYPED, bool ATTRACT>
-__device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, bool wantPr,
+__device__ __forceinline__ void deal_law(const KParams& P0, const KParams* __restrict__ table,
+                                         uint32_t spec, Deal<ATTRACT>& S, bool wantPr,
                                          uint32_t total, uint32_t mine, uint32_t cells, float2 p, float2 v,
                                          float w, float r, uint32_t mat,
                                          const float2* __restrict__ pos,
@@ -183,6 +188,7 @@ __device__ __forceinline__ void deal_law(const KParams& P, Deal<ATTRACT>& S, boo
         const float2 vA = make_float2(__shfl_sync(kAll, v.x, own), __shfl_sync(kAll, v.y, own));
         const float wA = __shfl_sync(kAll, w, own), rA = __shfl_sync(kAll, r, own);
         const uint32_t mA = TYPED ? __shfl_sync(kAll, mat, own) : 0u;
+        const KParams& P = table ? table[__shfl_sync(kAll, spec, own)] : P0;
         if (e < total) {
             const uint32_t j = S.j[code];
             const uint32_t sj = src ? __ldg(src + j) : j;

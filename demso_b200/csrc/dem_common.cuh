@@ -53,6 +53,8 @@ struct KParams {
     uint32_t cellOff;
     uint32_t log2gx;
     uint32_t cull;
+    // The specimen's first word in the bands' first-slot array (dem_bands.cuh).
+    uint32_t firstOff;
     // Row window: the context's cell rows are the scene's rows rowOff,
     // rowOff + 1, ... (gy of them, wrapping); gyf, Ly, cellH and invLy stay
     // the whole scene's, so positions give the scene's rows bit for bit.

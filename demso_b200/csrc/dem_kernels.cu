@@ -103,7 +103,7 @@ collide_kernel(const __grid_constant__ KParams P, const float2* __restrict__ pos
     Sums sum;
     uint32_t held = 0u, cells = 0u, total = 0u;  // candidates of the turn
     auto flush = [&]() {
-        deal_law<TYPED, ATTRACT>(P, S, pressure != nullptr, total, (1u << held) - 1u, cells, p, v, w, r, mat, pos, vel,
+        deal_law<TYPED, ATTRACT>(P, nullptr, 0u, S, pressure != nullptr, total, (1u << held) - 1u, cells, p, v, w, r, mat, pos, vel,
                                  omega, radius, type, nullptr, sum);
         held = cells = total = 0u;
     };

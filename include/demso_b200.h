@@ -180,11 +180,11 @@ typedef struct DemContext DemContext;
                                  (dem_get_step_variant) */
 #define DEM_CTX_CALLER_STATE 16u /* allocate no particle state: the caller's buffers
                                     are handed over by dem_adopt_state */
-#define DEM_CTX_RESIDENT 32u  /* run each dem_step call as one launch that keeps the
-                                 particles in shared memory: batches as bins of
-                                 specimens, one per multiprocessor (see
-                                 dem_batch_create); single scenes of up to 8,192 disks
-                                 as one thread-block cluster (see dem_step) */
+#define DEM_CTX_RESIDENT 32u  /* run a dem_step call as one launch that keeps the
+                                 particles in shared memory where that is the faster
+                                 form: batches as bins of specimens, one per
+                                 multiprocessor (see dem_batch_create); small single
+                                 scenes as one thread-block cluster (see dem_step) */
 
 int dem_create(const DemSystem* sys, uint32_t capacity, uint32_t flags, DemContext** out);
 /* A context over the cell rows [rowFirst, rowFirst + rowCount) of sys's grid
@@ -231,8 +231,9 @@ int dem_set_state(DemContext* ctx, uint32_t n, const float* pos, const float* ve
  * as it would alone.  No counterpart in the reference (one scene per
  * process).
  *
- * With DEM_CTX_RESIDENT in `flags`, a dem_step call on the batch is one
- * persistent kernel launch: the specimens are packed into bins of at most
+ * With DEM_CTX_RESIDENT in `flags`, a dem_step call of two or more steps on a
+ * batch of about one bin per multiprocessor is one persistent kernel launch
+ * (other batches step faster on the graph path): the specimens are packed into bins of at most
  * 8,192 particles, 8,192 cells and 64 specimens, and each thread block (one
  * per multiprocessor) takes bins from a queue and runs all the call's steps
  * of a bin inside its shared memory (positions, velocities, spins and radii;
@@ -321,8 +322,8 @@ int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
  * that completes the 24th waits for `stream` once and keeps the shape with
  * the smallest median time.  Every shape computes the same bits, so the
  * trajectory does not depend on the choice.
- * A single scene created with DEM_CTX_RESIDENT, of at most 8,192 disks and
- * 8,192 cells, one material, no attraction and no control particle, steps
+ * A single scene created with DEM_CTX_RESIDENT, of at most 1,536 disks (larger
+ * ones step faster on the graph path) and 8,192 cells, one material, no attraction and no control particle, steps
  * each call as ONE launch of a thread-block cluster of 8 blocks: every block
  * keeps the whole scene's positions, velocities, spins and radii in its
  * shared memory, steps an eighth of the disks and writes their new state
@@ -385,8 +386,8 @@ int dem_debug_sort_hold(DemContext* ctx, uint32_t holdTile, uint32_t spinLimit);
 int dem_row_slots(DemContext* ctx, uint32_t rowLo, uint32_t rowHi, uint32_t* first,
                   uint32_t* count, void* stream);
 
-/* Number of kernels one dem_step(ctx, 1, ...) launches (library kernels
- * only; the cellStart memset is not counted). */
+/* Number of library kernels of one step of a multi-step dem_step call (the
+ * kernels of the step loop itself and those of a call's end are not counted). */
 int dem_kernels_per_step(DemContext* ctx);
 
 /* Followed-particle rows, the reference's per-step output (writeOutputFile,
