@@ -1411,12 +1411,12 @@ extern "C" int dem_get_state(DemContext* c, float* pos, float* vel, float* theta
 namespace {
 
 // ------------------------------------------------------------ step in bands
-// Own buffers, no control particle.  The arrays are allocated at
+// The context's own buffers.  The arrays are allocated at
 // the first state a context takes (about 100 B per particle and 8 KB per
 // band, of its capacity); a context whose GPU has no room for them steps on
 // the packed path.
 bool steps_in_bands(DemContext* c) {
-    if (c->band.bands == 0 || c->ctlOn || c->dyn[0].pos != c->ownPos) return false;
+    if (c->band.bands == 0 || c->dyn[0].pos != c->ownPos) return false;
     if (c->bandBlock) return true;
     const bool pressure = c->flags & DEM_CTX_PRESSURE, accel = c->flags & DEM_CTX_ACCEL;
     const size_t bytes = band_bytes(c->band, c->capacity, c->typed, pressure, accel, c->nspec != 0);
@@ -1488,6 +1488,23 @@ cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
 constexpr int kBandPairs = 2;
 constexpr uint32_t kSkipDisks = 1u << 20;
 
+// The step of set q after its fix, with the control particle's kernels where
+// there is one.
+cudaError_t enqueue_band_step(DemContext* c, int q, bool everyStep, int variant, cudaStream_t st) {
+    ControlArgs ctl{};
+    cudaError_t e = cudaSuccess;
+    if (c->ctlOn) {
+        ctl = ControlArgs{c->dCtl, c->ctlVec, c->ctlVec + c->capacity,
+                          c->ctlVec + 2ull * c->capacity};
+        e = launch_band_gaps(c->band, st);
+    }
+    if (e == cudaSuccess) e = launch_band_step(c->P, c->band, q, everyStep, variant, ctl, st);
+    if (e == cudaSuccess && c->ctlOn)
+        e = launch_control_post(ctl, c->dCtl, c->n, c->ctlPartials, c->ctlOut, st, nullptr,
+                                c->band.ctrl + kBandAct + q);
+    return e;
+}
+
 // What follows every step of a call: nothing, its followed rows, its record for
 // the adjoint.
 enum class BandAfter { kNothing, kFollowed, kRecord };
@@ -1498,7 +1515,7 @@ cudaError_t enqueue_band_pairs(DemContext* c, BandAfter after, cudaStream_t st) 
         const int q = c->bandSet ^ (k & 1);
         e = launch_band_fix(c->band, q, st);
         if (e == cudaSuccess)
-            e = launch_band_step(c->P, c->band, q, after != BandAfter::kNothing, c->variant, st);
+            e = enqueue_band_step(c, q, after != BandAfter::kNothing, c->variant, st);
         if (e == cudaSuccess && after == BandAfter::kFollowed)
             e = launch_band_followed(c->band, q, c->followIds, c->loopCtl + kLoopFolCount,
                                      c->followRing, st);
@@ -1552,7 +1569,7 @@ cudaError_t enqueue_band_sort(DemContext* c, bool step, cudaStream_t st) {
         e = add_if(c, st, full, [&](cudaStream_t fb) { return enqueue_band_layout(c, fb); });
     if (e == cudaSuccess) e = launch_band_fix(c->band, c->bandSet, st);
     if (e == cudaSuccess && step)
-        e = launch_band_step(c->P, c->band, c->bandSet, false, c->variant, st);
+        e = enqueue_band_step(c, c->bandSet, false, c->variant, st);
     return e;
 }
 
@@ -1634,8 +1651,8 @@ int band_step_alone(DemContext* c, cudaStream_t st) {
         if (rc) return rc;
         DEM_TRY_CUDA(cudaEventRecord(c->tuneEv[2 * k], st), "tuner event");
     }
-    DEM_TRY_CUDA(launch_band_step(c->P, c->band, c->bandSet, false,
-                                  tune ? (int)(k % kStepVariants) : c->variant, st),
+    DEM_TRY_CUDA(enqueue_band_step(c, c->bandSet, false,
+                                   tune ? (int)(k % kStepVariants) : c->variant, st),
                  "band step");
     c->bandSet ^= 1;
     if (tune) {
@@ -2071,7 +2088,9 @@ extern "C" int dem_debug_sort_hold(DemContext* c, uint32_t holdTile, uint32_t sp
 
 extern "C" int dem_kernels_per_step(DemContext* c) {
     if (!c) return -1;
-    if (steps_in_bands(c)) return 2;  // band_fix_kernel, band_step_kernel
+    // band_fix_kernel, band_step_kernel; with a control particle the gaps, the
+    // reduction and the move too
+    if (steps_in_bands(c)) return c->ctlOn ? 5 : 2;
     if (!c->sortGraph[1][0] && c->n > 0) {
         if (build_graph(c, 1, 0) != DEM_OK) return -1;
     }

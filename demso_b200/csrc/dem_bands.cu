@@ -438,11 +438,11 @@ __device__ __forceinline__ void collide_warp(const KParams& P, const BandArgs& B
 
 // BATCH: the parameters are those of the slot's specimen (P0's only choose the
 // kernel).
-template <bool TYPED, bool ATTRACT, bool CULL, bool BATCH, int THREADS, int MINB>
+template <bool TYPED, bool ATTRACT, bool CULL, bool BATCH, bool CONTROL, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
 band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ BandArgs B,
                  const __grid_constant__ DynSet in, const __grid_constant__ DynSet out, uint32_t q,
-                 uint32_t everyStep) {
+                 uint32_t everyStep, ControlArgs ctl) {
     __shared__ Deal<ATTRACT> deal[CULL ? THREADS / 32 : 1];
     const uint32_t act = B.ctrl[kBandAct + q], now = B.ctrl[kBandNow + q];
     const uint32_t slot = blockIdx.x * THREADS + threadIdx.x;
@@ -500,6 +500,9 @@ band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ Ban
         collide_warp<TYPED, ATTRACT, BATCH>(P, B, in, deal[threadIdx.x >> 5], store && B.pressure,
                                             cand, base, key, spec, s.p, s.v, s.w, r, mat, o);
     if (!mine) return;
+    if (CONTROL)
+        meet_control<TYPED, ATTRACT>(P, ctl, i - B.gap[b0], s.p, s.v, s.w, r, mat, o.f, o.moment,
+                                     o.pr);
     // F/m and M/I as the reference divides them; without contacts both are
     // exactly +0 (see finish_particle)
     const bool quiet =
@@ -567,6 +570,34 @@ band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ Ban
 
 // --------------------------------------------------------- pack, layout
 constexpr int kPackThreads = 256;
+
+// One block: base less the running count of every band.
+constexpr int kGapThreads = 1024;
+__global__ void __launch_bounds__(kGapThreads) band_gap_kernel(BandArgs B) {
+    __shared__ uint32_t warpTot[kGapThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t carry = 0u;
+    for (uint32_t b0 = 0; b0 < B.bands; b0 += kGapThreads) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint32_t v = b < B.bands ? B.count[b] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (lane == 31u) warpTot[warp] = x;
+        __syncthreads();
+        uint32_t below = carry, all = 0u;
+        for (uint32_t k = 0; k < (uint32_t)kGapThreads / 32u; ++k) {
+            if (k < warp) below += warpTot[k];
+            all += warpTot[k];
+        }
+        if (b < B.bands) B.gap[b] = B.base[b] - (below + x - v);
+        carry += all;
+        __syncthreads();
+    }
+}
 
 // Packed slot of band b's first particle: those of its scene's or specimen's
 // bands below it are counted (every thread gets the sum).
@@ -837,6 +868,7 @@ void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool
     }
     b.base = static_cast<uint32_t*>(take(4ull * (b.bands + 1)));
     b.count = static_cast<uint32_t*>(take(4ull * b.bands));
+    b.gap = static_cast<uint32_t*>(take(4ull * b.bands));
     b.evCnt = static_cast<uint32_t*>(take(4ull * b.bands));
     b.ev = static_cast<BandEvent*>(take(sizeof(BandEvent) * (size_t)b.bands * kBandEvents));
     for (int k = 0; k < 2; ++k) b.dirty[k] = static_cast<uint32_t*>(take(4ull * b.bands));
@@ -887,8 +919,13 @@ cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+cudaError_t launch_band_gaps(const BandArgs& b, cudaStream_t st) {
+    band_gap_kernel<<<1, kGapThreads, 0, st>>>(b);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool everyStep,
-                             int variant, cudaStream_t st) {
+                             int variant, ControlArgs ctl, cudaStream_t st) {
     if (variant < 0 || variant >= kStepVariants) return cudaErrorInvalidValue;
     const bool typed = b.stat.type != nullptr && P.nmat > 1;
     const bool attract = attracts(P), batch = b.table != nullptr;
@@ -899,11 +936,14 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
     do {                                                                                       \
         const unsigned g = blocks_for(b.slots, TH);                                            \
         if (batch)                                                                             \
-            band_step_kernel<T, A, true, true, TH, MB><<<g, TH, 0, st>>>(P, b, in, out,        \
-                                                                         (uint32_t)q, e);      \
+            band_step_kernel<T, A, true, true, false, TH, MB><<<g, TH, 0, st>>>(               \
+                P, b, in, out, (uint32_t)q, e, ctl);                                           \
+        else if (ctl.c)                                                                        \
+            band_step_kernel<T, A, C, false, true, 128, 8>                                     \
+                <<<blocks_for(b.slots, 128), 128, 0, st>>>(P, b, in, out, (uint32_t)q, e, ctl); \
         else                                                                                   \
-            band_step_kernel<T, A, C, false, TH, MB><<<g, TH, 0, st>>>(P, b, in, out,          \
-                                                                       (uint32_t)q, e);        \
+            band_step_kernel<T, A, C, false, false, TH, MB><<<g, TH, 0, st>>>(                 \
+                P, b, in, out, (uint32_t)q, e, ctl);                                           \
     } while (0)
 #define DEM_BAND(T, A, C)                                    \
     do {                                                     \

@@ -117,6 +117,7 @@ struct BandArgs {
     uint32_t* first = nullptr;  // first slot of every cell, gx + 1 words a row (the last: row end)
     uint32_t* base = nullptr;   // bands + 1
     uint32_t* count = nullptr;  // particles of each band
+    uint32_t* gap = nullptr;    // slots less packed places of each band (launch_band_gaps)
     uint32_t* evCnt = nullptr;
     BandEvent* ev = nullptr;
     uint32_t* dirty[2] = {};
@@ -165,7 +166,10 @@ cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st);
 // everyStep: pressure and accelerations are stored on every step, not only on
 // the call's last one.
 cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool everyStep,
-                             int variant, cudaStream_t st);
+                             int variant, ControlArgs ctl, cudaStream_t st);
+// Before a step with a control particle, whose reactions are stored in packed
+// order: the bands' gaps.
+cudaError_t launch_band_gaps(const BandArgs& b, cudaStream_t st);
 cudaError_t launch_band_followed(const BandArgs& b, int q, const uint32_t* ids,
                                  const uint32_t* countWord, float* ring, cudaStream_t st);
 // The record of the step of set q (adj_record_step's, packed) at record block

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "dem_common.cuh"
+#include "dem_kernels.cuh"
 
 namespace dem {
 
@@ -357,6 +358,30 @@ __device__ __forceinline__ void collide_one(const KParams& P, uint32_t i, int2 g
             force.y += fc.y;
         }
     }
+}
+
+// particles_kernel.cuh:520-541: the contact (and attraction) with the control
+// particle after the 3x3 cells; its force is added once, the reaction is stored
+// (at `at`, the particle's place in sorted order) for the reduction.
+template <bool TYPED, bool ATTRACT>
+__device__ __forceinline__ void meet_control(const KParams& P, const ControlArgs& ctl, uint32_t at,
+                                             float2 p, float2 v, float w, float r, uint32_t mat,
+                                             float2& f, float& moment, float& pr) {
+    const ControlDev c = *ctl.c;
+    const float4 pc = TYPED ? P.pair[mat * P.nmat + c.mat] : P.pair[0];
+    float mc = 0.0f;
+    float2 fc = pair_force(p, c.pos, v, c.vel, w, c.omega, r, c.radius, pc, P.dt, mc, pr);
+    if (ATTRACT) {
+        const float2 fa = pair_attract(p, c.pos, r, c.radius, P.at[mat], P.at[c.mat], pr);
+        fc.x += fa.x;
+        fc.y += fa.y;
+    }
+    f.x += fc.x;
+    f.y += fc.y;
+    moment += mc;
+    ctl.fx[at] = -fc.x;
+    ctl.fy[at] = -fc.y;
+    ctl.fm[at] = -mc / r * c.radius;
 }
 
 // Row-interval form of collide_one for the context step (no attraction, no

@@ -322,27 +322,8 @@ __device__ __forceinline__ void step_particle(const KParams& P, uint32_t i, DynS
                                                in.omega, inS.radius, inS.type, src,
                                                PackedCells{cellRange}, f, moment, pr);
     }
-    if (CONTROL) {
-        // particles_kernel.cuh:520-541: the contact (and attraction) with the
-        // control particle after the 3x3 cells; its force is added once, the
-        // reaction is stored for the reduction
-        const ControlDev c = *ctl.c;
-        const float4 pc = TYPED ? P.pair[mat * P.nmat + c.mat] : P.pair[0];
-        float mc = 0.0f;
-        float2 fc = pair_force(s.p, c.pos, s.v, c.vel, s.w, c.omega, r, c.radius, pc, P.dt, mc,
-                               pr);
-        if (ATTRACT) {
-            const float2 fa = pair_attract(s.p, c.pos, r, c.radius, P.at[mat], P.at[c.mat], pr);
-            fc.x += fa.x;
-            fc.y += fa.y;
-        }
-        f.x += fc.x;
-        f.y += fc.y;
-        moment += mc;
-        ctl.fx[i] = -fc.x;
-        ctl.fy[i] = -fc.y;
-        ctl.fm[i] = -mc / r * c.radius;
-    }
+    if (CONTROL)
+        meet_control<TYPED, ATTRACT>(P, ctl, i, s.p, s.v, s.w, r, mat, f, moment, pr);
     finish_particle<TYPED>(P, i, s, f, moment, pr, r, m, mat, id, key, cellRange, out, outS, loc,
                            nextHash, pressure, acc, alpha, errFlag, sink);
 }
@@ -370,7 +351,9 @@ step_kernel(KParams P, DynSet in, StatSet inS, const uint32_t* __restrict__ src,
 // min(512, n) threads, a shared-memory tree that halves the block size.
 constexpr int kControlThreads = 512;
 __global__ void __launch_bounds__(kControlThreads)
-control_reduce_kernel(ControlArgs ctl, uint32_t n, float* __restrict__ partials) {
+control_reduce_kernel(ControlArgs ctl, uint32_t n, float* __restrict__ partials,
+                      const uint32_t* __restrict__ active) {
+    if (active && *active == 0u) return;
     __shared__ float cache[3][kControlThreads];
     const uint32_t index = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = threadIdx.x;
@@ -404,7 +387,9 @@ constexpr int kSumThreads = 256;
 constexpr uint32_t kSumTile = 1024;
 __global__ void __launch_bounds__(kSumThreads)
 control_sum_move_kernel(ControlDev* __restrict__ c, const float* __restrict__ partials,
-                        uint32_t blocks, float* __restrict__ out) {
+                        uint32_t blocks, float* __restrict__ out,
+                        const uint32_t* __restrict__ active) {
+    if (active && *active == 0u) return;
     __shared__ float tile[3][kSumTile];
     const uint32_t t = threadIdx.x, k = t >> 5;  // lane 0 of warp k < 3 adds component k
     float sum = 0.0f;
@@ -739,11 +724,12 @@ cudaError_t launch_loop_next(uint32_t* left, uint32_t* idx, int32_t idxStep,
 }
 
 cudaError_t launch_control_post(ControlArgs ctl, ControlDev* c, uint32_t n, float* partials,
-                                float* out, cudaStream_t st, int* launches) {
+                                float* out, cudaStream_t st, int* launches,
+                                const uint32_t* active) {
     const uint32_t threads = n < (uint32_t)kControlThreads ? (n ? n : 1u) : (uint32_t)kControlThreads;
     const uint32_t blocks = n ? (n + threads - 1) / threads : 0u;
-    if (blocks) control_reduce_kernel<<<blocks, threads, 0, st>>>(ctl, n, partials);
-    control_sum_move_kernel<<<1, kSumThreads, 0, st>>>(c, partials, blocks, out);
+    if (blocks) control_reduce_kernel<<<blocks, threads, 0, st>>>(ctl, n, partials, active);
+    control_sum_move_kernel<<<1, kSumThreads, 0, st>>>(c, partials, blocks, out, active);
     if (launches) *launches += blocks ? 2 : 1;
     return cudaGetLastError();
 }

@@ -148,9 +148,11 @@ struct StepShape {
 StepShape step_variant_shape(int variant);
 // After the step kernel: the reaction sums (reduceVecD's blocks, then their
 // sum in block order: out[0..2] = force x, force y, moment) and the control
-// particle's move.  partials: 3 * ceil(n / min(512, n)) floats.
+// particle's move.  partials: 3 * ceil(n / min(512, n)) floats.  With `active`,
+// nothing happens while that word is zero.
 cudaError_t launch_control_post(ControlArgs ctl, ControlDev* c, uint32_t n, float* partials,
-                                float* out, cudaStream_t st, int* launches);
+                                float* out, cudaStream_t st, int* launches,
+                                const uint32_t* active = nullptr);
 
 // Reorder with interleaved (start, end) cell ranges; resets the ranges first.
 cudaError_t launch_reorder_packed(uint2* cellRange, DynSet sorted, StatSet sortedS,
