@@ -1225,8 +1225,9 @@ bool has_state_sets(const DemContext* c) { return c->dyn[0].pos != nullptr; }
 bool steps_in_bands(DemContext* c);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
-    // the band arrays, unless a resident launch may step this scene or batch
-    if (!(c->flags & DEM_CTX_RESIDENT) || (!c->nspec && !cluster_scene_fits(n, c->numCells)))
+    // the band arrays, unless the cluster launch will step this scene
+    if (!(c->flags & DEM_CTX_RESIDENT) || c->nspec || n > kClusterBandDisks ||
+        !cluster_scene_fits(n, c->numCells))
         steps_in_bands(c);
     // the new state replaces the one any recorded error was about
     DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 4, st), "clear error word");
@@ -1439,13 +1440,14 @@ bool steps_in_bands(DemContext* c) {
 // path (one step: 79 against 115 us at 1,000,003 disks, 232 against 263 at
 // 4,194,304; five steps: 385 against 373, 1,151 against 896); longer ones leave
 // the packed path once they have made enough steps to earn the sort, and
-// kShortRun short calls in a row leave the bands.
-constexpr uint32_t kShortCall = 4, kPackedSteps = 16, kShortRun = 16;
+// kShortRun short calls in a row leave the bands.  A batch gains more by a step
+// in bands (63 against 42 us, 256 specimens of two materials): three steps do.
+constexpr uint32_t kShortCall = 4, kShortBatchCall = 3, kPackedSteps = 16, kShortRun = 16;
 bool band_call(DemContext* c, uint32_t nsteps) {
     if (!steps_in_bands(c)) return false;
     if (c->profiling || c->tuned < 0) return true;  // the bands' kernels are what is timed
     const bool packedOrder = c->keysValid && c->haveOrder;
-    if (nsteps >= kShortCall) {
+    if (nsteps >= (c->nspec ? kShortBatchCall : kShortCall)) {
         c->shortCalls = 0;
         c->packedSteps += std::min(nsteps, kPackedSteps);
         if (!c->bandValid && packedOrder && c->packedSteps < kPackedSteps) return false;
@@ -1782,28 +1784,18 @@ bool has_attraction_host(const KParams& P);
 
 constexpr int kNotResident = -1;
 
-// The resident launch steps a bin per multiprocessor at a time, whatever else
-// the GPU could do; the bands share all of it.  The launch is faster only with
-// about one bin for every multiprocessor, over enough steps to load and store
-// the bins: per step, resident against bands, 512 specimens (144 bins) 60.5 / 66
-// us, 4,096 (1,145 bins) 405 / 380, 32 (9 bins) 58 / 20; calls of one, three and
-// five steps of the 512, 155, 266 and 383 against 104, 317 and 421.
-constexpr uint32_t kResidentSteps = 2;
-bool resident_bins_fill(const DemContext* c) {
-    int sms = 148;
-    (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    return 8u * c->resBins >= 7u * (uint32_t)sms && c->resBins <= (uint32_t)sms;
-}
-
 // A multi-step call of a batch created with DEM_CTX_RESIDENT as one
 // persistent launch (dem_resident.cu).  Returns kNotResident, having done
-// nothing, when the batch has types, attraction, a control particle, stage
+// nothing, when the batch steps in bands -- faster for every batch measured:
+// per step, resident against bands, 512 specimens (1.17 M disks) 60.5 / 59 us,
+// 4,096 405 / 380, 32 58 / 20, 300 of 16 to 40 disks 16.3 / 11.0, 4 of 300
+// 10.6 / 7.9 -- or has types, attraction, a control particle, stage
 // profiling or a specimen too large for one bin: the graph path steps it.
 // After the launch the state is in the order of its last sort, as after the
 // graph path, but no mover record exists: the next graph-path step sorts
 // from scratch (the same permutation, the sort being stable).
 int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) || nsteps < kResidentSteps ||
+    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) || steps_in_bands(c) ||
         c->partOff.size() != (size_t)c->nspec + 1 || c->partOff.back() != c->n)
         return kNotResident;
     for (uint32_t s = 0; s < c->nspec; ++s)
@@ -1838,7 +1830,7 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
         c->resMaxC = maxC;
         c->resBlocks = blocks;
     }
-    if (c->resBins == 0 || !resident_bins_fill(c)) return kNotResident;
+    if (c->resBins == 0) return kNotResident;
     const int a = c->cur;
     ResIO io{c->dyn[0].pos, c->dyn[a].vel, c->dyn[a].theta, c->dyn[a].omega, c->stat[a].radius,
              c->stat[a].mass, c->stat[a].id, c->loc, c->pressure, c->acc, c->alpha};
@@ -1854,14 +1846,15 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
 // A multi-step call of a single scene created with DEM_CTX_RESIDENT as one
 // cluster launch (dem_resident.cu): every block of the cluster holds the
 // whole scene in shared memory and steps its share of the slots.  Returns
-// kNotResident, having done nothing, for scenes it does not take (more than
-// 1,536 disks or 8,192 cells, types, attraction, a control particle, profiling) or
+// kNotResident, having done nothing, for scenes that step faster in bands
+// (kClusterBandDisks) and those it does not take (more than 8,192 disks or cells, types, attraction, a control particle, profiling) or
 // when no such cluster can be resident on this GPU; the graph path steps
 // those.  The next graph-path step sorts from scratch.
 int cluster_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (c->typed || c->ctlOn || c->profiling || c->clusterUnsupported || c->rows ||
         !has_state_sets(c) ||
-        has_attraction_host(c->P) || !cluster_scene_fits(c->n, c->numCells))
+        has_attraction_host(c->P) || !cluster_scene_fits(c->n, c->numCells) ||
+        (c->n > kClusterBandDisks && steps_in_bands(c)))
         return kNotResident;
     const size_t bytes = cluster_scene_work_bytes(c->n);
     if (c->clusterWorkBytes < bytes) {

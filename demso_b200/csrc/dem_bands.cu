@@ -165,14 +165,13 @@ __device__ void fix_band(const BandArgs& B, const DynSet& d, FixShared& S, uint3
     fix_load<TYPED>(B, d, S, base, cell0, from, end, nl, na, now);
     // first slots (beside the loads): one more for every arrival in a lower
     // cell, one fewer for every leaver of one
-    const uint32_t rows = geo.cells >> geo.log2gx;
-    for (uint32_t r = 0; r < rows; ++r)
-        for (uint32_t x = tid; x <= gx; x += kFixThreads) {
-            const uint32_t c = r * gx + x;
-            const uint32_t up = lower_count(S.arrive, na, 2u * c);
-            const uint32_t down = lower_count(S.leaveCell, nl, c);
-            if (up != down) B.first[geo.first + r * (gx + 1u) + x] += up - down;
-        }
+    const uint32_t words = (geo.cells >> geo.log2gx) * (gx + 1u);
+    for (uint32_t k = tid; k < words; k += kFixThreads) {
+        const uint32_t row = k / (gx + 1u), c = k - row;  // row * gx + column
+        const uint32_t up = lower_count(S.arrive, na, 2u * c);
+        const uint32_t down = lower_count(S.leaveCell, nl, c);
+        if (up != down) B.first[geo.first + k] += up - down;
+    }
     for (uint32_t run = from; run < end; run += kFixRun) {
         fix_load<TYPED>(B, d, S, base, cell0, run + kFixRun, end, nl, na, next);
         __syncthreads();  // this run and the next are read

@@ -26,7 +26,7 @@
 // written only by the particle's own thread and live in the block's global
 // scratch, which stays in L2.
 //
-// The same file steps a single scene of up to kClusterMaxDisks disks as one
+// The same file steps a single scene of up to kResMaxParticles disks as one
 // thread-block cluster (cluster_kernel, below): every block holds the whole
 // scene, steps its share of the slots and broadcasts their new state to the
 // other blocks through distributed shared memory.
@@ -666,7 +666,7 @@ resident_kernel(const KParams* __restrict__ table, const ResBin* __restrict__ bi
 
 // ---------------------------------------------------------------------------
 // One scene across a thread-block cluster (DEM_CTX_RESIDENT on a single
-// scene of at most kClusterMaxDisks disks and kResMaxCells cells): the
+// scene of at most kResMaxParticles disks and kResMaxCells cells): the
 // cluster's kClusterCtas blocks, one per multiprocessor, each hold a full
 // copy of the scene's positions, velocities, spins and radii in shared
 // memory, and each steps its own share of the slots.  A step is
@@ -688,13 +688,6 @@ resident_kernel(const KParams* __restrict__ table, const ResBin* __restrict__ bi
 // read through L2 (__ldcg).
 
 constexpr int kClusterCtas = 8;  // blocks of a cluster (the portable size; 16 measured slower)
-
-// Larger scenes step faster in bands, where the whole GPU shares the law and the
-// sort: per step of 400-step calls, cluster against bands, 500 disks 6.3 / 6.4
-// us, 1,500 6.3 / 6.5, 2,000 fast ones 11.2 / 9.7, 4,096 in a dense packing
-// 11.2 / 8.4, 8,000 16.1 / 9.3; calls of one to five steps of 500 disks 25-49
-// against 25-104 us.
-constexpr uint32_t kClusterMaxDisks = 1536;
 
 // Global scratch of one cluster: angles, masses, ids (two sets), the cell of
 // every slot, the incremental sort's stash of those four, two mover counters
@@ -1074,7 +1067,7 @@ cudaError_t launch_resident(const KParams* table, const ResBin* bins, uint32_t n
 size_t cluster_scene_work_bytes(uint32_t n) { return cluster_work_bytes(n); }
 
 bool cluster_scene_fits(uint32_t n, uint32_t cells) {
-    return n >= 1u && n <= kClusterMaxDisks && cells <= kResMaxCells;
+    return n >= 1u && n <= kResMaxParticles && cells <= kResMaxCells;
 }
 
 cudaError_t launch_cluster_scene(const KParams& P, uint32_t n, uint32_t cells, void* work,
@@ -1109,8 +1102,9 @@ cudaError_t launch_cluster_scene(const KParams& P, uint32_t n, uint32_t cells, v
         return cudaLaunchKernelEx(&cfg, kernel, P, io, n, cells, static_cast<char*>(work),
                                   nsteps, errFlag);
     };
-    static_assert((kClusterMaxDisks + kClusterCtas - 1) / kClusterCtas <= 512, "a slot per thread");
-    return launch(cluster_kernel<512>, 512, kClusterCtas);
+    const uint32_t share = (n + (uint32_t)kClusterCtas - 1u) / (uint32_t)kClusterCtas;
+    return share <= 512u ? launch(cluster_kernel<512>, 512, kClusterCtas)
+                         : launch(cluster_kernel<1024>, 1024, kClusterCtas);
 }
 
 }  // namespace dem

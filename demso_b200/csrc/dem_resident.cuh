@@ -77,6 +77,13 @@ cudaError_t launch_resident(const KParams* table, const ResBin* bins, uint32_t n
 // most kResMaxParticles disks and kResMaxCells cells; `work` is
 // cluster_scene_work_bytes(n) bytes of device memory.  Returns
 // cudaErrorNotSupported when no cluster of this shape can be resident.
+//
+// Scenes of more than kClusterBandDisks disks step faster in bands
+// (dem_bands.cuh), where the whole GPU shares the law and the sort: per step of
+// 400-step calls, cluster against bands, 500 disks 6.3 / 6.4 us, 1,500 6.3 / 6.5,
+// 2,000 fast ones 11.2 / 9.7, 4,096 in a dense packing 11.2 / 8.4, 8,000
+// 16.1 / 9.3; calls of one to five steps of 500 disks 25-49 against 25-72 us.
+constexpr uint32_t kClusterBandDisks = 1536;
 bool cluster_scene_fits(uint32_t n, uint32_t cells);
 size_t cluster_scene_work_bytes(uint32_t n);
 cudaError_t launch_cluster_scene(const KParams& P, uint32_t n, uint32_t cells, void* work,

@@ -182,9 +182,10 @@ typedef struct DemContext DemContext;
                                     are handed over by dem_adopt_state */
 #define DEM_CTX_RESIDENT 32u  /* run a dem_step call as one launch that keeps the
                                  particles in shared memory where that is the faster
-                                 form: batches as bins of specimens, one per
-                                 multiprocessor (see dem_batch_create); small single
-                                 scenes as one thread-block cluster (see dem_step) */
+                                 form: small single scenes as one thread-block
+                                 cluster (see dem_step), batches in a caller's
+                                 buffers as bins of specimens, one per multiprocessor
+                                 (see dem_batch_create) */
 
 int dem_create(const DemSystem* sys, uint32_t capacity, uint32_t flags, DemContext** out);
 /* A context over the cell rows [rowFirst, rowFirst + rowCount) of sys's grid
@@ -231,9 +232,9 @@ int dem_set_state(DemContext* ctx, uint32_t n, const float* pos, const float* ve
  * as it would alone.  No counterpart in the reference (one scene per
  * process).
  *
- * With DEM_CTX_RESIDENT in `flags`, a dem_step call of two or more steps on a
- * batch of about one bin per multiprocessor is one persistent kernel launch
- * (other batches step faster on the graph path): the specimens are packed into bins of at most
+ * With DEM_CTX_RESIDENT in `flags`, a dem_step call on a batch that owns no
+ * state (DEM_CTX_CALLER_STATE; others step faster on the graph path) is one
+ * persistent kernel launch: the specimens are packed into bins of at most
  * 8,192 particles, 8,192 cells and 64 specimens, and each thread block (one
  * per multiprocessor) takes bins from a queue and runs all the call's steps
  * of a bin inside its shared memory (positions, velocities, spins and radii;
@@ -322,8 +323,9 @@ int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
  * that completes the 24th waits for `stream` once and keeps the shape with
  * the smallest median time.  Every shape computes the same bits, so the
  * trajectory does not depend on the choice.
- * A single scene created with DEM_CTX_RESIDENT, of at most 1,536 disks (larger
- * ones step faster on the graph path) and 8,192 cells, one material, no attraction and no control particle, steps
+ * A single scene created with DEM_CTX_RESIDENT, of at most 1,536 disks (with
+ * DEM_CTX_CALLER_STATE 8,192; larger ones step faster on the graph path) and
+ * 8,192 cells, one material, no attraction and no control particle, steps
  * each call as ONE launch of a thread-block cluster of 8 blocks: every block
  * keeps the whole scene's positions, velocities, spins and radii in its
  * shared memory, steps an eighth of the disks and writes their new state
