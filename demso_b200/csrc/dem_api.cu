@@ -305,6 +305,11 @@ extern "C" int dem_integrate_system(const DemSystem* sys, float* pos, float* vel
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
+// Steps of one pass of the band step loop: the loop is made in these lengths and
+// a call takes the one that skips the fewest steps (band_pass).
+constexpr int kBandPasses = 5;
+constexpr uint32_t kBandPassSteps[kBandPasses] = {4, 6, 8, 10, 12};
+
 struct DemContext {
     DemSystem sys;
     KParams P;
@@ -395,9 +400,9 @@ struct DemContext {
     // band_call: short calls in a row that stepped in bands; steps of longer
     // calls on the packed path since
     uint32_t shortCalls = 0, packedSteps = 0;
-    cudaGraphExec_t bandLoop[2][2] = {}, bandOne[2][2] = {}, bandFollow[2][2] = {};
-    cudaGraphExec_t bandSort[2][2] = {};
-    cudaGraphExec_t bandRec[2][2] = {};  // the loop recording every step for the adjoint
+    cudaGraphExec_t bandLoop[2][2][kBandPasses] = {}, bandFollow[2][2][kBandPasses] = {};
+    cudaGraphExec_t bandRec[2][2][kBandPasses] = {};  // recording every step for the adjoint
+    cudaGraphExec_t bandOne[2][2] = {}, bandSort[2][2] = {};
     // followed-particle staging (device), see dem_get_followed
     float* followRows = nullptr;
     // dem_step_followed: the ids (device copy), the ring of per-step rows,
@@ -496,12 +501,16 @@ void drop_tune_graphs(DemContext* c) {
         }
 }
 
+void drop_graph(cudaGraphExec_t& g) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+}
+
 void drop_adj_graphs(DemContext* c) {
     for (int p = 0; p < 2; ++p) {
-        for (cudaGraphExec_t* g : {&c->adjRecLoop[p], &c->bandRec[p][0], &c->bandRec[p][1]}) {
-            if (*g) cudaGraphExecDestroy(*g);
-            *g = nullptr;
-        }
+        drop_graph(c->adjRecLoop[p]);
+        for (int q = 0; q < 2; ++q)
+            for (int k = 0; k < kBandPasses; ++k) drop_graph(c->bandRec[p][q][k]);
     }
     if (c->adjRevLoop) cudaGraphExecDestroy(c->adjRevLoop);
     c->adjRevLoop = nullptr;
@@ -513,12 +522,14 @@ void drop_loop_graphs(DemContext* c) {
         c->loopGraph[p] = nullptr;
         if (c->followGraph[p]) cudaGraphExecDestroy(c->followGraph[p]);
         c->followGraph[p] = nullptr;
-        for (int q = 0; q < 2; ++q)
-            for (cudaGraphExec_t* g : {&c->bandLoop[p][q], &c->bandOne[p][q], &c->bandFollow[p][q],
-                                       &c->bandSort[p][q]}) {
-                if (*g) cudaGraphExecDestroy(*g);
-                *g = nullptr;
+        for (int q = 0; q < 2; ++q) {
+            drop_graph(c->bandOne[p][q]);
+            drop_graph(c->bandSort[p][q]);
+            for (int k = 0; k < kBandPasses; ++k) {
+                drop_graph(c->bandLoop[p][q][k]);
+                drop_graph(c->bandFollow[p][q][k]);
             }
+        }
     }
     drop_adj_graphs(c);
 }
@@ -1483,11 +1494,26 @@ cudaError_t enqueue_band_layout(DemContext* c, cudaStream_t st) {
 
 // The conditional nodes of the step loop, innermost last:
 //   while steps are left: { if (full) layout; while (steps left, not full)
-//                           { kBandPairs pairs of steps } }
+//                           { `pass` steps } }
 // A step the band layout cannot take (kBandFull) ends the inner loop, and
 // steps of the set that does not hold the state do nothing, so every pass of
 // the outer loop makes at least one step.
-constexpr int kBandPairs = 2;
+// A pass of the inner loop costs about 3 us, so its length is chosen for the
+// call: the one of kBandPassSteps that skips the fewest steps past the call's
+// last, the longest of those (10 steps a pass against 4: 13.7 -> 12.8 us a step
+// at 65,536 disks, 8.8 -> 8.0 at 4,096).
+int band_pass(uint32_t nsteps) {
+    int best = 0;
+    uint32_t least = 0xffffffffu;
+    for (int k = 0; k < kBandPasses; ++k) {
+        const uint32_t pass = kBandPassSteps[k], skipped = (pass - nsteps % pass) % pass;
+        if (skipped <= least) {
+            least = skipped;
+            best = k;
+        }
+    }
+    return best;
+}
 constexpr uint32_t kSkipDisks = 1u << 20;
 
 // The step of set q after its fix, with the control particle's kernels where
@@ -1511,10 +1537,10 @@ cudaError_t enqueue_band_step(DemContext* c, int q, bool everyStep, int variant,
 // the adjoint.
 enum class BandAfter { kNothing, kFollowed, kRecord };
 
-cudaError_t enqueue_band_pairs(DemContext* c, BandAfter after, cudaStream_t st) {
+cudaError_t enqueue_band_pass(DemContext* c, BandAfter after, uint32_t steps, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
-    for (int k = 0; k < 2 * kBandPairs && e == cudaSuccess; ++k) {
-        const int q = c->bandSet ^ (k & 1);
+    for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k) {
+        const int q = c->bandSet ^ (int)(k & 1u);
         e = launch_band_fix(c->band, q, st);
         if (e == cudaSuccess)
             e = enqueue_band_step(c, q, after != BandAfter::kNothing, c->variant, st);
@@ -1536,7 +1562,7 @@ cudaError_t conditional_handle(cudaStream_t st, cudaGraphConditionalHandle* h) {
     return e == cudaSuccess ? cudaGraphConditionalHandleCreate(h, g, 0, 0) : e;
 }
 
-cudaError_t enqueue_band_loop(DemContext* c, BandAfter after, cudaStream_t st) {
+cudaError_t enqueue_band_loop(DemContext* c, BandAfter after, uint32_t pass, cudaStream_t st) {
     cudaGraphConditionalHandle outer;
     cudaError_t e = conditional_handle(st, &outer);
     if (e == cudaSuccess) e = launch_band_next(c->band, outer, true, st);
@@ -1551,7 +1577,7 @@ cudaError_t enqueue_band_loop(DemContext* c, BandAfter after, cudaStream_t st) {
         if (eb == cudaSuccess)
             eb = add_conditional(ob, inner, cudaGraphCondTypeWhile, c->forkStream,
                                  [&](cudaStream_t ib) {
-                                     cudaError_t ei = enqueue_band_pairs(c, after, ib);
+                                     cudaError_t ei = enqueue_band_pass(c, after, pass, ib);
                                      return ei == cudaSuccess
                                                 ? launch_band_next(c->band, inner, false, ib)
                                                 : ei;
@@ -1687,23 +1713,25 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
     // cheaper: a step the loop skips costs its empty launches (7 us at 65,536
     // disks, 26 at 4,194,304), a graph of one step 12 us more than a step in the
     // loop.
-    const uint32_t pass = c->n >= kSkipDisks ? 2u * kBandPairs : 1u;
+    const bool whole = after == BandAfter::kNothing && c->n >= kSkipDisks;
     const int a = c->cur;
     while (done < nsteps) {
         uint32_t m = nsteps - done;
-        if (after == BandAfter::kNothing && m != 1u) m = m >= pass ? m - m % pass : 1u;
+        const int k = band_pass(m);
+        const uint32_t pass = kBandPassSteps[k];
+        if (whole) m = m >= pass ? m - m % pass : (m >= kBandPassSteps[0] ? kBandPassSteps[0] : 1u);
+        const bool one = after == BandAfter::kNothing && m == 1u;
         rc = band_begin(c, m, block + done, st);
         if (rc) return rc;
-        const int q = c->bandSet;
-        cudaGraphExec_t* g = after == BandAfter::kFollowed ? &c->bandFollow[a][q]
-                             : after == BandAfter::kRecord ? &c->bandRec[a][q]
-                             : m == 1u                     ? &c->bandOne[a][q]
-                                                           : &c->bandLoop[a][q];
+        const int q = c->bandSet, l = whole && m < pass ? 0 : k;
+        cudaGraphExec_t* g = one                            ? &c->bandOne[a][q]
+                             : after == BandAfter::kFollowed ? &c->bandFollow[a][q][l]
+                             : after == BandAfter::kRecord   ? &c->bandRec[a][q][l]
+                                                             : &c->bandLoop[a][q][l];
         rc = build_band_graph(c,
                               [&](cudaStream_t s) {
-                                  return m == 1u && after == BandAfter::kNothing
-                                             ? enqueue_band_sort(c, true, s)
-                                             : enqueue_band_loop(c, after, s);
+                                  return one ? enqueue_band_sort(c, true, s)
+                                             : enqueue_band_loop(c, after, kBandPassSteps[l], s);
                               },
                               g);
         if (rc) return rc;

@@ -627,26 +627,51 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     const float2* __restrict__ vel = one ? B.dyn[1].vel : B.dyn[0].vel;
     const float* __restrict__ theta = one ? B.dyn[1].theta : B.dyn[0].theta;
     const float* __restrict__ omega = one ? B.dyn[1].omega : B.dyn[0].omega;
-    for (uint32_t k = blockIdx.y * kPackThreads + threadIdx.x; k < cnt;
-         k += gridDim.y * kPackThreads) {
-        const uint32_t s = base + k, i = to + k;
-        // out of range only after a sort whose wait gave up
-        if (s >= B.slots || i >= B.n) break;
-        const uint32_t id = B.stat.id[s];
-        o.dyn.pos[i] = pos[s];
-        o.dyn.vel[i] = vel[s];
-        o.dyn.theta[i] = theta[s];
-        o.dyn.omega[i] = omega[s];
-        o.stat.radius[i] = B.stat.radius[s];
-        o.stat.mass[i] = B.stat.mass[s];
-        o.stat.id[i] = id;
-        if (TYPED) o.stat.type[i] = B.stat.type[s];
-        if (stateOnly) continue;
-        o.loc[id] = i;
-        if (B.pressure) o.pressure[i] = B.pressure[s];
-        if (B.acc) {
-            o.acc[i] = B.acc[s];
-            o.alpha[i] = B.alpha[s];
+    // two particles a thread in flight
+    const uint32_t step = gridDim.y * kPackThreads;
+    for (uint32_t k = blockIdx.y * kPackThreads + threadIdx.x; k < cnt; k += 2u * step) {
+        float2 p[2], v[2], ac[2];
+        float th[2], om[2], r[2], m[2], pr[2], al[2];
+        uint32_t id[2], type[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            // out of range only after a sort whose wait gave up
+            const uint32_t s = min(base + min(k + (uint32_t)u * step, cnt - 1u), B.slots - 1u);
+            p[u] = pos[s];
+            v[u] = vel[s];
+            th[u] = theta[s];
+            om[u] = omega[s];
+            r[u] = B.stat.radius[s];
+            m[u] = B.stat.mass[s];
+            id[u] = B.stat.id[s];
+            if (TYPED) type[u] = B.stat.type[s];
+            if (!stateOnly) {
+                pr[u] = B.pressure ? B.pressure[s] : 0.0f;
+                if (B.acc) {
+                    ac[u] = B.acc[s];
+                    al[u] = B.alpha[s];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t i = to + k + (uint32_t)u * step;
+            if (k + (uint32_t)u * step >= cnt || i >= B.n) break;
+            o.dyn.pos[i] = p[u];
+            o.dyn.vel[i] = v[u];
+            o.dyn.theta[i] = th[u];
+            o.dyn.omega[i] = om[u];
+            o.stat.radius[i] = r[u];
+            o.stat.mass[i] = m[u];
+            o.stat.id[i] = id[u];
+            if (TYPED) o.stat.type[i] = type[u];
+            if (stateOnly) continue;
+            o.loc[id[u]] = i;
+            if (B.pressure) o.pressure[i] = pr[u];
+            if (B.acc) {
+                o.acc[i] = ac[u];
+                o.alpha[i] = al[u];
+            }
         }
     }
 }
