@@ -1277,6 +1277,44 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
 }
 }  // namespace
 
+namespace {
+// Copies between the context's arrays and a caller's: one launch for the arrays
+// in this GPU's memory and aligned for it, a copy each for the others (host
+// memory, another GPU's, odd addresses).
+class ArrayCopies {
+public:
+    ArrayCopies(const DemContext* c, int host, cudaMemcpyKind kind, cudaStream_t st)
+        : device_(c->device), host_(host), kind_(kind), st_(st) {
+        list_.count = 0;
+    }
+    // `caller`: the end that is not the context's
+    cudaError_t add(void* dst, const void* src, size_t bytes, const void* caller) {
+        if (!bytes) return cudaSuccess;
+        cudaPointerAttributes at{};
+        const bool one = !host_ && bytes % 4 == 0 && !misaligned((const char*)dst, 16) &&
+                         !misaligned((const char*)src, 16) && list_.count < kCopyMax &&
+                         cudaPointerGetAttributes(&at, caller) == cudaSuccess &&
+                         at.type == cudaMemoryTypeDevice && at.device == device_;
+        if (!one) {
+            (void)cudaGetLastError();  // the query's error is not the caller's
+            return cudaMemcpyAsync(dst, src, bytes, kind_, st_);
+        }
+        const int k = list_.count++;
+        list_.src[k] = static_cast<const uint32_t*>(src);
+        list_.dst[k] = static_cast<uint32_t*>(dst);
+        list_.words[k] = bytes / 4;
+        return cudaSuccess;
+    }
+    cudaError_t run() { return list_.count ? launch_copy_arrays(list_, st_) : cudaSuccess; }
+
+private:
+    int device_, host_;
+    cudaMemcpyKind kind_;
+    cudaStream_t st_;
+    CopyList list_;
+};
+}  // namespace
+
 extern "C" int dem_set_state(DemContext* c, uint32_t n, const float* pos, const float* vel,
                              const float* theta, const float* omega, const float* radius,
                              const float* mass, const uint32_t* id, const uint32_t* type, int host,
@@ -1293,15 +1331,20 @@ extern "C" int dem_set_state(DemContext* c, uint32_t n, const float* pos, const 
     cudaStream_t st = (cudaStream_t)stream;
     const cudaMemcpyKind k = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     const int a = c->cur;
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[0].pos, pos, 8ull * n, k, st), "set pos");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].vel, vel, 8ull * n, k, st), "set vel");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].theta, theta, 4ull * n, k, st), "set theta");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].omega, omega, 4ull * n, k, st), "set omega");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].radius, radius, 4ull * n, k, st), "set radius");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].mass, mass, 4ull * n, k, st), "set mass");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].id, id, 4ull * n, k, st), "set id");
-    if (c->typed)
-        DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].type, type, 4ull * n, k, st), "set type");
+    ArrayCopies copies(c, host, k, st);
+    const struct { void* to; const void* from; size_t bytes; const char* what; } arrays[] = {
+        {c->dyn[0].pos, pos, 8, "set pos"},
+        {c->dyn[a].vel, vel, 8, "set vel"},
+        {c->dyn[a].theta, theta, 4, "set theta"},
+        {c->dyn[a].omega, omega, 4, "set omega"},
+        {c->stat[a].radius, radius, 4, "set radius"},
+        {c->stat[a].mass, mass, 4, "set mass"},
+        {c->stat[a].id, id, 4, "set id"},
+        {c->stat[a].type, c->typed ? type : nullptr, 4, "set type"},
+    };
+    for (const auto& x : arrays)
+        if (x.from) DEM_TRY_CUDA(copies.add(x.to, x.from, x.bytes * n, x.from), x.what);
+    DEM_TRY_CUDA(copies.run(), "set state");
     return accept_state(c, n, st);
 }
 
@@ -1404,19 +1447,24 @@ extern "C" int dem_get_state(DemContext* c, float* pos, float* vel, float* theta
     const cudaMemcpyKind k = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     const uint32_t n = c->n;
     const int a = c->cur;
-    if (pos) DEM_TRY_CUDA(cudaMemcpyAsync(pos, c->dyn[0].pos, 8ull * n, k, st), "get pos");
-    if (vel) DEM_TRY_CUDA(cudaMemcpyAsync(vel, c->dyn[a].vel, 8ull * n, k, st), "get vel");
-    if (theta) DEM_TRY_CUDA(cudaMemcpyAsync(theta, c->dyn[a].theta, 4ull * n, k, st), "get theta");
-    if (omega) DEM_TRY_CUDA(cudaMemcpyAsync(omega, c->dyn[a].omega, 4ull * n, k, st), "get omega");
-    if (radius) DEM_TRY_CUDA(cudaMemcpyAsync(radius, c->stat[a].radius, 4ull * n, k, st), "get radius");
-    if (mass) DEM_TRY_CUDA(cudaMemcpyAsync(mass, c->stat[a].mass, 4ull * n, k, st), "get mass");
-    if (id) DEM_TRY_CUDA(cudaMemcpyAsync(id, c->stat[a].id, 4ull * n, k, st), "get id");
-    if (type && c->typed)
-        DEM_TRY_CUDA(cudaMemcpyAsync(type, c->stat[a].type, 4ull * n, k, st), "get type");
-    if (loc) DEM_TRY_CUDA(cudaMemcpyAsync(loc, c->loc, 4ull * n, k, st), "get loc");
-    if (pressure) DEM_TRY_CUDA(cudaMemcpyAsync(pressure, c->pressure, 4ull * n, k, st), "get pressure");
-    if (acc) DEM_TRY_CUDA(cudaMemcpyAsync(acc, c->acc, 8ull * n, k, st), "get acc");
-    if (alpha) DEM_TRY_CUDA(cudaMemcpyAsync(alpha, c->alpha, 4ull * n, k, st), "get alpha");
+    ArrayCopies copies(c, host, k, st);
+    const struct { void* to; const void* from; size_t bytes; const char* what; } arrays[] = {
+        {pos, c->dyn[0].pos, 8, "get pos"},
+        {vel, c->dyn[a].vel, 8, "get vel"},
+        {theta, c->dyn[a].theta, 4, "get theta"},
+        {omega, c->dyn[a].omega, 4, "get omega"},
+        {radius, c->stat[a].radius, 4, "get radius"},
+        {mass, c->stat[a].mass, 4, "get mass"},
+        {id, c->stat[a].id, 4, "get id"},
+        {c->typed ? type : nullptr, c->stat[a].type, 4, "get type"},
+        {loc, c->loc, 4, "get loc"},
+        {pressure, c->pressure, 4, "get pressure"},
+        {acc, c->acc, 8, "get acc"},
+        {alpha, c->alpha, 4, "get alpha"},
+    };
+    for (const auto& x : arrays)
+        if (x.to) DEM_TRY_CUDA(copies.add(x.to, x.from, x.bytes * n, x.to), x.what);
+    DEM_TRY_CUDA(copies.run(), "get state");
     return DEM_OK;
 }
 
@@ -2475,13 +2523,15 @@ int step_recorded(DemContext* c, cudaStream_t st, char* rec) {
 int restore_checkpoint(DemContext* c, const Snapshot& s, cudaStream_t st) {
     const int a = c->cur;
     const size_t n = c->n;
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[0].pos, s.pos, 8 * n, cudaMemcpyDeviceToDevice, st), "restore pos");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].vel, s.vel, 8 * n, cudaMemcpyDeviceToDevice, st), "restore vel");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].theta, s.theta, 4 * n, cudaMemcpyDeviceToDevice, st), "restore theta");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->dyn[a].omega, s.omega, 4 * n, cudaMemcpyDeviceToDevice, st), "restore omega");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].radius, s.radius, 4 * n, cudaMemcpyDeviceToDevice, st), "restore radius");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].mass, s.mass, 4 * n, cudaMemcpyDeviceToDevice, st), "restore mass");
-    DEM_TRY_CUDA(cudaMemcpyAsync(c->stat[a].id, s.id, 4 * n, cudaMemcpyDeviceToDevice, st), "restore id");
+    ArrayCopies copies(c, 0, cudaMemcpyDeviceToDevice, st);
+    const struct { void* to; const void* from; size_t bytes; } arrays[] = {
+        {c->dyn[0].pos, s.pos, 8},      {c->dyn[a].vel, s.vel, 8},       {c->dyn[a].theta, s.theta, 4},
+        {c->dyn[a].omega, s.omega, 4},  {c->stat[a].radius, s.radius, 4}, {c->stat[a].mass, s.mass, 4},
+        {c->stat[a].id, s.id, 4},
+    };
+    for (const auto& x : arrays)
+        DEM_TRY_CUDA(copies.add(x.to, x.from, x.bytes * n, x.from), "restore checkpoint");
+    DEM_TRY_CUDA(copies.run(), "restore checkpoint");
     state_replaced(c);
     c->inSortOrder = false;
     return DEM_OK;

@@ -182,6 +182,17 @@ struct Words {
 };
 cudaError_t launch_set_words(uint32_t* dst, Words w, cudaStream_t st);
 
+// Up to kCopyMax device arrays (16-byte aligned at both ends, whole words) copied
+// by one launch.
+constexpr int kCopyMax = 12;
+struct CopyList {
+    const uint32_t* src[kCopyMax];
+    uint32_t* dst[kCopyMax];
+    size_t words[kCopyMax];
+    int count;
+};
+cudaError_t launch_copy_arrays(const CopyList& c, cudaStream_t st);
+
 // Adjoint (dem_adjoint.cu).
 size_t adj_step_bytes(uint32_t n, uint32_t numCells);
 // One recorded step: the sorted state the step kernel read, its cell ranges
