@@ -482,9 +482,10 @@ band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ Ban
     } else {
         b0 = band_of(B, key);
         // one round of loads: whether to search, and the rows of the candidates
-        // kept so far
+        // kept so far.  A cell stamped in the step before (`now`) may have been
+        // stamped again by a block of this step (`now` + 1).
         if (CULL) base = row_bases(P, B, key, cand & kCandNone ? 0ull : cand);
-        if (CULL && ((cand & kCandNone) || B.stamp[key] == now || B.search[b0])) {
+        if (CULL && ((cand & kCandNone) || B.stamp[key] - now <= 1u || B.search[b0])) {
             cand = search_candidates<ATTRACT>(P, i, key, s.p, r, B.skin, in.pos, B.stat.radius,
                                               B.first);
             B.cand[i] = cand;

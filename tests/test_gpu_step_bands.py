@@ -129,3 +129,23 @@ def sim_rows(sim, lo, hi):
     a, b = C.c_uint32(), C.c_uint32()
     D.check(D.load().dem_row_slots(sim.handle, lo, hi, C.byref(a), C.byref(b), D._stream()))
     return a.value, b.value
+
+
+def test_cells_entered_in_steps_after_each_other():
+    # more disks than the GPU has threads, so blocks of a step end before others
+    # of it begin; every other disk sits at the edge of two cells, so disks change
+    # cell in one step and in the next near each other, the rows beside the grid's
+    # wrap included (first and last blocks)
+    nx, ny = 8192, 64
+    sc = scenes.agitated_gas(n=nx * ny, seed=5, vel_std=0.5, grid=(4096, 32))
+    pitch = 2.05e-3
+    rng = np.random.default_rng(5)
+    ij = np.stack(np.meshgrid(np.arange(nx), np.arange(ny) + 0.5, indexing="xy"), -1)
+    at = (ij.reshape(-1, 2) + rng.uniform(-0.025, 0.025, size=(nx * ny, 2))) * pitch
+    sc.pos[:] = np.maximum(at, 1e-5)
+    sc.sys.Lx, sc.sys.Ly = nx * pitch, ny * pitch
+    # soft contacts: disks this slow search every few steps
+    m = sc.sys.materials[0]
+    m.normalStiffness, m.shearStiffness = 1e3, 5e2
+    sc.sys.knWall, sc.sys.ktWall = 1e3, 5e2
+    _check(sc, 40)
