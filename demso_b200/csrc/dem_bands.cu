@@ -221,11 +221,13 @@ band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynS
         __syncthreads();
     }
     // how far pairs may have approached since their bands searched, by the
-    // blocks from the last on (the first ones have the events).  Rows across a
-    // grid's wrap are out of reach, so the bands beside a band are enough.
+    // blocks from the last on (the first ones have the events).  A pair's bands
+    // are the same or beside each other, the first and the last one too (rows
+    // across the grid's wrap are out of reach in a whole scene; a disk that
+    // left a window of rows is met there).
     for (uint32_t b = (gridDim.x - 1u - blockIdx.x) * kFixThreads + threadIdx.x; b < B.bands;
          b += gridDim.x * kFixThreads) {
-        const uint32_t lo = b ? b - 1u : 0u, hi = min(b + 1u, B.bands - 1u);
+        const uint32_t lo = (b ? b : B.bands) - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
         const float own = __uint_as_float(B.moved[q][b]);
         // as bits, so that a NaN is the largest
         const float any = __uint_as_float(max(B.moved[q][b], max(B.moved[q][lo], B.moved[q][hi])));

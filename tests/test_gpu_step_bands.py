@@ -149,3 +149,23 @@ def test_cells_entered_in_steps_after_each_other():
     m.normalStiffness, m.shearStiffness = 1e3, 5e2
     sc.sys.knWall, sc.sys.ktWall = 1e3, 5e2
     _check(sc, 40)
+
+
+def test_disks_that_leave_a_row_window():
+    # they are met across the window's wrap, from the last band to the first; calls
+    # of 3 steps stay on the packed path
+    from demso_b200.slab import cell_rows
+    sc = scenes.agitated_gas(n=4096, seed=11, vel_std=0.5, grid=(64, 64), pitch_factor=1.15,
+                             gravity=(0.0, 0.0))
+    sc.pos[:, 1] = np.minimum(sc.pos[:, 1] + 1.15e-3, sc.sys.Ly - 1e-5)
+    rows = (16, 32)
+    r = cell_rows(sc.sys, sc.pos)
+    at = np.nonzero((r >= rows[0]) & (r < rows[0] + rows[1]))[0]
+    st = {k: (v[at].copy() if v is not None else None) for k, v in sc.state().items()}
+    st["id"] = np.arange(at.size, dtype=np.uint32)
+    a = gpu_run(sc.sys, st, 200, rows=rows)
+    b = gpu_run(sc.sys, st, 200, rows=rows, chunks=[3] * 66 + [2])
+    r = cell_rows(sc.sys, a["pos"])
+    assert np.any((r < rows[0]) | (r >= rows[0] + rows[1]))
+    for k in KEYS:
+        assert same(a[k], b[k]), k
