@@ -951,6 +951,14 @@ cudaError_t launch_band_gaps(const BandArgs& b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// From about this many slots on (80 B each against 126 MB of L2) a step reads its
+// state from DRAM, and ten blocks of 48 registers a multiprocessor hide more of
+// that than eight of 64 lose to spills: 154.8 -> 145.9 us a step at 4,194,304
+// disks, 65.4 -> 63.6 at 1,500,000, 343 -> 327 for 4,096 specimens, but 47.7 -> 48.5
+// at 1,100,001 and 13.7 -> 14.4 at 65,536.  Attraction spills more (450 -> 472 at
+// 4,000,003).
+constexpr uint32_t kFarSlots = 5u << 18;
+
 cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool everyStep,
                              int variant, ControlArgs ctl, cudaStream_t st) {
     if (variant < 0 || variant >= kStepVariants) return cudaErrorInvalidValue;
@@ -959,6 +967,7 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
     const bool cull = batch || P.cull != 0u;  // a specimen without culling searches in full
     const DynSet in = b.dyn[q], out = b.dyn[q ^ 1];
     const uint32_t e = everyStep ? 1u : 0u;
+    const bool far = !attract && b.slots >= kFarSlots;
 #define DEM_BAND_T(T, A, C, TH, MB)                                                            \
     do {                                                                                       \
         const unsigned g = blocks_for(b.slots, TH);                                            \
@@ -978,7 +987,10 @@ cudaError_t launch_band_step(const KParams& P, const BandArgs& b, int q, bool ev
             case 1: DEM_BAND_T(T, A, C, 64, 16); break;      \
             case 2: DEM_BAND_T(T, A, C, 256, 4); break;      \
             case 3: DEM_BAND_T(T, A, C, 128, 6); break;      \
-            default: DEM_BAND_T(T, A, C, 128, 8); break;     \
+            default:                                         \
+                if (far) DEM_BAND_T(T, A, C, 128, ((A) ? 8 : 10)); \
+                else DEM_BAND_T(T, A, C, 128, 8);            \
+                break;                                       \
         }                                                    \
     } while (0)
 #define DEM_BAND_AC(T)                                  \

@@ -161,10 +161,16 @@ int dem_integrate_system(const DemSystem* sys, float* pos, float* vel, const flo
 
 /* ---------------------------------------------------------------------------
  * Context API: the whole step (SimLooping's inner loop, main.cu:396-507)
- * on library-owned device buffers: a sort phase (incremental stable sort,
- * cell ranges, positions and radii moved to sorted order) and one step
- * kernel (collide, integrate, next hash, gathering the other fields into
- * sorted order), both replayed as CUDA graphs.  A context's calls share its
+ * on library-owned device buffers.  The particles lie in the reference's
+ * sorted order in bands of whole cell rows with free slots behind each: a
+ * step rewrites the bands that a particle left or entered (the stable sort,
+ * in place) and runs one step kernel (collide, integrate, next hash), as CUDA
+ * graphs; the state is packed into sorted order at the end of every call.
+ * Adopted buffers, rows of more than 4,096 cells, calls of fewer than 4
+ * steps (3 for a batch) on a state that is not in bands, and a context whose
+ * bands could not be allocated step packed instead: an incremental stable
+ * sort that moves positions and radii, and a step kernel that gathers the
+ * other fields.  The bits are the same.  A context's calls share its
  * device buffers and its loop counters: issue them on one stream, or
  * synchronise before a call on another stream.  Different contexts are
  * independent and may run on different streams and host threads.
@@ -309,15 +315,15 @@ int dem_adopt_state(DemContext* ctx, uint32_t n, const DemStateSet* first,
 int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
 
 /* Advances `nsteps` full steps (hash, sort, reorder, collide, integrate).
- * Once the context holds a previous order (after its first step) and is
- * neither tuning nor profiling nor created with DEM_CTX_DIRECT, a call of
- * two or more steps runs them in pairs inside ONE graph launch: a
- * device-side loop (a CUDA graph WHILE node, its pair count written to the
+ * Unless the context is tuning or profiling or was created with
+ * DEM_CTX_DIRECT, a call of several steps runs them inside ONE graph launch:
+ * a device-side loop (CUDA graph WHILE nodes, the step count written to the
  * device by a one-thread kernel before the launch and counted down there)
- * whose body is two whole steps, one per buffer parity; an odd
- * last step is one more ordinary step.  The loop runs the same kernels on
- * the same buffers as single calls, so the bits are those of nsteps calls
- * of one step.
+ * whose body is a pass of 4 to 12 steps in bands, or a pair of packed steps
+ * (which need a previous order, so not the first step); scenes of 1,048,576
+ * disks or more make the few steps that fill no pass by further launches.
+ * The loop runs the same kernels on the same buffers as single calls, so the
+ * bits are those of nsteps calls of one step.
  * With DEM_CTX_AUTOTUNE the context's first 24 steps run the step kernel's
  * launch shapes in turn, each timed by CUDA events on `stream`; the step
  * that completes the 24th waits for `stream` once and keeps the shape with
@@ -337,8 +343,9 @@ int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
 int dem_step(DemContext* ctx, uint32_t nsteps, void* stream);
 
 /* Launch shapes of the step kernel (threads per block x blocks per SM its
- * registers are capped for): 0 = 128 x 8 (the default), 1 = 64 x 16,
- * 2 = 256 x 4, 3 = 128 x 6. */
+ * registers are capped for): 0 = 128 x 8 (the default; without attraction and
+ * a control particle, states of about 1.25 million particles and more are
+ * stepped by a 128 x 10 form of it), 1 = 64 x 16, 2 = 256 x 4, 3 = 128 x 6. */
 #define DEM_STEP_VARIANTS 4
 typedef struct DemStepVariant {
     int32_t variant;       /* the shape in use */

@@ -169,3 +169,42 @@ def test_disks_that_leave_a_row_window():
     assert np.any((r < rows[0]) | (r >= rows[0] + rows[1]))
     for k in KEYS:
         assert same(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n", [1220000, 1250000])
+def test_sizes_beside_the_ten_block_shape(n):
+    # 1,296,250 and 1,328,125 slots: the last of the 8-block shape, the first of
+    # the 10-block one (from 1,310,720 on)
+    sc = scenes.agitated_gas(n=n, seed=31, vel_std=2.0, pitch_factor=1.1, jitter=0.1)
+    _check(sc, 8)
+
+
+@pytest.mark.parametrize("kind", ["typed", "batch"])
+def test_the_ten_block_shape_of_types_and_batches(kind):
+    import torch
+    import demso_b200 as D
+    t = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a)
+    if kind == "typed":
+        sc = scenes.agitated_gas(n=1400000, seed=33, vel_std=2.0, pitch_factor=1.1, jitter=0.1,
+                                 n_mat=3)
+        st = sc.state()
+        make = lambda: D.Simulation(sc.sys, capacity=sc.n, flags=D.CTX_PRESSURE | D.CTX_ACCEL)
+    else:
+        parts = [scenes.agitated_gas(n=n, seed=34 + n % 7, vel_std=2.0, pitch_factor=1.1,
+                                     jitter=0.1) for n in (700001, 699, 701003)]
+        st = scenes.concat_specimens(parts)
+        make = lambda: D.Batch([(p.sys, p.n) for p in parts],
+                               flags=D.CTX_PRESSURE | D.CTX_ACCEL)
+    got = []
+    for variant in (0, 1):  # 1 is one shape for every size
+        sim = make()
+        sim.set_step_variant(variant)
+        sim.set_state(*(t(st[k]) for k in ("pos", "vel", "theta", "omega", "radius", "mass",
+                                           "id")),
+                      *([t(st["type"])] if kind == "typed" else []))
+        sim.step(12)
+        got.append({k: v.numpy() for k, v in sim.get_state("cpu").items() if v is not None})
+        sim.check()
+        sim.close()
+    for k in got[0]:
+        assert same(got[0][k], got[1][k]), k
