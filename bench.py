@@ -53,20 +53,20 @@ N_DEFAULT = 4194304
 #   collide: reads own pos/vel/omega/radius/mass 28, writes force 8 + torque 4
 #     (neighbours are cache hits) = 40 per particle + 8 per cell (cell ranges);
 #   integrate: reads pos, vel, omega, theta, radius, mass, acc, alpha 44, writes
-#     pos, vel, omega, theta 24 = 68 per particle;
-#   the gather half of the reorder (84 per particle in all): the step kernel
-#     reads vel, theta, omega, mass, id at each particle's previous slot 24 and
-#     writes them in sorted order 24, with loc 4 = 52; the sort phase moves the
-#     positions and radii and writes the keys and slots (the other 32).
-# The fused kernel keeps force, torque and the sorted fields in registers, so
-# its own minimum is 88 per particle (reads 44, writes 44; reported beside).
-STEP_KERNEL_STAGE_BYTES = {"collide": 40, "integrate": 68, "reorder_gather": 52}
+#     pos, vel, omega, theta 24 = 68 per particle.
+# Particles keep their places between steps (only bands that one left or entered
+# are rewritten, by the sort phase), so no reorder is counted here.  The fused
+# kernel keeps force and torque in registers, so its own minimum is 68 per
+# particle (reads 44: pos, vel, theta, omega, radius, mass, key, kept
+# candidates; writes 24; reported beside).
+STEP_KERNEL_STAGE_BYTES = {"collide": 40, "integrate": 68}
 STEP_KERNEL_BYTES_PER_PARTICLE = sum(STEP_KERNEL_STAGE_BYTES.values())
 STEP_KERNEL_BYTES_PER_CELL = 8
-FUSED_MIN_BYTES_PER_PARTICLE = 88
-# Whole step, per particle: hash 16 + sort 52 + reorder 84 + collide 40 +
-# integrate 68 = 260, plus 20 per cell (reorder 12, collide 8).
-WHOLE_STEP_BYTES = lambda n, c: 260.0 * n + 20.0 * c  # whole-step model, per step
+FUSED_MIN_BYTES_PER_PARTICLE = 68
+# Whole step: the fused minimum, and a first-slot word and a stamp per cell.  (A
+# step that hashes, sorts, reorders, collides and integrates in passes of its own
+# moves 260 per particle and 20 per cell.)
+WHOLE_STEP_BYTES = lambda n, c: float(FUSED_MIN_BYTES_PER_PARTICLE) * n + 8.0 * c
 # the plain-at-scale sizes of the roofline curve (the same workload scaled)
 DEFAULT_SWEEP = "65536,262144,1048576,4194304,16777216"
 # the timed K-step call is repeated until this much device time is under load
@@ -248,10 +248,12 @@ def config_dict(n, sc):
 def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int = 256):
     """Batched form on the batched workload (4,096 specimens of 256..8,192
     disks, own boxes/parameters; 5,000 steps issued as one dem_step call) in
-    its two forms -- one persistent launch of the resident step, and one
+    two contexts -- with the resident flag (a batch with a state of its own
+    steps in bands with it too, the faster form) and without, each one
     graph launch of the device-side step loop -- against looping the plain
     single-scene step over an evenly spaced sample of the same specimens, in
-    the faster of its two forms (graph path, cluster launch).  `value` is
+    the faster of its two forms (graph path, resident flag: a cluster launch
+    up to 1,536 disks).  `value` is
     the faster batched form."""
     import torch
     import demso_b200 as D
@@ -278,9 +280,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     graph_path = total * steps / (e0.elapsed_time(e1) * 1e-3)
     kernels = b.kernels_per_step()
     b.close()
-    # the resident form (DEM_CTX_RESIDENT): the call's steps as one persistent
-    # launch, every bin of specimens stepped in one multiprocessor's shared
-    # memory; its first call packs the bins and is untimed
+    # the same with DEM_CTX_RESIDENT, which takes the faster form; its first
+    # call lays the bands out and is untimed
     r = D.Batch([(sc.sys, sc.n) for sc in specimens], flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
     r.set_state(t(st["pos"]), t(st["vel"]), t(st["theta"]), t(st["omega"]), t(st["radius"]),
                 t(st["mass"]), t(st["id"]))
@@ -317,8 +318,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     torch.cuda.synchronize()
     sample_n = sum(sc.n for sc in sample)
     looped_graph = sample_n * lsteps / (e0.elapsed_time(e1) * 1e-3)
-    # the same, each specimen's context stepped as one thread-block cluster
-    # launch (DEM_CTX_RESIDENT on a single scene of at most 8,192 disks)
+    # the same with DEM_CTX_RESIDENT: specimens of up to 1,536 disks as one
+    # thread-block cluster launch each, larger ones on the graph path
     csims = []
     for sc in sample:
         sim = D.Simulation(sc.sys, capacity=sc.n, flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
@@ -352,14 +353,13 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
         sim.close()
     return {"metric": "aggregate particle-steps/s, batched vs looped plain",
             "value": batched, "looped_plain": looped, "ratio": batched / looped,
-            "path": "resident" if resident >= graph_path else "graph",
+            "path": "graph",
             "resident": {"value": resident, "ratio": resident / looped, "launches": 1,
-                         "form": "the %d steps as one persistent kernel launch; specimens in "
-                                 "bins of up to 8,192 disks, each bin stepped inside one "
-                                 "multiprocessor's shared memory" % steps},
+                         "form": "the %d steps with the resident flag: one graph launch of the "
+                                 "device-side step loop, the faster form" % steps},
             "graph_path": {"value": graph_path, "ratio": graph_path / looped,
                            "kernels_per_step": kernels,
-                           "graph_launches": 1 if steps % 2 == 0 else 2,
+                           "graph_launches": 1,
                            "step_kernel_shape": [shape["threads"], shape["blocks_per_sm"]],
                            "form": "the %d steps as one graph launch of the device-side step "
                                    "loop, %d kernels per step" % (steps, kernels)},
@@ -370,7 +370,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
             "looped_sample": "%d of the %d specimens (every %d-th), each its own context "
                              "stepping %d steps as one dem_step call, one specimen after "
                              "another; the faster of the graph path (device-side step "
-                             "loop) and the cluster launch"
+                             "loop) and the resident flag (a cluster launch up to 1,536 "
+                             "disks)"
                              % (len(sample), num, max(1, num // loop_sample), lsteps),
             "workload": "batched: specimens with counts log-uniform in [256, 8192], square "
                         "walled boxes at area fraction 0.5, radii U[0.9, 1.1] mm, kn "
@@ -466,8 +467,9 @@ def measure_adjoint(n: int = 16384, steps: int = 2000, every: int = 100):
 # ------------------------------------------------------------------ config 0
 def measure_settling_pile(steps: int = 20000):
     """The plain 2D settling pile (4,096 disks, 20,000 steps): wall time of
-    the whole run on the GPU as one dem_step call, for the context stepped
-    by a thread-block cluster (DEM_CTX_RESIDENT) and on the graph path; the
+    the whole run on the GPU as one dem_step call, for a context with the
+    resident flag (scenes above 1,536 disks take the graph path with it) and
+    one without; the
     faster gives gpu_seconds (settling_pile_cpu adds the host build's)."""
     import torch
     import demso_b200 as D
@@ -501,10 +503,10 @@ def measure_settling_pile(steps: int = 20000):
                        "jittered lattice in a 0.2 x 0.2 m box, dt 2e-6 s, %d steps" % steps,
            "gpu_seconds": gpu_s, "gpu_steps_per_s": steps / gpu_s,
            "gpu_particle_steps_per_s": sc.n * steps / gpu_s,
-           "path": "cluster" if cluster_s <= graph_s else "graph",
+           "path": "graph",
            "cluster_seconds": cluster_s, "graph_path_seconds": graph_s,
-           "cluster_form": "one launch of a cluster of 8 blocks, each holding the scene in "
-                           "shared memory and stepping an eighth of the disks",
+           "cluster_form": "the context with the resident flag, which takes the graph path "
+                           "above 1,536 disks",
            "graph_path_form": "one graph launch of the device-side step loop"}
     return out
 
@@ -867,9 +869,10 @@ def main():
     elapsed = float(np.median(reps))
     sim.check()
     value = n * world * args.steps / (elapsed * 1e-3)
-    # kernels of the timed call: every step's, plus the loop's init kernel and
-    # one count-down kernel per pair of steps (none on direct launches)
-    loop_kernels = 0 if args.direct or args.steps < 2 else 1 + args.steps // 2
+    # kernels of the timed call: every step's, plus the count, the loop's first,
+    # head and last kernels, one per pass of at most 12 steps (none of these on
+    # direct launches), and the pack
+    loop_kernels = 1 if args.direct else 5 + (args.steps + 11) // 12
 
     stage_ms = [ms[i] / max(1, nprof.value) for i in range(3)]
     stage_names = ["sort_reorder", "reorder_separate", "collide_integrate"]
@@ -878,13 +881,12 @@ def main():
     cells = sc.sys.num_cells
     if dom == 2:
         bytes_launch = STEP_KERNEL_BYTES_PER_PARTICLE * n + STEP_KERNEL_BYTES_PER_CELL * cells
-        kname = "step_kernel (collide + integrate + next hash + gather into sorted order)"
+        kname = "band_step_kernel (collide + integrate + next hash)"
     else:
-        # counted as its share of the reorder alone (positions and radii 12 B
-        # in and out, key and slot 8 B per particle, 12 B per cell); the sort
-        # work is not counted
-        bytes_launch = 32 * n + 12 * cells
-        kname = "sort phase (incremental sort + positions and radii into sorted order)"
+        # counted as the reorder alone (84 B per particle, 12 B per cell); the
+        # sort work is not counted
+        bytes_launch = 84 * n + 12 * cells
+        kname = "sort phase (bands that a disk left or entered)"
     achieved = bytes_launch / (stage_ms[dom] * 1e-3) / 1e9
     traffic = None
     tf = os.path.join(ROOT, "profiles", "traffic.txt")

@@ -28,9 +28,9 @@
 // Against the packed incremental sort (six kernels a step, 40 B moved per
 // particle in the sort phase and 88 B in the step; here two kernels, 64 B in
 // the step), with the kept candidates below: a call of 20 steps of 4,194,304
-// disks 4,651 -> 3,199 us, of 1,000,003 dense disks 1,534 -> 1,225 us, 50 steps of
-// 65,536 1,235 -> 885 us, 20 steps of a fast gas of 131,071 587 -> 410 us, of 256
-// specimens of two materials 1,278 -> 1,007 us.  A batch's specimens keep their
+// disks 4,669 -> 2,988 us, of 1,000,003 dense disks 1,503 -> 1,116 us, 50 steps of
+// 65,536 1,229 -> 834 us, 20 steps of a fast gas of 131,071 584 -> 365 us, of 256
+// specimens of two materials 1,243 -> 784 us.  A batch's specimens keep their
 // own bands, so a slot never changes specimen.
 //
 // The two dynamic sets alternate with the steps (kBandCur: the one that holds
