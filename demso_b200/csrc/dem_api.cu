@@ -388,14 +388,15 @@ struct DemContext {
     void* block = nullptr;  // one allocation for every per-particle/per-cell array
     // The step in bands (dem_bands.cuh): its arrays, in bandBlock (band.bands
     // == 0: the context steps on the packed path); whether they hold the
-    // current state, and whether cells/first of set cur were made from them;
-    // the step loop, with and without followed rows, one step, and a step's
+    // current state; whether the cell ranges of the last sort are still to be
+    // made from them (band_cells: they describe that sort whatever replaces the
+    // state or its parameters, until the next step); the step loop, with and without followed rows, one step, and a step's
     // sort phase alone, by cur (the set the state is packed into) and bandSet.
     BandArgs band;
     std::vector<BandGeo> bandGeo;
     void* bandBlock = nullptr;
     float2* ownPos = nullptr;  // the block's positions: not an adopted set
-    bool bandValid = false, bandCells = false, bandInit = false;
+    bool bandValid = false, cellsInBands = false, bandInit = false;
     int bandSet = 0;  // the dynamic set of the bands that holds the state
     // band_call: short calls in a row that stepped in bands; steps of longer
     // calls on the packed path since
@@ -1687,7 +1688,7 @@ int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t s
     // as a step of the packed path would have left it
     state_replaced(c);
     c->bandValid = true;
-    c->bandCells = false;
+    c->cellsInBands = true;
     c->inSortOrder = true;
     return DEM_OK;
 }
@@ -1794,9 +1795,9 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
 // The packed cell ranges and first-particle array of set cur, made from the
 // bands on the first request after a call.
 int band_cells(DemContext* c, cudaStream_t st) {
-    if (!c->bandValid || c->bandCells) return DEM_OK;
+    if (!c->cellsInBands) return DEM_OK;
     DEM_TRY_CUDA(launch_band_cells(c->band, c->cells[c->cur], c->first[c->cur], st), "band cells");
-    c->bandCells = true;
+    c->cellsInBands = false;
     return DEM_OK;
 }
 
@@ -1979,6 +1980,7 @@ namespace {
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (band_call(c, nsteps)) return band_steps(c, nsteps, BandAfter::kNothing, 0, st);
     c->bandValid = false;
+    c->cellsInBands = false;  // the packed steps make their own
     if (!c->keysValid) {
         if (c->nspec)
             DEM_TRY_CUDA(launch_calc_hash_batched(c->dTable, c->spec, c->dyn[0].pos, c->keys, c->n,
@@ -2603,6 +2605,7 @@ constexpr uint32_t kRevSteps = 4;
 // slot, and an odd last step is host-launched.
 int rerun_recorded(DemContext* c, uint32_t k, size_t stepBytes, char* rec, cudaStream_t st) {
     const uint32_t n = c->n;
+    c->cellsInBands = false;
     if (!c->keysValid) {
         DEM_TRY_CUDA(c->nspec ? launch_calc_hash_batched(c->dTable, c->spec, c->dyn[0].pos, c->keys,
                                                          n, st)
