@@ -295,8 +295,8 @@ class Simulation:
 
     def state_view(self) -> dict:
         """The current state without a copy (dem_state_view): tensors over the
-        buffers that hold it, valid until the next step, set_state or
-        adopt_state, plus ``set`` (0 or 1), the set that holds every field but
+        buffers that hold it, valid until the next step (which takes what was
+        written through them), set_state or adopt_state, plus ``set`` (0 or 1), the set that holds every field but
         the positions."""
         import ctypes as C
         import torch

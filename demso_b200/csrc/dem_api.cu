@@ -1424,6 +1424,9 @@ extern "C" int dem_state_view(DemContext* c, DemStateSet* out, int* setIndex) {
     if (!out) return fail(DEM_ERR_INVALID_ARG, "dem_state_view: NULL output");
     if (!has_state_sets(c))
         return fail(DEM_ERR_INVALID_ARG, "no state buffers: call dem_adopt_state first");
+    // the caller may write through the view: the next step takes these arrays,
+    // not the bands they were packed from (one sort from scratch)
+    c->bandValid = false;
     const int a = c->cur;
     out->pos = reinterpret_cast<float*>(c->dyn[0].pos);
     out->vel = reinterpret_cast<float*>(c->dyn[a].vel);

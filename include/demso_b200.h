@@ -310,8 +310,10 @@ int dem_adopt_state(DemContext* ctx, uint32_t n, const DemStateSet* first,
  * adopted buffers or the context's own: positions in the first set's pos,
  * the other fields in set *setIndex (0 first, 1 second; may be NULL).
  * Valid until the next step, dem_set_state or dem_adopt_state; reading them
- * on another stream needs the usual synchronisation.  type is NULL with one
- * material. */
+ * on another stream needs the usual synchronisation.  The next step takes what
+ * was written through them (radii up to the largest of the state as set); a
+ * context that steps in bands sorts from scratch then, as after dem_set_state.
+ * type is NULL with one material. */
 int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
 
 /* Advances `nsteps` full steps (hash, sort, reorder, collide, integrate).
