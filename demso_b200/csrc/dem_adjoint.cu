@@ -81,7 +81,9 @@ adj_integrate_kernel(KParams P0, const KParams* __restrict__ table,
     if (i < n) {
         const StepRec rec = rec_at(rec0, at);
         const KParams& P = table ? table[seg] : P0;
-        const uint32_t id = rec.id[i];
+        // (a particle that a sort whose wait gave up has lost leaves its place of
+        // the record unwritten)
+        const uint32_t id = min(rec.id[i], n - 1u);
         const float r = rec.radius[i], m = rec.mass[i];
         const float I = inertia_of(m, r);
         const float2 x = rec.pos[i], v = rec.vel[i], a = rec.acc[i];
@@ -225,7 +227,7 @@ adj_pairs_kernel(KParams P0, const KParams* __restrict__ table, const uint32_t* 
                 }
             }
         }
-        const uint32_t k = rec.id[i];
+        const uint32_t k = min(rec.id[i], n - 1u);
         const float2 l = lx[i], u = lv[i];
         lamX[k] = make_float2(l.x + gx, l.y + gy);
         lamV[k] = make_float2(u.x + gvx, u.y + gvy);

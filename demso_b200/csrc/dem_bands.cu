@@ -503,8 +503,9 @@ band_step_kernel(const __grid_constant__ KParams P0, const __grid_constant__ Ban
                                             cand, base, key, spec, s.p, s.v, s.w, r, mat, o);
     if (!mine) return;
     if (CONTROL)
-        meet_control<TYPED, ATTRACT>(P, ctl, i - B.gap[b0], s.p, s.v, s.w, r, mat, o.f, o.moment,
-                                     o.pr);
+        // (within n, also after a sort whose wait gave up)
+        meet_control<TYPED, ATTRACT>(P, ctl, min(i - B.gap[b0], B.n - 1u), s.p, s.v, s.w, r, mat,
+                                     o.f, o.moment, o.pr);
     // F/m and M/I as the reference divides them; without contacts both are
     // exactly +0 (see finish_particle)
     const bool quiet =
@@ -680,12 +681,12 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
 }
 
 // Packed range of the band's cell c, the slots of the band `down` above their
-// packed places.
+// packed places (within n, also after a sort whose wait gave up).
 __device__ __forceinline__ uint2 packed_cell(const BandArgs& B, const BandGeo& geo, uint32_t c,
                                              uint32_t down) {
     const uint32_t* f = B.first + geo.first + (c >> geo.log2gx) * ((1u << geo.log2gx) + 1u) +
                         (c & ((1u << geo.log2gx) - 1u));
-    return make_uint2(f[0] - down, f[1] - down);
+    return make_uint2(min(f[0] - down, B.n), min(f[1] - down, B.n));
 }
 
 // Blocks (band, share), as band_pack_kernel: the state the step of set q
@@ -726,7 +727,10 @@ __global__ void band_cell_first_kernel(const uint32_t* __restrict__ keys, uint32
 }
 
 // A block per band: its base, count and first slots from the packed
-// first-particle array f; its empty slots; its counters.
+// first-particle array f; its empty slots; its counters.  A sort whose wait
+// gave up leaves keys in no order: a band may then count slots that
+// band_spread_kernel does not fill.  Those hold an id and a type that exist,
+// so that whoever indexes with them stays within the arrays.
 __global__ void __launch_bounds__(kPackThreads)
 band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
     const uint32_t b = blockIdx.x, tid = threadIdx.x;
@@ -744,6 +748,8 @@ band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
     }
     for (uint32_t s = b * kPackThreads + tid; s < B.slots; s += B.bands * kPackThreads) {
         B.key[s] = kBandEmpty;
+        B.stat.id[s] = 0u;
+        if (B.stat.type) B.stat.type[s] = 0u;
         if (B.slotSpec) B.slotSpec[s] = 0u;
     }
     const uint32_t gx = 1u << geo.log2gx, words = (geo.cells >> geo.log2gx) * (gx + 1u);
@@ -810,7 +816,9 @@ __global__ void band_followed_kernel(BandArgs B, DynSet d, uint32_t q,
     float* base = ring + (size_t)(B.ctrl[kBandDone] - 1u) * count * 12;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count;
          k += gridDim.x * blockDim.x)
-        followed_row(B.loc[ids[k]], base + 12ull * k, d, B.stat, B.acc, B.alpha, B.pressure);
+        // (an id that a sort whose wait gave up has lost keeps an old place, or none)
+        followed_row(min(B.loc[ids[k]], B.slots - 1u), base + 12ull * k, d, B.stat, B.acc, B.alpha,
+                     B.pressure);
 }
 
 // ---------------------------------------------------------- conditions
