@@ -1977,11 +1977,18 @@ extern "C" int dem_step(DemContext* c, uint32_t nsteps, void* stream) {
 }
 
 namespace {
-// dem_step on the graph path: the sort and step graphs, or the device-side
-// step loop for pairs of steps (also the steps of dem_step_followed, whose
-// per-step rows are gathered from this path's buffers).
+int packed_steps(DemContext* c, uint32_t nsteps, cudaStream_t st);
+
+// dem_step on the graph path.
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (band_call(c, nsteps)) return band_steps(c, nsteps, BandAfter::kNothing, 0, st);
+    return band_call(c, nsteps) ? band_steps(c, nsteps, BandAfter::kNothing, 0, st)
+                                : packed_steps(c, nsteps, st);
+}
+
+// The packed path: the sort and step graphs, or the device-side step loop for
+// pairs of steps (also the steps of dem_step_followed, whose per-step rows are
+// gathered from this path's buffers).
+int packed_steps(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     c->bandValid = false;
     c->cellsInBands = false;  // the packed steps make their own
     if (!c->keysValid) {
@@ -2278,8 +2285,11 @@ extern "C" int dem_step_followed(DemContext* c, uint32_t nsteps, const uint32_t*
                 DEM_TRY_CUDA(cudaGraphLaunch(c->followGraph[p], st), "graph launch");
                 j += 2 * pairs;
             } else {
-                // the graph path: the rows are gathered from its buffers
-                int rc = step_graph_path(c, 1, st);
+                // one step with the host around it, or the packed path's (the
+                // chunk's path is decided once: asked again for its single
+                // steps, band_call would keep a context in its bands); the
+                // rows are gathered from the packed state
+                int rc = alone ? step_graph_path(c, 1, st) : packed_steps(c, 1, st);
                 if (rc) return rc;
                 DEM_TRY_CUDA(enqueue_followed_ring(c, c->cur ^ 1, nullptr, j, st), "followed gather");
                 ++j;
