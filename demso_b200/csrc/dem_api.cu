@@ -399,8 +399,9 @@ struct DemContext {
     bool bandValid = false, cellsInBands = false, bandInit = false;
     int bandSet = 0;  // the dynamic set of the bands that holds the state
     // band_call: short calls in a row that stepped in bands; steps of longer
-    // calls on the packed path since
-    uint32_t shortCalls = 0, packedSteps = 0;
+    // calls on the packed path since.  cluster_call: steps of cluster launches
+    // since the graphs were dropped.
+    uint32_t shortCalls = 0, packedSteps = 0, clusterSteps = 0;
     cudaGraphExec_t bandLoop[2][2][kBandPasses] = {}, bandFollow[2][2][kBandPasses] = {};
     cudaGraphExec_t bandRec[2][2][kBandPasses] = {};  // recording every step for the adjoint
     cudaGraphExec_t bandOne[2][2] = {}, bandSort[2][2] = {};
@@ -536,6 +537,7 @@ void drop_loop_graphs(DemContext* c) {
 }
 
 void drop_graphs(DemContext* c) {
+    c->clusterSteps = 0;
     drop_tune_graphs(c);
     drop_loop_graphs(c);
     // a tuning interrupted by a change of the step starts again
@@ -1237,9 +1239,8 @@ bool has_state_sets(const DemContext* c) { return c->dyn[0].pos != nullptr; }
 bool steps_in_bands(DemContext* c);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
-    // the band arrays, unless the cluster launch will step this scene
-    if (!(c->flags & DEM_CTX_RESIDENT) || c->nspec || n > kClusterBandDisks ||
-        !cluster_scene_fits(n, c->numCells))
+    // the band arrays, unless the cluster launch will step this scene at first
+    if (!(c->flags & DEM_CTX_RESIDENT) || c->nspec || !cluster_scene_fits(n, c->numCells))
         steps_in_bands(c);
     // the new state replaces the one any recorded error was about
     DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 4, st), "clear error word");
@@ -1923,18 +1924,40 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     return DEM_OK;
 }
 
+// Whether a call of a resident scene of more than kClusterBandDisks disks, which
+// could step in bands, is a cluster launch.  The bands' arrays and graphs cost
+// a context about 1.5 ms (allocation, build and release; 4,096 disks, one call
+// of 100 steps: the context's life 2.3 ms with the cluster, 4.6 in bands), the
+// cluster 1 to 7 us a step more, so the first kClusterSteps steps are its own
+// unless one call is longer.  Afterwards calls too short for bands that are
+// not in them already: a single step is fastest on the packed path (24 us
+// against 36 to 66), two or three by the cluster up to kClusterBandDisks disks
+// a step (totals for 2 and 3 steps, cluster against packed: 2,000 disks 46 / 52
+// and 55 / 80 us, 4,096 63 / 53 and 75 / 81, 8,000 83 / 57 and 100 / 85).
+constexpr uint32_t kClusterSteps = 512;
+bool cluster_call(DemContext* c, uint32_t nsteps) {
+    if (c->clusterSteps < kClusterSteps && nsteps <= kClusterSteps - c->clusterSteps) {
+        c->clusterSteps += nsteps;
+        return true;
+    }
+    c->clusterSteps = kClusterSteps;
+    return nsteps >= 2 && nsteps < kShortCall && !c->bandValid &&
+           c->n <= kClusterBandDisks * nsteps;
+}
+
 // A multi-step call of a single scene created with DEM_CTX_RESIDENT as one
 // cluster launch (dem_resident.cu): every block of the cluster holds the
 // whole scene in shared memory and steps its share of the slots.  Returns
-// kNotResident, having done nothing, for scenes that step faster in bands
-// (kClusterBandDisks) and those it does not take (more than 8,192 disks or cells, types, attraction, a control particle, profiling) or
-// when no such cluster can be resident on this GPU; the graph path steps
-// those.  The next graph-path step sorts from scratch.
+// kNotResident, having done nothing, for calls that are faster in bands or
+// packed (cluster_call) and scenes it does not take (more than 8,192 disks or
+// cells, types, attraction, a control particle, profiling) or when no such
+// cluster can be resident on this GPU; the graph path steps those.  The next
+// graph-path step sorts from scratch.
 int cluster_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (c->typed || c->ctlOn || c->profiling || c->clusterUnsupported || c->rows ||
         !has_state_sets(c) ||
         has_attraction_host(c->P) || !cluster_scene_fits(c->n, c->numCells) ||
-        (c->n > kClusterBandDisks && steps_in_bands(c)))
+        (c->n > kClusterBandDisks && !cluster_call(c, nsteps) && steps_in_bands(c)))
         return kNotResident;
     const size_t bytes = cluster_scene_work_bytes(c->n);
     if (c->clusterWorkBytes < bytes) {

@@ -79,8 +79,8 @@ cudaError_t launch_resident(const KParams* table, const ResBin* bins, uint32_t n
 // cudaErrorNotSupported when no cluster of this shape can be resident.
 //
 // Scenes of more than kClusterBandDisks disks step faster in bands
-// (dem_bands.cuh), where the whole GPU shares the law and the sort: per step of
-// 400-step calls, cluster against bands, 500 disks 6.3 / 6.4 us, 1,500 6.3 / 6.5,
+// (dem_bands.cuh), where the whole GPU shares the law and the sort, once their
+// graphs are made (cluster_call): per step of 400-step calls, cluster against bands, 500 disks 6.3 / 6.4 us, 1,500 6.3 / 6.5,
 // 2,000 fast ones 11.2 / 9.7, 4,096 in a dense packing 11.2 / 8.4, 8,000
 // 16.1 / 9.3; calls of one to five steps of 500 disks 25-49 against 25-72 us.
 constexpr uint32_t kClusterBandDisks = 1536;

@@ -331,12 +331,12 @@ int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
  * that completes the 24th waits for `stream` once and keeps the shape with
  * the smallest median time.  Every shape computes the same bits, so the
  * trajectory does not depend on the choice.
- * A single scene created with DEM_CTX_RESIDENT, of at most 1,536 disks (with
- * DEM_CTX_CALLER_STATE 8,192; larger ones step faster on the graph path) and
+ * A single scene created with DEM_CTX_RESIDENT, of at most 8,192 disks and
  * 8,192 cells, one material, no attraction and no control particle, steps
- * each call as ONE launch of a thread-block cluster of 8 blocks: every block
- * keeps the whole scene's positions, velocities, spins and radii in its
- * shared memory, steps an eighth of the disks and writes their new state
+ * each call (above 1,536 disks, unless with DEM_CTX_CALLER_STATE: the first 512
+ * steps and short calls; the others are faster on the graph path) as ONE
+ * launch of a thread-block cluster of 8 blocks: every block keeps the whole
+ * scene's positions, velocities, spins and radii in its shared memory, steps an eighth of the disks and writes their new state
  * into every block's copy through distributed shared memory.  The bits are
  * the graph path's.  Its first call allocates the cluster's scratch (about
  * 270 B per disk); the next graph-path step sorts from scratch.  Other
