@@ -402,6 +402,12 @@ struct DemContext {
     // calls on the packed path since.  cluster_call: steps of cluster launches
     // since the graphs were dropped.
     uint32_t shortCalls = 0, packedSteps = 0, clusterSteps = 0;
+    // whether too many particles change cell for the bands (band_busy): the words
+    // the device reports to, whether an estimate is on its way, the estimates so
+    // far, the packed steps since the last one and those to wait
+    BandLoad* bandLoad = nullptr;
+    bool bandBusy = false, estimated = false;
+    uint32_t estimates = 0, busySteps = 0, busyWait = 0;
     cudaGraphExec_t bandLoop[2][2][kBandPasses] = {}, bandFollow[2][2][kBandPasses] = {};
     cudaGraphExec_t bandRec[2][2][kBandPasses] = {};  // recording every step for the adjoint
     cudaGraphExec_t bandOne[2][2] = {}, bandSort[2][2] = {};
@@ -481,6 +487,9 @@ KParams scene_kparams(const DemContext* c, uint32_t n) {
     }
     return P;
 }
+
+// Packed steps until the movers are looked at again (band_busy).
+constexpr uint32_t kBusySteps = 256;
 
 // The state or its cells are new: keys are recomputed and the next step sorts
 // from scratch.
@@ -1161,6 +1170,7 @@ extern "C" int dem_destroy(DemContext* c) {
     dev_free(c->incScratch);
     dev_free(c->sortScratch);
     dev_free(c->block);
+    if (c->bandLoad) cudaFreeHost(c->bandLoad);
     delete c;
     return DEM_OK;
 }
@@ -1234,26 +1244,42 @@ int check_count(const DemContext* c, uint32_t n) {
 bool has_state_sets(const DemContext* c) { return c->dyn[0].pos != nullptr; }
 
 // A new state of n particles is in the current sets (set c->cur, positions
-// in dyn[0].pos): clears the error word, reads the largest radius back and
-// keeps or drops the captured graphs.
+// in dyn[0].pos): clears the error word, reads the largest radius and the
+// expected movers back and keeps or drops the captured graphs.
 bool steps_in_bands(DemContext* c);
+int band_init(DemContext* c, cudaStream_t st);
+cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st);
+bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
     // the band arrays, unless the cluster launch will step this scene at first
     if (!(c->flags & DEM_CTX_RESIDENT) || c->nspec || !cluster_scene_fits(n, c->numCells))
         steps_in_bands(c);
-    // the new state replaces the one any recorded error was about
-    DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 4, st), "clear error word");
+    // the new state replaces the one any recorded error was about; the words
+    // behind the error word: the largest radius, the bands with expected movers,
+    // the movers
+    DEM_TRY_CUDA(cudaMemsetAsync(c->errFlag, 0, 16, st), "clear error word");
     const int a = c->cur;
     // the largest radius bounds every contact distance (neighbour culling)
-    uint32_t rbits = 0;
     DEM_TRY_CUDA(launch_max_radius(c->stat[a].radius, n, c->errFlag + 1, st), "max radius");
-    DEM_TRY_CUDA(cudaMemcpyAsync(&rbits, c->errFlag + 1, 4, cudaMemcpyDeviceToHost, st),
+    const bool bands = c->bandBlock && c->dyn[0].pos == c->ownPos;
+    if (bands) {
+        const int rc = band_init(c, st);
+        if (rc) return rc;
+        DEM_TRY_CUDA(estimate_movers(c, n, st), "expected movers");
+    }
+    uint32_t word[3] = {};
+    DEM_TRY_CUDA(cudaMemcpyAsync(word, c->errFlag + 1, sizeof(word), cudaMemcpyDeviceToHost, st),
                  "max radius copy");
     DEM_TRY_CUDA(cudaStreamSynchronize(st), "set_state sync");
+    if (c->bandLoad) c->bandLoad->dirty = kBandUnknown;
+    c->estimated = false;
+    c->busySteps = 0;
+    c->busyWait = kBusySteps;
     float rmax;
-    memcpy(&rmax, &rbits, 4);
+    memcpy(&rmax, &word[0], 4);
     rmax = (n > 0 && std::isfinite(rmax)) ? rmax : INFINITY;
+    c->bandBusy = bands && too_many_movers(c, n, word[1], word[2]);
     // the same particle count and largest radius give the same kernel
     // parameters (and specimen table), so the captured graphs stay valid;
     // only the first step's full sort is forced, as after every new state
@@ -1494,6 +1520,93 @@ bool steps_in_bands(DemContext* c) {
     carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel, c->nspec != 0);
     c->band.table = c->dTable;  // null for a single scene
     c->band.errFlag = c->errFlag;
+    // (without these words the bands are left and entered at a new state only)
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, sizeof(BandLoad), cudaHostAllocMapped) == cudaSuccess) {
+        c->bandLoad = static_cast<BandLoad*>(h);
+        c->bandLoad->dirty = kBandUnknown;
+        if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess)
+            c->band.load = static_cast<BandLoad*>(d);
+    }
+    (void)cudaGetLastError();
+    return true;
+}
+
+// What the band arrays hold from the start.
+int band_init(DemContext* c, cudaStream_t st) {
+    if (c->bandInit) return DEM_OK;
+    // stamps start below the first step's number
+    DEM_TRY_CUDA(cudaMemsetAsync(c->band.stamp, 0, 4ull * c->band.cells, st), "band stamps");
+    DEM_TRY_CUDA(cudaMemsetAsync(c->band.mark, 0, 4ull * c->band.bands, st), "band marks");
+    DEM_TRY_CUDA(cudaMemcpyAsync(const_cast<BandGeo*>(c->band.geo), c->bandGeo.data(),
+                                 sizeof(BandGeo) * c->bandGeo.size(), cudaMemcpyHostToDevice, st),
+                 "bands");
+    if (c->band.cellBand) DEM_TRY_CUDA(launch_band_cell_table(c->band, st), "band cells");
+    DEM_TRY_CUDA(cudaMemsetAsync(c->band.ctrl, 0, 4 * kBandCtrlWords, st), "band words");
+    DEM_TRY_CUDA(launch_set_words(c->band.ctrl + kBandStep, Words{{1u}, 1u}, st), "band step");
+    c->bandInit = true;
+    return DEM_OK;
+}
+
+// The words behind the largest radius: bands with expected movers, movers.
+cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st) {
+    return launch_band_estimate(c->P, c->band, c->dyn[0].pos, c->dyn[c->cur].vel, c->spec, n,
+                                ++c->estimates, c->errFlag + 2, st);
+}
+
+// Where the bands lose to the packed path's incremental sort, which moves every
+// particle but takes movers up to n / 8.  A fix rewrites a band for one mover
+// as for twenty: up to kFixBlocks bands that is one round of blocks, beyond it
+// costs what it moves.  With nearly all bands rewritten (0.9, at 1.5 movers a
+// band) the two meet -- us a step, bands against packed, at 1.0 / 2.0 / 4.9 movers
+// a band of 1,000,003 disks: 73 / 91 / 114 against 83 / 87 / 93; at 1.0 / 2.0 / 9.8 of
+// 4,194,304: 214 / 274 / 427 against 258 / 282 / 338; at 1.0 / 2.4 / 7.2 of 262,144:
+// 32 / 38 / 45 against 33 / 36 / 39.  And a band that runs out of free slots or
+// events makes every step a layout: at 14 movers a band of 65,536 disks (64
+// free slots) 28.6 against 29.3 us, at 29 of 262,144 116 against 47.
+bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers) {
+    const uint32_t b = c->band.bands;
+    return (b > kFixBlocks && dirty > b - b / 10) || movers > (uint64_t)b * (band_slack(c->band, n) / 4);
+}
+
+// Whether a call of `nsteps` steps stays on the packed path for its movers.  The
+// state was looked at when it was set; since then the calls in bands report the
+// bands they rewrote and their layouts, and on the packed path an estimate is
+// asked for every busyWait steps (more each time the bands were entered in
+// vain).  The words arrive when they do: the path never changes the bits.
+bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
+    if (!c->bandLoad) return c->bandBusy;
+    const volatile BandLoad* w = c->bandLoad;
+    const uint32_t b = c->band.bands;
+    if (!c->bandBusy) {
+        const uint32_t dirty = w->dirty;
+        if (dirty == kBandUnknown || !((b > kFixBlocks && dirty > b - b / 10) || w->layouts >= 4u))
+            return false;
+        c->bandBusy = true;
+        c->estimated = false;
+        c->busySteps = 0;
+        c->busyWait = std::min(2u * c->busyWait, 16u * kBusySteps);
+        return true;
+    }
+    c->busySteps += std::min(nsteps, 16u * kBusySteps);
+    if (c->estimated) {
+        const uint32_t dirty = w->estDirty, movers = w->estMovers;
+        if (dirty == kBandUnknown || movers == kBandUnknown) return true;
+        c->estimated = false;
+        // back with a tenth to spare
+        if (too_many_movers(c, c->n, dirty + dirty / 10, movers + movers / 10)) return true;
+        c->bandBusy = false;
+        c->bandLoad->dirty = kBandUnknown;
+        return false;
+    }
+    if (c->busySteps >= c->busyWait) {
+        c->busySteps = 0;
+        c->bandLoad->estDirty = c->bandLoad->estMovers = kBandUnknown;
+        c->estimated = cudaMemsetAsync(c->errFlag + 2, 0, 8, st) == cudaSuccess &&
+                       estimate_movers(c, c->n, st) == cudaSuccess &&
+                       cudaMemcpyAsync(&c->bandLoad->estDirty, c->errFlag + 2, 8,
+                                       cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    }
     return true;
 }
 
@@ -1507,9 +1620,10 @@ bool steps_in_bands(DemContext* c) {
 // kShortRun short calls in a row leave the bands.  A batch gains more by a step
 // in bands (63 against 42 us, 256 specimens of two materials): three steps do.
 constexpr uint32_t kShortCall = 4, kShortBatchCall = 3, kPackedSteps = 16, kShortRun = 16;
-bool band_call(DemContext* c, uint32_t nsteps) {
+bool band_call(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (!steps_in_bands(c)) return false;
     if (c->profiling || c->tuned < 0) return true;  // the bands' kernels are what is timed
+    if (band_busy(c, nsteps, st)) return false;
     const bool packedOrder = c->keysValid && c->haveOrder;
     if (nsteps >= (c->nspec ? kShortBatchCall : kShortCall)) {
         c->shortCalls = 0;
@@ -1676,16 +1790,8 @@ int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t s
     c->band.slack = band_slack(c->band, c->n);
     c->band.slots = (uint32_t)band_slots(c->band, c->n);
     c->band.skin = std::isfinite(c->rmax) ? kSkin * c->rmax : 0.0f;
-    if (!c->bandInit) {
-        // stamps start below the first step's number
-        DEM_TRY_CUDA(cudaMemsetAsync(c->band.stamp, 0, 4ull * c->band.cells, st), "band stamps");
-        DEM_TRY_CUDA(cudaMemcpyAsync(const_cast<BandGeo*>(c->band.geo), c->bandGeo.data(),
-                                     sizeof(BandGeo) * c->bandGeo.size(), cudaMemcpyHostToDevice, st),
-                     "bands");
-        if (c->band.cellBand) DEM_TRY_CUDA(launch_band_cell_table(c->band, st), "band cells");
-        DEM_TRY_CUDA(launch_set_words(c->band.ctrl + kBandStep, Words{{1u}, 1u}, st), "band step");
-        c->bandInit = true;
-    }
+    const int rc = band_init(c, st);
+    if (rc) return rc;
     const Words w = c->bandValid ? Words{{nsteps, rowBlock}, 2u}
                                  : Words{{nsteps, rowBlock, 1u, (uint32_t)c->bandSet, 0u}, 5u};
     DEM_TRY_CUDA(launch_set_words(c->band.ctrl, w, st), "band step count");
@@ -2004,7 +2110,7 @@ int packed_steps(DemContext* c, uint32_t nsteps, cudaStream_t st);
 
 // dem_step on the graph path.
 int step_graph_path(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    return band_call(c, nsteps) ? band_steps(c, nsteps, BandAfter::kNothing, 0, st)
+    return band_call(c, nsteps, st) ? band_steps(c, nsteps, BandAfter::kNothing, 0, st)
                                 : packed_steps(c, nsteps, st);
 }
 
@@ -2194,7 +2300,7 @@ extern "C" int dem_kernels_per_step(DemContext* c) {
     if (!c) return -1;
     // band_fix_kernel, band_step_kernel; with a control particle the gaps, the
     // reduction and the move too
-    if (steps_in_bands(c)) return c->ctlOn ? 5 : 2;
+    if (steps_in_bands(c) && !c->bandBusy) return c->ctlOn ? 5 : 2;
     if (!c->sortGraph[1][0] && c->n > 0) {
         if (build_graph(c, 1, 0) != DEM_OK) return -1;
     }
@@ -2288,7 +2394,7 @@ extern "C" int dem_step_followed(DemContext* c, uint32_t nsteps, const uint32_t*
     for (uint32_t s = 0; s < nsteps;) {
         const uint32_t m = std::min(chunk, nsteps - s);
         const bool alone = (c->flags & DEM_CTX_DIRECT) || c->profiling || c->tuned < 0;
-        if (!alone && band_call(c, m)) {
+        if (!alone && band_call(c, m, st)) {
             int rc = band_steps(c, m, BandAfter::kFollowed, 0, st);
             if (rc) return rc;
         } else for (uint32_t j = 0; j < m;) {

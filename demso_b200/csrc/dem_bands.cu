@@ -213,6 +213,10 @@ band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynS
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         B.ctrl[kBandAct + q] = active ? (c.x == 1u ? 2u : 1u) : 0u;
         B.ctrl[kBandNow + q] = B.ctrl[kBandStep];
+        if (active) {
+            atomicAdd(B.ctrl + kBandDirtySum, nd);
+            atomicAdd(B.ctrl + kBandFixes, 1u);
+        }
     }
     if (!active) return;
     for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
@@ -624,6 +628,15 @@ __global__ void __launch_bounds__(kPackThreads)
 band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     if (B.ctrl[kBandLaid] == 0u) return;
     const uint32_t b = blockIdx.x;
+    if (!stateOnly && b == 0u && blockIdx.y == 0u && threadIdx.x == 0u) {
+        const uint32_t fixes = B.ctrl[kBandFixes], layouts = B.ctrl[kBandLayouts];
+        if (fixes && B.load) {
+            volatile BandLoad* w = B.load;
+            w->dirty = B.ctrl[kBandDirtySum] / fixes;
+            w->layouts = (uint32_t)min(16ull * layouts / fixes, 16ull);
+        }
+        B.ctrl[kBandDirtySum] = B.ctrl[kBandFixes] = B.ctrl[kBandLayouts] = 0u;
+    }
     const uint32_t base = B.base[b], cnt = B.count[b];
     const uint32_t to = packed_base(B, b, B.geo[b]);
     const bool one = B.ctrl[kBandCur] != 0u;
@@ -765,6 +778,32 @@ __global__ void __launch_bounds__(kPackThreads) band_cell_table_kernel(BandArgs 
         B.cellBand[geo.cell0 + c] = blockIdx.x;
 }
 
+// See launch_band_estimate.  Bound by DRAM: position and velocity, 16 B a
+// particle.
+__global__ void __launch_bounds__(kPackThreads)
+band_estimate_kernel(const __grid_constant__ KParams P0, BandArgs B, const float2* __restrict__ pos,
+                     const float2* __restrict__ vel, const uint32_t* __restrict__ spec, uint32_t n,
+                     uint32_t serial, uint32_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
+    bool moves = false;
+    if (i < n) {
+        const KParams& P = spec ? B.table[spec[i]] : P0;
+        const float2 p = pos[i], v = vel[i];
+        const int2 g0 = grid_pos_fast(P, p);
+        const int2 g1 = grid_pos_fast(P, make_float2(p.x + v.x * P.dt, p.y + v.y * P.dt));
+        const uint32_t c[2] = {grid_hash(P, g0.x, g0.y), grid_hash(P, g1.x, g1.y)};
+        moves = c[0] != c[1];
+        for (int k = 0; k < 2 && moves; ++k) {
+            uint32_t* m = B.mark + band_of(B, c[k]);
+            if (*reinterpret_cast<volatile uint32_t*>(m) != serial &&
+                atomicExch(m, serial) != serial)
+                atomicAdd(out, 1u);
+        }
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, moves);
+    if ((threadIdx.x & 31u) == 0u && all) atomicAdd(out + 1, (uint32_t)__popc(all));
+}
+
 // The packed particles, in sorted order, into the slots of the current set.
 template <bool TYPED>
 __global__ void __launch_bounds__(kPackThreads)
@@ -772,6 +811,7 @@ band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys
                    const uint32_t* __restrict__ from) {
     const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
     if (i == 0u) {
+        if (B.ctrl[kBandLaid]) B.ctrl[kBandLayouts] += 1u;
         B.ctrl[kBandFull] = 0u;
         B.ctrl[kBandLaid] = 1u;
         B.ctrl[kBandDirty] = 0u;
@@ -913,6 +953,7 @@ void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool
     b.grown = static_cast<float*>(take(4ull * b.bands));
     b.search = static_cast<uint32_t*>(take(4ull * b.bands));
     b.ctrl = static_cast<uint32_t*>(take(4 * kBandCtrlWords));
+    b.mark = static_cast<uint32_t*>(take(4ull * b.bands));
     b.pressure = pressure ? static_cast<float*>(take(4 * S)) : nullptr;
     b.acc = accel ? static_cast<float2*>(take(8 * S)) : nullptr;
     b.alpha = accel ? static_cast<float*>(take(4 * S)) : nullptr;
@@ -945,8 +986,17 @@ cudaError_t launch_band_cell_table(const BandArgs& b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+cudaError_t launch_band_estimate(const KParams& P, const BandArgs& b, const float2* pos,
+                                 const float2* vel, const uint32_t* spec, uint32_t n,
+                                 uint32_t serial, uint32_t* out, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    band_estimate_kernel<<<blocks_for(n, kPackThreads), kPackThreads, 0, st>>>(P, b, pos, vel, spec,
+                                                                              n, serial, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st) {
-    const unsigned blocks = std::min(b.bands, 296u);  // two to a multiprocessor
+    const unsigned blocks = std::min(b.bands, kFixBlocks);
     if (b.stat.type)
         band_fix_kernel<true><<<blocks, kFixThreads, 0, st>>>(b, b.dyn[q], (uint32_t)q);
     else

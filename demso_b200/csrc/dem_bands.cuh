@@ -69,7 +69,13 @@ constexpr uint32_t kBandAct = 5;    // [2] step of set q: 0 skipped, 1 runs, 2 r
 constexpr uint32_t kBandDirty = 7;  // [2] bands with events, by the set the fix of which takes them
 constexpr uint32_t kBandStep = 9;   // steps since the context was made
 constexpr uint32_t kBandNow = 10;   // [2] kBandStep as the step of set q sees it
+constexpr uint32_t kBandDirtySum = 12;  // since the last pack of a call: bands the fixes rewrote,
+constexpr uint32_t kBandFixes = 13;     // fixes,
+constexpr uint32_t kBandLayouts = 14;   // layouts of a state that was in bands already
 constexpr uint32_t kBandCtrlWords = 16;
+// Blocks of the fix: that many bands are rewritten at once (two blocks to a
+// multiprocessor).
+constexpr uint32_t kFixBlocks = 296;
 
 // Kept candidates.  The search for neighbours (row intervals, radii and
 // distances of some twenty candidates) finds almost the same few pairs step
@@ -103,6 +109,16 @@ struct BandGeo {
     uint32_t sceneBand, scenePart, spec, pad;
 };
 
+// Words in host memory that the device writes for the host to read whenever they
+// arrive; kBandUnknown until then.
+constexpr uint32_t kBandUnknown = 0xffffffffu;
+struct BandLoad {
+    // the last call in bands: bands rewritten a step, layouts in 16 steps
+    uint32_t dirty, layouts;
+    // the last estimate (launch_band_estimate)
+    uint32_t estDirty, estMovers;
+};
+
 struct BandArgs {
     uint32_t bands = 0, shift = 0;  // band of a cell of a single scene: cell >> shift
     uint32_t cells = 0, firstWords = 0;
@@ -130,6 +146,8 @@ struct BandArgs {
     float* grown = nullptr;         // per band: bound on a pair's approach since the search
     uint32_t* search = nullptr;     // per band: this step searches anew
     uint32_t* ctrl = nullptr;
+    uint32_t* mark = nullptr;  // per band: the last estimate (launch_band_estimate) that met it
+    BandLoad* load = nullptr;  // may be null: dirty and layouts, written by a call's pack
     float* pressure = nullptr;  // slot-indexed, null when not kept
     float2* acc = nullptr;
     float* alpha = nullptr;
@@ -162,6 +180,13 @@ void carve_bands(BandArgs& b, void* base, uint32_t capacity, bool typed, bool pr
 
 // Band of every cell of a batch (once, after the arrays are made).
 cudaError_t launch_band_cell_table(const BandArgs& b, cudaStream_t st);
+
+// Adds to out[0] the bands that particles would leave or enter if all moved on
+// by a step at their velocities, to out[1] the particles; `serial`: another
+// number each time.  spec: a batch's specimen of every packed slot.
+cudaError_t launch_band_estimate(const KParams& P, const BandArgs& b, const float2* pos,
+                                 const float2* vel, const uint32_t* spec, uint32_t n,
+                                 uint32_t serial, uint32_t* out, cudaStream_t st);
 
 // The kernels; `q` is the dynamic set they step from.
 cudaError_t launch_band_fix(const BandArgs& b, int q, cudaStream_t st);

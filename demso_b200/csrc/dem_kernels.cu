@@ -538,8 +538,7 @@ cudaError_t launch_followed_ring(const uint32_t* ids, const uint32_t* countWord,
 }
 
 cudaError_t launch_max_radius(const float* radius, uint32_t n, uint32_t* out, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess || n == 0) return e;
+    if (n == 0) return cudaSuccess;
     const unsigned b = blocks_for(n, kThreads) < 1184 ? blocks_for(n, kThreads) : 1184;
     max_radius_kernel<<<b, kThreads, 0, st>>>(radius, n, out);
     return cudaGetLastError();

@@ -62,6 +62,7 @@ cudaError_t launch_followed_ring(const uint32_t* ids, const uint32_t* countWord,
                                  const float* pressure, float* ring, cudaStream_t st);
 
 // Upper bound of the radii: writes the largest radius's bit pattern to *out.
+// Raises *out to the bits of the largest radius.
 cudaError_t launch_max_radius(const float* radius, uint32_t n, uint32_t* out, cudaStream_t st);
 
 cudaError_t launch_calc_hash(const KParams& P, const float2* pos, uint32_t* hash, uint32_t* index,
