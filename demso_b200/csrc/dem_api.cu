@@ -1566,7 +1566,8 @@ cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st) {
 // free slots) 28.6 against 29.3 us, at 29 of 262,144 116 against 47.
 bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers) {
     const uint32_t b = c->band.bands;
-    return (b > kFixBlocks && dirty > b - b / 10) || movers > (uint64_t)b * (band_slack(c->band, n) / 4);
+    const uint32_t slack = c->nspec ? kBandMinSlack : band_slack(c->band, n);
+    return (b > kFixBlocks && dirty > b - b / 10) || movers > (uint64_t)b * (slack / 4);
 }
 
 // Whether a call of `nsteps` steps stays on the packed path for its movers.  The
@@ -1788,7 +1789,7 @@ int build_band_graph(DemContext* c, Body body, cudaGraphExec_t* out) {
 int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t st) {
     c->band.n = c->n;
     c->band.slack = band_slack(c->band, c->n);
-    c->band.slots = (uint32_t)band_slots(c->band, c->n);
+    c->band.slots = (uint32_t)band_slots(c->band, c->n, c->nspec != 0);
     c->band.skin = std::isfinite(c->rmax) ? kSkin * c->rmax : 0.0f;
     const int rc = band_init(c, st);
     if (rc) return rc;

@@ -27,6 +27,11 @@ __device__ __forceinline__ uint32_t band_of(const BandArgs& B, uint32_t cell) {
     return B.cellBand ? __ldg(B.cellBand + cell) : cell >> B.shift;
 }
 
+// Free slots before band b.
+__device__ __forceinline__ uint32_t free_before(const BandArgs& B, uint32_t b) {
+    return B.table ? B.geo[b].free & ~kBandWhole : b * B.slack;
+}
+
 // ------------------------------------------------------------------ fix
 // Bound by latency: four rounds of loads (the control words; the band's words
 // and events; its cells' first slots; its fields), each begun together: 153.8 ->
@@ -253,7 +258,8 @@ __device__ __forceinline__ BandEvent* push_event(const BandArgs& B, uint32_t b, 
         const uint32_t w = atomicAdd(B.ctrl + kBandDirty + nextSet, 1u);
         if (w < B.bands) B.dirty[nextSet][w] = b;
     }
-    const uint32_t room = B.base[b + 1u] - B.base[b] - B.count[b];
+    uint32_t room = B.base[b + 1u] - B.base[b] - B.count[b];
+    if (B.table && (B.geo[b].free & kBandWhole)) room = kBandEvents;
     if (k >= min(kBandEvents, room)) {
         B.ctrl[kBandFull] = 1u;
         return nullptr;
@@ -749,7 +755,8 @@ band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
     const uint32_t b = blockIdx.x, tid = threadIdx.x;
     const BandGeo geo = B.geo[b];
     const uint32_t p = f[geo.cell0], e = f[geo.cell0 + geo.cells];
-    const uint32_t base = min(p + b * B.slack, B.slots);
+    const uint32_t before = free_before(B, b);
+    const uint32_t base = min(p + before, B.slots);
     // e < p only after a sort whose wait gave up
     if (tid == 0) {
         B.base[b] = base;
@@ -768,7 +775,7 @@ band_layout_kernel(BandArgs B, const uint32_t* __restrict__ f) {
     const uint32_t gx = 1u << geo.log2gx, words = (geo.cells >> geo.log2gx) * (gx + 1u);
     for (uint32_t k = tid; k < words; k += kPackThreads) {
         const uint32_t row = k / (gx + 1u), x = k - row * (gx + 1u);
-        B.first[geo.first + k] = f[geo.cell0 + row * gx + x] + b * B.slack;
+        B.first[geo.first + k] = f[geo.cell0 + row * gx + x] + before;
     }
 }
 
@@ -820,7 +827,7 @@ band_spread_kernel(BandArgs B, PackedState in, const uint32_t* __restrict__ keys
     if (i >= B.n) return;
     // in range unless a wait of the sort gave up (stale words)
     const uint32_t key = min(keys[i], B.cells - 1u), src = min(from[i], B.n - 1u);
-    const uint32_t band = band_of(B, key), s = i + band * B.slack;
+    const uint32_t band = band_of(B, key), s = i + free_before(B, band);
     // a specimen's slots are its own: the fixes keep within a band
     if (B.slotSpec) B.slotSpec[s] = B.geo[band].spec;
     const bool one = B.ctrl[kBandCur] != 0u;
@@ -884,7 +891,7 @@ bool attracts(const KParams& P) {
 bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, bool batch,
                 BandArgs& b, std::vector<BandGeo>& geo) {
     geo.clear();
-    uint64_t cell = 0, first = 0, part = 0;
+    uint64_t cell = 0, first = 0, part = 0, free = 0;
     for (size_t s = 0; s < P.size(); ++s) {
         const uint32_t gx = P[s].gx, cells = P[s].gx * P[s].gy;
         if (gx > kBandMaxRow) return false;
@@ -892,18 +899,22 @@ bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, boo
         while (!batch && (uint64_t)per * kBandMaxBands < cells) per <<= 1;
         per = std::min(per, cells);  // both powers of two
         P[s].firstOff = (uint32_t)first;
-        const uint32_t sceneBand = (uint32_t)geo.size();
+        const uint32_t sceneBand = (uint32_t)geo.size(), bands = cells / per;
+        const uint32_t slack = bands == 1u ? 0u : std::max(kBandMinSlack, count[s] / (16u * bands));
         for (uint32_t c = 0; c < cells; c += per) {
             geo.push_back(BandGeo{(uint32_t)cell + c, per, (uint32_t)(first + (c / gx) * (gx + 1ull)),
-                                  P[s].log2gx, sceneBand, (uint32_t)part, (uint32_t)s, 0u});
+                                  P[s].log2gx, sceneBand, (uint32_t)part, (uint32_t)s,
+                                  (uint32_t)free | (bands == 1u ? kBandWhole : 0u)});
+            free += slack;
         }
         b.shift = 0;
         while ((1u << b.shift) < per) ++b.shift;
         cell += cells;
         first += (uint64_t)P[s].gy * (gx + 1ull);
         part += count[s];
-        if (first >= (1ull << 32)) return false;
+        if (first >= (1ull << 32) || free >= kBandWhole) return false;
     }
+    b.batchFree = batch ? (uint32_t)free : 0u;
     b.cells = (uint32_t)cell;
     b.firstWords = (uint32_t)first;
     b.bands = (uint32_t)geo.size();
@@ -913,8 +924,8 @@ bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, boo
 uint32_t band_slack(const BandArgs& b, uint32_t n) {
     return std::max(kBandMinSlack, n / (16u * b.bands));
 }
-size_t band_slots(const BandArgs& b, uint32_t n) {
-    return (size_t)n + (size_t)b.bands * band_slack(b, n);
+size_t band_slots(const BandArgs& b, uint32_t n, bool batch) {
+    return (size_t)n + (batch ? b.batchFree : (size_t)b.bands * band_slack(b, n));
 }
 
 namespace {
@@ -922,7 +933,7 @@ namespace {
 template <typename Take>
 void band_arrays(BandArgs& b, uint32_t capacity, bool typed, bool pressure, bool accel, bool batch,
                  Take take) {
-    const size_t S = band_slots(b, capacity) + kFilterPad;
+    const size_t S = band_slots(b, capacity, batch) + kFilterPad;
     for (int k = 0; k < 2; ++k) {
         b.dyn[k].pos = static_cast<float2*>(take(8 * S));
         b.dyn[k].vel = static_cast<float2*>(take(8 * S));
