@@ -231,12 +231,21 @@ band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynS
     }
     // how far pairs may have approached since their bands searched, by the
     // blocks from the last on (the first ones have the events).  A pair's bands
-    // are the same or beside each other, the first and the last one too (rows
-    // across the grid's wrap are out of reach in a whole scene; a disk that
-    // left a window of rows is met there).
+    // are the same or beside each other, the first and the last one of a scene
+    // too: a disk that left a window of rows is met across the grid's wrap, and
+    // so is one pushed against the top wall whose radius the wall's height
+    // swallows (Ly - r == Ly is in the row behind the last).
     for (uint32_t b = (gridDim.x - 1u - blockIdx.x) * kFixThreads + threadIdx.x; b < B.bands;
          b += gridDim.x * kFixThreads) {
-        const uint32_t lo = (b ? b : B.bands) - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
+        uint32_t lo = (b ? b : B.bands) - 1u, hi = b + 1u < B.bands ? b + 1u : 0u;
+        if (B.table) {
+            const BandGeo g = B.geo[b];
+            if (b == g.sceneBand) {
+                const KParams& P = B.table[g.spec];
+                lo = b + (P.gx * P.gy) / g.cells - 1u;
+            }
+            if (hi == 0u || B.geo[hi].sceneBand == hi) hi = g.sceneBand;
+        }
         const float own = __uint_as_float(B.moved[q][b]);
         // as bits, so that a NaN is the largest
         const float any = __uint_as_float(max(B.moved[q][b], max(B.moved[q][lo], B.moved[q][hi])));
