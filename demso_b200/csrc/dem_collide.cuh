@@ -199,12 +199,13 @@ __device__ __forceinline__ void deal_law(const KParams& P0, const KParams* __res
             const float rB = __ldg(radius + j);
             float2 f;
             float m, flen;
-            pair_terms(pA, pB, vA, __ldg(vel + sj), wA, __ldg(omega + sj), rA, rB, pc, P.dt, f, m,
-                       flen);
+            const bool touch = pair_terms(pA, pB, vA, __ldg(vel + sj), wA, __ldg(omega + sj), rA,
+                                          rB, pc, P.dt, f, m, flen);
             S.j[code] = __float_as_uint(f.x);
             S.fy[code] = f.y;
             S.moment[code] = m;
-            if (wantPr) S.q[code] = flen != 0.0f ? pressure_term(flen, rA) : 0.0;
+            // (a touching disk without a radius: 0 / 0, as the reference has it)
+            if (wantPr) S.q[code] = touch ? pressure_term(flen, rA) : 0.0;
             if (ATTRACT) {
                 const float2 g = pair_attract_terms(pA, pB, rA, rB, P.at[mA], P.at[mB]);
                 S.ax[code] = g.x;
