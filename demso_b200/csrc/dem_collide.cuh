@@ -106,8 +106,10 @@ __device__ __forceinline__ uint32_t filter8(const float2* __restrict__ pq,
             const float2 c2 = f32x2_mul(cd, cd);
             bound = f32x2_fma(c2, make_float2(2e-6f, 2e-6f), c2);
         }
-        if (d2a <= bound.x) m8 |= 1u << k;
-        if (d2b <= bound.y) m8 |= 2u << k;
+        // (with attraction a distance that is not a number stays: it adds 0 / (4 pi
+        // r^2) to the pressure, which is one to a disk without a radius)
+        if (ATTRACT ? !(d2a > bound.x) : d2a <= bound.x) m8 |= 1u << k;
+        if (ATTRACT ? !(d2b > bound.y) : d2b <= bound.y) m8 |= 2u << k;
     }
     return m8;
 }

@@ -153,7 +153,8 @@ collide_kernel(const __grid_constant__ KParams P, const float2* __restrict__ pos
                             const float rq = __ldg(radius + a + k);
                             const float dx = q.x - p.x, dq = q.y - p.y;
                             const float d2 = dx * dx + dq * dq, cd = r + rq;
-                            if (d2 <= (ATTRACT ? attract_reach2(r, rq) : cd * cd * 1.000002f))
+                            if (ATTRACT ? !attract_out_of_reach(r, rq, d2)
+                                        : d2 <= cd * cd * 1.000002f)
                                 hits |= 1u << k;
                         }
                     }

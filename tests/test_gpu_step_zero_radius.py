@@ -29,3 +29,18 @@ def test_pressure_of_a_disk_without_a_radius():
     st = gpu_stages(sc.sys, sc.state())
     ref = PortOracle("f32").run(sc.sys, sc.state(), 1)
     assert same(st["int_pressure"], ref["pressure"])
+
+
+@pytest.mark.parametrize("n", [3, 40])
+def test_attraction_beside_a_position_that_is_no_number(n):
+    # through the five stages, whose cell ranges hold the disk; 40: groups of eight
+    sc = scenes.agitated_gas(n=n, seed=2, grid=(4, 4), box=0.012, gravity=(0.0, 0.0),
+                             attraction=20.0)
+    sc.radius[0] = 0.0
+    sc.pos[1] = [np.nan, np.nan]
+    sc.vel[:] = 0.0
+    sc.omega[:] = 0.0
+    st = gpu_stages(sc.sys, sc.state())
+    ref = PortOracle("f32").run(sc.sys, sc.state(), 1)
+    assert np.isnan(ref["pressure"]).any()
+    assert same(st["int_pressure"], ref["pressure"])
