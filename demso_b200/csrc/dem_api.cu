@@ -1272,7 +1272,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     DEM_TRY_CUDA(cudaMemcpyAsync(word, c->errFlag + 1, sizeof(word), cudaMemcpyDeviceToHost, st),
                  "max radius copy");
     DEM_TRY_CUDA(cudaStreamSynchronize(st), "set_state sync");
-    if (c->bandLoad) c->bandLoad->dirty = kBandUnknown;
+    if (c->bandLoad) c->bandLoad->busy = 0u;
     c->estimated = false;
     c->busySteps = 0;
     c->busyWait = kBusySteps;
@@ -1524,7 +1524,7 @@ bool steps_in_bands(DemContext* c) {
     void *h = nullptr, *d = nullptr;
     if (cudaHostAlloc(&h, sizeof(BandLoad), cudaHostAllocMapped) == cudaSuccess) {
         c->bandLoad = static_cast<BandLoad*>(h);
-        c->bandLoad->dirty = kBandUnknown;
+        c->bandLoad->busy = 0u;
         if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess)
             c->band.load = static_cast<BandLoad*>(d);
     }
@@ -1567,22 +1567,20 @@ cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st) {
 bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers) {
     const uint32_t b = c->band.bands;
     const uint32_t slack = c->nspec ? kBandMinSlack : band_slack(c->band, n);
-    return (b > kFixBlocks && dirty > b - b / 10) || movers > (uint64_t)b * (slack / 4);
+    return band_overload(b, dirty) || movers > (uint64_t)b * (slack / 4);
 }
 
 // Whether a call of `nsteps` steps stays on the packed path for its movers.  The
-// state was looked at when it was set; since then the calls in bands report the
-// bands they rewrote and their layouts, and on the packed path an estimate is
-// asked for every busyWait steps (more each time the bands were entered in
-// vain).  The words arrive when they do: the path never changes the bits.
+// state was looked at when it was set; since then a call in bands reports when
+// it rewrote nearly all of them a step or laid out on a quarter of its steps,
+// and on the packed path an estimate is asked for every busyWait steps (more
+// each time the bands were entered in vain).  The words arrive when they do:
+// the path never changes the bits.
 bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (!c->bandLoad) return c->bandBusy;
     const volatile BandLoad* w = c->bandLoad;
-    const uint32_t b = c->band.bands;
     if (!c->bandBusy) {
-        const uint32_t dirty = w->dirty;
-        if (dirty == kBandUnknown || !((b > kFixBlocks && dirty > b - b / 10) || w->layouts >= 4u))
-            return false;
+        if (w->busy == 0u) return false;
         c->bandBusy = true;
         c->estimated = false;
         c->busySteps = 0;
@@ -1597,7 +1595,7 @@ bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
         // back with a tenth to spare
         if (too_many_movers(c, c->n, dirty + dirty / 10, movers + movers / 10)) return true;
         c->bandBusy = false;
-        c->bandLoad->dirty = kBandUnknown;
+        c->bandLoad->busy = 0u;
         return false;
     }
     if (c->busySteps >= c->busyWait) {

@@ -644,12 +644,12 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     if (B.ctrl[kBandLaid] == 0u) return;
     const uint32_t b = blockIdx.x;
     if (!stateOnly && b == 0u && blockIdx.y == 0u && threadIdx.x == 0u) {
+        // a write to host memory costs the call 4 us: only the news is written
         const uint32_t fixes = B.ctrl[kBandFixes], layouts = B.ctrl[kBandLayouts];
-        if (fixes && B.load) {
-            volatile BandLoad* w = B.load;
-            w->dirty = B.ctrl[kBandDirtySum] / fixes;
-            w->layouts = (uint32_t)min(16ull * layouts / fixes, 16ull);
-        }
+        if (fixes && B.load &&
+            (band_overload(B.bands, B.ctrl[kBandDirtySum] / fixes) ||
+             (layouts > 1u && 4u * layouts >= fixes)))
+            *reinterpret_cast<volatile uint32_t*>(&B.load->busy) = 1u;
         B.ctrl[kBandDirtySum] = B.ctrl[kBandFixes] = B.ctrl[kBandLayouts] = 0u;
     }
     const uint32_t base = B.base[b], cnt = B.count[b];

@@ -114,14 +114,13 @@ struct BandGeo {
 constexpr uint32_t kBandWhole = 0x80000000u;
 
 // Words in host memory that the device writes for the host to read whenever they
-// arrive; kBandUnknown until then.
-constexpr uint32_t kBandUnknown = 0xffffffffu;
+// arrive.
 struct BandLoad {
-    // the last call in bands: bands rewritten a step, layouts in 16 steps
-    uint32_t dirty, layouts;
-    // the last estimate (launch_band_estimate)
+    uint32_t busy;  // set by a call whose steps lost to the packed path (band_overload)
+    // the last estimate (launch_band_estimate); kBandUnknown until it arrives
     uint32_t estDirty, estMovers;
 };
+constexpr uint32_t kBandUnknown = 0xffffffffu;
 
 struct BandArgs {
     uint32_t bands = 0, shift = 0;  // band of a cell of a single scene: cell >> shift
@@ -152,7 +151,7 @@ struct BandArgs {
     uint32_t* search = nullptr;     // per band: this step searches anew
     uint32_t* ctrl = nullptr;
     uint32_t* mark = nullptr;  // per band: the last estimate (launch_band_estimate) that met it
-    BandLoad* load = nullptr;  // may be null: dirty and layouts, written by a call's pack
+    BandLoad* load = nullptr;  // may be null: `busy`, set by a call's pack
     float* pressure = nullptr;  // slot-indexed, null when not kept
     float2* acc = nullptr;
     float* alpha = nullptr;
@@ -212,6 +211,10 @@ cudaError_t launch_band_record(const BandArgs& b, int q, void* recBase, size_t s
 // stateOnly); nothing when the bands hold no state.
 cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool stateOnly,
                              cudaStream_t st);
+// Whether nearly all bands are rewritten on every step (see too_many_movers).
+__host__ __device__ inline bool band_overload(uint32_t bands, uint32_t dirty) {
+    return bands > kFixBlocks && dirty > bands - bands / 10u;
+}
 // New layout from the packed arrays, sorted by `keys` (their particles in
 // order `from`); cellFirst: numCells + 1 words of scratch.
 cudaError_t launch_band_layout(const BandArgs& b, const PackedState& in, const uint32_t* keys,
