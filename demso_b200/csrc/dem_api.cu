@@ -407,6 +407,7 @@ struct DemContext {
     // far, the packed steps since the last one and those to wait
     BandLoad* bandLoad = nullptr;
     bool bandBusy = false, estimated = false;
+    bool crowded = false;  // too many particles a cell for kept candidates (crowded_cells)
     uint32_t estimates = 0, busySteps = 0, busyWait = 0;
     cudaGraphExec_t bandLoop[2][2][kBandPasses] = {}, bandFollow[2][2][kBandPasses] = {};
     cudaGraphExec_t bandRec[2][2][kBandPasses] = {};  // recording every step for the adjoint
@@ -1250,6 +1251,7 @@ bool steps_in_bands(DemContext* c);
 int band_init(DemContext* c, cudaStream_t st);
 cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st);
 bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers);
+bool crowded_cells(const DemContext* c, uint32_t n);
 int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     c->inSortOrder = false;
     // the band arrays, unless the cluster launch will step this scene at first
@@ -1280,6 +1282,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     memcpy(&rmax, &word[0], 4);
     rmax = (n > 0 && std::isfinite(rmax)) ? rmax : INFINITY;
     c->bandBusy = bands && too_many_movers(c, n, word[1], word[2]);
+    c->crowded = crowded_cells(c, n);
     // the same particle count and largest radius give the same kernel
     // parameters (and specimen table), so the captured graphs stay valid;
     // only the first step's full sort is forced, as after every new state
@@ -1570,6 +1573,20 @@ bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t m
     return band_overload(b, dirty) || movers > (uint64_t)b * (slack / 4);
 }
 
+// Grids so coarse that the average row interval of three cells holds more
+// particles than it has candidate bits: most slots then search and walk their
+// cells on every step, and a walk of a band's slots is slower than one of the
+// packed order (a call of its own, bands of thousands of particles to rewrite).
+// Below about 8 million candidate tests a step latency decides and the bands
+// still win -- us a step, bands against packed: 65,536 disks, 48 a row 23.1 / 25.8;
+// 131,072, 24 a row 24.3 / 30.6 -- above it they lose: 550,000, 25 a row
+// 48.7 / 45.8 and 101 a row 92.4 / 74.4; 400,000, 73 a row 62.1 / 53.2; 262,144,
+// 48 a row 40.6 / 38.1.  (Grids of cells of about two radii hold 5 to 14.)
+bool crowded_cells(const DemContext* c, uint32_t n) {
+    return 3ull * n > (uint64_t)kCandBits * c->numCells &&
+           3ull * n * n / c->numCells > 8000000ull;
+}
+
 // Whether a call of `nsteps` steps stays on the packed path for its movers.  The
 // state was looked at when it was set; since then a call in bands reports when
 // it rewrote nearly all of them a step or laid out on a quarter of its steps,
@@ -1622,7 +1639,7 @@ constexpr uint32_t kShortCall = 4, kShortBatchCall = 3, kPackedSteps = 16, kShor
 bool band_call(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (!steps_in_bands(c)) return false;
     if (c->profiling || c->tuned < 0) return true;  // the bands' kernels are what is timed
-    if (band_busy(c, nsteps, st)) return false;
+    if (c->crowded || band_busy(c, nsteps, st)) return false;
     const bool packedOrder = c->keysValid && c->haveOrder;
     if (nsteps >= (c->nspec ? kShortBatchCall : kShortCall)) {
         c->shortCalls = 0;
@@ -2299,7 +2316,7 @@ extern "C" int dem_kernels_per_step(DemContext* c) {
     if (!c) return -1;
     // band_fix_kernel, band_step_kernel; with a control particle the gaps, the
     // reduction and the move too
-    if (steps_in_bands(c) && !c->bandBusy) return c->ctlOn ? 5 : 2;
+    if (steps_in_bands(c) && !c->bandBusy && !c->crowded) return c->ctlOn ? 5 : 2;
     if (!c->sortGraph[1][0] && c->n > 0) {
         if (build_graph(c, 1, 0) != DEM_OK) return -1;
     }

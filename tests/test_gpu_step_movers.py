@@ -118,3 +118,16 @@ def test_followed_rows_and_a_batch_with_many_movers():
         r = ref.run(parts[k].sys, parts[k].state(), 9)
         for x in ("pos", "vel", "theta", "omega", "pressure"):
             assert same(got[x].numpy()[60 * k:60 * k + 60], r[x]), x
+
+
+@pytest.mark.parametrize("n,grid,packed", [(40000, (32, 16), True), (22000, (16, 8), True),
+                                           (20000, (32, 16), False), (2000, (16, 4), False)])
+def test_crowded_cells(n, grid, packed):
+    # rows of 234, 515, 117 and 94 candidates; 9.4, 11, 2.3 and 0.2 million of them
+    import demso_b200 as D
+    sc = scenes.agitated_gas(n=n, seed=3, vel_std=0.5, grid=grid, pitch_factor=1.1, jitter=0.1)
+    sim = D.Simulation(sc.sys, capacity=n)
+    _load(sim, sc.state())
+    assert _call(sim, 5) == packed
+    _same(sim, PortOracle("f32").run(sc.sys, sc.state(), 5))
+    sim.close()
