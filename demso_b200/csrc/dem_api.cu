@@ -1720,6 +1720,32 @@ int band_pass(uint32_t nsteps) {
     return best;
 }
 constexpr uint32_t kSkipDisks = 1u << 20;
+// Above that many disks a skipped step costs its empty launches (about 12 us at
+// 1,048,576 disks, 26 at 4,194,304), a launch of the loop about 10 us and a graph
+// of one step 12 us more than a step in the loop.  The next launch of a call of
+// `nsteps`: its steps, and the pass of its loop (-1: the graph of one step).
+struct BandLaunch {
+    uint32_t steps;
+    int pass;
+};
+BandLaunch band_launch(uint32_t nsteps, uint32_t n) {
+    const uint32_t skip = 7 + (uint32_t)(19ull * n >> 22), one = 12, loop = 10;
+    BandLaunch best{1u, -1};
+    uint64_t least = nsteps < kBandPassSteps[0] ? (uint64_t)nsteps * one : UINT64_MAX;
+    for (int k = 0; k < kBandPasses; ++k) {
+        const uint32_t pass = kBandPassSteps[k], rest = nsteps % pass;
+        // the last pass not full, or the rest one by one (on a tie the longer pass)
+        if (loop + (uint64_t)(rest ? pass - rest : 0u) * skip <= least) {
+            least = loop + (uint64_t)(rest ? pass - rest : 0u) * skip;
+            best = BandLaunch{nsteps, k};
+        }
+        if (rest && nsteps > pass && loop + (uint64_t)rest * one <= least) {
+            least = loop + (uint64_t)rest * one;
+            best = BandLaunch{nsteps - rest, k};
+        }
+    }
+    return best;
+}
 
 // The step of set q after its fix, with the control particle's kernels where
 // there is one.
@@ -1906,21 +1932,16 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
         if (rc) return rc;
         ++done;
     }
-    // Whole passes of the loop, then the last few steps one by one where that is
-    // cheaper: a step the loop skips costs its empty launches (7 us at 65,536
-    // disks, 26 at 4,194,304), a graph of one step 12 us more than a step in the
-    // loop.
     const bool whole = after == BandAfter::kNothing && c->n >= kSkipDisks;
     const int a = c->cur;
     while (done < nsteps) {
-        uint32_t m = nsteps - done;
-        const int k = band_pass(m);
-        const uint32_t pass = kBandPassSteps[k];
-        if (whole) m = m >= pass ? m - m % pass : (m >= kBandPassSteps[0] ? kBandPassSteps[0] : 1u);
+        const uint32_t left = nsteps - done;
+        const BandLaunch next = whole ? band_launch(left, c->n) : BandLaunch{left, band_pass(left)};
+        const uint32_t m = next.steps;
         const bool one = after == BandAfter::kNothing && m == 1u;
         rc = band_begin(c, m, block + done, st);
         if (rc) return rc;
-        const int q = c->bandSet, l = whole && m < pass ? 0 : k;
+        const int q = c->bandSet, l = std::max(next.pass, 0);
         cudaGraphExec_t* g = one                            ? &c->bandOne[a][q]
                              : after == BandAfter::kFollowed ? &c->bandFollow[a][q][l]
                              : after == BandAfter::kRecord   ? &c->bandRec[a][q][l]
