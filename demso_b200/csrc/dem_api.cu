@@ -1867,10 +1867,10 @@ int band_begin(DemContext* c, uint32_t nsteps, uint32_t rowBlock, cudaStream_t s
     return DEM_OK;
 }
 
-// One step at a time with the host around each: profiling, the tuner, direct
+// One step (the call's after `done`) with the host around it: profiling, the tuner, direct
 // launches (the layout decided on the host).
-int band_step_alone(DemContext* c, cudaStream_t st) {
-    int rc = band_begin(c, 1, 0, st);
+int band_step_alone(DemContext* c, uint32_t done, cudaStream_t st) {
+    int rc = band_begin(c, 1, done, st);
     if (rc) return rc;
     const bool direct = c->flags & DEM_CTX_DIRECT;
     const int a = c->cur;
@@ -1928,7 +1928,7 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
     uint32_t done = 0;
     while (after == BandAfter::kNothing && done < nsteps &&
            (c->tuned < 0 || c->profiling || (c->flags & DEM_CTX_DIRECT))) {
-        rc = band_step_alone(c, st);
+        rc = band_step_alone(c, done, st);
         if (rc) return rc;
         ++done;
     }

@@ -218,10 +218,7 @@ band_fix_kernel(const __grid_constant__ BandArgs B, const __grid_constant__ DynS
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         B.ctrl[kBandAct + q] = active ? (c.x == 1u ? 2u : 1u) : 0u;
         B.ctrl[kBandNow + q] = B.ctrl[kBandStep];
-        if (active) {
-            atomicAdd(B.ctrl + kBandDirtySum, nd);
-            atomicAdd(B.ctrl + kBandFixes, 1u);
-        }
+        if (active && B.bands > kFixBlocks) atomicAdd(B.ctrl + kBandDirtySum, nd);
     }
     if (!active) return;
     for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
@@ -645,12 +642,12 @@ band_pack_kernel(BandArgs B, PackedState o, uint32_t stateOnly) {
     const uint32_t b = blockIdx.x;
     if (!stateOnly && b == 0u && blockIdx.y == 0u && threadIdx.x == 0u) {
         // a write to host memory costs the call 4 us: only the news is written
-        const uint32_t fixes = B.ctrl[kBandFixes], layouts = B.ctrl[kBandLayouts];
-        if (fixes && B.load &&
-            (band_overload(B.bands, B.ctrl[kBandDirtySum] / fixes) ||
-             (layouts > 1u && 4u * layouts >= fixes)))
+        const uint32_t steps = B.ctrl[kBandDone], layouts = B.ctrl[kBandLayouts];
+        if (steps && B.load &&
+            (band_overload(B.bands, B.ctrl[kBandDirtySum] / steps) ||
+             (layouts > 1u && 4u * layouts >= steps)))
             *reinterpret_cast<volatile uint32_t*>(&B.load->busy) = 1u;
-        B.ctrl[kBandDirtySum] = B.ctrl[kBandFixes] = B.ctrl[kBandLayouts] = 0u;
+        B.ctrl[kBandDirtySum] = B.ctrl[kBandLayouts] = 0u;
     }
     const uint32_t base = B.base[b], cnt = B.count[b];
     const uint32_t to = packed_base(B, b, B.geo[b]);

@@ -61,7 +61,7 @@ constexpr uint32_t kBandMaxRow = 4096, kBandMaxBands = 4096;
 
 // Words of BandArgs::ctrl.
 constexpr uint32_t kBandLeft = 0;   // steps left of the call
-constexpr uint32_t kBandDone = 1;   // steps done (the row block of the followed particles)
+constexpr uint32_t kBandDone = 1;   // steps of the call done (the row block of the followed particles)
 constexpr uint32_t kBandFull = 2;   // the next step needs a new layout
 constexpr uint32_t kBandCur = 3;    // dynamic set holding the state
 constexpr uint32_t kBandLaid = 4;   // the bands hold the state (0: only the packed arrays do)
@@ -69,9 +69,8 @@ constexpr uint32_t kBandAct = 5;    // [2] step of set q: 0 skipped, 1 runs, 2 r
 constexpr uint32_t kBandDirty = 7;  // [2] bands with events, by the set the fix of which takes them
 constexpr uint32_t kBandStep = 9;   // steps since the context was made
 constexpr uint32_t kBandNow = 10;   // [2] kBandStep as the step of set q sees it
-constexpr uint32_t kBandDirtySum = 12;  // since the last pack of a call: bands the fixes rewrote,
-constexpr uint32_t kBandFixes = 13;     // fixes,
-constexpr uint32_t kBandLayouts = 14;   // layouts of a state that was in bands already
+constexpr uint32_t kBandDirtySum = 12;  // bands the call's fixes rewrote (of more than kFixBlocks)
+constexpr uint32_t kBandLayouts = 13;   // the call's layouts of a state that was in bands already
 constexpr uint32_t kBandCtrlWords = 16;
 // Blocks of the fix: that many bands are rewritten at once (two blocks to a
 // multiprocessor).
