@@ -46,21 +46,15 @@ int cuda_fail(cudaError_t e, const char* what) {
 std::atomic<long long> g_liveAllocs{0};
 std::atomic<int> g_failCountdown{0};
 
-// `extra`: bytes behind them that are wanted too, zero when there is no room.
 template <typename T>
-cudaError_t dev_alloc(T** p, size_t bytes, size_t* extra = nullptr) {
+cudaError_t dev_alloc(T** p, size_t bytes) {
     *p = nullptr;
     int k = g_failCountdown.load();
     while (k > 0 && !g_failCountdown.compare_exchange_weak(k, k - 1)) {
     }
     if (k == 1) return cudaErrorMemoryAllocation;  // the injected failure
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, bytes + (extra ? *extra : 0));
-    if (e == cudaErrorMemoryAllocation && extra && *extra) {
-        (void)cudaGetLastError();
-        *extra = 0;
-        e = cudaMalloc(&q, bytes);
-    }
+    const cudaError_t e = cudaMalloc(&q, bytes);
     if (e == cudaSuccess) {
         *p = static_cast<T*>(q);
         ++g_liveAllocs;
@@ -392,9 +386,8 @@ struct DemContext {
     cudaGraphExec_t stepGraph[2] = {};
     int launchesPerStep = 0;
     void* block = nullptr;  // one allocation for every per-particle/per-cell array
-    // The step in bands (dem_bands.cuh): its arrays, in bandBlock, behind the
-    // others in `block` unless bandOwn (band.bands == 0: the context steps on the
-    // packed path; bandReady: the arrays have addresses); whether they hold the
+    // The step in bands (dem_bands.cuh): its arrays, in bandBlock (band.bands
+    // == 0: the context steps on the packed path); whether they hold the
     // current state; whether the cell ranges of the last sort are still to be
     // made from them (band_cells: they describe that sort whatever replaces the
     // state or its parameters, until the next step); the step loop, with and without followed rows, one step, and a step's
@@ -402,7 +395,6 @@ struct DemContext {
     BandArgs band;
     std::vector<BandGeo> bandGeo;
     void* bandBlock = nullptr;
-    bool bandOwn = false, bandReady = false;
     float2* ownPos = nullptr;  // the block's positions: not an adopted set
     bool bandValid = false, cellsInBands = false, bandInit = false;
     int bandSet = 0;  // the dynamic set of the bands that holds the state
@@ -1073,16 +1065,7 @@ int init_context(DemContext* c, uint32_t capacity, uint32_t numCells, DemContext
     total += 256;                                // step-loop counters
     const size_t sortBytes = onesweep_scratch_bytes(capacity, c->keyBits);
     const size_t incBytes = incsort_bytes(capacity, c->numCells, nullptr);
-    // the band arrays in the same allocation (another one costs a new context's
-    // first state 0.3 ms), unless cluster launches may be all that steps the scene
-    const size_t bandAt = al256(total);
-    size_t extra = 0;
-    if (c->band.bands &&
-        (c->nspec || !(c->flags & DEM_CTX_RESIDENT) || !cluster_scene_fits(capacity, numCells)))
-        extra = bandAt - total + band_bytes(c->band, capacity, c->typed, c->flags & DEM_CTX_PRESSURE,
-                                            c->flags & DEM_CTX_ACCEL, c->nspec != 0);
-    cudaError_t e = dev_alloc(&c->block, total, &extra);
-    if (e == cudaSuccess && extra) c->bandBlock = static_cast<char*>(c->block) + bandAt;
+    cudaError_t e = dev_alloc(&c->block, total);
     if (e == cudaSuccess) e = dev_alloc(&c->sortScratch, sortBytes);
     if (e == cudaSuccess) e = dev_alloc(&c->incScratch, incBytes);
     if (e != cudaSuccess) {
@@ -1180,7 +1163,7 @@ extern "C" int dem_destroy(DemContext* c) {
     dev_free(c->resQueue);
     dev_free(c->resWork);
     dev_free(c->clusterWork);
-    if (c->bandOwn) dev_free(c->bandBlock);
+    dev_free(c->bandBlock);
     dev_free(c->renderOwner);
     dev_free(c->ctlBlock);
     dev_free(c->dTable);
@@ -1281,7 +1264,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     const int a = c->cur;
     // the largest radius bounds every contact distance (neighbour culling)
     DEM_TRY_CUDA(launch_max_radius(c->stat[a].radius, n, c->errFlag + 1, st), "max radius");
-    const bool bands = c->bandReady && c->dyn[0].pos == c->ownPos;
+    const bool bands = c->bandBlock && c->dyn[0].pos == c->ownPos;
     if (bands) {
         const int rc = band_init(c, st);
         if (rc) return rc;
@@ -1522,26 +1505,21 @@ extern "C" int dem_get_state(DemContext* c, float* pos, float* vel, float* theta
 namespace {
 
 // ------------------------------------------------------------ step in bands
-// The context's own buffers.  The arrays (about 100 B per particle and 8 KB per
-// band, of its capacity) are allocated with the others, or here where cluster
-// launches came first; a context whose GPU has no room for them steps on the
-// packed path.
+// The context's own buffers.  The arrays are allocated at
+// the first state a context takes (about 100 B per particle and 8 KB per
+// band, of its capacity); a context whose GPU has no room for them steps on
+// the packed path.
 bool steps_in_bands(DemContext* c) {
     if (c->band.bands == 0 || c->dyn[0].pos != c->ownPos) return false;
-    if (c->bandReady) return true;
+    if (c->bandBlock) return true;
     const bool pressure = c->flags & DEM_CTX_PRESSURE, accel = c->flags & DEM_CTX_ACCEL;
-    if (!c->bandBlock) {
-        const size_t bytes =
-            band_bytes(c->band, c->capacity, c->typed, pressure, accel, c->nspec != 0);
-        if (dev_alloc(&c->bandBlock, bytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            c->bandBlock = nullptr;
-            c->band = BandArgs{};
-            return false;
-        }
-        c->bandOwn = true;
+    const size_t bytes = band_bytes(c->band, c->capacity, c->typed, pressure, accel, c->nspec != 0);
+    if (dev_alloc(&c->bandBlock, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->bandBlock = nullptr;
+        c->band = BandArgs{};
+        return false;
     }
-    c->bandReady = true;
     carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel, c->nspec != 0);
     c->band.table = c->dTable;  // null for a single scene
     c->band.errFlag = c->errFlag;
