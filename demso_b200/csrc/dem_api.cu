@@ -2778,6 +2778,18 @@ namespace {
 // Steps of one pass of the reverse loop; those past slot 0 do nothing.
 constexpr uint32_t kRevSteps = 4;
 
+// Whether the windows' steps re-run in bands: as a call of that many would, but
+// windows of one step -- a layout for a step, and a pass of the loop for it -- only
+// where the layout is what the packed sort from scratch costs too (a gradient
+// with a checkpoint every step, us a step, bands against packed: 2,000 disks
+// 150 / 138, 55,119 in 64 specimens 194 / 178, 16,384 176 / 174, 262,144 300 / 316;
+// every second step 101 / 106, 129 / 132, 116 / 130, 216 / 265).
+constexpr uint32_t kRerunOne = 1u << 17;
+bool rerun_in_bands(DemContext* c) {
+    return steps_in_bands(c) && !c->crowded && !c->bandBusy &&
+           (c->adjEvery > 1 || c->n >= kRerunOne);
+}
+
 // A window's `k` steps re-run from the restored checkpoint on the packed path,
 // each recorded: the first sorts from scratch (host-launched, record slot 0),
 // the rest run in pairs inside the recompute loop, recorded at the loop's
@@ -2894,7 +2906,7 @@ extern "C" int dem_adj_backward(DemContext* c, float* lamPos, float* lamVel, flo
                                 st);
         if (rc) break;
         const uint32_t k = std::min(c->adjEvery, c->adjSteps - (uint32_t)w * c->adjEvery);
-        const bool bands = steps_in_bands(c);
+        const bool bands = rerun_in_bands(c);
         if (bands) {
             rc = band_steps(c, k, BandAfter::kRecord, 0, st);
             if (rc) break;
