@@ -48,25 +48,18 @@ sys.path.insert(0, ROOT)
 METRIC = "particle-steps/s at 4M disks"
 UNIT = "particle-steps/s"
 N_DEFAULT = 4194304
-# Algorithmic bytes of the step kernel, counted per stage of the reference step
-# as the reference moves them, for the stages (or parts of them) it does:
-#   collide: reads own pos/vel/omega/radius/mass 28, writes force 8 + torque 4
-#     (neighbours are cache hits) = 40 per particle + 8 per cell (cell ranges);
-#   integrate: reads pos, vel, omega, theta, radius, mass, acc, alpha 44, writes
-#     pos, vel, omega, theta 24 = 68 per particle.
-# Particles keep their places between steps (only bands that one left or entered
-# are rewritten, by the sort phase), so no reorder is counted here.  The fused
-# kernel keeps force and torque in registers, so its own minimum is 68 per
-# particle (reads 44: pos, vel, theta, omega, radius, mass, key, kept
-# candidates; writes 24; reported beside).
-STEP_KERNEL_STAGE_BYTES = {"collide": 40, "integrate": 68}
+# Bytes the step kernel cannot do without, per particle: reads pos, vel, theta,
+# omega, radius, mass, key and kept candidates 44, writes pos, vel, theta and omega
+# 24 (force and torque stay in registers, neighbours are cache hits); per cell a
+# first-slot word and a stamp.
+STEP_KERNEL_STAGE_BYTES = {"read": 44, "write": 24}
 STEP_KERNEL_BYTES_PER_PARTICLE = sum(STEP_KERNEL_STAGE_BYTES.values())
 STEP_KERNEL_BYTES_PER_CELL = 8
-FUSED_MIN_BYTES_PER_PARTICLE = 68
-# Whole step: the fused minimum, and a first-slot word and a stamp per cell.  (A
-# step that hashes, sorts, reorders, collides and integrates in passes of its own
+# Whole step: the same (the fix rewrites only bands that a disk left or entered,
+# which is not counted).  (A step that hashes, sorts, reorders, collides and integrates in passes of its own
 # moves 260 per particle and 20 per cell.)
-WHOLE_STEP_BYTES = lambda n, c: float(FUSED_MIN_BYTES_PER_PARTICLE) * n + 8.0 * c
+WHOLE_STEP_BYTES = lambda n, c: (float(STEP_KERNEL_BYTES_PER_PARTICLE) * n
+                                 + float(STEP_KERNEL_BYTES_PER_CELL) * c)
 # the plain-at-scale sizes of the roofline curve (the same workload scaled)
 DEFAULT_SWEEP = "65536,262144,1048576,4194304,16777216"
 # the timed K-step call is repeated until this much device time is under load
@@ -244,17 +237,34 @@ def config_dict(n, sc):
     return d
 
 
+def adopt(sim, st):
+    """The state `st` (numpy arrays, one material) in two sets of buffers of the
+    caller's, handed to a context."""
+    import torch
+    n = st["pos"].shape[0]
+    sets = []
+    for _ in range(2):
+        d = {}
+        for k in ("pos", "vel", "theta", "omega", "radius", "mass", "id"):
+            a = np.ascontiguousarray(st[k])
+            a = torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a)
+            d[k] = torch.zeros((n + 8,) + tuple(a.shape[1:]), dtype=a.dtype, device="cuda")
+            d[k][:n] = a.cuda()
+        sets.append(d)
+    sim.adopt_state(sets[0], sets[1], n)
+
+
 # ------------------------------------------------------------------ batched form
 def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int = 256):
     """Batched form on the batched workload (4,096 specimens of 256..8,192
     disks, own boxes/parameters; 5,000 steps issued as one dem_step call) in
-    two contexts -- with the resident flag (a batch with a state of its own
-    steps in bands with it too, the faster form) and without, each one
-    graph launch of the device-side step loop -- against looping the plain
-    single-scene step over an evenly spaced sample of the same specimens, in
-    the faster of its two forms (graph path, resident flag: a cluster launch
-    up to 1,536 disks).  `value` is
-    the faster batched form."""
+    two contexts -- one with a state of its own, which steps in bands by one
+    graph launch of the device-side step loop, and one with the resident flag in
+    adopted buffers, one launch that keeps the specimens in shared memory --
+    against looping the plain single-scene step over an evenly spaced sample of
+    the same specimens, in the faster of its two forms (graph path, resident
+    flag: a cluster launch each).  `value` is the faster batched form and `path`
+    names it."""
     import torch
     import demso_b200 as D
     from demso_b200 import scenes
@@ -280,11 +290,10 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     graph_path = total * steps / (e0.elapsed_time(e1) * 1e-3)
     kernels = b.kernels_per_step()
     b.close()
-    # the same with DEM_CTX_RESIDENT, which takes the faster form; its first
-    # call lays the bands out and is untimed
-    r = D.Batch([(sc.sys, sc.n) for sc in specimens], flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
-    r.set_state(t(st["pos"]), t(st["vel"]), t(st["theta"]), t(st["omega"]), t(st["radius"]),
-                t(st["mass"]), t(st["id"]))
+    # the resident launch, in adopted buffers
+    r = D.Batch([(sc.sys, sc.n) for sc in specimens],
+                flags=D.CTX_PRESSURE | D.CTX_RESIDENT | D.CTX_CALLER_STATE)
+    adopt(r, st)
     r.step(max(3, warmup))
     torch.cuda.synchronize()
     e0.record()
@@ -318,8 +327,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     torch.cuda.synchronize()
     sample_n = sum(sc.n for sc in sample)
     looped_graph = sample_n * lsteps / (e0.elapsed_time(e1) * 1e-3)
-    # the same with DEM_CTX_RESIDENT: specimens of up to 1,536 disks as one
-    # thread-block cluster launch each, larger ones on the graph path
+    # the same with DEM_CTX_RESIDENT: a thread-block cluster launch each (the
+    # first 512 steps of a context)
     csims = []
     for sc in sample:
         sim = D.Simulation(sc.sys, capacity=sc.n, flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
@@ -353,10 +362,10 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
         sim.close()
     return {"metric": "aggregate particle-steps/s, batched vs looped plain",
             "value": batched, "looped_plain": looped, "ratio": batched / looped,
-            "path": "graph",
+            "path": "graph" if graph_path >= resident else "resident",
             "resident": {"value": resident, "ratio": resident / looped, "launches": 1,
-                         "form": "the %d steps with the resident flag: one graph launch of the "
-                                 "device-side step loop, the faster form" % steps},
+                         "form": "the %d steps as one launch that keeps the specimens in shared "
+                                 "memory, in adopted buffers" % steps},
             "graph_path": {"value": graph_path, "ratio": graph_path / looped,
                            "kernels_per_step": kernels,
                            "graph_launches": 1,
@@ -370,8 +379,7 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
             "looped_sample": "%d of the %d specimens (every %d-th), each its own context "
                              "stepping %d steps as one dem_step call, one specimen after "
                              "another; the faster of the graph path (device-side step "
-                             "loop) and the resident flag (a cluster launch up to 1,536 "
-                             "disks)"
+                             "loop) and the resident flag (a cluster launch each)"
                              % (len(sample), num, max(1, num // loop_sample), lsteps),
             "workload": "batched: specimens with counts log-uniform in [256, 8192], square "
                         "walled boxes at area fraction 0.5, radii U[0.9, 1.1] mm, kn "
@@ -467,10 +475,10 @@ def measure_adjoint(n: int = 16384, steps: int = 2000, every: int = 100):
 # ------------------------------------------------------------------ config 0
 def measure_settling_pile(steps: int = 20000):
     """The plain 2D settling pile (4,096 disks, 20,000 steps): wall time of
-    the whole run on the GPU as one dem_step call, for a context with the
-    resident flag (scenes above 1,536 disks take the graph path with it) and
-    one without; the
-    faster gives gpu_seconds (settling_pile_cpu adds the host build's)."""
+    the whole run on the GPU as one dem_step call, for a context with a state of
+    its own, which steps in bands, and as one cluster launch in adopted buffers;
+    the faster gives gpu_seconds and `path` names it (settling_pile_cpu adds the
+    host build's)."""
     import torch
     import demso_b200 as D
     from demso_b200 import scenes
@@ -479,13 +487,19 @@ def measure_settling_pile(steps: int = 20000):
                                    else np.ascontiguousarray(a))
     st = sc.state()
 
-    def run(flags):
-        sim = D.Simulation(sc.sys, capacity=sc.n, flags=flags)
-        sim.set_state(t(st["pos"]), t(st["vel"]), t(st["theta"]), t(st["omega"]), t(st["radius"]),
-                      t(st["mass"]), t(st["id"]))
+    def run(cluster):
+        flags = D.CTX_RESIDENT | D.CTX_CALLER_STATE if cluster else 0
+        sim = D.Simulation(sc.sys, capacity=sc.n, flags=D.CTX_PRESSURE | flags)
+
+        def load():
+            if cluster:
+                return adopt(sim, st)
+            sim.set_state(t(st["pos"]), t(st["vel"]), t(st["theta"]), t(st["omega"]),
+                          t(st["radius"]), t(st["mass"]), t(st["id"]))
+
+        load()
         sim.step(10)
-        sim.set_state(t(st["pos"]), t(st["vel"]), t(st["theta"]), t(st["omega"]), t(st["radius"]),
-                      t(st["mass"]), t(st["id"]))
+        load()
         torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
@@ -496,17 +510,16 @@ def measure_settling_pile(steps: int = 20000):
         sim.close()
         return e0.elapsed_time(e1) * 1e-3
 
-    cluster_s = run(D.CTX_PRESSURE | D.CTX_RESIDENT)
-    graph_s = run(D.CTX_PRESSURE)
+    cluster_s = run(True)
+    graph_s = run(False)
     gpu_s = min(cluster_s, graph_s)
     out = {"workload": "plain 2D settling pile: 4096 disks, radii U[0.9, 1.1] mm, 64x64 "
                        "jittered lattice in a 0.2 x 0.2 m box, dt 2e-6 s, %d steps" % steps,
            "gpu_seconds": gpu_s, "gpu_steps_per_s": steps / gpu_s,
            "gpu_particle_steps_per_s": sc.n * steps / gpu_s,
-           "path": "graph",
+           "path": "graph" if graph_s <= cluster_s else "cluster",
            "cluster_seconds": cluster_s, "graph_path_seconds": graph_s,
-           "cluster_form": "the context with the resident flag, which takes the graph path "
-                           "above 1,536 disks",
+           "cluster_form": "one launch of a thread-block cluster, in adopted buffers",
            "graph_path_form": "one graph launch of the device-side step loop"}
     return out
 
@@ -883,11 +896,10 @@ def main():
         bytes_launch = STEP_KERNEL_BYTES_PER_PARTICLE * n + STEP_KERNEL_BYTES_PER_CELL * cells
         kname = "band_step_kernel (collide + integrate + next hash)"
     else:
-        # counted as the reorder alone (84 B per particle, 12 B per cell); the
-        # sort work is not counted
-        bytes_launch = 84 * n + 12 * cells
+        # its bytes are those of the bands that disks left or entered: not counted
+        bytes_launch = None
         kname = "sort phase (bands that a disk left or entered)"
-    achieved = bytes_launch / (stage_ms[dom] * 1e-3) / 1e9
+    achieved = bytes_launch / (stage_ms[dom] * 1e-3) / 1e9 if bytes_launch else None
     traffic = None
     tf = os.path.join(ROOT, "profiles", "traffic.txt")
     if os.path.isfile(tf):
@@ -1021,14 +1033,12 @@ def main():
                                   "ms_per_step_min": float(np.min(reps)) / args.steps,
                                   "ms_per_step_max": float(np.max(reps)) / args.steps},
                 "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved,
-                             "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
+                             "peak": hbm, "unit": "GB/s",
+                             "frac": achieved / hbm if achieved else None,
                              "peak_kind": kind, "traffic": traffic,
                              "bytes_per_launch": bytes_launch,
                              "stage_bytes_per_particle": (STEP_KERNEL_STAGE_BYTES if dom == 2
-                                                          else {"reorder_move": 32}),
-                             "fused_minimum_frac": (FUSED_MIN_BYTES_PER_PARTICLE * n
-                                                    / (stage_ms[dom] * 1e-3) / 1e9 / hbm
-                                                    if dom == 2 else None)},
+                                                          else None)},
                 "stage_ms_per_step": {"sort_reorder": stage_ms[0],
                                       "collide_integrate": stage_ms[2]},
                 "whole_step": {"model_bytes_per_step": whole_bytes,

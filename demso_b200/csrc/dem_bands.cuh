@@ -26,7 +26,7 @@
 // sorted order, and the bits are its own.
 //
 // Against the packed incremental sort (six kernels a step, 40 B moved per
-// particle in the sort phase and 88 B in the step; here two kernels, 64 B in
+// particle in the sort phase and 88 B in the step; here two kernels, 68 B in
 // the step), with the kept candidates below: a call of 20 steps of 4,194,304
 // disks 4,669 -> 2,988 us, of 1,000,003 dense disks 1,503 -> 1,116 us, 50 steps of
 // 65,536 1,229 -> 834 us, 20 steps of a fast gas of 131,071 584 -> 365 us, of 256
