@@ -499,6 +499,15 @@ class Batch(Simulation):
         check(load().dem_batch_specimen(self._h, s, C.byref(a), C.byref(b)))
         return a.value, a.value + b.value
 
+    def cells(self, stream=None):
+        """(cellStart, cellEnd) over the cells of all specimens, one after another."""
+        import torch
+        nc = sum(sys.num_cells for sys, _ in self.specs)
+        cs = torch.empty(nc, dtype=torch.int32, device="cuda")
+        ce = torch.empty(nc, dtype=torch.int32, device="cuda")
+        check(load().dem_get_cells(self._h, cs.data_ptr(), ce.data_ptr(), _stream(stream)))
+        return cs, ce
+
     def get_state(self, device="cuda", stream=None) -> dict:
         # the typed layout follows the largest material count in the batch
         saved = self.sys

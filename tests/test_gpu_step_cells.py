@@ -113,3 +113,21 @@ def test_after_new_parameters_of_a_batch(steps):
                   lambda sim: _cells(sim, cells))
     assert np.count_nonzero(a[0] != 0xFFFFFFFF) > 100
     assert _equal(a, b)
+
+
+def test_cells_of_a_batch():
+    # the arrays hold every specimen's cells, not the first one's
+    import demso_b200 as D
+    parts = [scenes.agitated_gas(n=n, seed=n, vel_std=3.0, pitch_factor=1.1, jitter=0.1)
+             for n in (300, 2500, 40)]
+    sim = D.Batch([(p.sys, p.n) for p in parts])
+    _load(sim, scenes.concat_specimens(parts))
+    sim.step(5)
+    cs, ce = (x.cpu().numpy().view(np.uint32) for x in sim.cells())
+    n = sum(p.sys.num_cells for p in parts)
+    assert cs.size == ce.size == n
+    want = _cells(sim, n)
+    assert np.array_equal(cs, want[0])
+    assert np.array_equal(np.where(cs == 0xFFFFFFFF, 0, ce), want[1])
+    assert int((want[1] - np.where(cs == 0xFFFFFFFF, 0, cs)).sum()) == 2840
+    sim.close()
