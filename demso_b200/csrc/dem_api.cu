@@ -1282,7 +1282,7 @@ int accept_state(DemContext* c, uint32_t n, cudaStream_t st) {
     memcpy(&rmax, &word[0], 4);
     rmax = (n > 0 && std::isfinite(rmax)) ? rmax : INFINITY;
     c->bandBusy = bands && too_many_movers(c, n, word[1], word[2]);
-    c->crowded = crowded_cells(c, n);
+    if (!c->nspec || c->n == 0) c->crowded = crowded_cells(c, n);  // a batch's counts are fixed
     // the same particle count and largest radius give the same kernel
     // parameters (and specimen table), so the captured graphs stay valid;
     // only the first step's full sort is forced, as after every new state
@@ -1581,10 +1581,19 @@ bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t m
 // still win -- us a step, bands against packed: 65,536 disks, 48 a row 23.1 / 25.8;
 // 131,072, 24 a row 24.3 / 30.6 -- above it they lose: 550,000, 25 a row
 // 48.7 / 45.8 and 101 a row 92.4 / 74.4; 400,000, 73 a row 62.1 / 53.2; 262,144,
-// 48 a row 40.6 / 38.1.  (Grids of cells of about two radii hold 5 to 14.)
+// 48 a row 40.6 / 38.1; a batch's crowded specimens together: 512 of 2,000 to
+// 8,192 disks, 11 to 44 a row, 229 / 168.  (Grids of cells of about two radii hold
+// 5 to 14.)
 bool crowded_cells(const DemContext* c, uint32_t n) {
-    return 3ull * n > (uint64_t)kCandBits * c->numCells &&
-           3ull * n * n / c->numCells > 8000000ull;
+    const auto tests = [](uint64_t count, uint64_t cells) {  // 0 in a grid fine enough
+        return 3ull * count > kCandBits * cells ? 3ull * count * count / cells : 0ull;
+    };
+    constexpr uint64_t kCrowd = 8000000;
+    if (!c->nspec) return tests(n, c->numCells) > kCrowd;
+    uint64_t sum = 0;
+    for (uint32_t s = 0; s < c->nspec; ++s)
+        sum += tests(c->partOff[s + 1] - c->partOff[s], (uint64_t)c->hTable[s].gx * c->hTable[s].gy);
+    return sum > kCrowd;
 }
 
 // Whether a call of `nsteps` steps stays on the packed path for its movers.  The
@@ -1638,8 +1647,10 @@ bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
 constexpr uint32_t kShortCall = 4, kShortBatchCall = 3, kPackedSteps = 16, kShortRun = 16;
 bool band_call(DemContext* c, uint32_t nsteps, cudaStream_t st) {
     if (!steps_in_bands(c)) return false;
-    if (c->profiling || c->tuned < 0) return true;  // the bands' kernels are what is timed
-    if (c->crowded || band_busy(c, nsteps, st)) return false;
+    if (c->crowded) return false;
+    // the kernels of longer calls are what is timed
+    if (c->profiling || c->tuned < 0) return !c->bandBusy;
+    if (band_busy(c, nsteps, st)) return false;
     const bool packedOrder = c->keysValid && c->haveOrder;
     if (nsteps >= (c->nspec ? kShortBatchCall : kShortCall)) {
         c->shortCalls = 0;
@@ -2013,13 +2024,15 @@ constexpr int kNotResident = -1;
 // nothing, when the batch steps in bands -- faster for every batch measured:
 // per step, resident against bands, 512 specimens (1.17 M disks) 60.5 / 59 us,
 // 4,096 405 / 380, 32 58 / 20, 300 of 16 to 40 disks 16.3 / 11.0, 4 of 300
-// 10.6 / 7.9 -- or has types, attraction, a control particle, stage
+// 10.6 / 7.9; packed where too many disks change cell, 512 specimens 59 us against
+// 99 -- unless its cells are crowded (512 specimens 158 us, packed 164), or has types, attraction, a control particle, stage
 // profiling or a specimen too large for one bin: the graph path steps it.
 // After the launch the state is in the order of its last sort, as after the
 // graph path, but no mover record exists: the next graph-path step sorts
 // from scratch (the same permutation, the sort being stable).
 int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) || steps_in_bands(c) ||
+    if (c->typed || c->ctlOn || c->profiling || !has_state_sets(c) ||
+        (steps_in_bands(c) && !(c->crowded && nsteps >= kShortBatchCall)) ||
         c->partOff.size() != (size_t)c->nspec + 1 || c->partOff.back() != c->n)
         return kNotResident;
     for (uint32_t s = 0; s < c->nspec; ++s)

@@ -131,3 +131,49 @@ def test_crowded_cells(n, grid, packed):
     assert _call(sim, 5) == packed
     _same(sim, PortOracle("f32").run(sc.sys, sc.state(), 5))
     sim.close()
+
+
+@pytest.mark.parametrize("crowd,packed", [(30000, True), (9000, False)])
+def test_crowded_specimens(crowd, packed):
+    # the crowded specimen's tests decide (10.5 and 0.95 million), not the average
+    import demso_b200 as D
+    parts = [scenes.agitated_gas(n=crowd, seed=3, vel_std=0.5, grid=(16, 16), pitch_factor=1.1,
+                                 jitter=0.1),
+             scenes.agitated_gas(n=300, seed=4, vel_std=0.5, grid=(512, 256), box=1.0)]
+    st = scenes.concat_specimens(parts)
+    sim = D.Batch([(p.sys, p.n) for p in parts])
+    _load(sim, st)
+    assert _call(sim, 5) == packed
+    got = sim.get_state("cpu")
+    sim.check()
+    sim.close()
+    ref = PortOracle("f32").run(parts[0].sys, parts[0].state(), 5)
+    for x in ("pos", "vel", "theta", "omega", "pressure"):
+        assert same(got[x].numpy()[:crowd], ref[x]), x
+
+
+@pytest.mark.parametrize("crowded", [False, True])
+def test_a_resident_batch(crowded):
+    # with many movers it is packed (single steps alternate the sets), with crowded
+    # cells its calls of three steps or more are resident launches
+    import demso_b200 as D
+    if crowded:
+        parts = [scenes.agitated_gas(n=6000, seed=k, vel_std=0.5, grid=(8, 8), pitch_factor=1.1,
+                                     jitter=0.1) for k in range(6)]
+    else:
+        parts = [_gas((16, 16), 60, 200.0, seed=k) for k in range(320)]
+    st = scenes.concat_specimens(parts)
+    sim = D.Batch([(p.sys, p.n) for p in parts], flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
+    _load(sim, st)
+    assert _call(sim, 9) != crowded
+    assert _call(sim, 1)
+    sim.step(2)
+    sim.step(4)
+    got = sim.get_state("cpu")
+    sim.check()
+    sim.close()
+    n = parts[0].n
+    for k in (0, 3, len(parts) - 1):
+        r = PortOracle("f32").run(parts[k].sys, parts[k].state(), 16)
+        for x in ("pos", "vel", "theta", "omega", "pressure"):
+            assert same(got[x].numpy()[n * k:n * k + n], r[x]), x
