@@ -140,9 +140,9 @@ struct Sums {
 };
 
 // A warp's contacts, dealt to its lanes.  The contact law is some two hundred
-// instructions (five IEEE divisions, four square roots, a double division) and
-// the particles of a warp touch 0 to 6 others, so lane by lane it ran at a
-// third of the lanes.  Instead a turn takes up to kDeal kept candidates of
+// instructions (five IEEE divisions, four square roots; a double division for the
+// pressure where that is wanted) and the particles of a warp touch 0 to 6 others,
+// so lane by lane it ran at a third of the lanes.  Instead a turn takes up to kDeal kept candidates of
 // every lane, whose loads are in flight together, and writes the touching ones
 // into a list in shared memory; the warp evaluates the list 32 at a time, and
 // each lane adds up its own results in its own order.  In the band step, with

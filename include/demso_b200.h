@@ -167,8 +167,9 @@ int dem_integrate_system(const DemSystem* sys, float* pos, float* vel, const flo
  * in place) and runs one step kernel (collide, integrate, next hash), as CUDA
  * graphs; the state is packed into sorted order at the end of every call.
  * Adopted buffers, rows of more than 4,096 cells, calls of fewer than 4
- * steps (3 for a batch) on a state that is not in bands, and a context whose
- * bands could not be allocated step packed instead: an incremental stable
+ * steps (3 for a batch) on a state that is not in bands, scenes in which many
+ * particles change cell or whose cells are crowded, and a context whose bands
+ * could not be allocated step packed instead: an incremental stable
  * sort that moves positions and radii, and a step kernel that gathers the
  * other fields.  The bits are the same.  A context's calls share its
  * device buffers and its loop counters: issue them on one stream, or
