@@ -1044,15 +1044,10 @@ int init_context(DemContext* c, uint32_t capacity, uint32_t numCells, DemContext
     size_t total = 0;
     // single scenes step in bands (dem_bands.cuh)
     if (ownState) {
-        std::vector<KParams> grids{c->P};
-        std::vector<uint32_t> counts{0u};
-        if (c->nspec) {
-            grids = c->hTable;
-            for (uint32_t s = 1; s < c->nspec; ++s) counts.push_back(0u);
-            for (uint32_t s = 0; s < c->nspec; ++s) counts[s] = c->partOff[s + 1] - c->partOff[s];
-        }
-        if (!band_shape(grids, counts, c->nspec != 0, c->band, c->bandGeo)) c->band = BandArgs{};
-        for (uint32_t s = 0; s < c->nspec; ++s) c->hTable[s].firstOff = grids[s].firstOff;
+        KParams* const grids = c->nspec ? c->hTable.data() : &c->P;
+        if (!band_shape(grids, c->nspec ? c->nspec : 1u, c->nspec ? c->partOff.data() : nullptr,
+                        c->band, c->bandGeo))
+            c->band = BandArgs{};
     }
     if (ownState) {
         total += 2 * (f8p + f8 + 2 * f4);                    // dyn sets

@@ -894,11 +894,14 @@ bool attracts(const KParams& P) {
 
 }  // namespace
 
-bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, bool batch,
-                BandArgs& b, std::vector<BandGeo>& geo) {
+bool band_shape(KParams* P, uint32_t grids, const uint32_t* partOff, BandArgs& b,
+                std::vector<BandGeo>& geo) {
+    const bool batch = partOff != nullptr;
     geo.clear();
-    uint64_t cell = 0, first = 0, part = 0, free = 0;
-    for (size_t s = 0; s < P.size(); ++s) {
+    uint64_t cell = 0, first = 0, free = 0;
+    for (uint32_t s = 0; s < grids; ++s) {
+        const uint32_t part = batch ? partOff[s] : 0u;
+        const uint32_t count = batch ? partOff[s + 1] - part : 0u;
         const uint32_t gx = P[s].gx, cells = P[s].gx * P[s].gy;
         if (gx > kBandMaxRow) return false;
         uint32_t per = std::max(batch ? kBandBatchCells : kBandMinCells, gx);
@@ -906,10 +909,10 @@ bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, boo
         per = std::min(per, cells);  // both powers of two
         P[s].firstOff = (uint32_t)first;
         const uint32_t sceneBand = (uint32_t)geo.size(), bands = cells / per;
-        const uint32_t slack = bands == 1u ? 0u : std::max(kBandMinSlack, count[s] / (16u * bands));
+        const uint32_t slack = bands == 1u ? 0u : std::max(kBandMinSlack, count / (16u * bands));
         for (uint32_t c = 0; c < cells; c += per) {
             geo.push_back(BandGeo{(uint32_t)cell + c, per, (uint32_t)(first + (c / gx) * (gx + 1ull)),
-                                  P[s].log2gx, sceneBand, (uint32_t)part, (uint32_t)s,
+                                  P[s].log2gx, sceneBand, part, s,
                                   (uint32_t)free | (bands == 1u ? kBandWhole : 0u)});
             free += slack;
         }
@@ -917,7 +920,6 @@ bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, boo
         while ((1u << b.shift) < per) ++b.shift;
         cell += cells;
         first += (uint64_t)P[s].gy * (gx + 1ull);
-        part += count[s];
         if (first >= (1ull << 32) || free >= kBandWhole) return false;
     }
     b.batchFree = batch ? (uint32_t)free : 0u;

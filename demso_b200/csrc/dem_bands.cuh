@@ -167,11 +167,11 @@ struct PackedState {
     float* alpha;
 };
 
-// The bands of the grids `P` (one scene, or a batch's specimens of `count`
-// particles each), with the grids' firstOff; false when a grid takes the packed
-// path.
-bool band_shape(std::vector<KParams>& P, const std::vector<uint32_t>& count, bool batch,
-                BandArgs& b, std::vector<BandGeo>& geo);
+// The bands of the `grids` grids P (one scene, partOff null, or a batch's specimens
+// of partOff[s + 1] - partOff[s] particles), whose firstOff it sets; false when a
+// grid takes the packed path.
+bool band_shape(KParams* P, uint32_t grids, const uint32_t* partOff, BandArgs& b,
+                std::vector<BandGeo>& geo);
 // Free slots per band of a single scene, and slots in all, for n particles.
 uint32_t band_slack(const BandArgs& b, uint32_t n);
 size_t band_slots(const BandArgs& b, uint32_t n, bool batch);
