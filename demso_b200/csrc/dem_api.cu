@@ -402,6 +402,7 @@ struct DemContext {
     // calls on the packed path since.  cluster_call: steps of cluster launches
     // since the graphs were dropped.
     uint32_t shortCalls = 0, packedSteps = 0, clusterSteps = 0;
+    uint32_t bandSteps = 0;  // steps in bands, up to kLoadSteps (band_load)
     // whether too many particles change cell for the bands (band_busy): the words
     // the device reports to, whether an estimate is on its way, the estimates so
     // far, the packed steps since the last one and those to wait
@@ -1518,16 +1519,28 @@ bool steps_in_bands(DemContext* c) {
     carve_bands(c->band, c->bandBlock, c->capacity, c->typed, pressure, accel, c->nspec != 0);
     c->band.table = c->dTable;  // null for a single scene
     c->band.errFlag = c->errFlag;
-    // (without these words the bands are left and entered at a new state only)
+    return true;
+}
+
+// The words the device reports to.  Host memory costs a context about 1.5 ms, so
+// it is made once the context has stepped long enough for that to be little
+// (kLoadSteps steps in bands, or the first estimate on the packed path); without
+// it the bands are left and entered at a new state only.
+constexpr uint32_t kLoadSteps = 512;
+bool band_load(DemContext* c) {
+    if (c->bandLoad) return true;
     void *h = nullptr, *d = nullptr;
     if (cudaHostAlloc(&h, sizeof(BandLoad), cudaHostAllocMapped) == cudaSuccess) {
-        c->bandLoad = static_cast<BandLoad*>(h);
-        c->bandLoad->busy = 0u;
-        if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess)
+        if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
+            c->bandLoad = static_cast<BandLoad*>(h);
+            c->bandLoad->busy = 0u;
             c->band.load = static_cast<BandLoad*>(d);
+        } else {
+            cudaFreeHost(h);
+        }
     }
-    (void)cudaGetLastError();
-    return true;
+    (void)cudaGetLastError();  // no such memory is not the caller's error
+    return c->bandLoad != nullptr;
 }
 
 // What the band arrays hold from the start.
@@ -1598,10 +1611,9 @@ bool crowded_cells(const DemContext* c, uint32_t n) {
 // each time the bands were entered in vain).  The words arrive when they do:
 // the path never changes the bits.
 bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
-    if (!c->bandLoad) return c->bandBusy;
     const volatile BandLoad* w = c->bandLoad;
     if (!c->bandBusy) {
-        if (w->busy == 0u) return false;
+        if (!w || w->busy == 0u) return false;
         c->bandBusy = true;
         c->estimated = false;
         c->busySteps = 0;
@@ -1619,7 +1631,7 @@ bool band_busy(DemContext* c, uint32_t nsteps, cudaStream_t st) {
         c->bandLoad->busy = 0u;
         return false;
     }
-    if (c->busySteps >= c->busyWait) {
+    if (c->busySteps >= c->busyWait && band_load(c)) {
         c->busySteps = 0;
         c->bandLoad->estDirty = c->bandLoad->estMovers = kBandUnknown;
         c->estimated = cudaMemsetAsync(c->errFlag + 2, 0, 8, st) == cudaSuccess &&
@@ -1940,6 +1952,11 @@ int band_steps(DemContext* c, uint32_t nsteps, BandAfter after, uint32_t block, 
         DEM_TRY_CUDA(cudaGraphLaunch(*g, st), "graph launch");
         done += m;
         c->bandSet ^= (int)(m & 1u);
+    }
+    c->bandSteps += std::min(nsteps, kLoadSteps);
+    if (c->bandSteps >= kLoadSteps) {
+        c->bandSteps = kLoadSteps;
+        band_load(c);
     }
     DEM_TRY_CUDA(launch_band_pack(c->band, packed_state(c), false, st), "band pack");
     return DEM_OK;

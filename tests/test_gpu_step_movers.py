@@ -70,6 +70,8 @@ def test_new_states_and_scenes_that_change(grid, fast, slow):
         st["vel"] = (unit * np.float32(speed)).astype(np.float32)
         _load(sim, st)
 
+    go(slow)
+    sim.step(512)  # long enough for calls to report
     for speed, packed in ((slow, False), (fast, True), (slow, False)):
         go(speed)
         assert _call(sim, 7) == packed
