@@ -263,7 +263,7 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     adopted buffers, one launch that keeps the specimens in shared memory --
     against looping the plain single-scene step over an evenly spaced sample of
     the same specimens, in the faster of its two forms (graph path, resident
-    flag: a cluster launch each).  `value` is the faster batched form and `path`
+    flag: a cluster launch each up to 1,536 disks).  `value` is the faster batched form and `path`
     names it."""
     import torch
     import demso_b200 as D
@@ -327,8 +327,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
     torch.cuda.synchronize()
     sample_n = sum(sc.n for sc in sample)
     looped_graph = sample_n * lsteps / (e0.elapsed_time(e1) * 1e-3)
-    # the same with DEM_CTX_RESIDENT: a thread-block cluster launch each (the
-    # first 512 steps of a context)
+    # the same with DEM_CTX_RESIDENT: a thread-block cluster launch each up to
+    # 1,536 disks, larger ones on the graph path
     csims = []
     for sc in sample:
         sim = D.Simulation(sc.sys, capacity=sc.n, flags=D.CTX_PRESSURE | D.CTX_RESIDENT)
@@ -379,7 +379,8 @@ def measure_batched(steps: int, warmup: int, num: int = 4096, loop_sample: int =
             "looped_sample": "%d of the %d specimens (every %d-th), each its own context "
                              "stepping %d steps as one dem_step call, one specimen after "
                              "another; the faster of the graph path (device-side step "
-                             "loop) and the resident flag (a cluster launch each)"
+                             "loop) and the resident flag (a cluster launch each up to "
+                             "1,536 disks)"
                              % (len(sample), num, max(1, num // loop_sample), lsteps),
             "workload": "batched: specimens with counts log-uniform in [256, 8192], square "
                         "walled boxes at area fraction 0.5, radii U[0.9, 1.1] mm, kn "

@@ -2094,23 +2094,26 @@ int resident_step(DemContext* c, uint32_t nsteps, cudaStream_t st) {
 
 // Whether a call of a resident scene of more than kClusterBandDisks disks, which
 // could step in bands, is a cluster launch.  The bands' arrays and graphs cost
-// a context about 1.5 ms (allocation, build and release; 4,096 disks, one call
-// of 100 steps: the context's life 2.3 ms with the cluster, 4.6 in bands), the
-// cluster 1 to 7 us a step more, so the first kClusterSteps steps are its own
-// unless one call is longer.  Afterwards calls too short for bands that are
+// a context about 0.4 ms (allocation, build and release; 4,096 disks, create to
+// close around one call of 100 steps: 2.35 ms with the cluster, 2.75 in bands),
+// the cluster 1 to 7 us a step more, so the first kClusterSteps steps are its
+// own -- about as many as lose what they save -- unless one call is longer.  Afterwards calls too short for bands that are
 // not in them already: a single step is fastest on the packed path (24 us
 // against 36 to 66), two or three by the cluster up to kClusterBandDisks disks
 // a step (totals for 2 and 3 steps, cluster against packed: 2,000 disks 46 / 52
-// and 55 / 80 us, 4,096 63 / 53 and 75 / 81, 8,000 83 / 57 and 100 / 85).
-constexpr uint32_t kClusterSteps = 512;
+// and 55 / 80 us, 4,096 63 / 53 and 75 / 81, 8,000 83 / 57 and 100 / 85), and up to
+// seven in scenes of 2,048 disks or fewer (4 and 5 steps, cluster against bands:
+// 1,537 disks 59 / 64 and 69 / 73 us, 2,000 63 / 64 and 73 / 76, 8 steps equal).
+constexpr uint32_t kClusterSteps = 160;
 bool cluster_call(DemContext* c, uint32_t nsteps) {
     if (c->clusterSteps < kClusterSteps && nsteps <= kClusterSteps - c->clusterSteps) {
         c->clusterSteps += nsteps;
         return true;
     }
     c->clusterSteps = kClusterSteps;
-    return nsteps >= 2 && nsteps < kShortCall && !c->bandValid &&
-           c->n <= kClusterBandDisks * nsteps;
+    return nsteps >= 2 && !c->bandValid &&
+           (nsteps < kShortCall ? c->n <= kClusterBandDisks * nsteps
+                                : nsteps < 8 && c->n <= 2048);
 }
 
 // A multi-step call of a single scene created with DEM_CTX_RESIDENT as one

@@ -334,7 +334,7 @@ int dem_state_view(DemContext* ctx, DemStateSet* out, int* setIndex);
  * trajectory does not depend on the choice.
  * A single scene created with DEM_CTX_RESIDENT, of at most 8,192 disks and
  * 8,192 cells, one material, no attraction and no control particle, steps
- * each call (above 1,536 disks, unless with DEM_CTX_CALLER_STATE: the first 512
+ * each call (above 1,536 disks, unless with DEM_CTX_CALLER_STATE: the first 160
  * steps and short calls; the others are faster on the graph path) as ONE
  * launch of a thread-block cluster of 8 blocks: every block keeps the whole
  * scene's positions, velocities, spins and radii in its shared memory, steps an eighth of the disks and writes their new state

@@ -1,5 +1,5 @@
 """Which calls of a resident scene of more than 1,536 disks are cluster launches:
-the first 512 steps, then calls of two or three steps that are not in bands.
+the first 160 steps, then short calls that are not in bands.
 After a cluster launch the state is in no sort's order (dem_row_slots refuses),
 after the graph path it is.  The bits are the same on both."""
 import ctypes as C
@@ -28,8 +28,9 @@ def _by_cluster(sim):
     return D.load().dem_row_slots(sim.handle, 0, 1, C.byref(a), C.byref(b), D._stream()) != 0
 
 
-@pytest.mark.parametrize("n,short", [(1600, [False, True, True]), (3500, [False, False, True]),
-                                     (7000, [False, False, False])])
+@pytest.mark.parametrize("n,short", [(1600, [False, True, True, True, False]),
+                                     (3500, [False, False, True, False, False]),
+                                     (7000, [False, False, False, False, False])])
 def test_calls_of_a_resident_scene(n, short):
     import demso_b200 as D
     sc = scenes.agitated_gas(n=n, seed=n, vel_std=1.0, pitch_factor=1.1, jitter=0.1)
@@ -40,18 +41,18 @@ def test_calls_of_a_resident_scene(n, short):
     assert _by_cluster(sim)
     sim.step(100)
     assert _by_cluster(sim)
-    sim.step(409)
+    sim.step(57)
     assert _by_cluster(sim)
-    sim.step(8)  # the 513th step
+    sim.step(8)  # the 161st step
     assert not _by_cluster(sim)
     sim.step(2)  # stays in the bands
     assert not _by_cluster(sim)
     sim.check()
     got = sim.get_state("cpu")
-    ref = PortOracle("f32").run(sc.sys, sc.state(), 522)
+    ref = PortOracle("f32").run(sc.sys, sc.state(), 170)
     for k in ("pos", "vel", "theta", "omega", "pressure"):
         assert same(got[k].numpy(), ref[k]), k
-    for steps, cluster in zip((1, 2, 3), short):
+    for steps, cluster in zip((1, 2, 3, 7, 8), short):
         load()  # not in bands
         sim.step(steps)
         assert _by_cluster(sim) == cluster, steps
