@@ -98,6 +98,63 @@ row_scan_kernel(uint32_t* __restrict__ hist, uint32_t rows, uint32_t numTiles) {
     }
 }
 
+// The same for rows of more than kRowScanTiles tiles, a block a row, kRowItems
+// entries a thread: a warp's walk is a chain of numTiles / 32 loads, this one of
+// numTiles / 2,048 (50 M pairs by one bit 659 -> 647 us, 16 M 221 -> 210).
+constexpr uint32_t kRowScanTiles = 1024;
+constexpr int kRowItems = 8;
+// With `totals` the row's total goes there too.
+__global__ void __launch_bounds__(kScanThreads)
+row_scan_block_kernel(uint32_t* __restrict__ hist, uint32_t numTiles,
+                      uint32_t* __restrict__ totals) {
+    __shared__ uint32_t warpTot[kScanThreads / 32];
+    uint32_t* h = hist + (size_t)blockIdx.x * numTiles;
+    uint32_t carry = 0u;
+    for (uint32_t t0 = 0; t0 < numTiles; t0 += kScanThreads * kRowItems) {
+        const uint32_t t = t0 + threadIdx.x * kRowItems;
+        uint32_t v[kRowItems], sum = 0u;
+#pragma unroll
+        for (int k = 0; k < kRowItems; ++k) {
+            v[k] = t + k < numTiles ? h[t + k] : 0u;
+            sum += v[k];
+        }
+        uint32_t total;
+        uint32_t run = carry + block_exclusive_scan<kScanThreads>(sum, warpTot, total);
+#pragma unroll
+        for (int k = 0; k < kRowItems; ++k) {
+            run += v[k];
+            if (t + k < numTiles) h[t + k] = run;
+        }
+        carry += total;
+        __syncthreads();  // warpTot is used again
+    }
+    if (totals && threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+// One block: the digits' offsets from their totals, in place.  Where the totals
+// fit the spare words of the scratch (from 16.8 M pairs on) the downsweep's blocks
+// read them side by side instead of a word of every row (50 M pairs by 20 bits
+// 3,425 -> 3,278 us; by 11 bits 2,070 -> 1,974).
+__global__ void __launch_bounds__(kScanThreads)
+totals_scan_kernel(uint32_t* __restrict__ totals, uint32_t rows) {
+    __shared__ uint32_t warpTot[kScanThreads / 32];
+    const uint32_t d0 = threadIdx.x * kRowItems;
+    uint32_t v[kRowItems], sum = 0u;
+#pragma unroll
+    for (int k = 0; k < kRowItems; ++k) {
+        v[k] = d0 + k < rows ? totals[d0 + k] : 0u;
+        sum += v[k];
+    }
+    uint32_t all;
+    uint32_t run = block_exclusive_scan<kScanThreads>(sum, warpTot, all);
+#pragma unroll
+    for (int k = 0; k < kRowItems; ++k) {
+        if (d0 + k < rows) totals[d0 + k] = run;
+        run += v[k];
+    }
+}
+static_assert(kScanThreads * kRowItems >= 2048, "a digit of at most 11 bits");
+
 // Stable scatter.  Warp w of the tile owns the contiguous run of 512 keys
 // [w*512, (w+1)*512); it walks them 32 at a time in index order and ranks
 // equal digits with match_any, so ranks follow the input order inside the
@@ -107,7 +164,8 @@ template <int BITS, bool IDENT>
 __global__ void __launch_bounds__(kSortThreads)
 downsweep_kernel(const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
                  uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut, uint32_t n,
-                 int shift, uint32_t rows, const uint32_t* __restrict__ hist, uint32_t numTiles) {
+                 int shift, uint32_t rows, const uint32_t* __restrict__ hist, uint32_t numTiles,
+                 const uint32_t* __restrict__ offsets) {
     constexpr int R = 1 << BITS;
     __shared__ uint16_t cnt[kSortWarps][R];
     __shared__ uint32_t gbase[R];
@@ -115,24 +173,27 @@ downsweep_kernel(const uint32_t* __restrict__ keysIn, const uint32_t* __restrict
     const uint32_t mask = rows - 1u;
     uint16_t* flat = &cnt[0][0];
     for (int i = threadIdx.x; i < kSortWarps * R; i += kSortThreads) flat[i] = 0;
-    // the digits' offsets (an exclusive scan of their totals, PER consecutive
-    // digits a thread), then the tile's place within each digit
+    // the digits' offsets (`offsets`, or an exclusive scan of their totals, PER
+    // consecutive digits a thread), then the tile's place within each digit
     constexpr int PER = (R + kSortThreads - 1) / kSortThreads;
     __shared__ uint32_t warpTot[kSortWarps];
-    uint32_t tot[PER], sum = 0u;
+    uint32_t tot[PER], before[PER], sum = 0u;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const uint32_t d = threadIdx.x * PER + k;
-        tot[k] = d < rows ? __ldg(hist + (size_t)d * numTiles + (numTiles - 1u)) : 0u;
-        sum += tot[k];
+        const uint32_t* h = hist + (size_t)d * numTiles;
+        // (both loads of a digit in one round)
+        tot[k] = d >= rows ? 0u : offsets ? __ldg(offsets + d) : __ldg(h + (numTiles - 1u));
+        before[k] = d < rows && blockIdx.x ? __ldg(h + (blockIdx.x - 1u)) : 0u;
     }
-    uint32_t all;
-    uint32_t run0 = block_exclusive_scan<kSortThreads>(sum, warpTot, all);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) sum += tot[k];
+    uint32_t all, run0 = 0u;
+    if (!offsets) run0 = block_exclusive_scan<kSortThreads>(sum, warpTot, all);
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const uint32_t d = threadIdx.x * PER + k;
-        if (d < rows)
-            gbase[d] = run0 + (blockIdx.x ? __ldg(hist + (size_t)d * numTiles + blockIdx.x - 1u) : 0u);
+        if (d < rows) gbase[d] = before[k] + (offsets ? tot[k] : run0);
         run0 += tot[k];
     }
     __syncthreads();
@@ -364,21 +425,29 @@ __global__ void iota_kernel(uint32_t* __restrict__ v, uint32_t n) {
 
 template <int BITS>
 cudaError_t run_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
-                     uint32_t n, int shift, int bits, bool ident, uint32_t* hist, cudaStream_t st,
-                     int* launches) {
+                     uint32_t n, int shift, int bits, bool ident, uint32_t* hist,
+                     uint32_t* spare, size_t spareWords, cudaStream_t st, int* launches) {
     const uint32_t numTiles = (n + kSortTile - 1) / kSortTile;
     const uint32_t rows = 1u << bits;
     upsweep_kernel<BITS><<<numTiles, kSortThreads, 0, st>>>(kin, n, shift, rows, hist, numTiles);
     if (launches) ++*launches;
-    row_scan_kernel<<<(rows * 32u + kScanThreads - 1u) / kScanThreads, kScanThreads, 0, st>>>(
-        hist, rows, numTiles);
+    uint32_t* const offsets = numTiles > kRowScanTiles && rows <= spareWords ? spare : nullptr;
+    if (numTiles > kRowScanTiles)
+        row_scan_block_kernel<<<rows, kScanThreads, 0, st>>>(hist, numTiles, offsets);
+    else
+        row_scan_kernel<<<(rows * 32u + kScanThreads - 1u) / kScanThreads, kScanThreads, 0, st>>>(
+            hist, rows, numTiles);
     if (launches) ++*launches;
+    if (offsets) {
+        totals_scan_kernel<<<1, kScanThreads, 0, st>>>(offsets, rows);
+        if (launches) ++*launches;
+    }
     if (ident)
         downsweep_kernel<BITS, true><<<numTiles, kSortThreads, 0, st>>>(kin, vin, kout, vout, n,
-                                                                        shift, rows, hist, numTiles);
+                                                                        shift, rows, hist, numTiles, offsets);
     else
         downsweep_kernel<BITS, false><<<numTiles, kSortThreads, 0, st>>>(kin, vin, kout, vout, n,
-                                                                         shift, rows, hist, numTiles);
+                                                                         shift, rows, hist, numTiles, offsets);
     if (launches) ++*launches;
     return cudaGetLastError();
 }
@@ -563,7 +632,8 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_
         }
         return cudaGetLastError();
     }
-    if (sort_scan_partials(sort_hist_words(n, plan)) > kScanMaxPartials)
+    const size_t spare = sort_scan_partials(sort_hist_words(n, plan));
+    if (spare > kScanMaxPartials)
         return cudaErrorInvalidValue;
     uint32_t *ki = keys, *vi = vals, *ko = s.altKeys, *vo = s.altVals;
     for (int p = 0; p < plan.passes; ++p) {
@@ -572,19 +642,19 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_
         switch (plan.radixBits) {
             case 6:
                 e = run_pass<6>(ki, vi, ko, vo, n, plan.shift[p], plan.bits[p], ident, s.hist,
-                                st, launches);
+                                s.partials, spare, st, launches);
                 break;
             case 8:
                 e = run_pass<8>(ki, vi, ko, vo, n, plan.shift[p], plan.bits[p], ident, s.hist,
-                                st, launches);
+                                s.partials, spare, st, launches);
                 break;
             case 10:
                 e = run_pass<10>(ki, vi, ko, vo, n, plan.shift[p], plan.bits[p], ident, s.hist,
-                                 st, launches);
+                                 s.partials, spare, st, launches);
                 break;
             default:
                 e = run_pass<11>(ki, vi, ko, vo, n, plan.shift[p], plan.bits[p], ident, s.hist,
-                                 st, launches);
+                                 s.partials, spare, st, launches);
                 break;
         }
         if (e != cudaSuccess) return e;

@@ -36,7 +36,7 @@ struct SortScratch {
     uint32_t* altKeys;   // n
     uint32_t* altVals;   // n
     uint32_t* hist;      // sort_hist_words
-    uint32_t* partials;  // sort_scan_partials words, spare (the size query is part of the ABI)
+    uint32_t* partials;  // sort_scan_partials words: the digits' offsets, where they fit
 };
 
 // Bytes of scratch for the layout carve_sort_scratch produces.
