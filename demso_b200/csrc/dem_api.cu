@@ -1575,8 +1575,14 @@ cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st) {
 // 32 / 38 / 45 against 33 / 36 / 39.  And a band that runs out of free slots or
 // events makes every step a layout: at 14 movers a band of 65,536 disks (64
 // free slots) 28.6 against 29.3 us, at 29 of 262,144 116 against 47.
+// `dirty` and `movers` are an estimate's; where it looked at a part of the
+// particles, 1.5 movers a band stand for the bands.
 bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers) {
-    const uint32_t b = c->band.bands;
+    const uint32_t b = c->band.bands, stride = band_estimate_stride(n);
+    if (stride > 1) {
+        movers = (uint32_t)std::min<uint64_t>((uint64_t)movers * stride, UINT32_MAX);
+        dirty = movers / 3 > b / 2 ? b : 0u;
+    }
     const uint32_t slack = c->nspec ? kBandMinSlack : band_slack(c->band, n);
     return band_overload(b, dirty) || movers > (uint64_t)b * (slack / 4);
 }

@@ -792,12 +792,12 @@ __global__ void __launch_bounds__(kPackThreads) band_cell_table_kernel(BandArgs 
 }
 
 // See launch_band_estimate.  Bound by DRAM: position and velocity, 16 B a
-// particle.
+// particle (16 M of them 55 us, the sixteenth that is looked at 4).
 __global__ void __launch_bounds__(kPackThreads)
 band_estimate_kernel(const __grid_constant__ KParams P0, BandArgs B, const float2* __restrict__ pos,
                      const float2* __restrict__ vel, const uint32_t* __restrict__ spec, uint32_t n,
-                     uint32_t serial, uint32_t* __restrict__ out) {
-    const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
+                     uint32_t stride, uint32_t serial, uint32_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * stride * kPackThreads + threadIdx.x;
     bool moves = false;
     if (i < n) {
         const KParams& P = spec ? B.table[spec[i]] : P0;
@@ -1009,8 +1009,9 @@ cudaError_t launch_band_estimate(const KParams& P, const BandArgs& b, const floa
                                  const float2* vel, const uint32_t* spec, uint32_t n,
                                  uint32_t serial, uint32_t* out, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    band_estimate_kernel<<<blocks_for(n, kPackThreads), kPackThreads, 0, st>>>(P, b, pos, vel, spec,
-                                                                              n, serial, out);
+    const uint32_t stride = band_estimate_stride(n), all = blocks_for(n, kPackThreads);
+    band_estimate_kernel<<<(all + stride - 1u) / stride, kPackThreads, 0, st>>>(
+        P, b, pos, vel, spec, n, stride, serial, out);
     return cudaGetLastError();
 }
 

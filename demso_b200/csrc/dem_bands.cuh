@@ -186,7 +186,9 @@ cudaError_t launch_band_cell_table(const BandArgs& b, cudaStream_t st);
 
 // Adds to out[0] the bands that particles would leave or enter if all moved on
 // by a step at their velocities, to out[1] the particles; `serial`: another
-// number each time.  spec: a batch's specimen of every packed slot.
+// number each time.  spec: a batch's specimen of every packed slot.  Of many
+// particles a part is looked at, one block of 256 in band_estimate_stride.
+inline uint32_t band_estimate_stride(uint32_t n) { return n >> 20 ? n >> 20 : 1u; }
 cudaError_t launch_band_estimate(const KParams& P, const BandArgs& b, const float2* pos,
                                  const float2* vel, const uint32_t* spec, uint32_t n,
                                  uint32_t serial, uint32_t* out, cudaStream_t st);

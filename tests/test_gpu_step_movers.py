@@ -179,3 +179,17 @@ def test_a_resident_batch(crowded):
         r = PortOracle("f32").run(parts[k].sys, parts[k].state(), 16)
         for x in ("pos", "vel", "theta", "omega", "pressure"):
             assert same(got[x].numpy()[n * k:n * k + n], r[x]), x
+
+
+@pytest.mark.parametrize("vel,packed", [(0.5, False), (20.0, True)])
+def test_a_state_looked_at_in_part(vel, packed):
+    # 2.2 million disks in 1,024 bands: every second block of 256; about 0.8 and 31
+    # movers a band
+    import demso_b200 as D
+    sc = scenes.agitated_gas(n=2200000, seed=6, vel_std=vel, pitch_factor=1.5, jitter=0.1,
+                             gravity=(0.0, 0.0))
+    sim = D.Simulation(sc.sys, capacity=sc.n)
+    _load(sim, sc.state())
+    assert _call(sim, 5) == packed
+    _same(sim, PortOracle("f32").run(sc.sys, sc.state(), 5))
+    sim.close()
