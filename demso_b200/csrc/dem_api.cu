@@ -1568,23 +1568,23 @@ cudaError_t estimate_movers(DemContext* c, uint32_t n, cudaStream_t st) {
 // Where the bands lose to the packed path's incremental sort, which moves every
 // particle but takes movers up to n / 8.  A fix rewrites a band for one mover
 // as for twenty: up to kFixBlocks bands that is one round of blocks, beyond it
-// costs what it moves.  With nearly all bands rewritten (0.9, at 1.5 movers a
-// band) the two meet -- us a step, bands against packed, at 1.0 / 2.0 / 4.9 movers
-// a band of 1,000,003 disks: 73 / 91 / 114 against 83 / 87 / 93; at 1.0 / 2.0 / 9.8 of
-// 4,194,304: 214 / 274 / 427 against 258 / 282 / 338; at 1.0 / 2.4 / 7.2 of 262,144:
-// 32 / 38 / 45 against 33 / 36 / 39.  And a band that runs out of free slots or
-// events makes every step a layout: at 14 movers a band of 65,536 disks (64
-// free slots) 28.6 against 29.3 us, at 29 of 262,144 116 against 47.
-// `dirty` and `movers` are an estimate's; where it looked at a part of the
-// particles, 1.5 movers a band stand for the bands.
+// costs what it moves.  With nearly all bands rewritten the two meet, at about
+// 1.7 movers a band and, of 2,048 bands or more, 2.2 -- us a step, bands against
+// packed, at 1.0 / 2.0 / 4.9 movers a band of 1,000,003 disks: 73 / 91 / 114
+// against 83 / 87 / 93; at 1.0 / 2.0 / 9.8 of 4,194,304: 214 / 274 / 427 against
+// 258 / 282 / 338; at 1.7 / 3.4 / 6.7 of 12 million: 567 / 706 / 940 against
+// 726 / 778 / 869; at 1.0 / 2.4 / 7.2 of 262,144: 32 / 38 / 45 against 33 / 36 / 39.
+// And a band that runs out of free slots or events makes every step a layout: at
+// 14 movers a band of 65,536 disks (64 free slots) 28.6 against 29.3 us, at 29 of
+// 262,144 116 against 47.  `dirty` and `movers` are an estimate's; one of a part of
+// the particles says nothing of the bands.
 bool too_many_movers(const DemContext* c, uint32_t n, uint32_t dirty, uint32_t movers) {
     const uint32_t b = c->band.bands, stride = band_estimate_stride(n);
-    if (stride > 1) {
-        movers = (uint32_t)std::min<uint64_t>((uint64_t)movers * stride, UINT32_MAX);
-        dirty = movers / 3 > b / 2 ? b : 0u;
-    }
+    const uint64_t all = (uint64_t)movers * stride;
     const uint32_t slack = c->nspec ? kBandMinSlack : band_slack(c->band, n);
-    return band_overload(b, dirty) || movers > (uint64_t)b * (slack / 4);
+    return (stride == 1 && band_overload(b, dirty)) ||
+           (b > kFixBlocks && 10 * all > (uint64_t)b * (b < 2048 ? 17 : 22)) ||
+           all > (uint64_t)b * (slack / 4);
 }
 
 // Grids so coarse that the average row interval of three cells holds more

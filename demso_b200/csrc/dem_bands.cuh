@@ -214,7 +214,7 @@ cudaError_t launch_band_pack(const BandArgs& b, const PackedState& out, bool sta
                              cudaStream_t st);
 // Whether nearly all bands are rewritten on every step (see too_many_movers).
 __host__ __device__ inline bool band_overload(uint32_t bands, uint32_t dirty) {
-    return bands > kFixBlocks && dirty > bands - bands / 10u;
+    return bands > kFixBlocks && dirty > bands - bands / (bands < 2048u ? 10u : 25u);
 }
 // New layout from the packed arrays, sorted by `keys` (their particles in
 // order `from`); cellFirst: numCells + 1 words of scratch.
